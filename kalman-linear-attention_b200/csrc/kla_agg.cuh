@@ -88,7 +88,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
-            mbar_init(&full_in[s], 32);
+            mbar_init(&full_in[s], stage_arrivals(prm.use_tma, 32));
             mbar_init(&empty_in[s], NW);
         }
         mbar_fence_init();
@@ -270,11 +270,11 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
                     }
                 }
             } else {
-                stage_tile_plain<T, TT, MC, 32>(vstage(s), vb, prm.v.st, t0, L, m_cta, M, lane);
-                stage_tile_plain<T, TT, MC, 32>(lstage(s), lb, prm.lv.st, t0, L, m_cta, M, lane);
+                stage_tile<T, TT, MC, 32>(vstage(s), vb, prm.v.st, t0, L, m_cta, M, lane);
+                stage_tile<T, TT, MC, 32>(lstage(s), lb, prm.lv.st, t0, L, m_cta, M, lane);
                 if (ADJ) {
-                    stage_tile_plain<TO, TT, MC, 32>(dystage(s), dyb, prm.dy.st, t0, L, m_cta, M, lane);
-                    if (has_dyv) stage_tile_plain<TO, TT, MC, 32>(dyvstage(s), dyvb, prm.dyv.st, t0, L, m_cta, M, lane);
+                    stage_tile<TO, TT, MC, 32>(dystage(s), dyb, prm.dy.st, t0, L, m_cta, M, lane);
+                    if (has_dyv) stage_tile<TO, TT, MC, 32>(dyvstage(s), dyvb, prm.dyv.st, t0, L, m_cta, M, lane);
                 }
             }
             float *kq = kqstage(s);
@@ -288,10 +288,12 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
                 }
             }
             if (it + 1 < NT) load_kq(t0 + TT);
+            if (!prm.use_tma) stage_arrive(&full_in[s]);
             if (!(prm.use_tma && lane == 0)) mbar_arrive(&full_in[s]);
             produced = it + 1;
         }
-        // leaving early (a wait ran out): do not end the CTA with bulk copies still in flight into its shared memory
+        // leaving early (a wait ran out): do not end the CTA with copies still in flight into its shared memory
+        if (!ok && !prm.use_tma) cp_async_wait_all();
         if (!ok && prm.use_tma && lane == 0)
             for (int t = max(0, produced - NS); t < produced; ++t) mbar_wait(prm.wait, &full_in[t % NS], (t / NS) & 1, 33);
     }

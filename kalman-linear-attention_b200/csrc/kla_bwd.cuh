@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
-            mbar_init(&full_in[s], kProducers);
+            mbar_init(&full_in[s], stage_arrivals(prm.use_tma, kProducers));
             mbar_init(&empty_in[s], kStageUsers);
         }
         for (int bf = 0; bf < 2; ++bf) {
@@ -599,11 +599,11 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                         if (has_dyv) tma_load_3d(dyvstage(s), &prm.tm_dyv, m_cta, t_off + t0, b, &full_in[s]);
                     }
                 } else {
-                    stage_tile_plain<T, TT, MC, kProducers>(vstage(s), vb, prm.v.st, t0, L, m_cta, M, htid);
-                    stage_tile_plain<T, TT, MC, kProducers>(lstage(s), lb, prm.lv.st, t0, L, m_cta, M, htid);
-                    stage_tile_plain<TO, TT, MC, kProducers>(dystage(s), dyb, prm.dy.st, t0, L, m_cta, M, htid);
+                    stage_tile<T, TT, MC, kProducers>(vstage(s), vb, prm.v.st, t0, L, m_cta, M, htid);
+                    stage_tile<T, TT, MC, kProducers>(lstage(s), lb, prm.lv.st, t0, L, m_cta, M, htid);
+                    stage_tile<TO, TT, MC, kProducers>(dystage(s), dyb, prm.dy.st, t0, L, m_cta, M, htid);
                     if (has_dyv)
-                        stage_tile_plain<TO, TT, MC, kProducers>(dyvstage(s), dyvb, prm.dyv.st, t0, L, m_cta, M, htid);
+                        stage_tile<TO, TT, MC, kProducers>(dyvstage(s), dyvb, prm.dyv.st, t0, L, m_cta, M, htid);
                 }
                 float2 *kq = kqstage(s);
 #pragma unroll
@@ -612,6 +612,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                     if (idx < TT * SPAD) kq[idx] = make_float2(kr[e], qr[e]);
                 }
                 if (tile > 0) load_kq(t0 - TT);
+                if (!prm.use_tma) stage_arrive(&full_in[s]);
                 // (test hook, as in the forward: the wait for tile skip_tile runs out)
                 if (!(prm.use_tma && htid == 0) && !(it == prm.wait.skip_tile && htid == 1)) mbar_arrive(&full_in[s]);
                 produced = it + 1;
@@ -700,6 +701,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 }
             }
         }
+        if (!ok && !prm.use_tma) cp_async_wait_all();
         if (!ok && prm.use_tma && htid == 0) {
             for (int t = max(0, produced - NS); t < produced; ++t) mbar_wait(prm.wait, &full_in[t % NS], (t / NS) & 1, 15);
         }

@@ -351,17 +351,64 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// Cooperative fallback staging of a [TT x MC] tile (rows t0.., columns m0..) by
-// NTHR threads with plain loads, zero-filling rows past L and columns past M;
-// used when a tensor does not meet the tensor-map alignment rules.
+// Staging of a [TT x MC] tile (rows t0.., columns m0..) by NTHR threads for a tensor that does not meet the
+// tensor-map rules (a row length that is not a multiple of 16 bytes, an odd base), zero-filling rows past L and
+// columns past M. The copies are per-thread asynchronous 4-byte ones, so the loader never waits for global memory
+// and all input stages are in flight as with TMA; plain loads, one after the other behind their shared-memory
+// stores, made a 1001-channel training step ten times slower than a 1024-channel one (2.87 against 0.28 ms).
+// bfloat16 rows that are not even 4-byte aligned are loaded four elements at a time before the first is stored.
+// The caller's threads then signal the stage's barrier with stage_arrive(); the barrier counts two arrivals of
+// each (stage_arrivals).
+__device__ __forceinline__ void cp_async_4(void *dst, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Arrivals a stage filled by `threads` loader threads waits for: with TMA one each (the elected thread's also
+// announces the bytes); with per-thread copies one for the thread's own stores and one when its copies are done.
+__device__ __forceinline__ uint32_t stage_arrivals(bool tma, int threads) { return tma ? threads : 2 * threads; }
+__device__ __forceinline__ void stage_arrive(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 template <typename T, int TT, int MC, int NTHR>
-__device__ __forceinline__ void stage_tile_plain(T *smem, const T *base, long long st, int t0, int L, int m0, int M,
-                                                 int tid) {
-    for (int idx = tid; idx < TT * MC; idx += NTHR) {
-        const int row = idx / MC, c = idx % MC;
-        T v = from_f32<T>(0.0f);
-        if (t0 + row < L && m0 + c < M) v = base[(long long)(t0 + row) * st + m0 + c];
-        smem[row * MC + c] = v;
+__device__ __forceinline__ void stage_tile(T *smem, const T *base, long long st, int t0, int L, int m0, int M, int tid) {
+    constexpr int EPC = 4 / sizeof(T);  // elements per 4-byte copy
+    const T *src = base + (long long)t0 * st + m0;
+    if (EPC == 1 || ((reinterpret_cast<uintptr_t>(src) & 3) == 0 && st % EPC == 0)) {
+        // a thread keeps its column and walks down the rows, so a copy costs a pointer step and little else
+        constexpr int W = MC / EPC, STEP = NTHR / W > 0 ? NTHR / W : 1;
+        static_assert(NTHR % W == 0 || W % NTHR == 0, "whole rows, or whole parts of one, per pass");
+#pragma unroll 1
+        for (int c0 = tid % W; c0 < W; c0 += NTHR) {
+            const int c = c0 * EPC, cols = max(0, min(EPC, M - m0 - c)) * (int)sizeof(T);
+            int row = tid / W;
+            const T *from = cols > 0 ? src + (long long)row * st + c : base;
+            const long long down = cols > 0 ? STEP * st : 0;
+            T *to = smem + row * MC + c;
+            const int last = L - t0;
+#pragma unroll 1  // rolled: unrolled, the copies' addresses cost the whole kernel registers
+            for (; row < TT; row += STEP, from += down, to += STEP * MC) {
+                const bool in = row < last;
+                cp_async_4(to, in ? from : base, in ? cols : 0);
+            }
+        }
+    } else {
+        constexpr int PER = (TT * MC + NTHR - 1) / NTHR, NB = 4;
+#pragma unroll 1
+        for (int e0 = 0; e0 < PER; e0 += NB) {
+            T x[NB];
+#pragma unroll
+            for (int e = 0; e < NB; ++e) {
+                const int u = tid + (e0 + e) * NTHR, row = u / MC, c = u % MC;
+                const bool in = u < TT * MC && t0 + row < L && m0 + c < M;
+                x[e] = in ? src[(long long)row * st + c] : from_f32<T>(0.0f);
+            }
+#pragma unroll
+            for (int e = 0; e < NB; ++e) {
+                const int u = tid + (e0 + e) * NTHR;
+                if (u < TT * MC) smem[u] = x[e];
+            }
+        }
     }
 }
 

@@ -90,7 +90,7 @@ struct FwdSmem {
 // SEG: sequences cut into segments (FwdParams::seg, SegCtl). Again a separate instantiation: the unsegmented kernel
 // then carries none of that code (with it, one CTA per SM ran 3 % slower).
 template <typename T, typename TO, int SPT, int LPC, int CH, int NW, int NH, int TT, bool PRIOR, bool EPI, bool SEG>
-__global__ void __launch_bounds__((NW + NH) * 32) kla_fwd_kernel(const __grid_constant__ FwdParams prm) {
+__global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC <= 8 ? 3 : 1) kla_fwd_kernel(const __grid_constant__ FwdParams prm) {
     using Sh = ScanShape<SPT, LPC, CH, NW, NH, TT>;
     using Sm = FwdSmem<T, SPT, LPC, CH, NW, NH, TT>;
     constexpr int SPAD = Sh::kSPad, MC = Sh::kMC, MCP = Sh::kMCP;
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__((NW + NH) * 32) kla_fwd_kernel(const __grid_co
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
-            mbar_init(&full_in[s], kProducers);
+            mbar_init(&full_in[s], stage_arrivals(prm.use_tma, kProducers));
             mbar_init(&empty_in[s], NW);
         }
         for (int o = 0; o < NO; ++o) {
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__((NW + NH) * 32) kla_fwd_kernel(const __grid_co
         }
         if constexpr (EPI) {
             for (int e = 0; e < NE; ++e) {
-                mbar_init(&epi_full[e], kProducers);
+                mbar_init(&epi_full[e], stage_arrivals(prm.epi_tma, kProducers));
                 mbar_init(&epi_empty[e], kDrainers / 32);
             }
         }
@@ -445,8 +445,8 @@ __global__ void __launch_bounds__((NW + NH) * 32) kla_fwd_kernel(const __grid_co
                         tma_load_3d(lstage(s), &prm.tm_lv, m_cta, t_off + t0, b, &full_in[s]);
                     }
                 } else {
-                    stage_tile_plain<T, TT, MC, kProducers>(vstage(s), vb, prm.v.st, t0, L, m_cta, M, htid);
-                    stage_tile_plain<T, TT, MC, kProducers>(lstage(s), lb, prm.lv.st, t0, L, m_cta, M, htid);
+                    stage_tile<T, TT, MC, kProducers>(vstage(s), vb, prm.v.st, t0, L, m_cta, M, htid);
+                    stage_tile<T, TT, MC, kProducers>(lstage(s), lb, prm.lv.st, t0, L, m_cta, M, htid);
                 }
                 float *kq = kqstage(s);
 #pragma unroll
@@ -459,6 +459,7 @@ __global__ void __launch_bounds__((NW + NH) * 32) kla_fwd_kernel(const __grid_co
                     }
                 }
                 if (it + 1 < NT) load_kq(t0 + TT);
+                if (!prm.use_tma) stage_arrive(&full_in[s]);
                 // (test hook: one loader thread leaves out its arrive for tile skip_tile, so the wait for that tile runs out)
                 if (!(prm.use_tma && htid == 0) && !(it == prm.wait.skip_tile && htid == 1)) mbar_arrive(&full_in[s]);
                 produced = it + 1;
@@ -474,12 +475,13 @@ __global__ void __launch_bounds__((NW + NH) * 32) kla_fwd_kernel(const __grid_co
                         }
                     } else {
                         if (has_z)
-                            stage_tile_plain<T, TT, MC, kProducers>(
+                            stage_tile<T, TT, MC, kProducers>(
                                 zstage(e), static_cast<const T *>(prm.z.ptr) + (long long)b * prm.z.sb + (long long)t_off * prm.z.st, prm.z.st, t0, L, m_cta, M, htid);
                         if (has_g)
-                            stage_tile_plain<T, TT, MC, kProducers>(
+                            stage_tile<T, TT, MC, kProducers>(
                                 gstage(e), static_cast<const T *>(prm.gate.ptr) + (long long)b * prm.gate.sb + (long long)t_off * prm.gate.st, prm.gate.st, t0, L, m_cta, M, htid);
                     }
+                    if (!prm.epi_tma) stage_arrive(&epi_full[e]);
                     if (!(prm.epi_tma && htid == 0)) mbar_arrive(&epi_full[e]);
                     epi_issued = it + 1;
                 }
@@ -540,8 +542,9 @@ __global__ void __launch_bounds__((NW + NH) * 32) kla_fwd_kernel(const __grid_co
                 if (hlane == 0) mbar_arrive(&empty_out[o]);
             }
         }
-        // Leaving early (a wait ran out): do not end the CTA with bulk copies
+        // Leaving early (a wait ran out): do not end the CTA with copies
         // still in flight into its shared memory.
+        if (!ok) cp_async_wait_all();
         if (!ok && htid == 0) {
             if (prm.use_tma)
                 for (int t = max(0, produced - NS); t < produced; ++t) mbar_wait(prm.wait, &full_in[t % NS], (t / NS) & 1, 5);
