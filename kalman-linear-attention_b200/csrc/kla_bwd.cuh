@@ -4,49 +4,58 @@
 // the forward recurrence is replayed from the tile's checkpoint, every chain's
 // pre-step state (P', mean') going to shared memory, and then the adjoint is
 // walked back down the tile with the two carries (dL/dP, dL/dmean) in registers.
-// The same statements differentiated by hand (variance form, see kla_common.cuh):
+// The forward step, in variance form (kla_common.cuh), and its derivatives
+// written with the posterior (P, mean) wherever that takes fewer operations:
 //
-//   mean = g u,  u = a mean' + Pp r,  P = Pp g,  g = 1/d,  d = 1 + phi Pp,
-//   Pp = a2 P' + p
+//   Pp = a2 P' + p,  g = 1/(1 + phi Pp) = P/Pp,  P = Pp g,  mean = g (a mean' + Pp r)
+//   with phi = lambda_v k^2, r = lambda_v v k
 //
-//   mbar = c_mean + dy q            Pbar = c_P + dyvar q^2
-//   dbar = -g (mbar mean + Pbar P)  ubar = mbar g
-//   Ppbar = ubar r + Pbar g + dbar phi
-//   rbar = ubar Pp                  phibar = dbar Pp
-//   c_mean <- ubar a                c_P <- Ppbar a2
-//   da += ubar mean'   da2 += Ppbar P'   dp += Ppbar
+//   mbar = c_mean + dy q                    Pbar = c_P + dyvar q^2
+//   rbar = P mbar                           phibar = -P (mbar mean + Pbar P)
+//   ubar = g mbar                           Ppbar = g (g Pbar + mbar w),  w = lambda_v k (v - k mean)
+//   c_mean <- a ubar                        c_P <- a2 Ppbar
+//   da += ubar mean'   da2 += Ppbar P'      dp += Ppbar
+//   D = sum_s rbar k,  E = sum_s phibar k^2:  dv = D lambda_v,  dlambda_v = E + D v
+//   dk = sum_m lambda_v (rbar v + 2 k phibar)
+//
+// A thread owns two neighbouring channels x SPT states. The two channels are the
+// halves of every operand, so the whole walk runs on the paired fp32 instructions
+// of sm_100: inputs of the step arrive as pairs, k and q are staged duplicated,
+// and what a thread adds over its channels costs one addition per state. The mean
+// and the P carry travel negated (n = -mean, -c_P): every product above then has
+// the sign the next sum needs, since a pair instruction has no operand negation.
 //
 // The CTA is three groups of four warps, each with the registers its role needs
 // (the register file is re-divided between the groups when the kernel starts):
 //   replay warps   run the forward recurrence of tile n+1 into one of two
 //                  trajectory buffers while
 //   reverse warps  walk the adjoint down tile n from the other buffer, leaving
-//                  what crosses threads in shared memory:
-//                    sums over s (dv, dlambda_v): LPC partials per (t, channel);
-//                    sums over m (dk, dq): one partial per thread per (t, state),
-//                    parked in the slot its (P', mean') occupied;
+//                  what crosses threads where the trajectory was (a warp has read
+//                  a step's slots before it writes them):
+//                    sums over m (dk, dq): one float2 per thread and state;
+//                    sums over s (D, E): one float4 per thread;
 //                  sums over b and t (da, dp) stay in registers until the end;
 //   helper warps   one loads (TMA tiles of v, lambda_v, dy, dy_var issued by one
 //                  elected thread, and the (k, q) values of a tile, those
 //                  of the next tile already in registers); three finish the sums:
-//                  the CTA's channels of dk, dq and one atomic per (t, s), the
-//                  lane groups of dv, dlambda_v and their stores.
+//                  the CTA's channels of dk, dq and one vector atomic per (t, two
+//                  states), the lane groups of dv, dlambda_v and their stores.
 // Replay and reverse are different instruction streams with little in common but
 // the trajectory, so running them side by side doubles the warps a scheduler can
-// choose from without doubling the registers: the replay needs half of what
-// the reverse walk needs. All hand-overs go through mbarriers.
+// choose from without doubling the registers. All hand-overs go through mbarriers.
 //
 // With SEG a sequence is walked by several CTAs, last stretch first (SegCtl, kla_common.cuh): a CTA takes the two
 // carries and the running sums for da, dp from the CTA that walked the stretch after its own, and hands its own
 // on; the state its walk starts from needs no hand-over, the replay group computes it from the checkpoints.
 //
-// Measured on B200 at B=8, T=4096, M=1024, S=16 (1.49 ms unsegmented, 1.42 ms in 16 segments): the reverse walk alone takes 1.15 ms, the replay alone
-// 0.53 ms, the sums 0.12 ms; side by side they overlap only in part. Variants that were measured and are not kept:
-// the trajectory through tensor memory (tcgen05.st / tcgen05.ld, a third less shared-memory traffic: 1.56 ms),
-// the reverse walk on paired fp32 instructions (a third fewer instructions: 1.68 ms), other register splits between
-// the groups and deeper unrolling (1.54-1.79 ms), the reverse walk's shared-memory reads fetched one step ahead by hand
-// (1.62 ms). No single resource is the limit: issue slots, the FP32 pipe and
-// the shared-memory pipe are each a half to three quarters busy on the SMs that hold two CTAs.
+// Measured on B200 at T=4096, M=1024, S=16, float32, against the kernel with one channel per thread and scalar
+// arithmetic: B=8 1.42 -> 1.17 ms, B=4 0.88 -> 0.71 ms, B=16 2.59 -> 2.16 ms; 46 instead of 66 warp instructions per 32
+// lane-steps. What bounds it is the FP32 pipe's register reads: 30 pair operations per two chains and step in the
+// reverse walk and 8 in the replay, 12 and 2 of them three-operand FMAs at 3.75 cycles (kla_common.cuh), add up to about
+// 235 of the 291 cycles a scheduler spends on a warp's step. Not limits: shared memory (the trajectory through tensor
+// memory, a third less shared-memory traffic, takes the same 1.17 ms), the helpers (1.12 ms without their sums), the
+// replay (1.08 ms without its arithmetic). Scalar FMAs in place of the pair FMAs: 1.25 ms. Fetching a step's inputs
+// before the previous step's arithmetic and unrolling the whole tile gave 1.20 -> 1.17 ms.
 #pragma once
 
 #include "kla_fwd.cuh"
@@ -55,31 +64,36 @@ namespace kla {
 
 constexpr int kBwdStages = 3;  // input stages in flight
 #ifndef KLA_REV_UNROLL
-#define KLA_REV_UNROLL 2
+#define KLA_REV_UNROLL 8
 #endif
-constexpr int kRevUnroll = KLA_REV_UNROLL;  // steps of the reverse walk unrolled per loop trip
+template <int SPAD>
+constexpr int kRevUnroll = SPAD > 64 ? 2 : KLA_REV_UNROLL;  // steps of the reverse walk unrolled per loop trip
 #ifndef KLA_REP_UNROLL
-#define KLA_REP_UNROLL 4
+#define KLA_REP_UNROLL 8
 #endif
-constexpr int kRepUnroll = KLA_REP_UNROLL;  // steps of the replay unrolled per loop trip
+template <int SPAD>
+constexpr int kRepUnroll = SPAD > 64 ? 2 : KLA_REP_UNROLL;  // steps of the replay unrolled per loop trip
 
-// Registers per thread of the three warp groups after the kernel's start. The kernel is compiled for
+// Registers per thread of the three warp groups after the kernel's start (BwdRegs). The kernel is compiled for
 // kBwdRegsLaunch registers (384 threads, two CTAs per SM); the groups then hand registers to one another:
 // 128 * (reverse + replay + helpers) must not exceed 384 * the compiled count, which the launcher checks
 // against the compiled kernel before it launches (a group that asked for more than is there would wait for ever).
 constexpr int kBwdRegsLaunch = 80;
 #ifndef KLA_BWD_REGS_REVERSE
-#define KLA_BWD_REGS_REVERSE 128
+#define KLA_BWD_REGS_REVERSE 120
 #endif
 #ifndef KLA_BWD_REGS_REPLAY
-#define KLA_BWD_REGS_REPLAY 64
+#define KLA_BWD_REGS_REPLAY 72
 #endif
-constexpr int kBwdRegsReverse = KLA_BWD_REGS_REVERSE, kBwdRegsReplay = KLA_BWD_REGS_REPLAY;
-constexpr int kBwdRegsHelper = 3 * kBwdRegsLaunch - kBwdRegsReverse - kBwdRegsReplay;
-static_assert(kBwdRegsHelper >= 24 && kBwdRegsHelper % 8 == 0 && kBwdRegsReverse % 8 == 0 && kBwdRegsReplay % 8 == 0,
-              "register counts are multiples of 8, at least 24");
-static_assert(kBwdRegsReplay <= kBwdRegsLaunch && kBwdRegsHelper <= kBwdRegsLaunch && kBwdRegsReverse >= kBwdRegsLaunch,
-              "two groups give registers up, one takes them");
+template <int SPAD>  // at 128 states a reverse thread has twice the chains
+struct BwdRegs {
+    static constexpr int kReverse = SPAD > 64 ? 136 : KLA_BWD_REGS_REVERSE, kReplay = SPAD > 64 ? 64 : KLA_BWD_REGS_REPLAY;
+    static constexpr int kHelper = 3 * kBwdRegsLaunch - kReverse - kReplay;
+    static_assert(kHelper >= 24 && kHelper % 8 == 0 && kReverse % 8 == 0 && kReplay % 8 == 0,
+                  "register counts are multiples of 8, at least 24");
+    static_assert(kReplay <= kBwdRegsLaunch && kHelper <= kBwdRegsLaunch && kReverse >= kBwdRegsLaunch,
+                  "two groups give registers up, one takes them");
+};
 
 template <int R>
 __device__ __forceinline__ void regs_grow() {
@@ -100,6 +114,7 @@ struct alignas(64) BwdParams {
     const float *dlam_fin, *deta_fin;
     float *dk, *dq, *da, *dp, *dlam0, *deta0;
     int vec_dv, vec_dlv;
+    int vec_dkq;  // two neighbouring states of dk, dq can be added to at once
     // lv holds log-variances (see FwdParams); dlv then receives the gradient with respect to them
     int lv_log_sigma;
     float obs_var_min, obs_var_max;
@@ -107,36 +122,57 @@ struct alignas(64) BwdParams {
     SegCtl seg;  // hand: five planes [B, M, S]: the two carries and the running sums for da, da2, dp
 };
 
-template <typename T, typename TO, int SPT, int LPC, int CH, int NW, int NH, int TT>
+// How the backward's threads cover a state size, by the number of padded states SPAD = 4 .. 128 (a power of two):
+// two channels x SPT states per thread, LPC lanes per channel pair. Four states per thread only at 128, where two
+// would need more than a warp per channel pair.
+template <int SPAD>
+struct BwdShape {
+    static constexpr int kSPT = SPAD > 64 ? 4 : 2;
+    static constexpr int kLPC = SPAD / kSPT;
+    static constexpr int kCPW = (32 / kLPC) * 2;  // channels per warp
+    static constexpr int kMC = 4 * kCPW;          // channels per CTA
+    static constexpr int kCompute = 128;          // threads of a compute group
+};
+
+template <typename T, typename TO, int SPAD, int TT>
 struct BwdSmem {
-    using Sh = ScanShape<SPT, LPC, CH, NW, NH, TT>;
+    using Sh = BwdShape<SPAD>;
     static constexpr size_t kBars = 128;
     static constexpr size_t kTileI = ((sizeof(T) * TT * Sh::kMC + 127) / 128) * 128;   // v or lambda_v
     static constexpr size_t kTileO = ((sizeof(TO) * TT * Sh::kMC + 127) / 128) * 128;  // dy or dyvar
-    static constexpr size_t kKq = ((sizeof(float2) * TT * Sh::kSPad + 127) / 128) * 128;
+    static constexpr size_t kKq = sizeof(float4) * TT * SPAD;                          // (k, k, q, q) per (t, s)
     static constexpr size_t kLamF = sizeof(T) == 4 ? 0 : ((sizeof(float) * TT * Sh::kMC + 127) / 128) * 128;  // as in FwdSmem
     static constexpr size_t kIn = 2 * kTileI + 2 * kTileO + kKq + kLamF;
-    static constexpr int kRowPad = 4;  // slots; 8 words = the span of LPC lanes' float2 reads
-    static constexpr int kRow = Sh::kCompute + kRowPad;
-    static constexpr size_t kTraj = ((sizeof(float2) * TT * CH * SPT * kRow + 127) / 128) * 128;  // one of two
-    static constexpr size_t kDpart = ((sizeof(float2) * TT * LPC * Sh::kMCP + 127) / 128) * 128;  // one of two
-    static constexpr size_t kPost = ((sizeof(float2) * CH * SPT * kRow + 127) / 128) * 128;       // state after the last step
-    static constexpr size_t kTotal = kBars + kBwdStages * kIn + 2 * kTraj + 2 * kDpart + kPost;
+    // Trajectory: a row of one float4 (P', n' of two channels) per compute thread for every (step, state). Rows are
+    // padded by 64 bytes, so that helper lanes reading the same column of two neighbouring rows meet different banks.
+    static constexpr int kRow = Sh::kCompute + 4;  // float4s
+    static constexpr size_t kTraj = sizeof(float4) * TT * Sh::kSPT * kRow;  // one of two
+    static constexpr size_t kPost = sizeof(float4) * Sh::kSPT * kRow;       // state after the last step
+    static constexpr size_t kRawKq = SPAD <= 16 ? 0 : 2 * ((sizeof(T) * TT * SPAD + 127) / 128) * 128;  // k and q of a tile as they are in memory
+    static constexpr size_t kTotal = kBars + kBwdStages * kIn + 2 * kTraj + kPost + 2 * kRawKq;
 };
 
 constexpr int kBwdThreads = 384;  // reverse, replay and helper groups of four warps each
 
+// two neighbouring activations as a pair of floats
+__device__ __forceinline__ float2 load_pair(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+__device__ __forceinline__ float2 load_pair(const __nv_bfloat16 *p) {
+    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p));
+}
+__device__ __forceinline__ void store_pair(float *p, float x, float y) { *reinterpret_cast<float2 *>(p) = make_float2(x, y); }
+__device__ __forceinline__ void store_pair(__nv_bfloat16 *p, float x, float y) {
+    *reinterpret_cast<__nv_bfloat162 *>(p) = __floats2bfloat162_rn(x, y);
+}
+
 // LOGV: lambda_v arrives as a log-variance (BwdParams::lv_log_sigma). A separate instantiation, so that the plain
 // kernel does not carry that code.
-// SEG: sequences cut into segments (BwdParams::seg, SegCtl), also a separate instantiation: with that code in it the
-// unsegmented kernel ran 8 % slower at one CTA per SM.
-template <typename T, typename TO, int SPT, int LPC, int CH, int NW, int NH, int TT, bool PRIOR, bool LOGV, bool SEG>
+// SEG: sequences cut into segments (BwdParams::seg, SegCtl), also a separate instantiation.
+template <typename T, typename TO, int SPAD, int TT, bool PRIOR, bool LOGV, bool SEG>
 __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_constant__ BwdParams prm) {
-    using Sh = ScanShape<SPT, LPC, CH, NW, NH, TT>;
-    using Sm = BwdSmem<T, TO, SPT, LPC, CH, NW, NH, TT>;
-    constexpr int SPAD = Sh::kSPad, MC = Sh::kMC, MCP = Sh::kMCP, NTC = Sh::kCompute;
-    constexpr int NS = kBwdStages;
-    static_assert(NW == 4 && NH == 4, "three groups of four warps");
+    using Sh = BwdShape<SPAD>;
+    using Sm = BwdSmem<T, TO, SPAD, TT>;
+    constexpr int SPT = Sh::kSPT, LPC = Sh::kLPC, CPW = Sh::kCPW, MC = Sh::kMC, NTC = Sh::kCompute;
+    constexpr int NW = 4, NH = 4, NS = kBwdStages, ROW = Sm::kRow, CLS = 32 / LPC;
     static_assert(TT == kCkptInterval, "one checkpoint per tile");
     constexpr int kProducers = 32, kSummers = (NH - 1) * 32;
     constexpr int kStageUsers = 2 * NW + (NH - 1);  // warps that read an input stage: reverse, replay, summing helpers
@@ -152,20 +188,23 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
     static_assert((2 * NS + 6) * sizeof(uint64_t) <= Sm::kBars, "barriers fit their slot");
     unsigned char *in_base = smem + Sm::kBars;
     unsigned char *traj_base = in_base + NS * Sm::kIn;
-    unsigned char *dpart_base = traj_base + 2 * Sm::kTraj;
-    float2 *post = reinterpret_cast<float2 *>(dpart_base + 2 * Sm::kDpart);                       // [CH*SPT][ROW]
-    auto trajbuf = [&](int bf) { return reinterpret_cast<float2 *>(traj_base + bf * Sm::kTraj); };      // [TT*CH*SPT][ROW]
-    auto dpartbuf = [&](int bf) { return reinterpret_cast<float2 *>(dpart_base + bf * Sm::kDpart); };   // [TT][LPC][MCP]
+    unsigned char *raw_base = traj_base + 2 * Sm::kTraj + Sm::kPost;  // two tiles of k, q as they are in memory
+    float4 *post = reinterpret_cast<float4 *>(traj_base + 2 * Sm::kTraj);                                // [SPT][ROW]
+    auto trajbuf = [&](int bf) { return reinterpret_cast<float4 *>(traj_base + bf * Sm::kTraj); };      // [TT*SPT][ROW]
     auto vstage = [&](int s) { return reinterpret_cast<T *>(in_base + s * Sm::kIn); };
     auto lstage = [&](int s) { return reinterpret_cast<T *>(in_base + s * Sm::kIn + Sm::kTileI); };
     auto dystage = [&](int s) { return reinterpret_cast<TO *>(in_base + s * Sm::kIn + 2 * Sm::kTileI); };
     auto dyvstage = [&](int s) { return reinterpret_cast<TO *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + Sm::kTileO); };
-    auto kqstage = [&](int s) { return reinterpret_cast<float2 *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + 2 * Sm::kTileO); };
+    auto kqstage = [&](int s) { return reinterpret_cast<float4 *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + 2 * Sm::kTileO); };
+    // the precision tile the kernel computes with: float32 where lambda_v is float32 or formed from log-variances
     auto lfstage = [&](int s) {
         return reinterpret_cast<float *>(in_base + s * Sm::kIn +
                                          (sizeof(T) == 4 ? Sm::kTileI : 2 * Sm::kTileI + 2 * Sm::kTileO + Sm::kKq));
     };
-    constexpr bool pro = LOGV;
+    auto lam_pair = [&](int s, int at) {
+        if constexpr (sizeof(T) == 4 || LOGV) return load_pair(lfstage(s) + at);
+        else return load_pair(lstage(s) + at);
+    };
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // This CTA's sequence and, when sequences are cut into segments, its stretch of it: t_off steps in, L steps long
@@ -198,12 +237,9 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
     }
     __syncthreads();
 
-    // A trajectory buffer holds one float2 per compute thread for every (step u, channel ci, state i) of a tile:
-    // row = (u*CH + ci)*SPT + i, rows of NTC slots padded by kRowPad so that the helpers, whose lanes read
-    // different rows at the same column, do not collide on shared-memory banks. The replay thread and the
-    // reverse thread with the same index within their groups own the same chains and the same column.
-    constexpr int ROW = Sm::kRow;
-    auto trow = [&](int u, int ci, int i) { return ((u * CH + ci) * SPT + i) * ROW; };
+    // The replay thread and the reverse thread with the same index within their groups own the same chains and the
+    // same trajectory column: channels m_cta + cw, + 1 and states i * LPC + j.
+    auto trow = [&](int u, int i) { return (u * SPT + i) * ROW; };
 
     if (warp < 2 * NW) {
         // ======================================================= the two compute groups
@@ -211,35 +247,42 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
         const int ctid = tid & (NTC - 1);  // index within the group
         const int cwarp = ctid >> 5;
         const int j = lane % LPC, cl = lane / LPC;
-        const int cw = cwarp * Sh::kCPW + cl * CH;
+        const int cw = cwarp * CPW + cl * 2;
+        const int m0 = m_cta + cw;
+
+        // Per-chain constants as pairs over the two channels. Padding chains (s >= S or m >= M) get a = 0, p = 1.
+        float2 ca[SPT], ca2[SPT], cp[SPT];
+        auto load_constants = [&] {
+#pragma unroll
+            for (int i = 0; i < SPT; ++i) {
+                const int st = i * LPC + j;
+                float av[2], a2v[2], pv[2];
+#pragma unroll
+                for (int ci = 0; ci < 2; ++ci) {
+                    const bool live = (m0 + ci < M) && (st < S);
+                    av[ci] = live ? prm.a[(long long)(m0 + ci) * S + st] : 0.0f;
+                    a2v[ci] = live ? fmaxf(av[ci] * av[ci], kEps) : 0.0f;
+                    pv[ci] = fmaxf(live ? prm.p[(long long)(m0 + ci) * S + st] : 1.0f, kPMin);
+                }
+                ca[i] = make_float2(av[0], av[1]);
+                ca2[i] = make_float2(a2v[0], a2v[1]);
+                cp[i] = make_float2(pv[0], pv[1]);
+            }
+        };
 
         if (!is_reverse) {
             // ----------------------------------------------------------- replay
-            regs_shrink<kBwdRegsReplay>();
-            float ca[CH][SPT], ca2[CH][SPT], cp[CH][SPT];
-#pragma unroll
-            for (int ci = 0; ci < CH; ++ci) {
-                const int m = m_cta + cw + ci;
-#pragma unroll
-                for (int i = 0; i < SPT; ++i) {
-                    const int s = i * LPC + j;
-                    const bool live = (m < M) && (s < S);
-                    const float av = live ? prm.a[(long long)m * S + s] : 0.0f;
-                    const float pv = live ? prm.p[(long long)m * S + s] : 1.0f;
-                    ca[ci][i] = av;
-                    ca2[ci][i] = live ? fmaxf(av * av, kEps) : 0.0f;
-                    cp[ci][i] = fmaxf(pv, kPMin);
-                }
-            }
-            // checkpoint of the tile about to be replayed, fetched one tile ahead
-            float2 ck[CH][SPT];
+            regs_shrink<BwdRegs<SPAD>::kReplay>();
+            load_constants();
+            // checkpoint of the tile about to be replayed, fetched one tile ahead: (P, mean) per chain
+            float2 ck[SPT][2];
             auto load_ck = [&](int tile) {
-                const float2 *src = prm.ckpt + (((long long)b * prm.NT + tile_off + tile) * M + (m_cta + cw)) * S + j;
+                const float2 *src = prm.ckpt + (((long long)b * prm.NT + tile_off + tile) * M + m0) * S + j;
 #pragma unroll
-                for (int ci = 0; ci < CH; ++ci)
+                for (int i = 0; i < SPT; ++i)
 #pragma unroll
-                    for (int i = 0; i < SPT; ++i)
-                        ck[ci][i] = (m_cta + cw + ci < M && i * LPC + j < S) ? src[ci * S + i * LPC] : make_float2(1.0f, 0.0f);
+                    for (int ci = 0; ci < 2; ++ci)
+                        ck[i][ci] = (m0 + ci < M && i * LPC + j < S) ? src[ci * S + i * LPC] : make_float2(1.0f, 0.0f);
             };
             if (NT > 0) load_ck(NT - 1);
 
@@ -247,77 +290,58 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 const int tile = NT - 1 - ti, s = ti % NS, bf = ti & 1;
                 const int n = min(TT, L - tile * TT);
                 if (!mbar_wait(prm.wait, &full_in[s], (ti / NS) & 1, 11)) break;
-                if (pro) {  // this warp's channels of the tile: log-variance -> precision, float32
-                    const T *raw = lstage(s) + cwarp * Sh::kCPW;
-                    float *lf = lfstage(s) + cwarp * Sh::kCPW;
-                    for (int e = lane; e < TT * Sh::kCPW; e += 32) {
-                        const int at = (e / Sh::kCPW) * MC + e % Sh::kCPW;
+                if (LOGV) {  // this warp's channels of the tile: log-variance -> precision, float32
+                    const T *raw = lstage(s) + cwarp * CPW;
+                    float *lf = lfstage(s) + cwarp * CPW;
+                    for (int e = lane; e < TT * CPW; e += 32) {
+                        const int at = (e / CPW) * MC + e % CPW;
                         lf[at] = precision_from_log_variance_fast(to_f32<T>(raw[at]), prm.obs_var_min, prm.obs_var_max);
                     }
                     fence_proxy_async();  // these plain stores are ordered before the bulk copy that refills the stage
                     __syncwarp();
                 }
-                const T *lrow = lstage(s) + cw;
-                const float *lfrow = lfstage(s) + cw;
                 const T *vrow = vstage(s) + cw;
-                const float2 *kqrow = kqstage(s) + j;
-                float2 *traj = trajbuf(bf);
-                float P[CH][SPT], mean[CH][SPT];
+                const float4 *kqrow = kqstage(s) + j;
+                float4 *traj = trajbuf(bf) + ctid;
+                float2 P[SPT], nm[SPT];
 #pragma unroll
-                for (int ci = 0; ci < CH; ++ci)
-#pragma unroll
-                    for (int i = 0; i < SPT; ++i) {
-                        P[ci][i] = ck[ci][i].x;
-                        mean[ci][i] = ck[ci][i].y;
-                    }
+                for (int i = 0; i < SPT; ++i) {
+                    P[i] = make_float2(ck[i][0].x, ck[i][1].x);
+                    nm[i] = make_float2(-ck[i][0].y, -ck[i][1].y);
+                }
                 if (tile > 0) load_ck(tile - 1);
                 // the buffer still holds the partial sums of the tile before last until the helpers have consumed them
                 if (ti >= 2 && !mbar_wait(prm.wait, &buf_empty[bf], (ti / 2 - 1) & 1, 12)) break;
 
                 auto replay_step = [&](int u) {
-                    float lv[CH], vv[CH], Pp[CH][SPT], g[CH][SPT], r[CH][SPT];
-#pragma unroll
-                    for (int ci = 0; ci < CH; ++ci) {
-                        if constexpr (sizeof(T) == 4) lv[ci] = lfrow[u * MC + ci];  // the same tile as lrow
-                        else lv[ci] = pro ? lfrow[u * MC + ci] : to_f32<T>(lrow[u * MC + ci]);
-                        vv[ci] = to_f32<T>(vrow[u * MC + ci]);
-                    }
+                    const float2 lv = lam_pair(s, u * MC + cw), nv = neg2(load_pair(vrow + u * MC));
+                    float2 Pp[SPT], g[SPT], r[SPT];
 #pragma unroll
                     for (int i = 0; i < SPT; ++i) {
-                        const float kk = kqrow[u * SPAD + i * LPC].x;
-#pragma unroll
-                        for (int ci = 0; ci < CH; ++ci) {
-                            traj[trow(u, ci, i) + ctid] = make_float2(P[ci][i], mean[ci][i]);
-                            float phi;
-                            chain_inputs(lv[ci], vv[ci], kk, phi, r[ci][i]);
-                            g[ci][i] = chain_denominator(P[ci][i], phi, ca2[ci][i], cp[ci][i], Pp[ci][i]);
-                        }
+                        const float2 k = *reinterpret_cast<const float2 *>(&kqrow[u * SPAD + i * LPC]);
+                        traj[trow(u, i)] = make_float4(P[i].x, P[i].y, nm[i].x, nm[i].y);
+                        float2 phi;
+                        chain_inputs2(lv, nv, k, phi, r[i]);
+                        g[i] = chain_denominator2(P[i], phi, ca2[i], cp[i], Pp[i]);
                     }
 #pragma unroll
-                    for (int i = 0; i < SPT; ++i)
+                    for (int i = 0; i < SPT; ++i) g[i] = rcp_approx2(g[i]);
 #pragma unroll
-                        for (int ci = 0; ci < CH; ++ci) g[ci][i] = rcp_approx(g[ci][i]);
-#pragma unroll
-                    for (int i = 0; i < SPT; ++i)
-#pragma unroll
-                        for (int ci = 0; ci < CH; ++ci)
-                            chain_update(P[ci][i], mean[ci][i], Pp[ci][i], g[ci][i], r[ci][i], ca[ci][i]);
+                    for (int i = 0; i < SPT; ++i) chain_update2(P[i], nm[i], Pp[i], g[i], r[i], ca[i]);
                 };
                 if (n == TT) {
 #pragma unroll 1
-                    for (int h = 0; h < TT; h += kRepUnroll) {
+                    for (int h = 0; h < TT; h += kRepUnroll<SPAD>) {
 #pragma unroll
-                        for (int u = 0; u < kRepUnroll; ++u) replay_step(h + u);
+                        for (int u = 0; u < kRepUnroll<SPAD>; ++u) replay_step(h + u);
                     }
                 } else {
 #pragma unroll 1
                     for (int u = 0; u < n; ++u) replay_step(u);
                 }
-                if (ti == 0) {  // the state after the sequence's last step: where the reverse walk starts
+                if (ti == 0) {  // the state after the stretch's last step: where the reverse walk starts
 #pragma unroll
-                    for (int ci = 0; ci < CH; ++ci)
-#pragma unroll
-                        for (int i = 0; i < SPT; ++i) post[(ci * SPT + i) * ROW + ctid] = make_float2(P[ci][i], mean[ci][i]);
+                    for (int i = 0; i < SPT; ++i) post[i * ROW + ctid] = make_float4(P[i].x, P[i].y, nm[i].x, nm[i].y);
                 }
                 __syncwarp();
                 if (lane == 0) {
@@ -327,26 +351,15 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
             }
         } else {
             // ---------------------------------------------------------- reverse
-            regs_grow<kBwdRegsReverse>();
-            float ca[CH][SPT], ca2[CH][SPT], cp[CH][SPT];
-            float cP[CH][SPT], cm[CH][SPT], accA[CH][SPT], accA2[CH][SPT], accP[CH][SPT];
-            float Pn[CH][SPT], mn[CH][SPT];
+            regs_grow<BwdRegs<SPAD>::kReverse>();
+            load_constants();
+            // carries (that of P negated), running sums for da, da2, dp (negated), and the state after the step about
+            // to be walked (P, -mean)
+            float2 ncP[SPT], cm[SPT], naccA[SPT], naccA2[SPT], naccP[SPT], P[SPT], nm[SPT];
 #pragma unroll
-            for (int ci = 0; ci < CH; ++ci) {
-                const int m = m_cta + cw + ci;
-#pragma unroll
-                for (int i = 0; i < SPT; ++i) {
-                    const int s = i * LPC + j;
-                    const bool live = (m < M) && (s < S);
-                    const float av = live ? prm.a[(long long)m * S + s] : 0.0f;
-                    const float pv = live ? prm.p[(long long)m * S + s] : 1.0f;
-                    ca[ci][i] = av;
-                    ca2[ci][i] = live ? fmaxf(av * av, kEps) : 0.0f;
-                    cp[ci][i] = fmaxf(pv, kPMin);
-                    cP[ci][i] = cm[ci][i] = accA[ci][i] = accA2[ci][i] = accP[ci][i] = 0.0f;
-                    Pn[ci][i] = 1.0f;
-                    mn[ci][i] = 0.0f;
-                }
+            for (int i = 0; i < SPT; ++i) {
+                ncP[i] = cm[i] = naccA[i] = naccA2[i] = naccP[i] = nm[i] = make_float2(0.0f, 0.0f);
+                P[i] = make_float2(1.0f, 1.0f);
             }
 
             for (int ti = 0; ti < NT; ++ti) {
@@ -354,14 +367,12 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 const int n = min(TT, L - tile * TT);
                 if (!mbar_wait(prm.wait, &traj_full[bf], (ti / 2) & 1, 17)) break;
                 if (!mbar_wait(prm.wait, &full_in[s], (ti / NS) & 1, 18)) break;
-                const T *lrow = lstage(s) + cw;
-                const float *lfrow = lfstage(s) + cw;
                 const T *vrow = vstage(s) + cw;
                 const TO *dyrow = dystage(s) + cw;
                 const TO *dyvrow = dyvstage(s) + cw;
-                const float2 *kqrow = kqstage(s) + j;
-                float2 *traj = trajbuf(bf);
-                float2 *dpart = dpartbuf(bf);
+                const float4 *kqrow = kqstage(s) + j;
+                const float4 *traj = trajbuf(bf) + ctid;
+                float2 *parts = reinterpret_cast<float2 *>(trajbuf(bf)) + cwarp * 64 + lane;
 
                 if (ti == 0) {
                     // The walk starts from the state after the stretch's last step; at the end of the sequence the
@@ -372,128 +383,132 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                     if (!carried) break;
                     const long long plane = (long long)prm.B * M * S;
 #pragma unroll
-                    for (int ci = 0; ci < CH; ++ci) {
-                        const int m = m_cta + cw + ci;
+                    for (int i = 0; i < SPT; ++i) {
+                        const float4 fin = post[i * ROW + ctid];
+                        P[i] = make_float2(fin.x, fin.y);
+                        nm[i] = make_float2(fin.z, fin.w);
 #pragma unroll
-                        for (int i = 0; i < SPT; ++i) {
-                            const int st = i * LPC + j;
-                            const float2 fin = post[(ci * SPT + i) * ROW + ctid];
-                            Pn[ci][i] = fin.x;
-                            mn[ci][i] = fin.y;
+                        for (int ci = 0; ci < 2; ++ci) {
+                            const int m = m0 + ci, st = i * LPC + j;
+                            if (m >= M || st >= S) continue;
+                            const long long bms = ((long long)b * M + m) * S + st;
+                            auto at = [&](float2 &x) -> float & { return ci ? x.y : x.x; };
                             if (!last_seg) {
-                                if (m < M && st < S) {
-                                    const float *h = prm.seg.hand + ((long long)b * M + m) * S + st;
-                                    cP[ci][i] = __ldcg(h);
-                                    cm[ci][i] = __ldcg(h + plane);
-                                    accA[ci][i] = __ldcg(h + 2 * plane);
-                                    accA2[ci][i] = __ldcg(h + 3 * plane);
-                                    accP[ci][i] = __ldcg(h + 4 * plane);
-                                }
-                            } else if (prm.dlam_fin != nullptr && m < M && st < S) {
-                                const float Lb = prm.dlam_fin[((long long)b * M + m) * S + st];
-                                const float Eb = prm.deta_fin[((long long)b * M + m) * S + st];
-                                const float lam = 1.0f / fin.x;
-                                const float eta = fin.y * lam;
-                                cm[ci][i] = Eb * lam;
-                                cP[ci][i] = -lam * (lam * Lb + eta * Eb);
+                                const float *h = prm.seg.hand + bms;
+                                at(ncP[i]) = __ldcg(h);
+                                at(cm[i]) = __ldcg(h + plane);
+                                at(naccA[i]) = __ldcg(h + 2 * plane);
+                                at(naccA2[i]) = __ldcg(h + 3 * plane);
+                                at(naccP[i]) = __ldcg(h + 4 * plane);
+                            } else if (prm.dlam_fin != nullptr) {
+                                const float Lb = prm.dlam_fin[bms], Eb = prm.deta_fin[bms];
+                                const float lam = 1.0f / at(P[i]), eta = -at(nm[i]) * lam;
+                                at(cm[i]) = Eb * lam;
+                                at(ncP[i]) = lam * (lam * Lb + eta * Eb);
                             }
                         }
                     }
                 }
 
-                auto reverse_step = [&](int u) {
-                    float lv[CH], lv2[CH], vv[CH], vl[CH], dy[CH], dyv[CH], dyv2[CH], dvl[CH], dlphi[CH];
-#pragma unroll
-                    for (int ci = 0; ci < CH; ++ci) {
-                        if constexpr (sizeof(T) == 4) lv[ci] = lfrow[u * MC + ci];
-                        else lv[ci] = pro ? lfrow[u * MC + ci] : to_f32<T>(lrow[u * MC + ci]);
-                        vv[ci] = to_f32<T>(vrow[u * MC + ci]);
-                        dy[ci] = to_f32<TO>(dyrow[u * MC + ci]);
-                        dyv[ci] = to_f32<TO>(dyvrow[u * MC + ci]);
-                        vl[ci] = vv[ci] * lv[ci];
-                        lv2[ci] = lv[ci] + lv[ci];
-                        dyv2[ci] = dyv[ci] + dyv[ci];
-                        dvl[ci] = 0.0f;
-                        dlphi[ci] = 0.0f;
-                    }
-                    float2 prev[CH][SPT];
-                    float4 c[SPT];  // k^2, k, q, q^2
-                    float g[CH][SPT], Pp[CH][SPT], phi[CH][SPT], r[CH][SPT];
-#pragma unroll
-                    for (int i = 0; i < SPT; ++i) {
-                        // (k, q) from shared memory, the squares formed here: shared-memory bandwidth, not arithmetic,
-                        // is what this kernel runs out of
-                        const float2 kq2 = kqrow[u * SPAD + i * LPC];
-                        c[i] = make_float4(kq2.x * kq2.x, kq2.x, kq2.y, kq2.y * kq2.y);
-#pragma unroll
-                        for (int ci = 0; ci < CH; ++ci) {
-                            prev[ci][i] = traj[trow(u, ci, i) + ctid];  // P', mean'
-                            chain_inputs(lv[ci], vv[ci], c[i].y, phi[ci][i], r[ci][i]);
-                            g[ci][i] = chain_denominator(prev[ci][i].x, phi[ci][i], ca2[ci][i], cp[ci][i], Pp[ci][i]);
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < SPT; ++i)
-#pragma unroll
-                        for (int ci = 0; ci < CH; ++ci) g[ci][i] = rcp_approx(g[ci][i]);
-#pragma unroll
-                    for (int i = 0; i < SPT; ++i) {
-                        float X2 = 0.0f, Y = 0.0f, A_ = 0.0f, B2 = 0.0f;
-#pragma unroll
-                        for (int ci = 0; ci < CH; ++ci) {
-                            const float a = ca[ci][i], a2 = ca2[ci][i], p = cp[ci][i];
-                            const float gg = g[ci][i];
-                            float mbar, Pbar;
-                            if (PRIOR) {  // y reads a*mean and a2*P + p
-                                const float mob = dy[ci] * c[i].z, vob = dyv[ci] * c[i].w;
-                                mbar = fmaf(mob, a, cm[ci][i]);
-                                Pbar = fmaf(vob, a2, cP[ci][i]);
-                                accA[ci][i] = fmaf(mob, mn[ci][i], accA[ci][i]);
-                                accA2[ci][i] = fmaf(vob, Pn[ci][i], accA2[ci][i]);
-                                accP[ci][i] += vob;
-                                A_ = fmaf(dy[ci], a * mn[ci][i], A_);
-                                B2 = fmaf(dyv2[ci], fmaf(a2, Pn[ci][i], p), B2);
-                            } else {
-                                mbar = fmaf(dy[ci], c[i].z, cm[ci][i]);
-                                Pbar = fmaf(dyv[ci], c[i].w, cP[ci][i]);
-                                A_ = fmaf(dy[ci], mn[ci][i], A_);
-                                B2 = fmaf(dyv2[ci], Pn[ci][i], B2);
-                            }
-                            const float t2 = fmaf(Pbar, Pn[ci][i], mbar * mn[ci][i]);
-                            const float dbar = -(gg * t2);
-                            const float ubar = mbar * gg;
-                            const float Ppbar = fmaf(dbar, phi[ci][i], fmaf(Pbar, gg, ubar * r[ci][i]));
-                            const float rbar = ubar * Pp[ci][i];
-                            const float phibar = dbar * Pp[ci][i];
-                            cm[ci][i] = ubar * a;
-                            cP[ci][i] = Ppbar * a2;
-                            accA[ci][i] = fmaf(ubar, prev[ci][i].y, accA[ci][i]);
-                            accA2[ci][i] = fmaf(Ppbar, prev[ci][i].x, accA2[ci][i]);
-                            accP[ci][i] += Ppbar;
-                            dlphi[ci] = fmaf(phibar, c[i].x, dlphi[ci]);
-                            dvl[ci] = fmaf(rbar, c[i].y, dvl[ci]);
-                            X2 = fmaf(phibar, lv2[ci], X2);
-                            Y = fmaf(rbar, vl[ci], Y);
-                            Pn[ci][i] = prev[ci][i].x;
-                            mn[ci][i] = prev[ci][i].y;
-                        }
-                        // this thread's share of dk, dq for (t, s): parked where (P', mean') was
-                        traj[trow(u, 0, i) + ctid] = make_float2(fmaf(c[i].y, X2, Y), fmaf(c[i].z, B2, A_));
-                    }
-                    // this thread's share of the sums over s
-#pragma unroll
-                    for (int ci = 0; ci < CH; ++ci) dpart[(u * LPC + j) * MCP + cw + ci] = make_float2(dvl[ci], dlphi[ci]);
+                // A step's inputs are fetched, and its gain formed, while the step before it (later in time) is in its
+                // arithmetic: the stores at the end of a step could alias the next step's loads, so the compiler
+                // does not move them up by itself.
+                struct StepIn {
+                    float2 lv, v, dy, ndyv, k[SPT], q[SPT], P[SPT], nm[SPT];  // P, nm: the state before the step
                 };
-                if (n == TT) {
-                    // unrolled by kRevUnroll steps, not the whole tile: the walk's code then stays within the instruction cache
-#pragma unroll 1
-                    for (int h = TT - kRevUnroll; h >= 0; h -= kRevUnroll) {
+                auto fetch = [&](StepIn &in, int u) {
+                    in.lv = lam_pair(s, u * MC + cw);
+                    in.v = load_pair(vrow + u * MC);
+                    in.dy = load_pair(dyrow + u * MC);
+                    in.ndyv = neg2(load_pair(dyvrow + u * MC));
 #pragma unroll
-                        for (int u = kRevUnroll - 1; u >= 0; --u) reverse_step(h + u);
+                    for (int i = 0; i < SPT; ++i) {
+                        const float4 kq = kqrow[u * SPAD + i * LPC];
+                        in.k[i] = make_float2(kq.x, kq.y);
+                        in.q[i] = make_float2(kq.z, kq.w);
+                        const float4 x = traj[trow(u, i)];
+                        in.P[i] = make_float2(x.x, x.y);
+                        in.nm[i] = make_float2(x.z, x.w);
+                    }
+                };
+                auto gain = [&](float2 (&g)[SPT], const StepIn &in, const float2 (&Pn)[SPT]) {  // g = P/Pp
+#pragma unroll
+                    for (int i = 0; i < SPT; ++i) g[i] = mul2(Pn[i], rcp_approx2(fma2(ca2[i], in.P[i], cp[i])));
+                };
+                // P, nm: the state after the step on entry, before it on return; nxt, gn: fetched and formed for step un
+                auto reverse_step = [&](int u, const StepIn &in, const float2 (&g)[SPT], int un, StepIn &nxt, float2 (&gn)[SPT]) {
+                    fetch(nxt, un);
+                    const float2 nlv = neg2(in.lv), lv2 = add2(in.lv, in.lv), vl = mul2(in.v, in.lv);
+                    float2 D, E, share[SPT];
+#pragma unroll
+                    for (int i = 0; i < SPT; ++i) {
+                        const float2 k = in.k[i], q = in.q[i];
+                        const float2 e = fma2(k, nm[i], in.v);             // v - k mean
+                        const float2 nw = mul2(mul2(nlv, k), e);           // -w
+                        const float2 qd = mul2(q, in.ndyv);
+                        float2 mbar, nPbar, dq;
+                        if (PRIOR) {  // y reads a*mean and a2*P + p
+                            const float2 mob = mul2(in.dy, q), nvob = mul2(qd, q);
+                            mbar = fma2(mob, ca[i], cm[i]);
+                            nPbar = fma2(nvob, ca2[i], ncP[i]);
+                            naccA[i] = fma2(mob, nm[i], naccA[i]);
+                            naccA2[i] = fma2(nvob, P[i], naccA2[i]);
+                            naccP[i] = add2(naccP[i], nvob);
+                            dq = fma2(add2(qd, qd), fma2(ca2[i], P[i], cp[i]), mul2(in.dy, mul2(ca[i], nm[i])));
+                        } else {
+                            mbar = fma2(in.dy, q, cm[i]);
+                            nPbar = fma2(qd, q, ncP[i]);
+                            dq = fma2(add2(qd, qd), P[i], mul2(in.dy, nm[i]));
+                        }
+                        const float2 phibar = mul2(P[i], fma2(mbar, nm[i], mul2(nPbar, P[i])));
+                        const float2 rbar = mul2(P[i], mbar);
+                        const float2 ubar = mul2(mbar, g[i]);
+                        const float2 nPpbar = mul2(g[i], fma2(mbar, nw, mul2(nPbar, g[i])));
+                        const float2 z = mul2(phibar, k);
+                        const float2 dk = fma2(z, lv2, mul2(rbar, vl));
+                        D = i == 0 ? mul2(rbar, k) : fma2(rbar, k, D);
+                        E = i == 0 ? mul2(z, k) : fma2(z, k, E);
+                        cm[i] = mul2(ubar, ca[i]);
+                        ncP[i] = mul2(nPpbar, ca2[i]);
+                        naccA[i] = fma2(ubar, in.nm[i], naccA[i]);
+                        naccA2[i] = fma2(nPpbar, in.P[i], naccA2[i]);
+                        naccP[i] = add2(naccP[i], nPpbar);
+                        P[i] = in.P[i];
+                        nm[i] = in.nm[i];
+                        share[i] = make_float2(dk.x + dk.y, dq.x + dq.y);  // this thread's dk, -dq for (t, s)
+                    }
+                    gain(gn, nxt, P);
+                    // parked where the warp's own trajectory slots of this step were: row (u, i) of the warp is 64 float2s,
+                    // the shares in its first half, D / E in the second half of rows i = 0 / 1
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < SPT; ++i) parts[2 * trow(u, i)] = share[i];
+                    parts[2 * trow(u, 0) + 32] = D;
+                    parts[2 * trow(u, 1) + 32] = E;
+                };
+                StepIn in[2];
+                float2 g[2][SPT];
+                fetch(in[0], n - 1);
+                gain(g[0], in[0], P);
+                if (n == TT) {
+                    static_assert(kRevUnroll<SPAD> % 2 == 0, "the two register sets swap roles from step to step");
+#pragma unroll 1
+                    for (int h = TT - kRevUnroll<SPAD>; h >= 0; h -= kRevUnroll<SPAD>) {
+#pragma unroll
+                        for (int u = kRevUnroll<SPAD> - 1; u >= 0; --u) {
+                            const int c = (kRevUnroll<SPAD> - 1 - u) & 1;
+                            // (the fetch past the tile's first step re-reads that step and is not used)
+                            reverse_step(h + u, in[c], g[c], max(h + u - 1, 0), in[c ^ 1], g[c ^ 1]);
+                        }
                     }
                 } else {
 #pragma unroll 1
-                    for (int u = n - 1; u >= 0; --u) reverse_step(u);
+                    for (int u = n - 1; u >= 0; --u) {
+                        reverse_step(u, in[0], g[0], max(u - 1, 0), in[1], g[1]);
+                        in[0] = in[1];
+#pragma unroll
+                        for (int i = 0; i < SPT; ++i) g[0][i] = g[1][i];
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) {
@@ -506,38 +521,37 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 // ---- start of an inner segment: hand the carries and the running sums to the segment before it
                 const long long plane = (long long)prm.B * M * S;
 #pragma unroll
-                for (int ci = 0; ci < CH; ++ci) {
-                    const int m = m_cta + cw + ci;
+                for (int i = 0; i < SPT; ++i)
 #pragma unroll
-                    for (int i = 0; i < SPT; ++i) {
-                        const int st = i * LPC + j;
-                        if (m < M && st < S) {
-                            float *h = prm.seg.hand + ((long long)b * M + m) * S + st;
-                            __stcg(h, cP[ci][i]);
-                            __stcg(h + plane, cm[ci][i]);
-                            __stcg(h + 2 * plane, accA[ci][i]);
-                            __stcg(h + 3 * plane, accA2[ci][i]);
-                            __stcg(h + 4 * plane, accP[ci][i]);
-                        }
+                    for (int ci = 0; ci < 2; ++ci) {
+                        const int m = m0 + ci, st = i * LPC + j;
+                        if (m >= M || st >= S) continue;
+                        auto at = [&](const float2 &x) { return ci ? x.y : x.x; };
+                        float *h = prm.seg.hand + ((long long)b * M + m) * S + st;
+                        __stcg(h, at(ncP[i]));
+                        __stcg(h + plane, at(cm[i]));
+                        __stcg(h + 2 * plane, at(naccA[i]));
+                        __stcg(h + 3 * plane, at(naccA2[i]));
+                        __stcg(h + 4 * plane, at(naccP[i]));
                     }
-                }
                 __threadfence();
                 group_barrier_128();
                 if (tid == 0) st_release_gpu(prm.seg.done + unit.seq, prm.seg.nseg - unit.seg);
             }
             // ---- start of the sequence: gradients of a, p and of the carried-in state
+            if (first_seg) {
 #pragma unroll
-            for (int ci = 0; ci < CH; ++ci) {
-                const int m = m_cta + cw + ci;
+                for (int i = 0; i < SPT; ++i)
 #pragma unroll
-                for (int i = 0; i < SPT; ++i) {
-                    const int st = i * LPC + j;
-                    if (first_seg && m < M && st < S) {
+                    for (int ci = 0; ci < 2; ++ci) {
+                        const int m = m0 + ci, st = i * LPC + j;
+                        if (m >= M || st >= S) continue;
+                        auto at = [&](const float2 &x) { return ci ? x.y : x.x; };
                         const long long ms = (long long)m * S + st, bms = ((long long)b * M + m) * S + st;
-                        const float a = ca[ci][i];
+                        const float a = at(ca[i]);
                         const float da2_da = (a * a >= kEps) ? 2.0f * a : 0.0f;  // clamp_min subgradient
-                        atomicAdd(prm.da + ms, fmaf(accA2[ci][i], da2_da, accA[ci][i]));
-                        if (prm.p[ms] >= kPMin) atomicAdd(prm.dp + ms, accP[ci][i]);
+                        atomicAdd(prm.da + ms, -fmaf(at(naccA2[i]), da2_da, at(naccA[i])));
+                        if (prm.p[ms] >= kPMin) atomicAdd(prm.dp + ms, -at(naccP[i]));
                         float lam0 = 1.0f, eta0 = 0.0f;
                         if (prm.lam0 != nullptr) {
                             lam0 = prm.lam0[bms];
@@ -545,15 +559,14 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                         }
                         // P0 = 1/max(lam0, floor), mean0 = eta0 * P0
                         const float P0 = 1.0f / fmaxf(lam0, kLamMin);
-                        prm.deta0[bms] = cm[ci][i] * P0;
-                        prm.dlam0[bms] = (lam0 >= kLamMin) ? -(cP[ci][i] + cm[ci][i] * eta0) * P0 * P0 : 0.0f;
+                        prm.deta0[bms] = at(cm[i]) * P0;
+                        prm.dlam0[bms] = (lam0 >= kLamMin) ? (at(ncP[i]) - at(cm[i]) * eta0) * P0 * P0 : 0.0f;
                     }
-                }
             }
         }
     } else {
         // ================================================================ helpers
-        regs_shrink<kBwdRegsHelper>();
+        regs_shrink<BwdRegs<SPAD>::kHelper>();
         const int htid = tid - 2 * NTC;
         const int hlane = htid & 31;
         constexpr uint32_t kBytesI = sizeof(T) * TT * MC, kBytesO = sizeof(TO) * TT * MC;
@@ -572,24 +585,40 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 for (int s = 0; s < NS; ++s)
                     for (int idx = htid; idx < TT * MC; idx += kProducers) dyvstage(s)[idx] = from_f32<TO>(0.0f);
             }
-            // (k, q) of the next tile are fetched into registers while the current one
-            // is handed over, so the loader never sits on a global-memory latency
-            constexpr int KQP = (TT * SPAD + kProducers - 1) / kProducers;
-            float kr[KQP], qr[KQP];
+            // (k, q) of the next tile are on their way while the current one is handed over, so the loader never sits on a
+            // global-memory latency: in registers up to 16 states, by per-thread asynchronous copies into shared memory
+            // beyond, where a tile in registers spilled up to 500 bytes per thread, and a tile fetched when its stage was
+            // free set the pace (B=4 L=2048 M=512 S=64: 1.61 and 1.10 ms, with the copies 0.80 ms). With one CTA per SM
+            // the registers are the shorter way (B=4 of the headline shape 0.71 against 0.75 ms).
+            constexpr int KQP = TT * SPAD / kProducers;
+            constexpr bool kInRegs = KQP <= 4;
+            float kr[kInRegs ? KQP : 1], qr[kInRegs ? KQP : 1];
             auto load_kq = [&](int t0) {
 #pragma unroll
-                for (int e = 0; e < KQP; ++e) {
+                for (int e = 0; e < (kInRegs ? KQP : 0); ++e) {
                     const int idx = htid + e * kProducers, row = idx / SPAD, sidx = idx % SPAD;
-                    const bool in = idx < TT * SPAD && sidx < S && t0 + row < L;
+                    const bool in = sidx < S && t0 + row < L;
                     kr[e] = in ? to_f32<T>(kb[(long long)(t0 + row) * prm.k.st + sidx]) : 0.0f;
                     qr[e] = in ? to_f32<T>(qb[(long long)(t0 + row) * prm.q.st + sidx]) : 0.0f;
                 }
             };
-            if (NT > 0) load_kq((NT - 1) * TT);
+            auto raw = [&](int bf, int which) { return reinterpret_cast<T *>(raw_base + bf * Sm::kRawKq + which * (Sm::kRawKq / 2)); };
+            auto fetch_kq = [&](int t0, int bf) {
+                stage_tile<T, TT, SPAD, kProducers>(raw(bf, 0), kb, prm.k.st, t0, L, 0, S, htid);
+                stage_tile<T, TT, SPAD, kProducers>(raw(bf, 1), qb, prm.q.st, t0, L, 0, S, htid);
+            };
+            if (NT > 0) {
+                if (kInRegs) load_kq((NT - 1) * TT);
+                else fetch_kq((NT - 1) * TT, 0);
+            }
             for (int it = 0; it < NT; ++it) {
                 const int tile = NT - 1 - it, s = it % NS, t0 = tile * TT;
                 // the stage is free once the compute groups and the summing helpers are done with it
                 if (it >= NS && !mbar_wait(prm.wait, &empty_in[s], (it / NS - 1) & 1, 13, 100)) { ok = false; break; }
+                if (!kInRegs) {
+                    cp_async_wait_all();  // k, q of this tile, asked for a tile ago
+                    __syncwarp();
+                }
                 if (prm.use_tma) {
                     if (htid == 0) {
                         mbar_arrive_expect_tx(&full_in[s], 2 * kBytesI + (has_dyv ? 2 : 1) * kBytesO);
@@ -605,14 +634,22 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                     if (has_dyv)
                         stage_tile<TO, TT, MC, kProducers>(dyvstage(s), dyvb, prm.dyv.st, t0, L, m_cta, M, htid);
                 }
-                float2 *kq = kqstage(s);
-#pragma unroll
-                for (int e = 0; e < KQP; ++e) {
-                    const int idx = htid + e * kProducers;
-                    if (idx < TT * SPAD) kq[idx] = make_float2(kr[e], qr[e]);
-                }
-                if (tile > 0) load_kq(t0 - TT);
                 if (!prm.use_tma) stage_arrive(&full_in[s]);
+                float4 *kq = kqstage(s);
+                if (kInRegs) {
+#pragma unroll
+                    for (int e = 0; e < (kInRegs ? KQP : 0); ++e) kq[htid + e * kProducers] = make_float4(kr[e], kr[e], qr[e], qr[e]);
+                    if (tile > 0) load_kq(t0 - TT);
+                } else {
+                    if (tile > 0) fetch_kq(t0 - TT, (it + 1) & 1);
+                    const T *rk = raw(it & 1, 0), *rq = raw(it & 1, 1);
+#pragma unroll 8
+                    for (int idx = htid; idx < TT * SPAD; idx += kProducers) {
+                        const float k = to_f32<T>(rk[idx]), q = to_f32<T>(rq[idx]);
+                        kq[idx] = make_float4(k, k, q, q);
+                    }
+                    __syncwarp();
+                }
                 // (test hook, as in the forward: the wait for tile skip_tile runs out)
                 if (!(prm.use_tma && htid == 0) && !(it == prm.wait.skip_tile && htid == 1)) mbar_arrive(&full_in[s]);
                 produced = it + 1;
@@ -625,73 +662,85 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
             for (int jt = 0; jt < NT; ++jt) {
                 const int tile = NT - 1 - jt, s = jt % NS, t0 = tile * TT, bf = jt & 1;
                 const int n = min(TT, L - t0);
-                const T *lt = lstage(s), *vt = vstage(s);
-                const float *lft = lfstage(s);
-                const float2 *traj = trajbuf(bf);
-                const float2 *dpart = dpartbuf(bf);
+                const T *vt = vstage(s);
+                const float2 *parts = reinterpret_cast<const float2 *>(trajbuf(bf));
                 if (!mbar_wait(prm.wait, &part_full[bf], (jt / 2) & 1, 14, 100)) break;
-                // dk, dq: add the CTA's channels. Compute thread t holds lane group j = t % LPC, so the partials
-                // of state s = i*LPC + jj sit at columns jj, jj + LPC, ... of row (u, i).
-                for (int pidx = ctid; pidx < TT * SPAD; pidx += kSummers) {
-                    const int jj = pidx % LPC, row = pidx / LPC;  // row = (step, i)
-                    const int u = row / SPT, i = row % SPT;
-                    const int st = i * LPC + jj;
-                    const float2 *src = traj + trow(u, 0, i) + jj;
-                    float sk0 = 0.0f, sq0 = 0.0f, sk1 = 0.0f, sq1 = 0.0f;
+                // dk, dq: add the CTA's channels. A unit is two neighbouring states of one step (the shares of lanes
+                // jj, jj + 1 of every channel pair).
+                for (int unit_id = ctid; unit_id < TT * SPT * (LPC / 2); unit_id += kSummers) {
+                    const int jj = (unit_id % (LPC / 2)) * 2, row = unit_id / (LPC / 2);  // row = (step, i)
+                    const int u = row / SPT, st = (row % SPT) * LPC + jj;
+                    const float2 *src = parts + 2 * row * ROW + jj;
+                    float2 x0 = make_float2(0.0f, 0.0f), x1 = x0;
 #pragma unroll
-                    for (int c = 0; c < NTC / LPC; c += 2) {
-                        const float2 x0 = src[c * LPC], x1 = src[(c + 1) * LPC];
-                        sk0 += x0.x; sq0 += x0.y;
-                        sk1 += x1.x; sq1 += x1.y;
-                    }
+                    for (int w = 0; w < NW; ++w)
+#pragma unroll
+                        for (int c = 0; c < CLS; ++c) {
+                            const float4 x = *reinterpret_cast<const float4 *>(src + w * 64 + c * LPC);
+                            x0 = add2(x0, make_float2(x.x, x.y));
+                            x1 = add2(x1, make_float2(x.z, x.w));
+                        }
                     if (st < S && u < n) {
-                        atomicAdd(prm.dk + ((long long)b * prm.L + t_off + t0 + u) * S + st, sk0 + sk1);
-                        atomicAdd(prm.dq + ((long long)b * prm.L + t_off + t0 + u) * S + st, sq0 + sq1);
+                        const long long at = ((long long)b * prm.L + t_off + t0 + u) * S + st;
+                        if (prm.vec_dkq) {
+                            atomicAdd(reinterpret_cast<float2 *>(prm.dk + at), make_float2(x0.x, x1.x));
+                            atomicAdd(reinterpret_cast<float2 *>(prm.dq + at), make_float2(-x0.y, -x1.y));
+                        } else {
+                            atomicAdd(prm.dk + at, x0.x);
+                            atomicAdd(prm.dq + at, -x0.y);
+                            if (st + 1 < S) {
+                                atomicAdd(prm.dk + at + 1, x1.x);
+                                atomicAdd(prm.dq + at + 1, -x1.y);
+                            }
+                        }
                     }
                 }
-                // dv, dlambda_v: add the lane groups. v enters only through v*lambda_v (kla_ops.py:177): with
-                // D = sum_s rbar k, dv = D lambda_v and dlambda_v = sum_s phibar k^2 + D v.
+                // dv, dlambda_v: add the lane group of a channel pair. v enters only through v*lambda_v
+                // (kla_ops.py:177): dv = D lambda_v and dlambda_v = E + D v.
                 // (threads taken from the other end, so the two loops spread over the warps)
-                for (int uidx = kSummers - 1 - ctid; uidx < TT * (MC / 2); uidx += kSummers) {
-                    const int u = uidx / (MC / 2), c = (uidx % (MC / 2)) * 2;
-                    if (u >= n || m_cta + c >= M) continue;
-                    float ax = 0.0f, ay = 0.0f, bx = 0.0f, by = 0.0f;
+                // A wide lane group is split over kParts threads, eight lanes each, whose sums meet by shuffles.
+                constexpr int kParts = LPC > 8 ? LPC / 8 : 1, kLanes = LPC / kParts;
+                static_assert(32 % kParts == 0 && (TT * (MC / 2) * kParts) % 32 == 0, "parts of a unit share a warp, whole warps work");
+                for (int uidx = kSummers - 1 - ctid; uidx < TT * (MC / 2) * kParts; uidx += kSummers) {
+                    const int u = uidx / (MC / 2 * kParts), pp = uidx % (MC / 2 * kParts), pr = pp / kParts, c = pr * 2;
+                    const float2 *src = parts + 2 * u * SPT * ROW + (pr / CLS) * 64 + 32 + (pr % CLS) * LPC + (pp % kParts) * kLanes;
+                    float2 D0 = make_float2(0.0f, 0.0f), E0 = D0;
 #pragma unroll
-                    for (int jj = 0; jj < LPC; ++jj) {
-                        const float4 x = *reinterpret_cast<const float4 *>(dpart + (u * LPC + jj) * MCP + c);
-                        ax += x.x; ay += x.y; bx += x.z; by += x.w;
+                    for (int h = 0; h < kLanes / 2; ++h) {
+                        // every other lane starts 16 bytes further on: neighbouring threads read 64 bytes (eight lanes) apart
+                        const int at = 2 * ((h + (pp >> 1)) % (kLanes / 2));
+                        const float4 x = *reinterpret_cast<const float4 *>(src + at);
+                        const float4 y = *reinterpret_cast<const float4 *>(src + 2 * ROW + at);
+                        D0 = add2(D0, add2(make_float2(x.x, x.y), make_float2(x.z, x.w)));
+                        E0 = add2(E0, add2(make_float2(y.x, y.y), make_float2(y.z, y.w)));
                     }
-                    float l0, l1;
-                    if (pro || sizeof(T) == 4) {
-                        l0 = lft[u * MC + c];
-                        l1 = lft[u * MC + c + 1];
-                    } else {
-                        l0 = to_f32<T>(lt[u * MC + c]);
-                        l1 = to_f32<T>(lt[u * MC + c + 1]);
+#pragma unroll
+                    for (int o = kParts / 2; o > 0; o /= 2) {
+                        D0 = add2(D0, make_float2(__shfl_xor_sync(0xffffffffu, D0.x, o), __shfl_xor_sync(0xffffffffu, D0.y, o)));
+                        E0 = add2(E0, make_float2(__shfl_xor_sync(0xffffffffu, E0.x, o), __shfl_xor_sync(0xffffffffu, E0.y, o)));
                     }
-                    const float v0 = to_f32<T>(vt[u * MC + c]), v1 = to_f32<T>(vt[u * MC + c + 1]);
-                    const float dv0 = ax * l0, dv1 = bx * l1;
-                    float dl0 = fmaf(ax, v0, ay), dl1 = fmaf(bx, v1, by);
-                    if (pro) {  // chain through Lambda_v = 1 / min(softplus(x) + floor, ceiling)
-                        dl0 *= precision_slope(l0, prm.obs_var_min, prm.obs_var_max);
-                        dl1 *= precision_slope(l1, prm.obs_var_min, prm.obs_var_max);
+                    if (pp % kParts != 0 || u >= n || m_cta + c >= M) continue;
+                    const float2 lam = lam_pair(s, u * MC + c), v = load_pair(vt + u * MC + c);
+                    const float2 dv = mul2(D0, lam);
+                    float2 dl = fma2(D0, v, E0);
+                    if (LOGV) {  // chain through Lambda_v = 1 / min(softplus(x) + floor, ceiling)
+                        dl.x *= precision_slope(lam.x, prm.obs_var_min, prm.obs_var_max);
+                        dl.y *= precision_slope(lam.y, prm.obs_var_min, prm.obs_var_max);
                     }
                     T *p0 = dvb + (long long)(t0 + u) * prm.dv.st + m_cta + c;
                     T *p1 = dlvb + (long long)(t0 + u) * prm.dlv.st + m_cta + c;
                     const bool full = m_cta + c + 1 < M;
                     if (full && prm.vec_dv) {
-                        if constexpr (sizeof(T) == 4) *reinterpret_cast<float2 *>(p0) = make_float2(dv0, dv1);
-                        else *reinterpret_cast<__nv_bfloat162 *>(p0) = __floats2bfloat162_rn(dv0, dv1);
+                        store_pair(p0, dv.x, dv.y);
                     } else {
-                        p0[0] = from_f32<T>(dv0);
-                        if (full) p0[1] = from_f32<T>(dv1);
+                        p0[0] = from_f32<T>(dv.x);
+                        if (full) p0[1] = from_f32<T>(dv.y);
                     }
                     if (full && prm.vec_dlv) {
-                        if constexpr (sizeof(T) == 4) *reinterpret_cast<float2 *>(p1) = make_float2(dl0, dl1);
-                        else *reinterpret_cast<__nv_bfloat162 *>(p1) = __floats2bfloat162_rn(dl0, dl1);
+                        store_pair(p1, dl.x, dl.y);
                     } else {
-                        p1[0] = from_f32<T>(dl0);
-                        if (full) p1[1] = from_f32<T>(dl1);
+                        p1[0] = from_f32<T>(dl.x);
+                        if (full) p1[1] = from_f32<T>(dl.y);
                     }
                 }
                 __syncwarp();
@@ -701,7 +750,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 }
             }
         }
-        if (!ok && !prm.use_tma) cp_async_wait_all();
+        if (!ok) cp_async_wait_all();
         if (!ok && prm.use_tma && htid == 0) {
             for (int t = max(0, produced - NS); t < produced; ++t) mbar_wait(prm.wait, &full_in[t % NS], (t / NS) & 1, 15);
         }

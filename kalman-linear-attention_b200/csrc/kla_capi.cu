@@ -217,11 +217,10 @@ int plan_segments(int64_t ctas, int64_t L, bool backward, int *seg_len) {
 // Fill prm.seg for one direction and clear its ticket and done words. The working memory is the bytes behind the
 // checkpoints, or, for a forward without checkpoints, the caller's `work` buffer of the same layout.
 template <typename Params>
-int seg_setup(Params &prm, void *ckpt, void *work, int64_t B, int64_t L, int64_t M, int64_t S, int lpc, bool backward,
+int seg_setup(Params &prm, void *ckpt, void *work, int64_t B, int64_t L, int64_t M, int64_t S, int mc, bool backward,
               cudaStream_t st) {
     prm.seg = SegCtl{1, (int)L, nullptr, nullptr, nullptr};
     if ((ckpt == nullptr && work == nullptr) || L <= 0) return KLA_B200_OK;
-    const int mc = scan_channels_per_cta(lpc);
     const int64_t ctas = ((M + mc - 1) / mc) * B;
     int seg_len = (int)L;
     const int nseg = plan_segments(ctas, L, backward, &seg_len);
@@ -246,7 +245,7 @@ int seg_setup(Params &prm, void *ckpt, void *work, int64_t B, int64_t L, int64_t
 template <typename T, typename TO, int LPC, bool PRIOR>
 int prep_fwd(FwdParams &prm, const kla_b200_fwd_args &a, cudaStream_t st) {
     const int mc = scan_channels_per_cta(LPC);
-    if (int rc = seg_setup(prm, a.ckpt, a.work, a.B, a.L, a.M, a.S, LPC, false, st)) return rc;
+    if (int rc = seg_setup(prm, a.ckpt, a.work, a.B, a.L, a.M, a.S, mc, false, st)) return rc;
     prm.use_tma = !g_no_tma && make_tile_map<T>(&prm.tm_v, a.v, a.B, a.L, a.M, mc, kTT) &&
                   make_tile_map<T>(&prm.tm_lv, a.lambda_v, a.B, a.L, a.M, mc, kTT);
     if (prm.epilogue)  // z and gate tiles travel like v and lambda_v when they meet the tensor-map rules
@@ -259,8 +258,8 @@ int prep_fwd(FwdParams &prm, const kla_b200_fwd_args &a, cudaStream_t st) {
 
 template <typename T, typename TO, int LPC, bool PRIOR>
 int prep_bwd(BwdParams &prm, const kla_b200_bwd_args &a, cudaStream_t st) {
-    const int mc = scan_channels_per_cta(LPC);
-    if (int rc = seg_setup(prm, const_cast<void *>(a.ckpt), nullptr, a.B, a.L, a.M, a.S, LPC, true, st)) return rc;
+    const int mc = bwd_channels_per_cta<LPC>();
+    if (int rc = seg_setup(prm, const_cast<void *>(a.ckpt), nullptr, a.B, a.L, a.M, a.S, mc, true, st)) return rc;
     prm.use_tma = !g_no_tma && make_tile_map<T>(&prm.tm_v, a.v, a.B, a.L, a.M, mc, kBwdTT) &&
                   make_tile_map<T>(&prm.tm_lv, a.lambda_v, a.B, a.L, a.M, mc, kBwdTT) &&
                   make_tile_map<TO>(&prm.tm_dy, a.dy, a.B, a.L, a.M, mc, kBwdTT) &&
@@ -529,6 +528,7 @@ int kla_b200_scan_bwd(const kla_b200_bwd_args *a, void *stream) {
     prm.dlam0 = a->dlam0; prm.deta0 = a->deta0;
     if ((rc = wait_ctl(&prm.wait))) return rc;
     prm.vec_dv = a->in_dtype == KLA_B200_F32 ? vec2_ok<float>(a->dv) : vec2_ok<__nv_bfloat16>(a->dv);
+    prm.vec_dkq = a->S % 2 == 0 && aligned(a->dk, 8) && aligned(a->dq, 8);
     prm.vec_dlv = a->in_dtype == KLA_B200_F32 ? vec2_ok<float>(a->dlambda_v) : vec2_ok<__nv_bfloat16>(a->dlambda_v);
     return dispatch_bwd(a->in_dtype, a->out_dtype, a->decode_from_prior != 0, lpc_for(a->S), prm, *a, st);
 }

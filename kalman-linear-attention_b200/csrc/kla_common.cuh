@@ -178,10 +178,13 @@ __device__ __forceinline__ void chain_update(float &P, float &mean, float Pp, fl
     mean = __fmul_rn(g, __fmaf_rn(Pp, r, __fmul_rn(a, mean)));
 }
 
-// The same pieces for two chains at a time. sm_100 issues an fp32 multiply, add
-// or FMA on a pair of values held in an aligned register pair as one
-// instruction; every lane of it rounds like the scalar instruction, so the pair
-// forms give bit-identical results while taking half the issue slots.
+// The same pieces for two chains at a time, held in aligned register pairs. sm_100 issues an fp32 multiply, add or FMA
+// on a pair as one instruction; every lane of it rounds like the scalar instruction, so the pair forms give
+// bit-identical results while taking half the issue slots. They do not take half the time: measured on B200, in cycles
+// of a scheduler per instruction with all operands different, a pair multiply or add takes 2.25 and a pair FMA 3.75
+// (2.9 / 2.4 when one / two operands repeat those of the instruction before, 2.2 with a constant addend), where two
+// scalar instructions take 2.06: what a pair FMA waits for is its six register reads. Mixing in scalar FMAs does not
+// help where the operands live in pairs: their halves then sit in the same register bank.
 __device__ __forceinline__ float2 mul2(float2 x, float2 y) { return __fmul2_rn(x, y); }
 __device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) { return __ffma2_rn(x, y, z); }
 __device__ __forceinline__ float2 add2(float2 x, float2 y) { return __fadd2_rn(x, y); }

@@ -32,6 +32,10 @@ constexpr int kCH = KLA_CH;            // channels per thread
 // channels per CTA of the scan kernels for a given number of lanes per channel
 inline int scan_channels_per_cta(int lpc) { return kNW * (32 / lpc) * kCH; }
 
+// channels per CTA of the backward kernel
+template <int LPC>
+constexpr int bwd_channels_per_cta() { return BwdShape<kSPT * LPC>::kMC; }
+
 // channels per CTA of the aggregate kernel
 inline int agg_channels_per_cta(int lpc) { return kNW * (32 / lpc); }
 

@@ -27,13 +27,14 @@ cudaError_t launch_fwd(const FwdParams &prm, cudaStream_t st) {
 
 template <typename T, typename TO, int LPC, bool PRIOR>
 cudaError_t launch_bwd(const BwdParams &prm, cudaStream_t st) {
-    using Sh = ScanShape<kSPT, LPC, kCH, kNW, kNH, kBwdTT>;
-    using Sm = BwdSmem<T, TO, kSPT, LPC, kCH, kNW, kNH, kBwdTT>;
+    constexpr int SPAD = kSPT * LPC;
+    using Sm = BwdSmem<T, TO, SPAD, kBwdTT>;
+    constexpr int MC = BwdShape<SPAD>::kMC;
     const bool seg = prm.seg.nseg > 1;
-    auto kern = prm.lv_log_sigma ? (seg ? kla_bwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kBwdTT, PRIOR, true, true>
-                                        : kla_bwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kBwdTT, PRIOR, true, false>)
-                                 : (seg ? kla_bwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kBwdTT, PRIOR, false, true>
-                                        : kla_bwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kBwdTT, PRIOR, false, false>);
+    auto kern = prm.lv_log_sigma ? (seg ? kla_bwd_kernel<T, TO, SPAD, kBwdTT, PRIOR, true, true>
+                                        : kla_bwd_kernel<T, TO, SPAD, kBwdTT, PRIOR, true, false>)
+                                 : (seg ? kla_bwd_kernel<T, TO, SPAD, kBwdTT, PRIOR, false, true>
+                                        : kla_bwd_kernel<T, TO, SPAD, kBwdTT, PRIOR, false, false>);
     // The kernel's warp groups re-divide the registers the CTA was launched with; if the compiled kernel holds
     // fewer than the division assumes, the group that grows would wait for registers that never come. Checked
     // once per instantiation, before anything is launched.
@@ -43,12 +44,12 @@ cudaError_t launch_bwd(const BwdParams &prm, cudaStream_t st) {
         cudaFuncAttributes attr;
         cudaError_t e = cudaFuncGetAttributes(&attr, kern);
         if (e != cudaSuccess) return e;
-        ok = attr.numRegs * kBwdThreads >= 128 * (kBwdRegsReverse + kBwdRegsReplay + kBwdRegsHelper) ? 1 : 0;
+        ok = attr.numRegs * kBwdThreads >= 128 * (BwdRegs<SPAD>::kReverse + BwdRegs<SPAD>::kReplay + BwdRegs<SPAD>::kHelper) ? 1 : 0;
     }
     if (!ok) return cudaErrorLaunchOutOfResources;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sm::kTotal);
     if (e != cudaSuccess) return e;
-    dim3 grid((unsigned)((prm.M + Sh::kMC - 1) / Sh::kMC), (unsigned)prm.B, (unsigned)prm.seg.nseg);
+    dim3 grid((unsigned)((prm.M + MC - 1) / MC), (unsigned)prm.B, (unsigned)prm.seg.nseg);
     kern<<<grid, kBwdThreads, Sm::kTotal, st>>>(prm);
     return cudaGetLastError();
 }
