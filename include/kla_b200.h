@@ -107,6 +107,11 @@ typedef struct kla_b200_fwd_args {
      * working memory, with which this forward too can hand its sequences from CTA to CTA in segments; NULL: it runs
      * unsegmented. Ignored when ckpt is given (the working memory then sits behind the checkpoints). */
     void *work;
+    /* Sequences cut into chunks (the time-parallel form, see kla_b200_chunk_fold): with chunks > 1 every sequence is
+     * scanned as that many pieces of chunk_len steps, the last one shorter when they do not divide L, each from a start
+     * state of its own. lam0, eta0, lam_fin, eta_fin then hold [B*chunks, M, S] (entry b*chunks + c is chunk c of batch
+     * element b) and ckpt is kla_b200_ckpt_bytes(B*chunks, chunk_len, M, S) bytes. 0 or 1: sequences are whole. */
+    int64_t chunks, chunk_len;
 } kla_b200_fwd_args;
 
 /* Bytes of the scratch the forward writes for the backward: the filter state
@@ -183,6 +188,7 @@ typedef struct kla_b200_bwd_args {
     /* as in kla_b200_fwd_args; dlambda_v then receives the gradient with respect to the log-variances */
     int32_t lambda_v_is_log_variance;
     float obs_var_min, obs_var_max;
+    int64_t chunks, chunk_len; /* as in kla_b200_fwd_args; dlam_fin, deta_fin, dlam0, deta0 are then per entry too */
 } kla_b200_bwd_args;
 
 int kla_b200_scan_bwd(const kla_b200_bwd_args *args, void *stream);
@@ -214,6 +220,7 @@ typedef struct kla_b200_slab_args {
     const float *lam0, *eta0;           /* adjoint only; both NULL = unit prior */
     kla_b200_tensor3 dy, dy_var;        /* adjoint only; dy_var.ptr may be NULL */
     float *out;                         /* [B, M, S, 8] float32 */
+    int64_t chunks, chunk_len;          /* as in kla_b200_fwd_args: lam0, eta0 and out are then per entry */
 } kla_b200_slab_args;
 
 int kla_b200_slab_aggregate(const kla_b200_slab_args *args, void *stream);
@@ -254,9 +261,9 @@ int kla_b200_epilogue_bwd(const kla_b200_epilogue_bwd_args *args, void *stream);
  * is the carry pass of the same idea at chunk granularity.
  *
  * A [B, L, ...] problem whose (b, m) grid is too small to fill the GPU is cut
- * into C chunks of L/C steps that are scanned as B*C batch entries (entry
- * b*C + c is chunk c of batch element b; for tensors whose batch stride is
- * L times their time stride this is the same memory with other strides):
+ * into C chunks that are scanned as B*C batch entries (the chunks and chunk_len
+ * fields of the three argument structures; entry b*C + c is chunk c of batch
+ * element b):
  *   1. kla_b200_slab_aggregate (adjoint = 0) over the B*C entries;
  *   2. kla_b200_chunk_fold (adjoint = 0): the state before each chunk,
  *      lam_in / eta_in [B*C, M, S], from the aggregates and the initial state;

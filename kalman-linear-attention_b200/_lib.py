@@ -111,7 +111,7 @@ class FwdArgs(Structure):
         ("lambda_v_is_log_variance", c_int32), ("obs_var_min", c_float), ("obs_var_max", c_float),
         ("z", Tensor3), ("gate", Tensor3), ("lambda_skip", c_void_p),
         ("lambda_skip_len", c_int32), ("gate_activation", c_int32),
-        ("y_raw", Tensor3), ("y_var_raw", Tensor3), ("work", c_void_p),
+        ("y_raw", Tensor3), ("y_var_raw", Tensor3), ("work", c_void_p), ("chunks", c_int64), ("chunk_len", c_int64),
     ]
 
 
@@ -138,6 +138,7 @@ class BwdArgs(Structure):
         ("dk", c_void_p), ("dq", c_void_p), ("da", c_void_p), ("dp", c_void_p),
         ("dlam0", c_void_p), ("deta0", c_void_p),
         ("lambda_v_is_log_variance", c_int32), ("obs_var_min", c_float), ("obs_var_max", c_float),
+        ("chunks", c_int64), ("chunk_len", c_int64),
     ]
 
 
@@ -147,7 +148,7 @@ class SlabArgs(Structure):
         ("in_dtype", c_int32), ("out_dtype", c_int32), ("decode_from_prior", c_int32), ("adjoint", c_int32),
         ("v", Tensor3), ("lambda_v", Tensor3), ("k", Tensor3), ("q", Tensor3),
         ("a", c_void_p), ("p", c_void_p), ("lam0", c_void_p), ("eta0", c_void_p),
-        ("dy", Tensor3), ("dy_var", Tensor3), ("out", c_void_p),
+        ("dy", Tensor3), ("dy_var", Tensor3), ("out", c_void_p), ("chunks", c_int64), ("chunk_len", c_int64),
     ]
 
 
@@ -233,6 +234,31 @@ def load() -> ctypes.CDLL:
     lib.kla_b200_test_hooks.argtypes = [c_int64, c_int32]
     _lib = lib
     return lib
+
+
+_host = None
+_HOST_ENTRIES = (
+    "scan_fwd", "scan_bwd", "slab_aggregate", "chunk_fold", "epilogue_bwd", "step", "conv_step", "step_layer",
+    "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
+    "ckpt_bytes", "segment_scratch_bytes", "strerror",
+)
+
+
+def host():
+    """The extension module of ``csrc/kla_host.cpp``, bound to the loaded library's entry points."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            from . import _kla_host
+        except ImportError as e:
+            raise LibraryMissing(
+                f"the extension module _kla_host is not built or does not fit this torch ({e}). Build it with "
+                "`python kalman-linear-attention_b200/build.py`."
+            ) from e
+        _kla_host.bind({"kla_b200_" + n: ctypes.cast(getattr(lib, "kla_b200_" + n), c_void_p).value for n in _HOST_ENTRIES})
+        _host = _kla_host
+    return _host
 
 
 def device_status() -> int:

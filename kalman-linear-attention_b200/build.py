@@ -10,7 +10,9 @@ channel, prior read-out) combination, a few hundred kernels in all, so the
 instantiations are cut into slices (``csrc/kla_scan_inst.cu`` compiled with
 different ``-DKLA_INST_*``) that compile in parallel; ``csrc/kla_capi.cu`` holds
 the entry points and the small kernels. Objects are kept under ``build/`` and
-only recompiled when a file they include has changed.
+only recompiled when a file they include has changed. ``csrc/kla_host.cpp``, the
+native half of the Python wrappers, becomes the extension module ``_kla_host.so``
+beside the library, compiled by g++ against the installed torch.
 """
 
 from __future__ import annotations
@@ -26,6 +28,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libkla_b200.so")
+HOST = os.path.join(HERE, "_kla_host.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -69,7 +72,27 @@ def _newer(target: str, deps) -> bool:
 
 
 def is_stale() -> bool:
-    return _newer(LIB, _sources() + [os.path.abspath(__file__)])
+    return _newer(LIB, _sources() + [os.path.abspath(__file__)]) or _newer(HOST, _host_deps())
+
+
+def _host_deps():
+    return [os.path.join(CSRC, "kla_host.cpp"), os.path.join(INCLUDE, "kla_b200.h"), os.path.abspath(__file__)]
+
+
+def _host_cmd():
+    """The extension module that fills the C-ABI structures from torch tensors (no device code)."""
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc),
+            os.path.join(CSRC, "kla_host.cpp"), "-o", HOST, f"-L{os.path.join(root, 'lib')}",
+            "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
 
 
 def build(force: bool = False, verbose: bool = False, jobs: int | None = None) -> str:
@@ -90,6 +113,8 @@ def build(force: bool = False, verbose: bool = False, jobs: int | None = None) -
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             todo.append((name, cmd))
+    if force or _newer(HOST, _host_deps()):
+        todo.append(("host", _host_cmd()))
 
     def run(item):
         name, cmd = item
@@ -100,7 +125,7 @@ def build(force: bool = False, verbose: bool = False, jobs: int | None = None) -
     with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, jobs)) as pool:
         for name, cmd, res in pool.map(run, todo):
             if res.returncode != 0:
-                raise RuntimeError(f"nvcc failed on {name}:\n{' '.join(cmd)}\n{res.stdout}{res.stderr}")
+                raise RuntimeError(f"compiler failed on {name}:\n{' '.join(cmd)}\n{res.stdout}{res.stderr}")
             if verbose:
                 print(f"== {name}\n{res.stderr}")
     link = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC", "-o", LIB, *objs]

@@ -43,7 +43,8 @@ struct alignas(64) AggParams {
     int use_tma;
     Tensor3 v, lv, k, q, dy, dyv;      // dy, dyv, q: adjoint only
     const float *a, *p, *lam0, *eta0;  // lam0/eta0: adjoint only (nullptr = unit prior)
-    float *out;                        // [B, M, S, 8]
+    float *out;                        // [entries, M, S, 8]
+    ChunkCtl chunk;
     WaitCtl wait;
 };
 
@@ -81,8 +82,9 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
     };
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int b = blockIdx.y, m_cta = blockIdx.x * MC;
-    const int L = prm.L, M = prm.M, S = prm.S;
+    const int be = blockIdx.y, m_cta = blockIdx.x * MC;  // be: batch entry, what states and records are indexed by
+    const ChunkSpan span = chunk_span(prm.chunk, be, prm.L);
+    const int b = span.b, t_off = span.t_off, L = span.L, M = prm.M, S = prm.S;
     const int NT = (L + TT - 1) / TT;
     const bool has_dyv = ADJ && prm.dyv.ptr != nullptr;
 
@@ -115,8 +117,8 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
             if (ADJ) {
                 float lam = 1.0f, eta = 0.0f;
                 if (live && prm.lam0 != nullptr) {
-                    lam = prm.lam0[((long long)b * M + m) * S + s];
-                    eta = prm.eta0[((long long)b * M + m) * S + s];
+                    lam = prm.lam0[((long long)be * M + m) * S + s];
+                    eta = prm.eta0[((long long)be * M + m) * S + s];
                 }
                 const float P0 = 1.0f / fmaxf(lam, kLamMin);
                 pair_el(A[0], i) = 1.0f; pair_el(A[1], i) = 0.0f; pair_el(A[2], i) = 1.0f;
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
         for (int i = 0; i < SPT; ++i) {
             const int s = i * LPC + j;
             if (m < M && s < S) {
-                float4 *o = reinterpret_cast<float4 *>(prm.out + (((long long)b * M + m) * S + s) * 8);
+                float4 *o = reinterpret_cast<float4 *>(prm.out + (((long long)be * M + m) * S + s) * 8);
                 o[0] = make_float4(pair_el(A[0], i), pair_el(A[1], i), pair_el(A[2], i), pair_el(A[3], i));
                 o[1] = make_float4(pair_el(A[4], i), pair_el(A[5], i), pair_el(A[6], i), 0.0f);
             }
@@ -231,12 +233,12 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
     } else {
         // ================================================================ loader warp
         constexpr uint32_t kBytesI = sizeof(T) * TT * MC, kBytesO = sizeof(TO) * TT * MC;
-        const T *vb = static_cast<const T *>(prm.v.ptr) + (long long)b * prm.v.sb;
-        const T *lb = static_cast<const T *>(prm.lv.ptr) + (long long)b * prm.lv.sb;
-        const T *kb = static_cast<const T *>(prm.k.ptr) + (long long)b * prm.k.sb;
-        const T *qb = ADJ ? static_cast<const T *>(prm.q.ptr) + (long long)b * prm.q.sb : nullptr;
-        const TO *dyb = ADJ ? static_cast<const TO *>(prm.dy.ptr) + (long long)b * prm.dy.sb : nullptr;
-        const TO *dyvb = has_dyv ? static_cast<const TO *>(prm.dyv.ptr) + (long long)b * prm.dyv.sb : nullptr;
+        const T *vb = static_cast<const T *>(prm.v.ptr) + (long long)b * prm.v.sb + (long long)t_off * prm.v.st;
+        const T *lb = static_cast<const T *>(prm.lv.ptr) + (long long)b * prm.lv.sb + (long long)t_off * prm.lv.st;
+        const T *kb = static_cast<const T *>(prm.k.ptr) + (long long)b * prm.k.sb + (long long)t_off * prm.k.st;
+        const T *qb = ADJ ? static_cast<const T *>(prm.q.ptr) + (long long)b * prm.q.sb + (long long)t_off * prm.q.st : nullptr;
+        const TO *dyb = ADJ ? static_cast<const TO *>(prm.dy.ptr) + (long long)b * prm.dy.sb + (long long)t_off * prm.dy.st : nullptr;
+        const TO *dyvb = has_dyv ? static_cast<const TO *>(prm.dyv.ptr) + (long long)b * prm.dyv.sb + (long long)t_off * prm.dyv.st : nullptr;
         if (ADJ && !has_dyv) {  // dyvar absent: its stage buffers stay zero for the whole kernel
             for (int s = 0; s < NS; ++s)
                 for (int idx = lane; idx < TT * MC; idx += 32) dyvstage(s)[idx] = from_f32<TO>(0.0f);
@@ -262,11 +264,11 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
             if (prm.use_tma) {
                 if (lane == 0) {
                     mbar_arrive_expect_tx(&full_in[s], 2 * kBytesI + (ADJ ? (has_dyv ? 2 : 1) * kBytesO : 0));
-                    tma_load_3d(vstage(s), &prm.tm_v, m_cta, t0, b, &full_in[s]);
-                    tma_load_3d(lstage(s), &prm.tm_lv, m_cta, t0, b, &full_in[s]);
+                    tma_load_3d(vstage(s), &prm.tm_v, m_cta, t_off + t0, b, &full_in[s]);
+                    tma_load_3d(lstage(s), &prm.tm_lv, m_cta, t_off + t0, b, &full_in[s]);
                     if (ADJ) {
-                        tma_load_3d(dystage(s), &prm.tm_dy, m_cta, t0, b, &full_in[s]);
-                        if (has_dyv) tma_load_3d(dyvstage(s), &prm.tm_dyv, m_cta, t0, b, &full_in[s]);
+                        tma_load_3d(dystage(s), &prm.tm_dy, m_cta, t_off + t0, b, &full_in[s]);
+                        if (has_dyv) tma_load_3d(dyvstage(s), &prm.tm_dyv, m_cta, t_off + t0, b, &full_in[s]);
                     }
                 }
             } else {

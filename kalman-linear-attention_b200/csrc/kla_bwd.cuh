@@ -106,7 +106,7 @@ __device__ __forceinline__ void regs_shrink() {
 
 struct alignas(64) BwdParams {
     CUtensorMap tm_v, tm_lv, tm_dy, tm_dyv;
-    int B, L, M, S, NT;  // NT tiles of kCkptInterval steps = checkpoints per sequence
+    int B, L, M, S, NT;  // B entries; NT tiles of kCkptInterval steps = checkpoints per entry
     int use_tma;
     Tensor3 v, lv, k, q, dy, dyv, dv, dlv;
     const float *a, *p, *lam0, *eta0;
@@ -119,6 +119,7 @@ struct alignas(64) BwdParams {
     int lv_log_sigma;
     float obs_var_min, obs_var_max;
     WaitCtl wait;
+    ChunkCtl chunk;
     SegCtl seg;  // hand: five planes [B, M, S]: the two carries and the running sums for da, da2, dp
 };
 
@@ -214,12 +215,14 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
         unit = seg_assign(prm.seg, true);
         if (unit.seg < 0) return;
     }
-    const int b = unit.b;
+    const int be = unit.b;  // batch entry: what states and checkpoints are indexed by
     const int m_cta = unit.bx * MC;
     const int M = prm.M, S = prm.S;
-    const int t_off = SEG ? unit.seg * prm.seg.seg_len : 0, tile_off = t_off / TT;
-    const int L = SEG ? min(prm.seg.seg_len, prm.L - t_off) : prm.L;
-    const int NT = SEG ? (L + TT - 1) / TT : prm.NT;
+    const ChunkSpan span = chunk_span(prm.chunk, be, prm.L);
+    const int b = span.b;
+    const int t_off = SEG ? unit.seg * prm.seg.seg_len : span.t_off, tile_off = SEG ? t_off / TT : 0;
+    const int L = SEG ? min(prm.seg.seg_len, prm.L - t_off) : span.L;
+    const int NT = (L + TT - 1) / TT;
     const bool first_seg = !SEG || unit.seg == 0, last_seg = !SEG || unit.seg == prm.seg.nseg - 1;
     const bool has_dyv = prm.dyv.ptr != nullptr;
 
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
             // checkpoint of the tile about to be replayed, fetched one tile ahead: (P, mean) per chain
             float2 ck[SPT][2];
             auto load_ck = [&](int tile) {
-                const float2 *src = prm.ckpt + (((long long)b * prm.NT + tile_off + tile) * M + m0) * S + j;
+                const float2 *src = prm.ckpt + (((long long)be * prm.NT + tile_off + tile) * M + m0) * S + j;
 #pragma unroll
                 for (int i = 0; i < SPT; ++i)
 #pragma unroll
@@ -391,7 +394,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                         for (int ci = 0; ci < 2; ++ci) {
                             const int m = m0 + ci, st = i * LPC + j;
                             if (m >= M || st >= S) continue;
-                            const long long bms = ((long long)b * M + m) * S + st;
+                            const long long bms = ((long long)be * M + m) * S + st;
                             auto at = [&](float2 &x) -> float & { return ci ? x.y : x.x; };
                             if (!last_seg) {
                                 const float *h = prm.seg.hand + bms;
@@ -527,7 +530,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                         const int m = m0 + ci, st = i * LPC + j;
                         if (m >= M || st >= S) continue;
                         auto at = [&](const float2 &x) { return ci ? x.y : x.x; };
-                        float *h = prm.seg.hand + ((long long)b * M + m) * S + st;
+                        float *h = prm.seg.hand + ((long long)be * M + m) * S + st;
                         __stcg(h, at(ncP[i]));
                         __stcg(h + plane, at(cm[i]));
                         __stcg(h + 2 * plane, at(naccA[i]));
@@ -547,7 +550,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                         const int m = m0 + ci, st = i * LPC + j;
                         if (m >= M || st >= S) continue;
                         auto at = [&](const float2 &x) { return ci ? x.y : x.x; };
-                        const long long ms = (long long)m * S + st, bms = ((long long)b * M + m) * S + st;
+                        const long long ms = (long long)m * S + st, bms = ((long long)be * M + m) * S + st;
                         const float a = at(ca[i]);
                         const float da2_da = (a * a >= kEps) ? 2.0f * a : 0.0f;  // clamp_min subgradient
                         atomicAdd(prm.da + ms, -fmaf(at(naccA2[i]), da2_da, at(naccA[i])));

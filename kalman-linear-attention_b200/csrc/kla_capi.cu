@@ -105,6 +105,51 @@ bool pair_ok(const kla_b200_tensor3 &t, size_t esz) {
     return (reinterpret_cast<uintptr_t>(t.ptr) % (2 * esz)) == 0 && t.stride_b % 2 == 0 && t.stride_t % 2 == 0;
 }
 
+// A sequence of L steps cut into `chunks` pieces of chunk_len steps (the last one may be shorter); chunks <= 1: whole.
+int check_chunks(int64_t B, int64_t L, int64_t chunks, int64_t chunk_len, ChunkCtl *cc) {
+    *cc = ChunkCtl{1, (int)L};
+    if (chunks <= 1) return chunks < 0 ? KLA_B200_EINVAL : KLA_B200_OK;
+    if (chunk_len <= 0 || chunk_len > L || chunks > L || (chunks - 1) * chunk_len >= L || chunks * chunk_len < L) return KLA_B200_EINVAL;
+    if (B * chunks > 65535) return KLA_B200_EUNSUPPORTED;
+    *cc = ChunkCtl{(int)chunks, (int)chunk_len};
+    return KLA_B200_OK;
+}
+
+// One launch that clears up to five stretches of words, in place of as many memory-set operations.
+constexpr int kZeroRanges = 5;
+struct ZeroParams {
+    int *ptr[kZeroRanges];
+    unsigned long long end[kZeroRanges];  // running totals of the stretches' words
+};
+__global__ void __launch_bounds__(256) kla_zero_kernel(const __grid_constant__ ZeroParams prm) {
+    const unsigned long long n = prm.end[kZeroRanges - 1];
+    for (unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (unsigned long long)gridDim.x * 256) {
+        unsigned long long from = 0;
+#pragma unroll
+        for (int r = 0; r < kZeroRanges; ++r) {
+            if (i >= from && i < prm.end[r]) prm.ptr[r][i - from] = 0;
+            from = prm.end[r];
+        }
+    }
+}
+struct ZeroList {
+    ZeroParams prm{};
+    int n = 0;
+    void add(void *p, size_t words) {
+        if (words == 0) return;
+        prm.ptr[n] = static_cast<int *>(p);
+        prm.end[n] = (n ? prm.end[n - 1] : 0) + words;
+        ++n;
+    }
+    cudaError_t run(cudaStream_t st) {
+        if (n == 0) return cudaSuccess;
+        for (int r = n; r < kZeroRanges; ++r) { prm.end[r] = prm.end[n - 1]; prm.ptr[r] = prm.ptr[0]; }
+        const unsigned long long blocks = (prm.end[kZeroRanges - 1] + 1023) / 1024;
+        kla_zero_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), 256, 0, st>>>(prm);
+        return cudaGetLastError();
+    }
+};
+
 int check_t3(const kla_b200_tensor3 &t, size_t esz, bool required) {
     if (t.ptr == nullptr) return required ? KLA_B200_EINVAL : KLA_B200_OK;
     if (!aligned(t.ptr, esz)) return KLA_B200_EALIGN;
@@ -214,13 +259,13 @@ int plan_segments(int64_t ctas, int64_t L, bool backward, int *seg_len) {
     return plan_segments_for(ctas, L, backward, sms, forced, seg_len);
 }
 
-// Fill prm.seg for one direction and clear its ticket and done words. The working memory is the bytes behind the
+// Fill prm.seg for one direction; its ticket and done words go on the list of what to clear before the launch. The working memory is the bytes behind the
 // checkpoints, or, for a forward without checkpoints, the caller's `work` buffer of the same layout.
 template <typename Params>
 int seg_setup(Params &prm, void *ckpt, void *work, int64_t B, int64_t L, int64_t M, int64_t S, int mc, bool backward,
-              cudaStream_t st) {
+              ZeroList &zero) {
     prm.seg = SegCtl{1, (int)L, nullptr, nullptr, nullptr};
-    if ((ckpt == nullptr && work == nullptr) || L <= 0) return KLA_B200_OK;
+    if ((ckpt == nullptr && work == nullptr) || L <= 0 || prm.chunk.n > 1) return KLA_B200_OK;
     const int64_t ctas = ((M + mc - 1) / mc) * B;
     int seg_len = (int)L;
     const int nseg = plan_segments(ctas, L, backward, &seg_len);
@@ -231,8 +276,7 @@ int seg_setup(Params &prm, void *ckpt, void *work, int64_t B, int64_t L, int64_t
     if (base == SIZE_MAX) return KLA_B200_OK;
     unsigned char *p = static_cast<unsigned char *>(ckpt != nullptr ? ckpt : work) + base;
     unsigned char *flags = p + (backward ? sc.flags : 0);
-    const cudaError_t e = cudaMemsetAsync(flags, 0, sc.flags, st);
-    if (e != cudaSuccess) return cuda_fail(e);
+    zero.add(flags, sc.flags / sizeof(int));
     prm.seg.nseg = nseg;
     prm.seg.seg_len = seg_len;
     prm.seg.ticket = reinterpret_cast<int *>(flags);
@@ -245,7 +289,9 @@ int seg_setup(Params &prm, void *ckpt, void *work, int64_t B, int64_t L, int64_t
 template <typename T, typename TO, int LPC, bool PRIOR>
 int prep_fwd(FwdParams &prm, const kla_b200_fwd_args &a, cudaStream_t st) {
     const int mc = scan_channels_per_cta(LPC);
-    if (int rc = seg_setup(prm, a.ckpt, a.work, a.B, a.L, a.M, a.S, mc, false, st)) return rc;
+    ZeroList zero;
+    if (int rc = seg_setup(prm, a.ckpt, a.work, a.B, a.L, a.M, a.S, mc, false, zero)) return rc;
+    if (const cudaError_t e = zero.run(st); e != cudaSuccess) return cuda_fail(e);
     prm.use_tma = !g_no_tma && make_tile_map<T>(&prm.tm_v, a.v, a.B, a.L, a.M, mc, kTT) &&
                   make_tile_map<T>(&prm.tm_lv, a.lambda_v, a.B, a.L, a.M, mc, kTT);
     if (prm.epilogue)  // z and gate tiles travel like v and lambda_v when they meet the tensor-map rules
@@ -259,7 +305,13 @@ int prep_fwd(FwdParams &prm, const kla_b200_fwd_args &a, cudaStream_t st) {
 template <typename T, typename TO, int LPC, bool PRIOR>
 int prep_bwd(BwdParams &prm, const kla_b200_bwd_args &a, cudaStream_t st) {
     const int mc = bwd_channels_per_cta<LPC>();
-    if (int rc = seg_setup(prm, const_cast<void *>(a.ckpt), nullptr, a.B, a.L, a.M, a.S, mc, true, st)) return rc;
+    ZeroList zero;
+    zero.add(a.dk, (size_t)a.B * a.L * a.S);
+    zero.add(a.dq, (size_t)a.B * a.L * a.S);
+    zero.add(a.da, (size_t)a.M * a.S);
+    zero.add(a.dp, (size_t)a.M * a.S);
+    if (int rc = seg_setup(prm, const_cast<void *>(a.ckpt), nullptr, a.B, a.L, a.M, a.S, mc, true, zero)) return rc;
+    if (const cudaError_t e = zero.run(st); e != cudaSuccess) return cuda_fail(e);
     prm.use_tma = !g_no_tma && make_tile_map<T>(&prm.tm_v, a.v, a.B, a.L, a.M, mc, kBwdTT) &&
                   make_tile_map<T>(&prm.tm_lv, a.lambda_v, a.B, a.L, a.M, mc, kBwdTT) &&
                   make_tile_map<TO>(&prm.tm_dy, a.dy, a.B, a.L, a.M, mc, kBwdTT) &&
@@ -438,9 +490,9 @@ int kla_b200_scan_fwd(const kla_b200_fwd_args *a, void *stream) {
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     FwdParams prm{};
-    prm.B = (int)a->B; prm.L = (int)a->L; prm.M = (int)a->M; prm.S = (int)a->S;
-    prm.NT = (int)((a->L + kTT - 1) / kTT);
-    prm.NC = (int)((a->L + kCkptInterval - 1) / kCkptInterval);
+    if ((rc = check_chunks(a->B, a->L, a->chunks, a->chunk_len, &prm.chunk))) return rc;
+    prm.B = (int)a->B * prm.chunk.n; prm.L = (int)a->L; prm.M = (int)a->M; prm.S = (int)a->S;
+    prm.NC = (int)((prm.chunk.len + kCkptInterval - 1) / kCkptInterval);
     prm.v = t3(a->v); prm.lv = t3(a->lambda_v); prm.k = t3(a->k); prm.q = t3(a->q);
     prm.y = t3(a->y); prm.yv = t3(a->y_var);
     prm.a = a->a; prm.p = a->p; prm.lam0 = a->lam0; prm.eta0 = a->eta0;
@@ -488,13 +540,13 @@ int kla_b200_scan_bwd(const kla_b200_bwd_args *a, void *stream) {
     if ((a->lam0 == nullptr) != (a->eta0 == nullptr)) return KLA_B200_EINVAL;
     if ((a->dlam_fin == nullptr) != (a->deta_fin == nullptr)) return KLA_B200_EINVAL;
     cudaError_t e;
-    if (n_bls) {
-        if ((e = cudaMemsetAsync(a->dk, 0, n_bls * 4, st)) != cudaSuccess) return cuda_fail(e);
-        if ((e = cudaMemsetAsync(a->dq, 0, n_bls * 4, st)) != cudaSuccess) return cuda_fail(e);
-    }
-    if (n_ms) {
-        if ((e = cudaMemsetAsync(a->da, 0, n_ms * 4, st)) != cudaSuccess) return cuda_fail(e);
-        if ((e = cudaMemsetAsync(a->dp, 0, n_ms * 4, st)) != cudaSuccess) return cuda_fail(e);
+    if (n_bms == 0 || a->L == 0) {  // no kernel below: the sums are empty
+        ZeroList zero;
+        zero.add(a->dk, n_bls);
+        zero.add(a->dq, n_bls);
+        zero.add(a->da, n_ms);
+        zero.add(a->dp, n_ms);
+        if ((e = zero.run(st)) != cudaSuccess) return cuda_fail(e);
     }
     if (n_bms == 0) return KLA_B200_OK;
     if (a->L == 0) {  // nothing to scan: the state gradient passes straight through
@@ -515,8 +567,9 @@ int kla_b200_scan_bwd(const kla_b200_bwd_args *a, void *stream) {
     if ((rc = check_t3(a->dy_var, osz, false))) return rc;
 
     BwdParams prm{};
-    prm.B = (int)a->B; prm.L = (int)a->L; prm.M = (int)a->M; prm.S = (int)a->S;
-    prm.NT = (int)((a->L + kBwdTT - 1) / kBwdTT);
+    if ((rc = check_chunks(a->B, a->L, a->chunks, a->chunk_len, &prm.chunk))) return rc;
+    prm.B = (int)a->B * prm.chunk.n; prm.L = (int)a->L; prm.M = (int)a->M; prm.S = (int)a->S;
+    prm.NT = (int)((prm.chunk.len + kBwdTT - 1) / kBwdTT);
     prm.v = t3(a->v); prm.lv = t3(a->lambda_v); prm.k = t3(a->k); prm.q = t3(a->q);
     prm.dy = t3(a->dy); prm.dyv = t3(a->dy_var); prm.dv = t3(a->dv); prm.dlv = t3(a->dlambda_v);
     prm.a = a->a; prm.p = a->p; prm.lam0 = a->lam0; prm.eta0 = a->eta0;
@@ -549,7 +602,8 @@ int kla_b200_slab_aggregate(const kla_b200_slab_args *a, void *stream) {
             return rc;
     }
     AggParams prm{};
-    prm.B = (int)a->B; prm.L = (int)a->L; prm.M = (int)a->M; prm.S = (int)a->S;
+    if ((rc = check_chunks(a->B, a->L, a->chunks, a->chunk_len, &prm.chunk))) return rc;
+    prm.B = (int)a->B * prm.chunk.n; prm.L = (int)a->L; prm.M = (int)a->M; prm.S = (int)a->S;
     prm.v = t3(a->v); prm.lv = t3(a->lambda_v); prm.k = t3(a->k); prm.q = t3(a->q);
     prm.dy = t3(a->dy); prm.dyv = t3(a->dy_var);
     prm.a = a->a; prm.p = a->p; prm.lam0 = a->lam0; prm.eta0 = a->eta0; prm.out = a->out;

@@ -70,6 +70,21 @@ struct SegCtl {
     float *hand;  // carried state between segments, planes of [B, M, S] floats
 };
 
+// A sequence cut into `n` chunks of `len` steps (the last may be shorter) that run side by side as n batch entries from
+// start states of their own: entry e is chunk e % n of batch element e / n. States, their gradients and checkpoints are
+// indexed by entry, activations by (batch element, time). n = 1: entries are batch elements.
+struct ChunkCtl {
+    int n, len;
+};
+struct ChunkSpan {
+    int b, t_off, L;  // batch element, first step, steps
+};
+__device__ __forceinline__ ChunkSpan chunk_span(const ChunkCtl &cc, int entry, int L) {
+    if (cc.n <= 1) return ChunkSpan{entry, 0, L};
+    const int b = entry / cc.n, t_off = (entry - b * cc.n) * cc.len;
+    return ChunkSpan{b, t_off, min(cc.len, L - t_off)};
+}
+
 // What a CTA works on: its channel block, batch element and segment.
 struct SegUnit {
     int bx, b, seg, seq;

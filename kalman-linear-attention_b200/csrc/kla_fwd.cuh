@@ -41,13 +41,13 @@ constexpr int kFwdUnroll = KLA_FWD_UNROLL;  // steps unrolled per trip of the ti
 
 struct alignas(64) FwdParams {
     CUtensorMap tm_v, tm_lv;  // rank-3 (M, L, B) maps with box (MC, TT, 1); valid when use_tma
-    int B, L, M, S, NT;  // NT tiles of TT steps
-    int NC;              // checkpoints per sequence: one per kCkptInterval steps
+    int B, L, M, S;  // B entries (ChunkCtl) of up to L steps
+    int NC;          // checkpoints per entry: one per kCkptInterval steps
     int use_tma;
     Tensor3 v, lv, k, q, y, yv;
     const float *a, *p, *lam0, *eta0;
     float *lam_fin, *eta_fin;
-    float2 *ckpt;  // [B, NC, M, S] (P, mean) before every kCkptInterval-th step, or nullptr
+    float2 *ckpt;  // [entries, NC, M, S] (P, mean) before every kCkptInterval-th step, or nullptr
     int vec_y, vec_yv;
     // lv holds the sensor projection's raw log-variance output instead of the precision:
     // Lambda_v = 1 / min(softplus(lv) + obs_var_min, obs_var_max) is formed in shared memory by the compute warps,
@@ -65,6 +65,7 @@ struct alignas(64) FwdParams {
     int skip_len, gate_act, epilogue, epi_tma;
     WaitCtl wait;
     SegCtl seg;  // hand: one plane pair (P, mean) as float2 [B, M, S]
+    ChunkCtl chunk;
     alignas(64) CUtensorMap tm_z, tm_gate;  // maps of the epilogue operands, like tm_v; valid when epi_tma
 };
 
@@ -139,12 +140,14 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
         unit = seg_assign(prm.seg, false);
         if (unit.seg < 0) return;
     }
-    const int b = unit.b;
+    const int be = unit.b;  // batch entry: what states and checkpoints are indexed by
     const int m_cta = unit.bx * MC;
     const int M = prm.M, S = prm.S;
-    const int t_off = SEG ? unit.seg * prm.seg.seg_len : 0;
-    const int L = SEG ? min(prm.seg.seg_len, prm.L - t_off) : prm.L;
-    const int NT = SEG ? (L + TT - 1) / TT : prm.NT;
+    const ChunkSpan span = chunk_span(prm.chunk, be, prm.L);
+    const int b = span.b;
+    const int t_off = SEG ? unit.seg * prm.seg.seg_len : span.t_off;
+    const int L = SEG ? min(prm.seg.seg_len, prm.L - t_off) : span.L;
+    const int NT = (L + TT - 1) / TT;
     const bool first_seg = !SEG || unit.seg == 0, last_seg = !SEG || unit.seg == prm.seg.nseg - 1;
 
     if (tid == 0) {
@@ -190,8 +193,8 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
                 pair_el(cp[ci], i) = fmaxf(pv, kPMin);
                 float lam = 1.0f, eta = 0.0f;
                 if (live && prm.lam0 != nullptr) {
-                    lam = prm.lam0[((long long)b * M + m) * S + s];
-                    eta = prm.eta0[((long long)b * M + m) * S + s];
+                    lam = prm.lam0[((long long)be * M + m) * S + s];
+                    eta = prm.eta0[((long long)be * M + m) * S + s];
                 }
                 const float P0 = 1.0f / fmaxf(lam, kLamMin);
                 pair_el(P[ci], i) = P0;
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
                 for (int i = 0; i < SPT; ++i) {
                     const int s = i * LPC + j;
                     if (carried && m < M && s < S) {
-                        const float2 h = __ldcg(hand + ((long long)b * M + m) * S + s);
+                        const float2 h = __ldcg(hand + ((long long)be * M + m) * S + s);
                         pair_el(P[ci], i) = h.x;
                         pair_el(mean[ci], i) = h.y;
                     }
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
         }
         // checkpoint pointer of chain (ci = 0, i = 0); advanced by one tile per tile
         float2 *ck = prm.ckpt;
-        if (ck != nullptr) ck += (((long long)b * prm.NC + t_off / kCkptInterval) * M + (m_cta + cw)) * S + j;
+        if (ck != nullptr) ck += (((long long)be * prm.NC + (SEG ? t_off / kCkptInterval : 0)) * M + (m_cta + cw)) * S + j;
         const long long ck_tile = (long long)M * S;
         auto store_ckpt = [&]() {  // the state before the step about to be taken; advances to the next checkpoint
 #pragma unroll
@@ -395,10 +398,10 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
                 if (m < M && s < S) {
                     if (last_seg) {
                         const float lam = 1.0f / pair_el(P[ci], i);
-                        prm.lam_fin[((long long)b * M + m) * S + s] = lam;
-                        prm.eta_fin[((long long)b * M + m) * S + s] = pair_el(mean[ci], i) * lam;
+                        prm.lam_fin[((long long)be * M + m) * S + s] = lam;
+                        prm.eta_fin[((long long)be * M + m) * S + s] = pair_el(mean[ci], i) * lam;
                     } else {
-                        __stcg(hand + ((long long)b * M + m) * S + s, make_float2(pair_el(P[ci], i), pair_el(mean[ci], i)));
+                        __stcg(hand + ((long long)be * M + m) * S + s, make_float2(pair_el(P[ci], i), pair_el(mean[ci], i)));
                     }
                 }
             }

@@ -1,0 +1,451 @@
+// Native half of the Python wrappers: argument structures, output allocations and launches of the C-ABI library
+// (include/kla_b200.h) on torch tensors, one Python call per operation. Filling the structures through ctypes and
+// allocating from Python cost 25-40 us per launch, more than most of these kernels run: a decode step of 2.5 us of GPU
+// time took 30 us, a small training step of 220 us took 500 us.
+//
+// The module holds no state but the library's entry points, which bind() receives as addresses, so that it uses the very
+// library the Python side loaded. Every function here takes tensors the wrappers have found canonical (same device, dtypes
+// and unit last strides checked); canonical() and step() do that check themselves and answer "not this route" otherwise,
+// which sends the wrapper to its general path with its error messages.
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/core/GradMode.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <optional>
+#include <string>
+#include <tuple>
+#include <vector>
+
+#include "../../include/kla_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+struct Entry {
+    int (*scan_fwd)(const kla_b200_fwd_args *, void *) = nullptr;
+    int (*scan_bwd)(const kla_b200_bwd_args *, void *) = nullptr;
+    int (*slab_aggregate)(const kla_b200_slab_args *, void *) = nullptr;
+    int (*chunk_fold)(const kla_b200_chunk_fold_args *, void *) = nullptr;
+    int (*epilogue_bwd)(const kla_b200_epilogue_bwd_args *, void *) = nullptr;
+    int (*step)(const kla_b200_step_args *, void *) = nullptr;
+    int (*conv_step)(const kla_b200_conv_step_args *, void *) = nullptr;
+    int (*step_layer)(const kla_b200_step_layer_args *, void *) = nullptr;
+    int (*conv_seq)(const kla_b200_conv_seq_args *, void *) = nullptr;
+    int (*conv_seq_bwd)(const kla_b200_conv_seq_bwd_args *, void *) = nullptr;
+    int (*rawscan[4])(const kla_b200_rawscan_args *, void *) = {};  // Moebius forward, backward, affine forward, backward
+    size_t (*ckpt_bytes)(int64_t, int64_t, int64_t, int64_t) = nullptr;
+    size_t (*segment_scratch_bytes)(int64_t, int64_t, int64_t) = nullptr;
+    const char *(*strerror)(int) = nullptr;
+} lib;
+
+template <typename F>
+void take(F &f, const py::dict &d, const char *name) {
+    f = reinterpret_cast<F>(d[name].cast<uintptr_t>());
+}
+
+void bind(const py::dict &d) {
+    take(lib.scan_fwd, d, "kla_b200_scan_fwd");
+    take(lib.scan_bwd, d, "kla_b200_scan_bwd");
+    take(lib.slab_aggregate, d, "kla_b200_slab_aggregate");
+    take(lib.chunk_fold, d, "kla_b200_chunk_fold");
+    take(lib.epilogue_bwd, d, "kla_b200_epilogue_bwd");
+    take(lib.step, d, "kla_b200_step");
+    take(lib.conv_step, d, "kla_b200_conv_step");
+    take(lib.step_layer, d, "kla_b200_step_layer");
+    take(lib.conv_seq, d, "kla_b200_conv_seq");
+    take(lib.conv_seq_bwd, d, "kla_b200_conv_seq_bwd");
+    take(lib.rawscan[0], d, "kla_b200_mobius_scan_fwd");
+    take(lib.rawscan[1], d, "kla_b200_mobius_scan_bwd");
+    take(lib.rawscan[2], d, "kla_b200_affine_scan_fwd");
+    take(lib.rawscan[3], d, "kla_b200_affine_scan_bwd");
+    take(lib.ckpt_bytes, d, "kla_b200_ckpt_bytes");
+    take(lib.segment_scratch_bytes, d, "kla_b200_segment_scratch_bytes");
+    take(lib.strerror, d, "kla_b200_strerror");
+}
+
+// The C-ABI status as the exception the Python side's _lib.check raises for it.
+void check(int rc) {
+    if (rc == KLA_B200_OK) return;
+    const std::string msg = lib.strerror(rc);
+    if (rc == KLA_B200_EUNSUPPORTED) {
+        PyErr_SetString(PyExc_NotImplementedError, ("The b200 KLA backend: " + msg + ". Use backend='torch' for this case.").c_str());
+        throw py::error_already_set();
+    }
+    if (rc == KLA_B200_EINVAL || rc == KLA_B200_EALIGN || rc == KLA_B200_ETOOBIG) throw py::value_error("kla_b200: " + msg);
+    throw std::runtime_error("kla_b200: " + msg);
+}
+
+kla_b200_tensor3 t3(const Tensor &t) { return kla_b200_tensor3{t.data_ptr(), t.stride(0), t.stride(1)}; }
+kla_b200_tensor3 t3(const OptTensor &t) { return t ? t3(*t) : kla_b200_tensor3{nullptr, 0, 0}; }
+float *fp(const Tensor &t) { return static_cast<float *>(t.data_ptr()); }
+float *fp(const OptTensor &t) { return t ? fp(*t) : nullptr; }
+int32_t dt(at::ScalarType t) { return t == at::kBFloat16 ? KLA_B200_BF16 : KLA_B200_F32; }
+at::ScalarType out_type(bool bf16) { return bf16 ? at::kBFloat16 : at::kFloat; }
+void *stream_of(const Tensor &t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+Tensor f32(const Tensor &like, at::IntArrayRef sizes) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
+
+struct Sensors {
+    bool on = false;
+    float vmin = 0.0f, vmax = 0.0f;
+    explicit Sensors(const std::optional<std::tuple<double, std::optional<double>>> &s) {
+        if (!s) return;
+        on = true;
+        vmin = (float)std::get<0>(*s);
+        vmax = (float)std::get<1>(*s).value_or(0.0);
+    }
+};
+using SensorArg = std::optional<std::tuple<double, std::optional<double>>>;
+
+bool rows_ok(const Tensor &t) { return t.size(-1) <= 1 || t.stride(-1) == 1; }
+bool sm100(const at::Device &d) { return at::cuda::getDeviceProperties(d.index())->major == 10; }
+
+// Whether the scan's arguments need no conversion, copy or error message.
+bool canonical(const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p,
+               const OptTensor &lam0, const OptTensor &eta0) {
+    if (!v.is_cuda() || v.dim() != 3 || k.dim() != 3 || a.dim() != 2) return false;
+    const auto T = v.scalar_type();
+    if (T != at::kFloat && T != at::kBFloat16) return false;
+    if (lv.scalar_type() != T || k.scalar_type() != T || q.scalar_type() != T) return false;
+    if (a.scalar_type() != at::kFloat || p.scalar_type() != at::kFloat || !a.is_contiguous() || !p.is_contiguous()) return false;
+    const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2);
+    if (S > KLA_B200_MAX_DSTATE || lv.sizes() != v.sizes() || q.sizes() != k.sizes() || k.size(0) != B || k.size(1) != L) return false;
+    if (a.size(0) != M || a.size(1) != S || p.sizes() != a.sizes()) return false;
+    const auto dev = v.device();
+    if (lv.device() != dev || k.device() != dev || q.device() != dev || a.device() != dev || p.device() != dev) return false;
+    if (!rows_ok(v) || !rows_ok(lv) || !rows_ok(k) || !rows_ok(q)) return false;
+    if (lam0.has_value() != eta0.has_value()) return false;
+    if (lam0) {
+        for (const Tensor *t : {&*lam0, &*eta0})
+            if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->device() != dev || t->dim() != 3 || t->size(0) != B ||
+                t->size(1) != M || t->size(2) != S)
+                return false;
+    }
+    return sm100(dev);
+}
+
+// ------------------------------------------------------------------------------------------------------ the scan
+
+// kla_b200_scan_fwd. segments: give the kernel working memory so that a forward without checkpoints can hand sequences
+// from CTA to CTA. chunks > 1: lam0, eta0 and the returned states are per chunk.
+std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> scan_fwd(
+    const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const OptTensor &lam0,
+    const OptTensor &eta0, bool prior, bool out_bf16, bool need_ckpt, bool segments, const SensorArg &sensors, const OptTensor &z,
+    const OptTensor &skip, const OptTensor &gate, int gate_act, const OptTensor &y_raw, const OptTensor &yv_raw, int64_t chunks,
+    int64_t chunk_len) {
+    const c10::cuda::CUDAGuard guard(v.device());
+    const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2), E = B * chunks;
+    const auto opt = v.options().dtype(out_type(out_bf16)), bytes = v.options().dtype(at::kByte);
+    Tensor y = at::empty({B, L, M}, opt), yv = at::empty({B, L, M}, opt);
+    Tensor lam = f32(v, {E, M, S}), eta = f32(v, {E, M, S});
+    OptTensor ckpt, work;
+    if (need_ckpt && L > 0) ckpt = at::empty({(int64_t)lib.ckpt_bytes(E, chunks > 1 ? chunk_len : L, M, S)}, bytes);
+    else if (segments) work = at::empty({(int64_t)lib.segment_scratch_bytes(B, M, S)}, bytes);
+    const Sensors sen(sensors);
+    kla_b200_fwd_args f{};
+    f.B = B; f.L = L; f.M = M; f.S = S;
+    f.in_dtype = dt(v.scalar_type()); f.out_dtype = dt(opt.dtype().toScalarType()); f.decode_from_prior = prior;
+    f.v = t3(v); f.lambda_v = t3(lv); f.k = t3(k); f.q = t3(q);
+    f.a = fp(a); f.p = fp(p); f.lam0 = fp(lam0); f.eta0 = fp(eta0);
+    f.y = t3(y); f.y_var = t3(yv); f.lam_fin = fp(lam); f.eta_fin = fp(eta);
+    f.ckpt = ckpt ? ckpt->data_ptr() : nullptr;
+    f.work = work ? work->data_ptr() : nullptr;
+    f.lambda_v_is_log_variance = sen.on; f.obs_var_min = sen.vmin; f.obs_var_max = sen.vmax;
+    if (skip) { f.z = t3(z); f.lambda_skip = fp(*skip); f.lambda_skip_len = (int32_t)skip->numel(); }
+    if (gate) { f.gate = t3(*gate); f.gate_activation = gate_act; }
+    f.y_raw = t3(y_raw); f.y_var_raw = t3(yv_raw);
+    if (chunks > 1) { f.chunks = chunks; f.chunk_len = chunk_len; }
+    check(lib.scan_fwd(&f, stream_of(v)));
+    return {y, yv, lam, eta, ckpt};
+}
+
+// kla_b200_scan_bwd -> dv, dlambda_v, dk, dq, da, dp, dlam0, deta0
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_bwd(
+    const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const OptTensor &lam0,
+    const OptTensor &eta0, const OptTensor &ckpt, const Tensor &dy, const OptTensor &dyv, const OptTensor &dlam_fin,
+    const OptTensor &deta_fin, bool prior, bool out_bf16, const SensorArg &sensors, int64_t chunks, int64_t chunk_len) {
+    const c10::cuda::CUDAGuard guard(v.device());
+    const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2), E = B * chunks;
+    Tensor dv = at::empty({B, L, M}, v.options()), dlv = at::empty({B, L, M}, v.options());
+    Tensor dk = f32(v, {B, L, S}), dq = f32(v, {B, L, S}), da = f32(v, {M, S}), dp = f32(v, {M, S});
+    Tensor dlam0 = f32(v, {E, M, S}), deta0 = f32(v, {E, M, S});
+    const Sensors sen(sensors);
+    kla_b200_bwd_args b{};
+    b.B = B; b.L = L; b.M = M; b.S = S;
+    b.in_dtype = dt(v.scalar_type()); b.out_dtype = out_bf16 ? KLA_B200_BF16 : KLA_B200_F32; b.decode_from_prior = prior;
+    b.v = t3(v); b.lambda_v = t3(lv); b.k = t3(k); b.q = t3(q);
+    b.a = fp(a); b.p = fp(p); b.lam0 = fp(lam0); b.eta0 = fp(eta0);
+    b.ckpt = ckpt ? ckpt->data_ptr() : nullptr;
+    b.dy = t3(dy); b.dy_var = t3(dyv); b.dlam_fin = fp(dlam_fin); b.deta_fin = fp(deta_fin);
+    b.dv = t3(dv); b.dlambda_v = t3(dlv); b.dk = fp(dk); b.dq = fp(dq); b.da = fp(da); b.dp = fp(dp);
+    b.dlam0 = fp(dlam0); b.deta0 = fp(deta0);
+    b.lambda_v_is_log_variance = sen.on; b.obs_var_min = sen.vmin; b.obs_var_max = sen.vmax;
+    if (chunks > 1) { b.chunks = chunks; b.chunk_len = chunk_len; }
+    check(lib.scan_bwd(&b, stream_of(v)));
+    return {dv, dlv, dk, dq, da, dp, dlam0, deta0};
+}
+
+// kla_b200_slab_aggregate -> [B*chunks, M, S, 8]; the adjoint aggregate when dy is given
+Tensor slab_aggregate(const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &a, const Tensor &p, const OptTensor &q,
+                      const OptTensor &dy, const OptTensor &dyv, const OptTensor &lam0, const OptTensor &eta0, bool prior,
+                      int64_t chunks, int64_t chunk_len) {
+    const c10::cuda::CUDAGuard guard(v.device());
+    const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2);
+    Tensor out = f32(v, {B * chunks, M, S, 8});
+    kla_b200_slab_args s{};
+    s.B = B; s.L = L; s.M = M; s.S = S;
+    s.in_dtype = dt(v.scalar_type()); s.out_dtype = dy ? dt(dy->scalar_type()) : KLA_B200_F32;
+    s.decode_from_prior = prior; s.adjoint = dy.has_value();
+    s.v = t3(v); s.lambda_v = t3(lv); s.k = t3(k); s.q = t3(q);
+    s.a = fp(a); s.p = fp(p); s.lam0 = fp(lam0); s.eta0 = fp(eta0);
+    s.dy = t3(dy); s.dy_var = t3(dyv); s.out = fp(out);
+    if (chunks > 1) { s.chunks = chunks; s.chunk_len = chunk_len; }
+    check(lib.slab_aggregate(&s, stream_of(v)));
+    return out;
+}
+
+// kla_b200_chunk_fold over aggregates [B*C, M, S, 8] -> two [B*C, M, S]
+std::tuple<Tensor, Tensor> chunk_fold(const Tensor &agg, int64_t C, const OptTensor &in_a, const OptTensor &in_b, bool adjoint) {
+    const c10::cuda::CUDAGuard guard(agg.device());
+    const int64_t E = agg.size(0), M = agg.size(1), S = agg.size(2);
+    Tensor out_a = f32(agg, {E, M, S}), out_b = f32(agg, {E, M, S});
+    kla_b200_chunk_fold_args c{};
+    c.B = E / C; c.C = C; c.M = M; c.S = S; c.adjoint = adjoint;
+    c.agg = fp(agg); c.in_a = fp(in_a); c.in_b = fp(in_b); c.out_a = fp(out_a); c.out_b = fp(out_b);
+    check(lib.chunk_fold(&c, stream_of(agg)));
+    return {out_a, out_b};
+}
+
+// The time-parallel forward: aggregates, fold, scan over the chunks. -> y, y_var, the sequences' final state, the
+// checkpoints and every chunk's start state (both for the backward).
+std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor, Tensor, Tensor> scan_fwd_chunked(
+    const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const OptTensor &lam0,
+    const OptTensor &eta0, bool prior, bool out_bf16, bool need_ckpt, int64_t chunks, int64_t chunk_len) {
+    const Tensor agg = slab_aggregate(v, lv, k, a, p, {}, {}, {}, {}, {}, false, chunks, chunk_len);
+    auto [lam_in, eta_in] = chunk_fold(agg, chunks, lam0, eta0, false);
+    auto [y, yv, lam, eta, ckpt] = scan_fwd(v, lv, k, q, a, p, lam_in, eta_in, prior, out_bf16, need_ckpt, false, {}, {}, {}, {}, 0, {},
+                                            {}, chunks, chunk_len);
+    const int64_t B = v.size(0), M = v.size(2), S = k.size(2);
+    auto last = [&](const Tensor &t) { return t.view({B, chunks, M, S}).select(1, chunks - 1); };
+    return {y, yv, last(lam), last(eta), ckpt, lam_in, eta_in};
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_bwd_chunked(
+    const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const Tensor &lam_in,
+    const Tensor &eta_in, const OptTensor &ckpt, const Tensor &dy, const OptTensor &dyv, const OptTensor &dlam_fin,
+    const OptTensor &deta_fin, bool prior, bool out_bf16, int64_t chunks, int64_t chunk_len) {
+    const Tensor agg = slab_aggregate(v, lv, k, a, p, q, dy, dyv, lam_in, eta_in, prior, chunks, chunk_len);
+    auto [dlam_seed, deta_seed] = chunk_fold(agg, chunks, dlam_fin, deta_fin, true);
+    auto r = scan_bwd(v, lv, k, q, a, p, lam_in, eta_in, ckpt, dy, dyv, dlam_seed, deta_seed, prior, out_bf16, {}, chunks, chunk_len);
+    const int64_t B = v.size(0), M = v.size(2), S = k.size(2);
+    auto first = [&](const Tensor &t) { return t.view({B, chunks, M, S}).select(1, 0); };
+    std::get<6>(r) = first(std::get<6>(r));
+    std::get<7>(r) = first(std::get<7>(r));
+    return r;
+}
+
+// kla_b200_epilogue_bwd -> dy, dy_var for the scan's backward, and dz, dgate, dskip of the halves that are there
+std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> epilogue_bwd(const Tensor &v, bool out_bf16, const Tensor &dout,
+                                                                        const OptTensor &dout_var, const OptTensor &y_raw,
+                                                                        const OptTensor &yv_raw, const OptTensor &z,
+                                                                        const OptTensor &gate, const OptTensor &skip, int gate_act) {
+    const c10::cuda::CUDAGuard guard(v.device());
+    const int64_t B = v.size(0), L = v.size(1), M = v.size(2);
+    const auto opt = v.options().dtype(out_type(out_bf16));
+    Tensor dy = at::empty({B, L, M}, opt), dyv = at::empty({B, L, M}, opt);
+    OptTensor dz, dgate, dskip;
+    if (z) dz = at::empty({B, L, M}, v.options());
+    if (gate) dgate = at::empty({B, L, M}, v.options());
+    if (skip) dskip = at::empty_like(*skip);
+    kla_b200_epilogue_bwd_args e{};
+    e.B = B; e.L = L; e.M = M;
+    e.in_dtype = dt(v.scalar_type()); e.out_dtype = dt(opt.dtype().toScalarType());
+    e.gate_activation = gate ? gate_act : KLA_B200_ACT_NONE;
+    e.lambda_skip_len = skip ? (int32_t)skip->numel() : 0;
+    e.dout = t3(dout); e.dout_var = t3(dout_var); e.y_raw = t3(y_raw); e.y_var_raw = t3(yv_raw);
+    e.z = t3(z); e.gate = t3(gate); e.lambda_skip = fp(skip);
+    e.dy = t3(dy); e.dy_var = t3(dyv); e.dz = t3(dz); e.dgate = t3(dgate); e.dlambda_skip = fp(dskip);
+    check(lib.epilogue_bwd(&e, stream_of(v)));
+    return {dy, dyv, dz, dgate, dskip};
+}
+
+// kla_b200_conv_seq -> z, the window after the sequence
+std::tuple<Tensor, Tensor> conv_seq(const Tensor &x, const Tensor &w, const OptTensor &bias, const Tensor &state, int act) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t B = x.size(0), L = x.size(1), D = x.size(2);
+    Tensor z = at::empty({B, L, D}, x.options()), next = at::empty_like(state);
+    kla_b200_conv_seq_args c{};
+    c.B = B; c.L = L; c.D = D; c.K = w.size(1); c.dtype = dt(x.scalar_type()); c.activation = act;
+    c.x = t3(x); c.weight = fp(w); c.bias = fp(bias); c.state = state.data_ptr(); c.state_out = next.data_ptr(); c.z = t3(z);
+    check(lib.conv_seq(&c, stream_of(x)));
+    return {z, next};
+}
+
+// kla_b200_conv_seq_bwd -> dx, dweight, dbias
+std::tuple<Tensor, Tensor, OptTensor> conv_seq_bwd(const Tensor &x, const Tensor &dz, const Tensor &w, const OptTensor &bias,
+                                                   const Tensor &state, int act) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t B = x.size(0), L = x.size(1), D = x.size(2), K = w.size(1);
+    Tensor dx = at::empty({B, L, D}, x.options());
+    Tensor sums = at::zeros({bias ? D * (K + 1) : D * K}, x.options().dtype(at::kFloat));  // dweight, then dbias
+    Tensor dw = sums.narrow(0, 0, D * K).view({D, K});
+    OptTensor db;
+    if (bias) db = sums.narrow(0, D * K, D);
+    kla_b200_conv_seq_bwd_args c{};
+    c.B = B; c.L = L; c.D = D; c.K = K; c.dtype = dt(x.scalar_type()); c.activation = act;
+    c.x = t3(x); c.dz = t3(dz); c.weight = fp(w); c.bias = fp(bias); c.state = state.data_ptr(); c.dx = t3(dx);
+    c.dweight = fp(dw); c.dbias = fp(db);
+    check(lib.conv_seq_bwd(&c, stream_of(x)));
+    return {dx, dw, db};
+}
+
+// One of the four raw scans over [B, L, M, S] coefficients.
+void rawscan(int which, const std::vector<Tensor> &ins, const std::vector<Tensor> &outs, const OptTensor &state0, const OptTensor &dstate0) {
+    const Tensor &x = ins[0];
+    const c10::cuda::CUDAGuard guard(x.device());
+    kla_b200_rawscan_args r{};
+    r.B = x.size(0); r.L = x.size(1); r.N = x.size(2) * x.size(3);
+    for (size_t i = 0; i < ins.size(); ++i) r.in[i] = fp(ins[i]);
+    for (size_t i = 0; i < outs.size(); ++i) r.out[i] = fp(outs[i]);
+    r.state0 = fp(state0); r.dstate0 = fp(dstate0);
+    check(lib.rawscan[which](&r, stream_of(x)));
+}
+
+// --------------------------------------------------------------------------------------------------- decode steps
+
+bool wants_grad(std::initializer_list<const Tensor *> ts) {
+    if (!c10::GradMode::is_enabled()) return false;
+    for (const Tensor *t : ts)
+        if (t->requires_grad()) return true;
+    return false;
+}
+
+// kla_b200_step -> (y, y_var, lam, eta), or None when the arguments need the wrapper's general path.
+py::object step(const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const Tensor &lam,
+                const Tensor &eta, bool prior, bool inplace) {
+    if (!v.is_cuda() || v.dim() != 2 || k.dim() != 2 || a.dim() != 2 || lam.dim() != 3) return py::none();
+    const auto T = v.scalar_type();
+    const int64_t B = v.size(0), M = v.size(1), S = k.size(1);
+    if ((T != at::kFloat && T != at::kBFloat16) || lv.scalar_type() != T || k.scalar_type() != T || q.scalar_type() != T) return py::none();
+    if (S > KLA_B200_MAX_DSTATE || lv.sizes() != v.sizes() || q.sizes() != k.sizes() || k.size(0) != B || a.size(0) != M || a.size(1) != S ||
+        p.sizes() != a.sizes() || lam.size(0) != B || lam.size(1) != M || lam.size(2) != S || eta.sizes() != lam.sizes())
+        return py::none();
+    for (const Tensor *t : {&a, &p, &lam, &eta})
+        if (t->scalar_type() != at::kFloat || !t->is_contiguous()) return py::none();
+    for (const Tensor *t : {&lv, &k, &q, &a, &p, &lam, &eta})
+        if (t->device() != v.device()) return py::none();
+    if (!rows_ok(v) || !rows_ok(lv) || !rows_ok(k) || !rows_ok(q) || !sm100(v.device())) return py::none();
+    if (wants_grad({&v, &lv, &k, &q, &a, &p, &lam, &eta})) return py::none();
+    const c10::cuda::CUDAGuard guard(v.device());
+    Tensor y = f32(v, {B, M}), yv = f32(v, {B, M});
+    Tensor lo = inplace ? lam : at::empty_like(lam), eo = inplace ? eta : at::empty_like(eta);
+    kla_b200_step_args s{};
+    s.B = B; s.M = M; s.S = S;
+    s.in_dtype = dt(T); s.out_dtype = KLA_B200_F32; s.decode_from_prior = prior;
+    s.v = v.data_ptr(); s.lambda_v = lv.data_ptr(); s.v_stride_b = v.stride(0); s.lambda_v_stride_b = lv.stride(0);
+    s.k = k.data_ptr(); s.q = q.data_ptr(); s.k_stride_b = k.stride(0); s.q_stride_b = q.stride(0);
+    s.a = fp(a); s.p = fp(p); s.lam = fp(lam); s.eta = fp(eta);
+    s.y = y.data_ptr(); s.y_var = yv.data_ptr(); s.lam_out = fp(lo); s.eta_out = fp(eo);
+    check(lib.step(&s, stream_of(v)));
+    return py::make_tuple(y, yv, lo, eo);
+}
+
+int act_code(const py::object &name) {  // the activation's name in a config, or None
+    if (name.is_none()) return KLA_B200_ACT_NONE;
+    const std::string s = name.cast<std::string>();
+    if (s == "silu") return KLA_B200_ACT_SILU;
+    if (s == "gelu") return KLA_B200_ACT_GELU;
+    if (s == "relu") return KLA_B200_ACT_RELU;
+    throw py::key_error(s);
+}
+
+struct Weights {  // a layer's weights by name; what a dict does not hold is absent
+    const py::dict &d;
+    Tensor at(const char *name) const { return d[name].cast<Tensor>(); }
+    OptTensor get(const char *name) const {
+        const PyObject *o = PyDict_GetItemString(d.ptr(), name);
+        return o ? OptTensor(py::handle(const_cast<PyObject *>(o)).cast<Tensor>()) : OptTensor();
+    }
+    Tensor linear(const Tensor &x, const char *w, const char *b) const { return at::linear(x, at(w), get(b)); }
+};
+
+// One token of a layer (LayerDecoder.step): three projections, the convolution's step and the fused filter step. conv_state
+// (absent without a convolution), lam and eta are updated in place. Returns the layer's output and the gated variance, which
+// a config that returns variances projects as well.
+std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, const Tensor &x, const OptTensor &conv_state,
+                                      const Tensor &lam, const Tensor &eta, const Tensor &a_bar, const Tensor &p_bar,
+                                      const OptTensor &skip, const OptTensor &conv_w, const OptTensor &conv_b, int64_t w_value,
+                                      int64_t w_var) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Weights w{w_};
+    void *stream = stream_of(x);
+    const int64_t B = x.size(0), M = a_bar.size(0), S = a_bar.size(1);
+    const int32_t type = dt(x.scalar_type());
+    const Tensor projected = w.linear(x, "in_proj.weight", "in_proj.bias");
+    const bool gated = cfg["use_gating"].cast<bool>();
+    Tensor z = gated ? projected.narrow(1, 0, M) : projected;
+    OptTensor gate;
+    if (gated) gate = projected.narrow(1, M, projected.size(1) - M);
+    if (conv_w) {
+        Tensor zc = at::empty({B, M}, x.options());
+        kla_b200_conv_step_args c{};
+        c.B = B; c.D = M; c.K = cfg["conv_kernel_size"].cast<int64_t>(); c.dtype = type;
+        c.activation = act_code(cfg["conv_activation"]);
+        c.x = z.data_ptr(); c.x_stride_b = z.stride(0); c.weight = fp(*conv_w); c.bias = fp(conv_b);
+        c.state = conv_state ? conv_state->data_ptr() : nullptr; c.z = zc.data_ptr();
+        check(lib.conv_step(&c, stream));
+        z = zc;
+    }
+    const Tensor sens = w.linear(z, "sensor_proj.weight", "sensor_proj.bias");
+    // the four sensor signals, raw, as KLALayer._project_sensors splits them (src/kla/layers/kla_layer.py:199-216)
+    const bool from_conv = w_value == 0;
+    Tensor v = from_conv ? z : sens.narrow(1, 0, w_value);
+    if (!from_conv && w_.contains("value_expand.weight")) v = w.linear(v, "value_expand.weight", "value_expand.bias");
+    Tensor ls = sens.narrow(1, w_value, w_var);
+    if (w_.contains("var_expand.weight")) ls = w.linear(ls, "var_expand.weight", "var_expand.bias");
+    const int64_t at_k = (w_value + w_var), row = sens.stride(0), esz = sens.element_size();
+    char *kq = static_cast<char *>(sens.data_ptr()) + at_k * esz;
+    Tensor y = at::empty({B, M}, x.options()), yv = at::empty({B, M}, x.options());
+    const py::object vmax = cfg["obs_var_max"], clip = cfg["clip_value"];
+    kla_b200_step_layer_args s{};
+    s.B = B; s.M = M; s.S = S; s.in_dtype = type; s.out_dtype = type;
+    s.decode_from_prior = cfg["decode_from_prior"].cast<bool>();
+    s.qk_norm = cfg["qk_norm"].cast<bool>();
+    s.gate_activation = gated ? act_code(cfg["gating_activation"]) : KLA_B200_ACT_NONE;
+    s.lambda_skip_len = skip ? (int32_t)skip->numel() : 0;
+    s.obs_var_min = cfg["obs_var_min"].cast<float>();
+    s.obs_var_max = vmax.is_none() ? 0.0f : vmax.cast<float>();
+    s.clip_value = clip.is_none() ? 0.0f : clip.cast<float>();
+    s.v = v.data_ptr(); s.log_sigma_v = ls.data_ptr(); s.v_stride_b = v.stride(0); s.log_sigma_v_stride_b = ls.stride(0);
+    s.k = kq; s.q = kq + S * esz; s.k_stride_b = row; s.q_stride_b = row;
+    s.z = z.data_ptr(); s.z_stride_b = z.stride(0);
+    s.gate = gate ? gate->data_ptr() : nullptr; s.gate_stride_b = gate ? gate->stride(0) : 0;
+    s.lambda_skip = fp(skip); s.a = fp(a_bar); s.p = fp(p_bar); s.lam = fp(lam); s.eta = fp(eta);
+    s.y = y.data_ptr(); s.y_var = yv.data_ptr(); s.lam_out = fp(lam); s.eta_out = fp(eta);
+    check(lib.step_layer(&s, stream));
+    return {w.linear(y, "out_proj.weight", "out_proj.bias"), yv};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_kla_host, m) {
+    m.doc() = "Launches of the kla_b200 library on torch tensors";
+    m.def("bind", &bind);
+    m.def("canonical", &canonical);
+    m.def("scan_fwd", &scan_fwd);
+    m.def("scan_bwd", &scan_bwd);
+    m.def("slab_aggregate", &slab_aggregate);
+    m.def("chunk_fold", &chunk_fold);
+    m.def("scan_fwd_chunked", &scan_fwd_chunked);
+    m.def("scan_bwd_chunked", &scan_bwd_chunked);
+    m.def("epilogue_bwd", &epilogue_bwd);
+    m.def("conv_seq", &conv_seq);
+    m.def("conv_seq_bwd", &conv_seq_bwd);
+    m.def("rawscan", &rawscan);
+    m.def("step", &step);
+    m.def("layer_step", &layer_step);
+}

@@ -34,14 +34,20 @@ __global__ void __launch_bounds__(128) kla_chunk_fold_kernel(const ChunkFoldPara
     if (gid >= (long long)prm.B * lanes) return;
     const long long b = gid / lanes, ms = gid % lanes;
     const int C = prm.C;
-    // The fold itself is serial over c, but a chunk's record does not depend on the carry: the next record is
-    // fetched while the current one is applied, so the loop pays one memory latency, not C of them.
+    // The fold itself is serial over c, but a chunk's record does not depend on the carry: records are fetched kAhead
+    // chunks before they are applied, so the loop pays C / kAhead memory latencies (16 chunks, one ahead: 7.2 us).
+    constexpr int kAhead = 4;
     auto fetch = [&](int c, float4 &lo, float4 &hi) {
         const float4 *src = reinterpret_cast<const float4 *>(prm.agg + (((b * C + c) * lanes) + ms) * 8);
         lo = src[0];
         hi = src[1];
     };
-    float4 lo, hi, nlo = make_float4(0, 0, 0, 0), nhi = nlo;
+    float4 lo[kAhead], hi[kAhead];  // slot i: the i-th record from here in the order of the fold
+    auto fetch_nth = [&](int n, float4 &l, float4 &h) {  // record number n in that order (nothing past the last)
+        if (n < C) fetch(ADJ ? C - 1 - n : n, l, h);
+    };
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) fetch_nth(i, lo[i], hi[i]);
     if (!ADJ) {
         // the state in homogeneous coordinates (x, w, z), P = w/x, mean = z/x: applying a record is a 3x3
         // product, and lam = x/w, eta = z/w need one reciprocal per chunk. Records are normalised, so the
@@ -51,41 +57,44 @@ __global__ void __launch_bounds__(128) kla_chunk_fold_kernel(const ChunkFoldPara
             w = 1.0 / fmax((double)prm.in_a[gid], (double)kLamMin);
             z = (double)prm.in_b[gid] * w;
         }
-        if (C > 1) fetch(0, nlo, nhi);
-        for (int c = 0; c < C; ++c) {
-            const long long o = (b * C + c) * lanes + ms;
-            const double rw = 1.0 / w;
-            prm.out_a[o] = (float)(x * rw);
-            prm.out_b[o] = (float)(z * rw);
-            if (c + 1 < C) {
-                lo = nlo; hi = nhi;
-                if (c + 2 < C) fetch(c + 1, nlo, nhi);
-                const double nx = (double)lo.x * x + (double)lo.y * w, nw = (double)lo.z * x + (double)lo.w * w;
-                z = (double)hi.x * x + (double)hi.y * w + (double)hi.z * z;
+        for (int c0 = 0; c0 < C; c0 += kAhead) {
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const int c = c0 + i;
+                if (c >= C) break;
+                const long long o = (b * C + c) * lanes + ms;
+                const double rw = 1.0 / w;
+                prm.out_a[o] = (float)(x * rw);
+                prm.out_b[o] = (float)(z * rw);
+                const float4 l = lo[i], h = hi[i];
+                fetch_nth(c + kAhead, lo[i], hi[i]);
+                const double nx = (double)l.x * x + (double)l.y * w, nw = (double)l.z * x + (double)l.w * w;
+                z = (double)h.x * x + (double)h.y * w + (double)h.z * z;
                 x = nx;
                 w = nw;
             }
         }
     } else {
-        fetch(C - 1, lo, hi);
-        if (C > 1) fetch(C - 2, nlo, nhi);
         const double dl = prm.in_a ? (double)prm.in_a[gid] : 0.0, de = prm.in_b ? (double)prm.in_b[gid] : 0.0;
         // (dL/dP, dL/dmean) at the end of the sequence from the gradient of (lam, eta) = (1/P, mean/P)
-        const double lam = 1.0 / (double)hi.y, eta = (double)hi.z * lam;
+        const double lam = 1.0 / (double)hi[0].y, eta = (double)hi[0].z * lam;
         double cP = -lam * (lam * dl + eta * de), cm = de * lam;
-        for (int c = C - 1; c >= 0; --c) {
-            if (c != C - 1) {
-                lo = nlo; hi = nhi;
-                if (c > 0) fetch(c - 1, nlo, nhi);
+        for (int n0 = 0; n0 < C; n0 += kAhead) {
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const int n = n0 + i;
+                if (n >= C) break;
+                const float4 l = lo[i], h = hi[i];
+                fetch_nth(n + kAhead, lo[i], hi[i]);
+                const long long o = (b * C + (C - 1 - n)) * lanes + ms;
+                const double P_end = h.y, mean_end = h.z;  // record: K00 K01 K11 b0 | b1 P_end mean_end
+                const double deta = cm * P_end;
+                prm.out_b[o] = (float)deta;
+                prm.out_a[o] = (float)(-(cP * P_end * P_end + mean_end * deta));
+                const double nP = (double)l.x * cP + (double)l.y * cm + (double)l.w;
+                cm = (double)l.z * cm + (double)h.x;
+                cP = nP;
             }
-            const long long o = (b * C + c) * lanes + ms;
-            const double P_end = hi.y, mean_end = hi.z;  // record: K00 K01 K11 b0 | b1 P_end mean_end
-            const double deta = cm * P_end;
-            prm.out_b[o] = (float)deta;
-            prm.out_a[o] = (float)(-(cP * P_end * P_end + mean_end * deta));
-            const double nP = (double)lo.x * cP + (double)lo.y * cm + (double)lo.w;
-            cm = (double)lo.z * cm + (double)hi.x;
-            cP = nP;
         }
     }
 }

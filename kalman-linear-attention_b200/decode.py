@@ -14,8 +14,6 @@ reference package at run time; ``LayerDecoder.from_layer`` reads both off a refe
 
 from __future__ import annotations
 
-import ctypes
-
 import torch
 import torch.nn.functional as F
 
@@ -137,17 +135,7 @@ class LayerDecoder:
         z, gate = (projected[..., :M], projected[..., M:]) if cfg["use_gating"] else (projected, None)
         if cfg["use_conv"]:
             # the causal convolution over the prompt, in place of cat + transpose + conv1d + activation + transpose
-            zc = torch.empty(B, L, M, device=x.device, dtype=x.dtype)
-            new_window = torch.empty_like(conv_state)
-            dt = _lib.F32 if x.dtype == torch.float32 else _lib.BF16
-            P = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())
-            ca = _lib.ConvSeqArgs(B=B, L=L, D=M, K=cfg["conv_kernel_size"], dtype=dt,
-                                  activation=_lib.ACT[cfg["conv_activation"]],
-                                  x=_lib.Tensor3(z.data_ptr(), z.stride(0), z.stride(1)), weight=P(self.conv_w),
-                                  bias=P(self.conv_b), state=P(conv_state), state_out=P(new_window),
-                                  z=_lib.Tensor3(zc.data_ptr(), zc.stride(0), zc.stride(1)))
-            with torch.cuda.device(x.device):
-                _lib.check(_lib.load().kla_b200_conv_seq(ctypes.byref(ca), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            zc, new_window = _lib.host().conv_seq(z, self.conv_w, self.conv_b, conv_state, _lib.ACT[cfg["conv_activation"]])
             conv_state.copy_(new_window)
             z = zc
         v, ls, k, q = self._sensors(z, self._linear(z, "sensor_proj"))
@@ -180,42 +168,12 @@ class LayerDecoder:
             raise NotImplementedError("The b200 decode kernels need CUDA tensors; use the reference layer on this device.")
         if x.dtype not in (torch.float32, torch.bfloat16):
             raise NotImplementedError(f"The b200 decode kernels take float32 or bfloat16 activations, not {x.dtype}.")
-        cfg, M, S = self.cfg, self.M, self.S
         conv_state, lam, eta = state
-        B = x.shape[0]
-        dt = _lib.F32 if x.dtype == torch.float32 else _lib.BF16
-        lib = _lib.load()
-        P = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())
-        with torch.cuda.device(x.device):
-            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-            projected = self._linear(x, "in_proj")
-            z, gate = (projected[:, :M], projected[:, M:]) if cfg["use_gating"] else (projected, None)
-            if cfg["use_conv"]:
-                zc = torch.empty(B, M, device=x.device, dtype=x.dtype)
-                ca = _lib.ConvStepArgs(B=B, D=M, K=cfg["conv_kernel_size"], dtype=dt,
-                                       activation=_lib.ACT[cfg["conv_activation"]], x=P(z), x_stride_b=z.stride(0),
-                                       weight=P(self.conv_w), bias=P(self.conv_b), state=P(conv_state), z=P(zc))
-                _lib.check(lib.kla_b200_conv_step(ctypes.byref(ca), stream))
-                z = zc
-            sens = self._linear(z, "sensor_proj")
-            v, ls, k, q = self._sensors(z, sens)
-            y = torch.empty(B, M, device=x.device, dtype=x.dtype)
-            y_var = torch.empty_like(y)
-            sa = _lib.StepLayerArgs(
-                B=B, M=M, S=S, in_dtype=dt, out_dtype=dt, decode_from_prior=int(cfg["decode_from_prior"]),
-                qk_norm=int(cfg["qk_norm"]), gate_activation=_lib.ACT[cfg["gating_activation"] if gate is not None else None],
-                lambda_skip_len=0 if self.skip is None else self.skip.numel(),
-                obs_var_min=cfg["obs_var_min"], obs_var_max=cfg["obs_var_max"] or 0.0, clip_value=cfg["clip_value"] or 0.0,
-                v=P(v), log_sigma_v=P(ls), v_stride_b=v.stride(0), log_sigma_v_stride_b=ls.stride(0),
-                k=P(k), q=P(q), k_stride_b=k.stride(0), q_stride_b=q.stride(0),
-                z=P(z), gate=P(gate), z_stride_b=z.stride(0), gate_stride_b=0 if gate is None else gate.stride(0),
-                lambda_skip=P(self.skip), a=P(self.a_bar), p=P(self.p_bar), lam=P(lam), eta=P(eta),
-                y=P(y), y_var=P(y_var), lam_out=P(lam), eta_out=P(eta))
-            _lib.check(lib.kla_b200_step_layer(ctypes.byref(sa), stream))
-            out = self._linear(y, "out_proj")
-            if cfg["return_variance"]:
-                return out, F.linear(y_var, self.w["out_proj.weight"].pow(2))
-            return out
+        out, y_var = _lib.host().layer_step(self.w, self.cfg, x, conv_state, lam, eta, self.a_bar, self.p_bar, self.skip,
+                                            self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var)
+        if self.cfg["return_variance"]:
+            return out, F.linear(y_var, self.w["out_proj.weight"].pow(2))
+        return out
 
 
 MODEL_KEYS = ("n_layers", "norm_eps", "mlp", "logit_softcap")

@@ -23,14 +23,13 @@ to the original method. ``disable()`` restores it.
 
 from __future__ import annotations
 
-import ctypes
 import sys
 
 import torch
 import torch.nn.functional as F
 
 from . import _lib
-from .ops import _on, _rowmajor_last, _stream, _t3, kla_scan_b200
+from .ops import _rowmajor_last, kla_scan_b200
 
 _ORIG_FORWARD = None
 
@@ -43,7 +42,6 @@ class _CausalConvB200(torch.autograd.Function):
     def forward(ctx, x, weight, bias, state, activation):
         B, L, D = x.shape
         K = weight.shape[-1]
-        lib = _lib.load()
         w = weight.detach().float().reshape(D, K).contiguous()
         b = None if bias is None else bias.detach().float().contiguous()
         x = _rowmajor_last(x)
@@ -51,14 +49,7 @@ class _CausalConvB200(torch.autograd.Function):
             state = torch.zeros((B, D, K - 1), device=x.device, dtype=x.dtype)
         else:
             state = state.detach().to(x.dtype).contiguous()
-        z = torch.empty((B, L, D), device=x.device, dtype=x.dtype)
-        new_state = torch.empty_like(state)
-        args = _lib.ConvSeqArgs(B=B, L=L, D=D, K=K, dtype=_lib.F32 if x.dtype == torch.float32 else _lib.BF16,
-                                activation=_lib.ACT[activation], x=_t3(x), weight=w.data_ptr(),
-                                bias=None if b is None else b.data_ptr(), state=state.data_ptr(),
-                                state_out=new_state.data_ptr(), z=_t3(z))
-        with _on(x.device):
-            _lib.check(lib.kla_b200_conv_seq(ctypes.byref(args), _stream(x.device)))
+        z, new_state = _lib.host().conv_seq(x, w, b, state, _lib.ACT[activation])
         ctx.save_for_backward(x, w, b, state)
         ctx.activation, ctx.wshape = activation, weight.shape
         ctx.wdtype, ctx.bdtype = weight.dtype, None if bias is None else bias.dtype
@@ -69,18 +60,8 @@ class _CausalConvB200(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, dz, _dstate):
         x, w, b, state = ctx.saved_tensors
-        B, L, D = x.shape
-        K = w.shape[1]
         dz = _rowmajor_last(dz if dz.dtype == x.dtype else dz.to(x.dtype))
-        dx = torch.empty((B, L, D), device=x.device, dtype=x.dtype)
-        dw = torch.zeros((D, K), device=x.device, dtype=torch.float32)
-        db = None if b is None else torch.zeros((D,), device=x.device, dtype=torch.float32)
-        args = _lib.ConvSeqBwdArgs(B=B, L=L, D=D, K=K, dtype=_lib.F32 if x.dtype == torch.float32 else _lib.BF16,
-                                   activation=_lib.ACT[ctx.activation], x=_t3(x), dz=_t3(dz), weight=w.data_ptr(),
-                                   bias=None if b is None else b.data_ptr(), state=state.data_ptr(), dx=_t3(dx),
-                                   dweight=dw.data_ptr(), dbias=None if db is None else db.data_ptr())
-        with _on(x.device):
-            _lib.check(_lib.load().kla_b200_conv_seq_bwd(ctypes.byref(args), _stream(x.device)))
+        dx, dw, db = _lib.host().conv_seq_bwd(x, dz, w, b, state, _lib.ACT[ctx.activation])
         return dx, dw.reshape(ctx.wshape).to(ctx.wdtype), None if db is None else db.to(ctx.bdtype), None, None
 
 

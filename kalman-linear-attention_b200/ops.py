@@ -16,15 +16,13 @@ can; nothing falls back silently, and there is no CPU or Triton path.
 
 from __future__ import annotations
 
-import contextlib
-import ctypes
 import sys
 from typing import NamedTuple, Optional
 
 import torch
 
 from . import _lib
-from ._lib import BF16, F32, MAX_DSTATE, BwdArgs, ChunkFoldArgs, EpilogueBwdArgs, FwdArgs, SlabArgs, StepArgs, Tensor3
+from ._lib import MAX_DSTATE
 
 
 class KLAState(NamedTuple):
@@ -76,62 +74,12 @@ def _require_sm100(device: torch.device) -> None:
         raise _unsupported("is compiled for sm_100a (B200) only and this device is not one")
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
-
-
-def _t3(t: Optional[torch.Tensor]) -> Tensor3:
-    if t is None:
-        return Tensor3(None, 0, 0)
-    return Tensor3(t.data_ptr(), t.stride(0), t.stride(1))
-
-
 def _rowmajor_last(t: torch.Tensor) -> torch.Tensor:
     """The kernels take a batch and a time stride per tensor but need unit stride
     on the last dimension; anything else is copied once."""
     if t.dim() == 3 and (t.shape[-1] <= 1 or t.stride(-1) == 1):
         return t
     return t.contiguous()
-
-
-_NULL_CTX = contextlib.nullcontext()
-
-
-def _on(device: torch.device):
-    """Context that makes ``device`` current for a launch; free when it already is (the usual case)."""
-    idx = device.index
-    if idx is None or idx == torch.cuda.current_device():
-        return _NULL_CTX
-    return torch.cuda.device(device)
-
-
-def _stream(device: torch.device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
-
-
-def _dt(t: torch.dtype) -> int:
-    return BF16 if t == torch.bfloat16 else F32
-
-
-def _sensor_fields(sensors):
-    """C-ABI fields of the fused sensor prologue: ``sensors`` is None or (obs_var_min, obs_var_max or None)."""
-    if sensors is None:
-        return dict(lambda_v_is_log_variance=0, obs_var_min=0.0, obs_var_max=0.0)
-    return dict(lambda_v_is_log_variance=1, obs_var_min=float(sensors[0]), obs_var_max=float(sensors[1] or 0.0))
-
-
-def _epilogue_fields(epilogue):
-    """C-ABI fields of the forward-only layer epilogue: ``epilogue`` is None or a dict with any of
-    ``z`` + ``lambda_skip`` (float32, one value or [M]) and ``gate`` + ``gate_activation``."""
-    if not epilogue:
-        return {}
-    out = {}
-    skip = epilogue.get("lambda_skip")
-    if skip is not None:
-        out.update(z=_t3(epilogue["z"]), lambda_skip=_ptr(skip), lambda_skip_len=skip.numel())
-    if epilogue.get("gate") is not None:
-        out.update(gate=_t3(epilogue["gate"]), gate_activation=_lib.ACT[epilogue.get("gate_activation", "silu")])
-    return out
 
 
 _SM_COUNT: dict = {}
@@ -153,98 +101,29 @@ def _launch_fwd(v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype, nee
                 epilogue=None, raw=None):
     """Allocate outputs (and the checkpoint scratch when a backward will follow)
     and enqueue ``kla_b200_scan_fwd`` on the current stream of the inputs' device."""
-    lib = _lib.load()
-    B, L, M = v.shape
-    S = k.shape[2]
-    dev = v.device
-    y = torch.empty((B, L, M), device=dev, dtype=out_dtype)
-    y_var = torch.empty((B, L, M), device=dev, dtype=out_dtype)
-    lam_fin = torch.empty((B, M, S), device=dev, dtype=torch.float32)
-    eta_fin = torch.empty((B, M, S), device=dev, dtype=torch.float32)
-    ckpt = work = None
-    if need_ckpt and L > 0:
-        ckpt = torch.empty(lib.kla_b200_ckpt_bytes(B, L, M, S), device=dev, dtype=torch.uint8)
-    elif _forward_segments(lib, dev, B, L, M, S):
-        # no backward will follow, but the sequences are many enough for the kernel to hand them from CTA to CTA in
-        # segments: that needs a little working memory
-        work = torch.empty(lib.kla_b200_segment_scratch_bytes(B, M, S), device=dev, dtype=torch.uint8)
-    args = FwdArgs(
-        B=B, L=L, M=M, S=S, in_dtype=_dt(v.dtype), out_dtype=_dt(out_dtype),
-        decode_from_prior=int(prior),
-        v=_t3(v), lambda_v=_t3(lambda_v), k=_t3(k), q=_t3(q),
-        a=_ptr(a), p=_ptr(p), lam0=_ptr(lam0), eta0=_ptr(eta0),
-        y=_t3(y), y_var=_t3(y_var), lam_fin=_ptr(lam_fin), eta_fin=_ptr(eta_fin),
-        ckpt=_ptr(ckpt), work=_ptr(work), **_sensor_fields(sensors), **_epilogue_fields(epilogue),
-        **({} if raw is None else dict(y_raw=_t3(raw[0]), y_var_raw=_t3(raw[1]))),
-    )
-    with _on(dev):
-        _lib.check(lib.kla_b200_scan_fwd(ctypes.byref(args), _stream(dev)))
-    return y, y_var, lam_fin, eta_fin, ckpt
+    # without checkpoints the kernel still hands long lists of sequences from CTA to CTA in segments, given a little
+    # working memory
+    segments = not need_ckpt and _forward_segments(_lib.load(), v.device, v.shape[0], v.shape[1], v.shape[2], k.shape[2])
+    epi = epilogue or {}
+    gate = epi.get("gate")
+    return _lib.host().scan_fwd(
+        v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype == torch.bfloat16, need_ckpt, segments, sensors,
+        epi.get("z"), epi.get("lambda_skip"), gate, 0 if gate is None else _lib.ACT[epi.get("gate_activation", "silu")],
+        *(raw or (None, None)), 1, 0)
 
 
 def _launch_bwd(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin,
                 prior: bool, out_dtype, sensors=None):
     """Allocate the gradients and enqueue ``kla_b200_scan_bwd``."""
-    lib = _lib.load()
-    B, L, M = v.shape
-    S = k.shape[2]
-    dev = v.device
-    dv = torch.empty((B, L, M), device=dev, dtype=v.dtype)
-    dlv = torch.empty((B, L, M), device=dev, dtype=v.dtype)
-    dk = torch.empty((B, L, S), device=dev, dtype=torch.float32)
-    dq = torch.empty((B, L, S), device=dev, dtype=torch.float32)
-    da = torch.empty((M, S), device=dev, dtype=torch.float32)
-    dp = torch.empty((M, S), device=dev, dtype=torch.float32)
-    dlam0 = torch.empty((B, M, S), device=dev, dtype=torch.float32)
-    deta0 = torch.empty((B, M, S), device=dev, dtype=torch.float32)
-    args = BwdArgs(
-        B=B, L=L, M=M, S=S, in_dtype=_dt(v.dtype), out_dtype=_dt(out_dtype),
-        decode_from_prior=int(prior),
-        v=_t3(v), lambda_v=_t3(lambda_v), k=_t3(k), q=_t3(q),
-        a=_ptr(a), p=_ptr(p), lam0=_ptr(lam0), eta0=_ptr(eta0), ckpt=_ptr(ckpt),
-        dy=_t3(dy), dy_var=_t3(dy_var), dlam_fin=_ptr(dlam_fin), deta_fin=_ptr(deta_fin),
-        dv=_t3(dv), dlambda_v=_t3(dlv), dk=_ptr(dk), dq=_ptr(dq), da=_ptr(da), dp=_ptr(dp),
-        dlam0=_ptr(dlam0), deta0=_ptr(deta0), **_sensor_fields(sensors),
-    )
-    with _on(dev):
-        _lib.check(lib.kla_b200_scan_bwd(ctypes.byref(args), _stream(dev)))
-    return dv, dlv, dk, dq, da, dp, dlam0, deta0
+    return _lib.host().scan_bwd(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin, prior,
+                                out_dtype == torch.bfloat16, sensors, 1, 0)
 
 
 def slab_aggregate(v, lambda_v, k, a, p, *, q=None, dy=None, dy_var=None, lam0=None, eta0=None,
                    prior: bool = False) -> torch.Tensor:
     """Launch ``kla_b200_slab_aggregate``: one record per lane that describes how a whole time slab acts on
     the filter state (``dy`` None) or on the backward carry (``dy`` given). Returns [B, M, S, 8] float32."""
-    lib = _lib.load()
-    B, L, M = v.shape
-    S = k.shape[2]
-    out = torch.empty((B, M, S, 8), device=v.device, dtype=torch.float32)
-    adjoint = dy is not None
-    od = dy.dtype if adjoint else torch.float32
-    args = SlabArgs(
-        B=B, L=L, M=M, S=S, in_dtype=_dt(v.dtype), out_dtype=_dt(od),
-        decode_from_prior=int(prior), adjoint=int(adjoint),
-        v=_t3(v), lambda_v=_t3(lambda_v), k=_t3(k), q=_t3(q),
-        a=_ptr(a), p=_ptr(p), lam0=_ptr(lam0), eta0=_ptr(eta0),
-        dy=_t3(dy), dy_var=_t3(dy_var), out=_ptr(out),
-    )
-    with _on(v.device):
-        _lib.check(lib.kla_b200_slab_aggregate(ctypes.byref(args), _stream(v.device)))
-    return out
-
-
-def chunk_fold(agg: torch.Tensor, C: int, in_a, in_b, adjoint: bool):
-    """Launch ``kla_b200_chunk_fold`` over aggregates [B*C, M, S, 8]; returns two [B*C, M, S] float32 tensors:
-    the state before each chunk (forward) or the state-gradient seeds of each chunk (adjoint)."""
-    lib = _lib.load()
-    BC, M, S, _ = agg.shape
-    out_a = torch.empty((BC, M, S), device=agg.device, dtype=torch.float32)
-    out_b = torch.empty((BC, M, S), device=agg.device, dtype=torch.float32)
-    args = ChunkFoldArgs(B=BC // C, C=C, M=M, S=S, adjoint=int(adjoint), agg=_ptr(agg),
-                         in_a=_ptr(in_a), in_b=_ptr(in_b), out_a=_ptr(out_a), out_b=_ptr(out_b))
-    with _on(agg.device):
-        _lib.check(lib.kla_b200_chunk_fold(ctypes.byref(args), _stream(agg.device)))
-    return out_a, out_b
+    return _lib.host().slab_aggregate(v, lambda_v, k, a, p, q, dy, dy_var, lam0, eta0, prior, 1, 0)
 
 
 # CTAs the backward kernel keeps resident on a B200: 148 SMs x 2
@@ -264,8 +143,9 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
     When that grid leaves most of the GPU empty, the sequence is cut into C chunks that run as B*C batch entries;
     building the chunks' start states costs about 0.7x of a forward + backward pass on top, so chunking is only
     chosen when the plain grid fills less than a third of the resident CTA slots; then up to 16 chunks, enough
-    for about four waves of CTAs. C divides L, chunks keep at least 64 steps. ``requested`` (or the environment variable KLA_B200_TIME_CHUNKS) overrides the choice; it is
-    lowered to the nearest usable divisor of L."""
+    for about four waves of CTAs. Chunks keep at least 64 steps and are equally long where the count divides L, else
+    a multiple of 16 steps with a shorter last one (:func:`_chunk_len`). ``requested`` (or the environment variable
+    KLA_B200_TIME_CHUNKS) overrides the choice; it is lowered to the nearest usable divisor of L."""
     import os
 
     if requested is None and os.environ.get("KLA_B200_TIME_CHUNKS"):
@@ -283,10 +163,19 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
     else:
         want = max(1, int(requested))
     want = min(want, max(1, L // _MIN_CHUNK_STEPS), max(1, 65535 // max(B, 1)))
+    if requested is None:
+        while want > 1 and -(-L // _chunk_len(L, want)) != want:  # rounding the length up can leave fewer chunks
+            want = -(-L // _chunk_len(L, want))
+        return want
     for c in range(want, 0, -1):
         if L % c == 0:
             return c
     return 1
+
+
+def _chunk_len(L: int, C: int) -> int:
+    """Steps per chunk when ``L`` steps are cut into ``C`` chunks."""
+    return L // C if L % C == 0 else (-(-L // C) + 15) // 16 * 16
 
 
 def _as_chunks(t: Optional[torch.Tensor], C: int) -> Optional[torch.Tensor]:
@@ -310,21 +199,15 @@ class _KLAScanB200(torch.autograd.Function):
     def forward(ctx, v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype: torch.dtype, sensors=None,
                 chunks: int = 1):
         need_grad = any(ctx.needs_input_grad[:8])
-        B, L, M = v.shape
-        C = chunks if (chunks > 1 and sensors is None and all(_chunkable(t, B, L) for t in (v, lambda_v, k, q))) else 1
+        ctx.set_materialize_grads(False)  # an output without a gradient costs nothing below
+        C = chunks if sensors is None else 1
         ctx.chunks = C
         if C > 1:
-            # time-parallel: the chunks of every sequence run as B*C batch entries from exact start states
-            vc, lc, kc, qc = (_as_chunks(t, C) for t in (v, lambda_v, k, q))
-            agg = slab_aggregate(vc, lc, kc, a, p)
-            lam_in, eta_in = chunk_fold(agg, C, lam0, eta0, adjoint=False)
-            y, y_var, lam_all, eta_all, ckpt = _launch_fwd(
-                vc, lc, kc, qc, a, p, lam_in, eta_in, prior, out_dtype, need_grad)
-            S = k.shape[2]
-            lam_fin = lam_all.view(B, C, M, S)[:, C - 1]  # views: the last chunk's posterior is the sequence's
-            eta_fin = eta_all.view(B, C, M, S)[:, C - 1]
+            # time-parallel: the chunks of every sequence run side by side from exact start states
+            y, y_var, lam_fin, eta_fin, ckpt, lam_in, eta_in = _lib.host().scan_fwd_chunked(
+                v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype == torch.bfloat16, need_grad, C,
+                _chunk_len(v.shape[1], C))
             ctx.save_for_backward(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, lam_in, eta_in)
-            y, y_var = y.view(B, L, M), y_var.view(B, L, M)
         else:
             y, y_var, lam_fin, eta_fin, ckpt = _launch_fwd(
                 v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, need_grad, sensors)
@@ -363,19 +246,9 @@ class _KLAScanB200(torch.autograd.Function):
             deta_fin = deta_fin.float().contiguous()
         C = ctx.chunks
         if C > 1:
-            lam_in, eta_in = chunk_state
-            if not (_chunkable(dy, B, L) and _chunkable(dy_var, B, L)):
-                dy = dy.contiguous()
-                dy_var = None if dy_var is None else dy_var.contiguous()
-            vc, lc, kc, qc, dyc, dyvc = (_as_chunks(t, C) for t in (v, lambda_v, k, q, dy, dy_var))
-            adj = slab_aggregate(vc, lc, kc, a, p, q=qc, dy=dyc, dy_var=dyvc, lam0=lam_in, eta0=eta_in, prior=ctx.prior)
-            dlam_seed, deta_seed = chunk_fold(adj, C, dlam_fin, deta_fin, adjoint=True)
-            dv, dlv, dk, dq, da, dp, dlam_all, deta_all = _launch_bwd(
-                vc, lc, kc, qc, a, p, lam_in, eta_in, ckpt, dyc, dyvc, dlam_seed, deta_seed, ctx.prior, od)
-            dv, dlv = dv.view(B, L, M), dlv.view(B, L, M)
-            dk, dq = dk.view(B, L, S), dq.view(B, L, S)
-            dlam0 = dlam_all.view(B, C, M, S)[:, 0]
-            deta0 = deta_all.view(B, C, M, S)[:, 0]
+            dv, dlv, dk, dq, da, dp, dlam0, deta0 = _lib.host().scan_bwd_chunked(
+                v, lambda_v, k, q, a, p, *chunk_state, ckpt, dy, dy_var, dlam_fin, deta_fin, ctx.prior,
+                od == torch.bfloat16, C, _chunk_len(L, C))
         else:
             dv, dlv, dk, dq, da, dp, dlam0, deta0 = _launch_bwd(
                 v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin, ctx.prior, od, ctx.sensors)
@@ -393,6 +266,7 @@ class _KLAScanEpilogueB200(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, v, lambda_v, k, q, a, p, lam0, eta0, z, gate, skip, prior, out_dtype, sensors, gate_act):
+        ctx.set_materialize_grads(False)
         need_grad = any(ctx.needs_input_grad[:11])
         B, L, M = v.shape
         epi = {}
@@ -419,7 +293,6 @@ class _KLAScanEpilogueB200(torch.autograd.Function):
         B, L, M = v.shape
         S = k.shape[2]
         dev, od = v.device, ctx.out_dtype
-        lib = _lib.load()
 
         def grad_in(g):
             return None if g is None else _rowmajor_last(g if g.dtype == od else g.to(od))
@@ -427,20 +300,8 @@ class _KLAScanEpilogueB200(torch.autograd.Function):
         dout, dout_var = grad_in(dout), grad_in(dout_var)
         if dout is None:
             dout = torch.zeros((B, L, M), device=dev, dtype=od)
-        dy = torch.empty((B, L, M), device=dev, dtype=od)
-        dy_var = torch.empty((B, L, M), device=dev, dtype=od)
-        dz = None if z is None else torch.empty((B, L, M), device=dev, dtype=v.dtype)
-        dgate = None if gate is None else torch.empty((B, L, M), device=dev, dtype=v.dtype)
-        dskip = None if skip_flat is None else torch.empty_like(skip_flat)
-        args = EpilogueBwdArgs(
-            B=B, L=L, M=M, in_dtype=_dt(v.dtype), out_dtype=_dt(od),
-            gate_activation=_lib.ACT[ctx.gate_act if gate is not None else None],
-            lambda_skip_len=0 if skip_flat is None else skip_flat.numel(),
-            dout=_t3(dout), dout_var=_t3(dout_var), y_raw=_t3(raw[0] if raw else None), y_var_raw=_t3(raw[1] if raw else None),
-            z=_t3(z), gate=_t3(gate), lambda_skip=_ptr(skip_flat),
-            dy=_t3(dy), dy_var=_t3(dy_var), dz=_t3(dz), dgate=_t3(dgate), dlambda_skip=_ptr(dskip))
-        with _on(dev):
-            _lib.check(lib.kla_b200_epilogue_bwd(ctypes.byref(args), _stream(dev)))
+        dy, dy_var, dz, dgate, dskip = _lib.host().epilogue_bwd(
+            v, od == torch.bfloat16, dout, dout_var, *(raw or (None, None)), z, gate, skip_flat, _lib.ACT[ctx.gate_act])
         if (dlam_fin is None) != (deta_fin is None):
             zero = torch.zeros((B, M, S), device=dev, dtype=torch.float32)
             dlam_fin = zero if dlam_fin is None else dlam_fin
@@ -505,6 +366,12 @@ def kla_scan_b200(
     the adjoint carry). ``None`` picks C from the shape (:func:`pick_time_chunks`:
     1 unless B*M is too small to fill the GPU), ``1`` switches it off.
     """
+    if not epilogue and v.is_cuda:
+        lam0, eta0 = initial_state if initial_state is not None else (None, None)
+        if _lib.host().canonical(v, lambda_v, k, q, a, p, lam0, eta0) and (
+                out_dtype is None or out_dtype == torch.float32 or out_dtype == v.dtype == torch.bfloat16):
+            return _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, decode_from_prior, out_dtype or torch.float32,
+                             log_variance, time_chunks)
     _require_device(v)
     if a.dim() != 2:
         raise _unsupported("expects a/p of shape [M, S]")
@@ -543,11 +410,8 @@ def kla_scan_b200(
         lam0 = lam0.float().contiguous()
         eta0 = eta0.float().contiguous()
 
-    if log_variance is not None:
-        if len(log_variance) != 2 or not log_variance[0] >= 0.0:
-            raise ValueError("log_variance must be (obs_var_min >= 0, obs_var_max or None)")
-        log_variance = (float(log_variance[0]), None if log_variance[1] is None else float(log_variance[1]))
     if epilogue:
+        log_variance = _check_log_variance(log_variance)
         epi = dict(epilogue)
         unknown = set(epi) - {"z", "lambda_skip", "gate", "gate_activation"}
         if unknown:
@@ -573,9 +437,26 @@ def kla_scan_b200(
             v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip, bool(decode_from_prior),
             out_dtype, log_variance, gate_act)
         return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)
-    chunks = pick_time_chunks(B, L, M, S, time_chunks) if L > 0 else 1
+    return _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, decode_from_prior, out_dtype, log_variance, time_chunks)
+
+
+def _check_log_variance(log_variance):
+    if log_variance is None:
+        return None
+    if len(log_variance) != 2 or not log_variance[0] >= 0.0:
+        raise ValueError("log_variance must be (obs_var_min >= 0, obs_var_max or None)")
+    return float(log_variance[0]), None if log_variance[1] is None else float(log_variance[1])
+
+
+def _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, log_variance, time_chunks):
+    """The scan of canonical arguments, without an epilogue."""
+    log_variance = _check_log_variance(log_variance)
+    B, L, M = v.shape
+    chunks = pick_time_chunks(B, L, M, k.shape[2], time_chunks) if L > 0 and log_variance is None else 1
+    if chunks > 1 and time_chunks is not None and not all(_chunkable(t, B, L) for t in (v, lambda_v, k, q)):
+        chunks = 1  # an explicit count is taken for sequences that lie back to back
     y, y_var, lam_fin, eta_fin = _KLAScanB200.apply(
-        v, lambda_v, k, q, a, p, lam0, eta0, bool(decode_from_prior), out_dtype, log_variance, chunks)
+        v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype, log_variance, chunks)
     return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)
 
 
@@ -603,10 +484,14 @@ def kla_step_b200(
     (kla_ops.py:310-312, 323), the scan leaves ``phi`` unfloored (kla_ops.py:238);
     the values agree except for keys that are zero to within 1e-6.
     """
+    lam, eta = state
+    if v.is_cuda:
+        out = _lib.host().step(v, lambda_v, k, q, a, p, lam, eta, bool(decode_from_prior), bool(inplace))
+        if out is not None:
+            return out[0], out[1], _state_cls()(lam=out[2], eta=out[3])
     _require_device(v)
     if v.dim() != 2 or k.dim() != 2:
         raise ValueError("v, lambda_v must be [B, M] and k, q [B, S]")
-    lam, eta = state
     if torch.is_grad_enabled() and any(
         t.requires_grad for t in (v, lambda_v, k, q, a, p, lam, eta)
     ):
@@ -622,7 +507,6 @@ def kla_step_b200(
         raise _unsupported(f"supports d_state <= {MAX_DSTATE} (got {S})")
     if any(t.dtype == torch.float64 for t in (v, lambda_v, k, q, a, p, lam, eta)):
         raise _unsupported("runs in float32 only")
-    lib = _lib.load()
     act = torch.bfloat16 if all(t.dtype == torch.bfloat16 for t in (v, lambda_v, k, q)) else torch.float32
 
     def row(t):
@@ -635,20 +519,11 @@ def kla_step_b200(
     if inplace:
         if lam.dtype != torch.float32 or not lam.is_contiguous() or eta.dtype != torch.float32 or not eta.is_contiguous():
             raise ValueError("inplace=True needs float32 contiguous state tensors")
-        lam_out, eta_out = lam, eta
     else:
         lam, eta = lam.float().contiguous(), eta.float().contiguous()
-        lam_out, eta_out = torch.empty_like(lam), torch.empty_like(eta)
-    dev = v.device
-    y = torch.empty((B, M), device=dev, dtype=torch.float32)
-    y_var = torch.empty((B, M), device=dev, dtype=torch.float32)
-    args = StepArgs(
-        B=B, M=M, S=S, in_dtype=_dt(act), out_dtype=F32, decode_from_prior=int(decode_from_prior),
-        v=_ptr(v), lambda_v=_ptr(lambda_v), v_stride_b=v.stride(0), lambda_v_stride_b=lambda_v.stride(0),
-        k=_ptr(k), q=_ptr(q), k_stride_b=k.stride(0), q_stride_b=q.stride(0),
-        a=_ptr(a), p=_ptr(p), lam=_ptr(lam), eta=_ptr(eta),
-        y=_ptr(y), y_var=_ptr(y_var), lam_out=_ptr(lam_out), eta_out=_ptr(eta_out),
-    )
-    with _on(dev):
-        _lib.check(lib.kla_b200_step(ctypes.byref(args), _stream(dev)))
-    return y, y_var, _state_cls()(lam=lam_out, eta=eta_out)
+    with torch.no_grad():
+        out = _lib.host().step(v, lambda_v, k, q, a, p, lam, eta, bool(decode_from_prior), bool(inplace))
+    if out is None:
+        raise ValueError("v, lambda_v [B, M], k, q [B, S], a, p [M, S] and the state [B, M, S] must agree in shape and device")
+    y, y_var, lam, eta = out
+    return y, y_var, _state_cls()(lam=lam, eta=eta)

@@ -14,8 +14,6 @@ Triton or eager path: a tensor that is not a CUDA float32 tensor raises ``NotImp
 
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import _lib
@@ -34,19 +32,7 @@ def _require(name: str, t: torch.Tensor) -> None:
         )
 
 
-def _launch(name: str, shape, ins, outs, state0=None, dstate0=None) -> None:
-    B, L, M, S = shape
-    args = _lib.RawScanArgs(B=B, L=L, N=M * S)
-    for i, t in enumerate(ins):
-        args.inp[i] = t.data_ptr()
-    for i, t in enumerate(outs):
-        args.out[i] = t.data_ptr()
-    args.state0 = state0.data_ptr() if state0 is not None else None
-    args.dstate0 = dstate0.data_ptr() if dstate0 is not None else None
-    lib = _lib.load()
-    with torch.cuda.device(ins[0].device):
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        _lib.check(getattr(lib, "kla_b200_" + name)(ctypes.byref(args), stream))
+_MOBIUS_FWD, _MOBIUS_BWD, _AFFINE_FWD, _AFFINE_BWD = range(4)  # the native module's numbering
 
 
 class _MobiusScanB200(torch.autograd.Function):
@@ -55,7 +41,7 @@ class _MobiusScanB200(torch.autograd.Function):
         A, B, C, D = (t.contiguous() for t in (A, B, C, D))
         lam0c = lam0.contiguous() if lam0 is not None else None
         lam = torch.empty_like(A)
-        _launch("mobius_scan_fwd", A.shape, (A, B, C, D), (lam,), state0=lam0c)
+        _lib.host().rawscan(_MOBIUS_FWD, (A, B, C, D), (lam,), lam0c, None)
         ctx.save_for_backward(A, B, C, D, lam, *((lam0c,) if lam0c is not None else ()))
         ctx.has_lam0 = lam0c is not None
         return lam
@@ -68,7 +54,7 @@ class _MobiusScanB200(torch.autograd.Function):
         dlam = dlam.contiguous()
         dA, dB, dC, dD = (torch.empty_like(A) for _ in range(4))
         dlam0 = torch.empty_like(lam0) if (lam0 is not None and ctx.needs_input_grad[4]) else None
-        _launch("mobius_scan_bwd", A.shape, (A, B, C, D, lam, dlam), (dA, dB, dC, dD), state0=lam0, dstate0=dlam0)
+        _lib.host().rawscan(_MOBIUS_BWD, (A, B, C, D, lam, dlam), (dA, dB, dC, dD), lam0, dlam0)
         return dA, dB, dC, dD, dlam0
 
 
@@ -77,7 +63,7 @@ class _AffineScanB200(torch.autograd.Function):
     def forward(ctx, alpha, r):
         alpha, r = alpha.contiguous(), r.contiguous()
         eta = torch.empty_like(alpha)
-        _launch("affine_scan_fwd", alpha.shape, (alpha, r), (eta,))
+        _lib.host().rawscan(_AFFINE_FWD, (alpha, r), (eta,), None, None)
         ctx.save_for_backward(alpha, eta)
         return eta
 
@@ -87,7 +73,7 @@ class _AffineScanB200(torch.autograd.Function):
         alpha, eta = ctx.saved_tensors
         deta = deta.contiguous()
         dalpha, dr = torch.empty_like(alpha), torch.empty_like(alpha)
-        _launch("affine_scan_bwd", alpha.shape, (alpha, eta, deta), (dalpha, dr))
+        _lib.host().rawscan(_AFFINE_BWD, (alpha, eta, deta), (dalpha, dr), None, None)
         return dalpha, dr
 
 

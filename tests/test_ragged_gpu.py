@@ -1,0 +1,60 @@
+"""Shapes that divide into nothing, against the float64 oracle: rows that are not multiples of 16 bytes (or of 4, in
+bfloat16), odd channel counts, odd state sizes, sequences cut into chunks of unequal length."""
+
+import importlib
+import os
+import sys
+
+import numpy as np
+import pytest
+import torch
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+sys.path.insert(0, os.path.dirname(HERE))
+import kla_b200  # noqa: E402
+from oracle import kla_oracle as O  # noqa: E402
+
+ops = importlib.import_module("kalman-linear-attention_b200.ops")
+
+
+
+def _rel(got, ref):
+    ref = torch.as_tensor(np.asarray(ref), dtype=torch.float64)
+    return ((got.detach().double().cpu() - ref).norm() / (ref.norm() + 1e-30)).item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,L,M,S,dtype", [
+    (1, 1037, 33, 16, torch.float32),    # 16 chunks of 80 steps, the last one 77 short; odd channels
+    (2, 129, 1001, 16, torch.float32),   # two chunks, 80 + 49
+    (1, 65, 7, 16, torch.float32),       # one chunk of 64 steps would leave a step over
+    (3, 200, 35, 16, torch.bfloat16),    # bfloat16 rows off every 4-byte boundary
+    (2, 77, 34, 24, torch.bfloat16),     # even bfloat16 rows, padded states
+    (2, 150, 19, 40, torch.float32),     # k, q of wide states, S not a power of two
+    (1, 90, 9, 100, torch.float32),
+])
+def test_ragged_shapes_match_the_oracle(B, L, M, S, dtype):
+    g = torch.Generator().manual_seed(B * L + M)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    F = torch.nn.functional
+    ins = [rn(B, L, M), 1 / F.softplus(rn(B, L, M)), F.normalize(rn(B, L, S), dim=-1), F.normalize(rn(B, L, S), dim=-1)]
+    ins = [t.to(dtype).float() for t in ins] + [torch.sigmoid(rn(M, S)), F.softplus(rn(M, S))]
+    dy, dyv, dlam, deta = rn(B, L, M), rn(B, L, M), rn(B, M, S), rn(B, M, S)
+    n = lambda t: t.double().numpy()
+    f = O.scan_fwd(*map(n, ins))
+    b = O.scan_bwd(*map(n, ins), n(dy), n(dyv), None, None, n(dlam), n(deta))
+    dev = [t.to("cuda", dtype if i < 4 else torch.float32).requires_grad_() for i, t in enumerate(ins)]
+    y, y_var, st = kla_b200.kla_scan_b200(*dev)
+    grads = torch.autograd.grad([y, y_var, st.lam, st.eta], dev, [t.cuda() for t in (dy, dyv, dlam, deta)])
+    for name, got, ref in (("y", y, f.y), ("y_var", y_var, f.y_var), ("lam", st.lam, f.lam), ("eta", st.eta, f.eta)):
+        assert _rel(got, ref) < 2e-6, name
+    for name, got in zip(("dv", "dlambda_v", "dk", "dq", "da", "dp"), grads):
+        assert _rel(got, getattr(b, name)) < (2e-5 if got.dtype == torch.float32 else 4e-3), name
+
+
+def test_chunks_cover_every_length():
+    for L in list(range(1, 300)) + [1040, 1501, 4096, 65537]:
+        for B, M in ((1, 16), (2, 1000), (1, 3000)):
+            c = ops.pick_time_chunks(B, L, M, 16)
+            n = ops._chunk_len(L, c)
+            assert (c - 1) * n < L <= c * n and (c == 1 or n >= 64), (L, c, n)
