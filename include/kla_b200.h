@@ -417,6 +417,35 @@ typedef struct kla_b200_step_layer_args {
 int kla_b200_step_layer(const kla_b200_step_layer_args *args, void *stream);
 
 /*
+ * A projection of single-token decode with its neighbours: out = f(norm(x) W^T + bias) + residual for up to
+ * KLA_B200_LINEAR_MAX_ROWS rows of bfloat16, float32 accumulation, one rounding at the store. Replaces, for one token,
+ * nn.Linear with the RMSNorm before it (src/kla/layers/common.py:45-55) and what follows it: the causal convolution's
+ * step on the first conv_D outputs (common.py:87-96, as kla_b200_conv_step), silu(gate) * up (common.py:99-122: weight's
+ * first N/2 rows are the gate, the others up, out has N/2 columns), or the block's residual sum
+ * (src/kla/models/sequence_model.py:47-98). x and weight are 16-byte aligned, K and x_stride_b multiples of 8.
+ */
+#define KLA_B200_LINEAR_MAX_ROWS 64
+typedef struct kla_b200_linear_args {
+    int64_t B, N, K;
+    const void *x;              /* in  [B, K] */
+    int64_t x_stride_b;
+    const void *weight, *bias;  /* in  [N, K] contiguous; [N] or NULL */
+    void *out;                  /* out [B, N], or [B, N/2] with swiglu */
+    int64_t out_stride_b;
+    const void *norm_weight;    /* in  [K]: x is RMS-normalised first; NULL: taken as it is */
+    float norm_eps;
+    int32_t swiglu;
+    const void *residual;       /* in  added to the result, shape of out; NULL: none */
+    int64_t residual_stride_b;
+    int64_t conv_D, conv_taps;  /* conv_D = 0: no convolution */
+    int32_t conv_activation;    /* KLA_B200_ACT_* */
+    const float *conv_weight, *conv_bias; /* [conv_D, conv_taps]; [conv_D] or NULL */
+    void *conv_state;           /* in/out [B, conv_D, conv_taps-1] bfloat16 contiguous */
+} kla_b200_linear_args;
+
+int kla_b200_linear(const kla_b200_linear_args *args, void *stream);
+
+/*
  * Raw scan pair over materialised coefficients. Replaces the reference's
  * tiled_mobius_scan(A, B, C, D, lam0) and tiled_affine_scan(alpha, r)
  * (src/kla/ops/kernels/triton/tiled_mobius_scan.py:301-311) and their exact

@@ -31,6 +31,7 @@ SYMBOLS = (
     "kla_b200_conv_seq",
     "kla_b200_conv_seq_bwd",
     "kla_b200_step_layer",
+    "kla_b200_linear",
     "kla_b200_mobius_scan_fwd",
     "kla_b200_mobius_scan_bwd",
     "kla_b200_affine_scan_fwd",
@@ -239,7 +240,7 @@ def load() -> ctypes.CDLL:
 _host = None
 _HOST_ENTRIES = (
     "scan_fwd", "scan_bwd", "slab_aggregate", "chunk_fold", "epilogue_bwd", "step", "conv_step", "step_layer",
-    "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
+    "linear", "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
     "ckpt_bytes", "segment_scratch_bytes", "strerror",
 )
 

@@ -11,6 +11,7 @@
 #include "kla_decode.cuh"
 #include "kla_epilogue.cuh"
 #include "kla_launch.cuh"
+#include "kla_linear.cuh"
 #include "kla_rawscan.cuh"
 #include "kla_slab.cuh"
 #include "kla_step.cuh"
@@ -32,6 +33,23 @@ const bool g_no_tma = [] { const char *e = getenv("KLA_B200_NO_TMA"); return e &
 int cuda_fail(cudaError_t e) {
     g_last_cuda = e;
     return KLA_B200_ECUDA;
+}
+
+// A launch that may start before the kernel in front of it has ended (programmatic dependent launch): the kernel itself
+// waits (grid_dep_wait) before it touches anything that kernel could have written.
+template <typename Params>
+cudaError_t launch_dependent(void (*kern)(const Params), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const Params &prm) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, prm);
 }
 
 Tensor3 t3(const kla_b200_tensor3 &t) { return Tensor3{t.ptr, t.stride_b, t.stride_t}; }
@@ -389,9 +407,8 @@ int launch_step_layer(const StepLayerParams &prm, cudaStream_t st) {
     const long long threads = (long long)prm.B * prm.M * LPC;
     if ((threads + 127) / 128 > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;  // grid.x limit
     const unsigned blocks = (unsigned)((threads + 127) / 128);
-    kla_step_layer_kernel<T, TO, LPC, PRIOR><<<blocks, 128, 0, st>>>(prm);
+    const cudaError_t e = launch_dependent(kla_step_layer_kernel<T, TO, LPC, PRIOR>, dim3(blocks), 128, 0, st, prm);
     g_launches++;
-    cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
 }
 int dispatch_step_layer(int din, int dout, bool prior, int lpc, const StepLayerParams &prm, cudaStream_t st) {
@@ -442,6 +459,30 @@ int launch_rawscan(const kla_b200_rawscan_args *a, void *stream, bool takes_stat
     g_launches++;
     e = cudaGetLastError();
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+
+template <int NT, int MODE, bool NORM>
+int launch_linear(const LinearParams &prm, cudaStream_t st) {
+    auto kern = kla_linear_kernel<NT, MODE, NORM>;
+    const size_t smem = kLinearRedBytes<NT, MODE> + (NORM ? linear_norm_bytes(NT, prm.K) : 0);
+    if (smem > 200 * 1024) return KLA_B200_EUNSUPPORTED;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e);
+    const int n_out = MODE == kLinearSwiglu ? prm.N / 2 : prm.N;
+    // A CTA per tile up to two per SM, which is what fits; beyond (a language model's head) a CTA walks several tiles, the
+    // next one's W on its way while it adds up the last one, and normalises x once.
+    constexpr int rows = MODE == kLinearSwiglu ? 16 : 16 * kLinearTiles<NT, MODE>;
+    const int tiles = (n_out + rows - 1) / rows;
+    e = launch_dependent(kern, dim3((unsigned)(tiles < 296 ? tiles : 296)), kLinearWarps * 32, smem, st, prm);
+    g_launches++;
+    return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+template <int NT>
+int dispatch_linear(const LinearParams &prm, int mode, cudaStream_t st) {
+    const bool norm = prm.norm_w != nullptr;
+    if (mode == kLinearSwiglu) return norm ? launch_linear<NT, kLinearSwiglu, true>(prm, st) : launch_linear<NT, kLinearSwiglu, false>(prm, st);
+    if (mode == kLinearConv) return norm ? launch_linear<NT, kLinearConv, true>(prm, st) : launch_linear<NT, kLinearConv, false>(prm, st);
+    return norm ? launch_linear<NT, kLinearPlain, true>(prm, st) : launch_linear<NT, kLinearPlain, false>(prm, st);
 }
 }  // namespace
 
@@ -817,6 +858,35 @@ int kla_b200_conv_seq_bwd(const kla_b200_conv_seq_bwd_args *a, void *stream) {
     g_launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+
+int kla_b200_linear(const kla_b200_linear_args *a, void *stream) {
+    if (a == nullptr || a->B < 0 || a->N < 0 || a->K < 0) return KLA_B200_EINVAL;
+    if (a->B > KLA_B200_LINEAR_MAX_ROWS || a->N > (1 << 30) || a->K > (1 << 20) || a->K % 8 || a->x_stride_b % 8) return KLA_B200_EUNSUPPORTED;
+    if (a->B == 0 || a->N == 0) return KLA_B200_OK;
+    if (a->K == 0 || !a->x || !a->weight || !a->out || a->x_stride_b < 0 || a->out_stride_b < 0) return KLA_B200_EINVAL;
+    if (!aligned(a->x, 16) || !aligned(a->weight, 16) || (a->norm_weight && !aligned(a->norm_weight, 16)) || !aligned(a->out, 2)) return KLA_B200_EALIGN;
+    if (a->swiglu && (a->N % 2 || a->conv_D)) return KLA_B200_EINVAL;
+    LinearParams prm{};
+    prm.B = (int)a->B; prm.N = (int)a->N; prm.K = (int)a->K;
+    prm.x = static_cast<const __nv_bfloat16 *>(a->x); prm.x_sb = a->x_stride_b;
+    prm.w = static_cast<const __nv_bfloat16 *>(a->weight); prm.bias = static_cast<const __nv_bfloat16 *>(a->bias);
+    prm.out = static_cast<__nv_bfloat16 *>(a->out); prm.out_sb = a->out_stride_b;
+    prm.norm_w = static_cast<const __nv_bfloat16 *>(a->norm_weight); prm.norm_eps = a->norm_eps;
+    prm.res = static_cast<const __nv_bfloat16 *>(a->residual); prm.res_sb = a->residual_stride_b;
+    if (a->conv_D) {
+        if (a->conv_D < 0 || a->conv_D > a->N || a->conv_taps < 1 || a->conv_taps > KLA_B200_MAX_CONV_TAPS) return KLA_B200_EUNSUPPORTED;
+        if (!a->conv_weight || (a->conv_taps > 1 && !a->conv_state)) return KLA_B200_EINVAL;
+        if (a->conv_activation < KLA_B200_ACT_SILU || a->conv_activation > KLA_B200_ACT_NONE) return KLA_B200_EINVAL;
+        prm.D = (int)a->conv_D; prm.taps = (int)a->conv_taps; prm.conv_act = a->conv_activation;
+        prm.conv_w = a->conv_weight; prm.conv_b = a->conv_bias; prm.conv_state = static_cast<__nv_bfloat16 *>(a->conv_state);
+    }
+    const int mode = a->swiglu ? kLinearSwiglu : a->conv_D ? kLinearConv : kLinearPlain;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (a->B <= 8) return dispatch_linear<1>(prm, mode, st);
+    if (a->B <= 16) return dispatch_linear<2>(prm, mode, st);
+    if (a->B <= 32) return dispatch_linear<4>(prm, mode, st);
+    return dispatch_linear<8>(prm, mode, st);
 }
 
 int kla_b200_step_layer(const kla_b200_step_layer_args *a, void *stream) {

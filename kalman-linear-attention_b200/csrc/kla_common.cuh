@@ -364,6 +364,11 @@ __device__ __forceinline__ void bulk_load_1d(void *dst, const void *src, uint32_
         : "memory");
 }
 
+// Programmatic dependent launch: the next kernel of the stream may be scheduled / the kernel before has ended and its
+// writes are visible. Both do nothing in a kernel launched the ordinary way.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Named barrier over a subset of the CTA's warps (id 1..15).
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

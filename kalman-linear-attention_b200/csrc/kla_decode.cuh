@@ -192,6 +192,8 @@ __global__ void __launch_bounds__(128) kla_step_layer_kernel(const StepLayerPara
     const bool row_live = bm < (long long)prm.B * M;
     const int b = row_live ? (int)(bm / M) : 0, m = row_live ? (int)(bm % M) : 0;
 
+    grid_dep_launch();
+    grid_dep_wait();  // launched before the sensor projection's kernel has ended
     // this lane's four k, q values and its share of their squared norms
     const T *kb = static_cast<const T *>(prm.k) + (long long)b * prm.k_sb;
     const T *qb = static_cast<const T *>(prm.q) + (long long)b * prm.q_sb;

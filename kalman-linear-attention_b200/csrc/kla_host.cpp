@@ -35,6 +35,7 @@ struct Entry {
     int (*step)(const kla_b200_step_args *, void *) = nullptr;
     int (*conv_step)(const kla_b200_conv_step_args *, void *) = nullptr;
     int (*step_layer)(const kla_b200_step_layer_args *, void *) = nullptr;
+    int (*linear)(const kla_b200_linear_args *, void *) = nullptr;
     int (*conv_seq)(const kla_b200_conv_seq_args *, void *) = nullptr;
     int (*conv_seq_bwd)(const kla_b200_conv_seq_bwd_args *, void *) = nullptr;
     int (*rawscan[4])(const kla_b200_rawscan_args *, void *) = {};  // Moebius forward, backward, affine forward, backward
@@ -57,6 +58,7 @@ void bind(const py::dict &d) {
     take(lib.step, d, "kla_b200_step");
     take(lib.conv_step, d, "kla_b200_conv_step");
     take(lib.step_layer, d, "kla_b200_step_layer");
+    take(lib.linear, d, "kla_b200_linear");
     take(lib.conv_seq, d, "kla_b200_conv_seq");
     take(lib.conv_seq_bwd, d, "kla_b200_conv_seq_bwd");
     take(lib.rawscan[0], d, "kla_b200_mobius_scan_fwd");
@@ -363,6 +365,55 @@ int act_code(const py::object &name) {  // the activation's name in a config, or
     throw py::key_error(s);
 }
 
+// Whether kla_b200_linear takes the projection: a few bfloat16 rows, nothing to differentiate, vectors aligned; with a norm
+// the normalised rows must fit shared memory.
+bool few_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const OptTensor &norm_w) {
+    const int64_t K = w.size(1);
+    auto plain = [](const Tensor &t) { return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.is_cuda(); };
+    return x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.size(0) >= 1 && x.size(0) <= KLA_B200_LINEAR_MAX_ROWS && x.stride(1) == 1 &&
+           x.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && K % 8 == 0 && plain(w) &&
+           reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0 && (!bias || plain(*bias)) &&
+           (!norm_w || (plain(*norm_w) && reinterpret_cast<uintptr_t>(norm_w->data_ptr()) % 16 == 0 &&
+                        (x.size(0) + 7) / 8 * 16 * (K + 8) <= 128 * 1024)) &&
+           !wants_grad({&x, &w}) && sm100(x.device());
+}
+
+struct Extra {  // what kla_b200_linear does besides the projection
+    const OptTensor &norm_w;
+    double norm_eps = 0.0;
+    OptTensor residual;
+    bool swiglu = false;
+    kla_b200_linear_args conv{};  // its conv_* fields
+};
+
+Tensor linear_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const Extra &e) {
+    Tensor out = at::empty({x.size(0), e.swiglu ? w.size(0) / 2 : w.size(0)}, x.options());
+    kla_b200_linear_args l = e.conv;
+    l.B = x.size(0); l.N = w.size(0); l.K = w.size(1);
+    l.x = x.data_ptr(); l.x_stride_b = x.stride(0);
+    l.weight = w.data_ptr(); l.bias = bias ? bias->data_ptr() : nullptr;
+    l.out = out.data_ptr(); l.out_stride_b = out.stride(0);
+    l.norm_weight = e.norm_w ? e.norm_w->data_ptr() : nullptr; l.norm_eps = (float)e.norm_eps;
+    l.swiglu = e.swiglu;
+    if (e.residual) { l.residual = e.residual->data_ptr(); l.residual_stride_b = e.residual->stride(0); }
+    check(lib.linear(&l, stream_of(x)));
+    return out;
+}
+
+Tensor rms_norm(const Tensor &x, const Tensor &w, double eps) {  // RMSNorm, src/kla/layers/common.py:45-55
+    const Tensor xf = x.to(at::kFloat);
+    return (xf * at::rsqrt(xf.pow(2).mean(-1, true) + eps) * w.to(at::kFloat)).to(x.scalar_type());
+}
+
+// norm (when norm_w is given), projection, residual sum (when given)
+Tensor project(const Tensor &x, const Tensor &w, const OptTensor &bias, const OptTensor &norm_w, double eps, const OptTensor &residual) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    if (few_rows(x, w, bias, norm_w) && (!residual || (residual->scalar_type() == at::kBFloat16 && residual->stride(-1) == 1)))
+        return linear_rows(x, w, bias, Extra{norm_w, eps, residual});
+    const Tensor out = at::linear(norm_w ? rms_norm(x, *norm_w, eps) : x, w, bias);
+    return residual ? *residual + out : out;
+}
+
 struct Weights {  // a layer's weights by name; what a dict does not hold is absent
     const py::dict &d;
     Tensor at(const char *name) const { return d[name].cast<Tensor>(); }
@@ -370,27 +421,59 @@ struct Weights {  // a layer's weights by name; what a dict does not hold is abs
         const PyObject *o = PyDict_GetItemString(d.ptr(), name);
         return o ? OptTensor(py::handle(const_cast<PyObject *>(o)).cast<Tensor>()) : OptTensor();
     }
-    Tensor linear(const Tensor &x, const char *w, const char *b) const { return at::linear(x, at(w), get(b)); }
+    Tensor linear(const Tensor &x, const char *w, const char *b) const { return project(x, at(w), get(b), {}, 0.0, {}); }
 };
 
-// One token of a layer (LayerDecoder.step): three projections, the convolution's step and the fused filter step. conv_state
+// x + mlp(norm(x)) of one token (src/kla/layers/common.py:99-122): w12, w3 of a swiglu MLP
+Tensor swiglu_step(const Tensor &x, const Tensor &norm_w_, double eps, const Tensor &w12, const OptTensor &b12, const Tensor &w3,
+                   const OptTensor &b3) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const OptTensor norm_w = norm_w_;
+    Tensor h;
+    if (few_rows(x, w12, b12, norm_w) && w12.size(0) % 2 == 0) {
+        Extra e{norm_w, eps};
+        e.swiglu = true;
+        h = linear_rows(x, w12, b12, e);
+    } else {
+        const auto gu = at::linear(rms_norm(x, norm_w_, eps), w12, b12).chunk(2, -1);
+        h = at::silu(gu[0]) * gu[1];
+    }
+    return project(h, w3, b3, {}, 0.0, x);
+}
+
+// One token of a layer (LayerDecoder.step), with the block's norm before it and its residual sum after it when norm_w is given
+// (ModelDecoder): three projections, the convolution's step and the fused filter step. conv_state
 // (absent without a convolution), lam and eta are updated in place. Returns the layer's output and the gated variance, which
 // a config that returns variances projects as well.
 std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, const Tensor &x, const OptTensor &conv_state,
                                       const Tensor &lam, const Tensor &eta, const Tensor &a_bar, const Tensor &p_bar,
                                       const OptTensor &skip, const OptTensor &conv_w, const OptTensor &conv_b, int64_t w_value,
-                                      int64_t w_var) {
+                                      int64_t w_var, const OptTensor &norm_w, double norm_eps) {
     const c10::cuda::CUDAGuard guard(x.device());
     const Weights w{w_};
     void *stream = stream_of(x);
     const int64_t B = x.size(0), M = a_bar.size(0), S = a_bar.size(1);
     const int32_t type = dt(x.scalar_type());
-    const Tensor projected = w.linear(x, "in_proj.weight", "in_proj.bias");
     const bool gated = cfg["use_gating"].cast<bool>();
+    const Tensor in_w = w.at("in_proj.weight");
+    const OptTensor in_b = w.get("in_proj.bias");
+    const bool fused = few_rows(x, in_w, in_b, norm_w);  // the convolution's step then rides on the projection
+    Tensor projected;
+    if (fused) {
+        Extra e{norm_w, norm_eps};
+        if (conv_w) {
+            e.conv.conv_D = M; e.conv.conv_taps = conv_w->size(1); e.conv.conv_activation = act_code(cfg["conv_activation"]);
+            e.conv.conv_weight = fp(*conv_w); e.conv.conv_bias = fp(conv_b);
+            e.conv.conv_state = conv_state ? conv_state->data_ptr() : nullptr;
+        }
+        projected = linear_rows(x, in_w, in_b, e);
+    } else {
+        projected = at::linear(norm_w ? rms_norm(x, *norm_w, norm_eps) : x, in_w, in_b);
+    }
     Tensor z = gated ? projected.narrow(1, 0, M) : projected;
     OptTensor gate;
     if (gated) gate = projected.narrow(1, M, projected.size(1) - M);
-    if (conv_w) {
+    if (conv_w && !fused) {
         Tensor zc = at::empty({B, M}, x.options());
         kla_b200_conv_step_args c{};
         c.B = B; c.D = M; c.K = cfg["conv_kernel_size"].cast<int64_t>(); c.dtype = type;
@@ -427,7 +510,7 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     s.lambda_skip = fp(skip); s.a = fp(a_bar); s.p = fp(p_bar); s.lam = fp(lam); s.eta = fp(eta);
     s.y = y.data_ptr(); s.y_var = yv.data_ptr(); s.lam_out = fp(lam); s.eta_out = fp(eta);
     check(lib.step_layer(&s, stream));
-    return {w.linear(y, "out_proj.weight", "out_proj.bias"), yv};
+    return {project(y, w.at("out_proj.weight"), w.get("out_proj.bias"), {}, 0.0, norm_w ? OptTensor(x) : OptTensor()), yv};
 }
 
 }  // namespace
@@ -448,4 +531,6 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("rawscan", &rawscan);
     m.def("step", &step);
     m.def("layer_step", &layer_step);
+    m.def("project", &project);
+    m.def("swiglu_step", &swiglu_step);
 }

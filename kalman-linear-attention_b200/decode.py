@@ -14,6 +14,9 @@ reference package at run time; ``LayerDecoder.from_layer`` reads both off a refe
 
 from __future__ import annotations
 
+import contextlib
+import threading
+
 import torch
 import torch.nn.functional as F
 
@@ -161,6 +164,14 @@ class LayerDecoder:
             return (out, F.linear(y_var, self.w["out_proj.weight"].pow(2))), state
         return out, state
 
+    def block_step(self, x: torch.Tensor, state, norm_weight: torch.Tensor, norm_eps: float) -> torch.Tensor:
+        """``x + step(rms_norm(x), state)``: a block's mixer half for one token (the mean path of a layer that returns
+        variances, src/kla/models/sequence_model.py:47-98)."""
+        conv_state, lam, eta = state
+        return _lib.host().layer_step(self.w, self.cfg, x, conv_state, lam, eta, self.a_bar, self.p_bar, self.skip,
+                                      self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var, norm_weight,
+                                      norm_eps)[0]
+
     def step(self, x: torch.Tensor, state):
         """One token. ``x``: [B, d_model]; ``state``: the tuple of ``init_state``, updated in place.
         Returns ``out`` [B, d_model], or ``(out, out_var)`` when the config returns variances."""
@@ -170,10 +181,60 @@ class LayerDecoder:
             raise NotImplementedError(f"The b200 decode kernels take float32 or bfloat16 activations, not {x.dtype}.")
         conv_state, lam, eta = state
         out, y_var = _lib.host().layer_step(self.w, self.cfg, x, conv_state, lam, eta, self.a_bar, self.p_bar, self.skip,
-                                            self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var)
+                                            self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var, None, 0.0)
         if self.cfg["return_variance"]:
             return out, F.linear(y_var, self.w["out_proj.weight"].pow(2))
         return out
+
+
+class _TokenGraph:
+    """The decode step of a :class:`ModelDecoder` captured once: state, token and logits buffers and the graph that
+    advances them by one token."""
+
+    def __init__(self, dec: "ModelDecoder", batch: int, device, dtype, greedy: bool):
+        self.state = dec.init_state(batch, device, dtype)
+        self.token = torch.zeros(batch, device=device, dtype=torch.long)
+        self.done = None  # recorded behind the last use
+        side = torch.cuda.Stream(device)
+        side.wait_stream(torch.cuda.current_stream(device))
+        with torch.cuda.stream(side):  # libraries set themselves up outside the capture
+            dec.step(self.token, self.state).argmax(dim=-1)
+        torch.cuda.current_stream(device).wait_stream(side)
+        self.graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(self.graph):
+            self.logits = dec.step(self.token, self.state)
+            if greedy:
+                self.token.copy_(self.logits.argmax(dim=-1))
+
+    def reset(self):
+        """The prior state, ordered behind whatever used the buffers last."""
+        if self.done is not None:
+            torch.cuda.current_stream(self.token.device).wait_event(self.done)
+        for conv, lam, eta in self.state:
+            if conv is not None:
+                conv.zero_()
+            lam.fill_(1.0)
+            eta.zero_()
+        return self.state
+
+    def release(self):
+        self.done = torch.cuda.Event()
+        self.done.record(torch.cuda.current_stream(self.token.device))
+
+
+class _GraphSlot:
+    """One captured decode step kept for the next call with the same batch, types and weights. A call that finds the slot
+    taken (another thread generates) captures a step of its own. Copies of a decoder start with an empty slot."""
+
+    def __init__(self):
+        self.lock = threading.Lock()
+        self.key = self.graph = None
+
+    def __deepcopy__(self, memo):
+        return _GraphSlot()
+
+    def __reduce__(self):
+        return _GraphSlot, ()
 
 
 MODEL_KEYS = ("n_layers", "norm_eps", "mlp", "logit_softcap")
@@ -208,7 +269,7 @@ class ModelDecoder:
             pre = f"blocks.{i}.mixer."
             lw = {k[len(pre):]: v for k, v in weights.items() if k.startswith(pre)}
             self.layers.append(LayerDecoder(lw, layer_configs[i]))
-        self._graph = None
+        self._slot = _GraphSlot()
 
     @classmethod
     def from_model(cls, model) -> "ModelDecoder":
@@ -225,7 +286,7 @@ class ModelDecoder:
         out.__dict__.update(self.__dict__)
         out.w = {k: v.to(device) for k, v in self.w.items()}
         out.layers = [layer.to(device) for layer in self.layers]
-        out._graph = None
+        out._slot = _GraphSlot()
         return out
 
     def init_state(self, batch: int, device, dtype=torch.float32):
@@ -245,14 +306,30 @@ class ModelDecoder:
                         self.w[pre + "w2.weight"], self.w.get(pre + "w2.bias"))
 
     def _head(self, x):
-        logits = F.linear(self._norm(x, "norm_f"), self.w["lm_head.weight"])
+        return self._cap(F.linear(self._norm(x, "norm_f"), self.w["lm_head.weight"]))
+
+    def _cap(self, logits):
         cap = self.cfg["logit_softcap"]
         return logits if cap is None else cap * torch.tanh(logits / cap)
 
-    def _blocks(self, x, state, prompt: bool):
+    def _step_blocks(self, x, state):
+        """One token through the blocks: norm, mixer and residual sum of a block are the layer's step with the norm folded
+        into its first projection and the sum into its last; the MLP likewise."""
+        host, w, eps = _lib.host(), self.w, self.cfg["norm_eps"]
         for i, layer in enumerate(self.layers):
-            h = self._norm(x, f"blocks.{i}.mixer_norm")
-            mixed = layer.prefill(h, state[i])[0] if prompt else layer.step(h, state[i])
+            pre = f"blocks.{i}."
+            x = layer.block_step(x, state[i], w[pre + "mixer_norm.weight"], eps)
+            if self.cfg["mlp"] == "swiglu":
+                m = pre + "mlp."
+                x = host.swiglu_step(x, w[pre + "mlp_norm.weight"], eps, w[m + "w12.weight"], w.get(m + "w12.bias"),
+                                     w[m + "w3.weight"], w.get(m + "w3.bias"))
+            elif self.cfg["mlp"] != "none":
+                x = x + self._mlp(i, self._norm(x, pre + "mlp_norm"))
+        return x
+
+    def _prompt_blocks(self, x, state):
+        for i, layer in enumerate(self.layers):
+            mixed = layer.prefill(self._norm(x, f"blocks.{i}.mixer_norm"), state[i])[0]
             if isinstance(mixed, tuple):  # a layer that returns variances: the mean path (sequence_model.py:85-86)
                 mixed = mixed[0]
             x = x + mixed
@@ -266,13 +343,13 @@ class ModelDecoder:
         x = F.embedding(input_ids, self.w["embedding.weight"])
         if state is None:
             state = self.init_state(x.shape[0], x.device, x.dtype)
-        return self._head(self._blocks(x, state, prompt=True)), state
+        return self._head(self._prompt_blocks(x, state)), state
 
     @torch.no_grad()
     def step(self, token: torch.Tensor, state):
         """One token per sequence: ``token`` [B] -> logits [B, vocab]; ``state`` is updated in place."""
-        x = F.embedding(token, self.w["embedding.weight"])
-        return self._head(self._blocks(x, state, prompt=False))
+        x = self._step_blocks(F.embedding(token, self.w["embedding.weight"]), state)
+        return self._cap(_lib.host().project(x, self.w["lm_head.weight"], None, self.w["norm_f.weight"], self.cfg["norm_eps"], None))
 
     @torch.no_grad()
     def generate(self, input_ids: torch.Tensor, max_new_tokens: int, temperature: float = 0.0, top_k=None,
@@ -280,38 +357,55 @@ class ModelDecoder:
         """``SequenceModel.generate`` (sequence_model.py:200-220): prefill, then one token at a time from the
         recurrent state. ``temperature <= 0`` is greedy. With ``use_graph`` the per-token work of all layers is
         one CUDA graph replay; sampling happens between replays, on the device."""
-        logits, state = self.prefill(input_ids)
-        token = self._sample(logits[:, -1], temperature, top_k)
-        out = [input_ids, token]
-        if max_new_tokens <= 1:
-            return torch.cat(out, dim=1)
-        tok_buf = token[:, 0].clone()
-        graph = None
-        if use_graph:
-            side = torch.cuda.Stream()
-            side.wait_stream(torch.cuda.current_stream())
-            snapshot = [[None if t is None else t.clone() for t in st] for st in state]
-            with torch.cuda.stream(side):  # warm-up on a side stream, as graph capture requires
-                for _ in range(2):
-                    self.step(tok_buf, state)
-            torch.cuda.current_stream().wait_stream(side)
-            for st, snap in zip(state, snapshot):  # the warm-up advanced the state: put it back
-                for t, s_ in zip(st, snap):
-                    if t is not None:
-                        t.copy_(s_)
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
-                logits_buf = self.step(tok_buf, state)
-        for _ in range(max_new_tokens - 1):
-            if graph is not None:
-                graph.replay()
-                logits = logits_buf
+        x = F.embedding(input_ids, self.w["embedding.weight"])
+        B, P = input_ids.shape
+        greedy = temperature <= 0
+        graph_ctx = self._token_graph(B, x.device, x.dtype, greedy) if use_graph and max_new_tokens > 1 else contextlib.nullcontext()
+        with graph_ctx as graph:
+            state = graph.reset() if graph is not None else self.init_state(B, x.device, x.dtype)
+            last = self._prompt_blocks(x, state)[:, -1]  # the prompt's other logits are not needed
+            token = self._sample(self._head(last), temperature, top_k)
+            if max_new_tokens <= 1:
+                return torch.cat((input_ids, token), dim=1)
+            out = torch.empty(B, P + max_new_tokens, device=x.device, dtype=input_ids.dtype)
+            out[:, :P] = input_ids
+            out[:, P] = token[:, 0]
+            tok_buf = token[:, 0].clone() if graph is None else graph.token.copy_(token[:, 0])
+            for i in range(P + 1, P + max_new_tokens):
+                if graph is None:
+                    tok_buf.copy_(self._sample(self.step(tok_buf, state), temperature, top_k)[:, 0])
+                else:
+                    graph.graph.replay()
+                    if not greedy:
+                        tok_buf.copy_(self._sample(graph.logits, temperature, top_k)[:, 0])
+                out[:, i] = tok_buf
+        return out
+
+    @contextlib.contextmanager
+    def _token_graph(self, batch: int, device, dtype, greedy: bool):
+        """The captured decode step for this batch: the kept one when it fits and is free, else a new one."""
+        weights = [t for d in (self.w, *(layer.w for layer in self.layers)) for t in d.values()]
+        key = (batch, device, dtype, greedy, torch.is_autocast_enabled("cuda"), tuple(t.data_ptr() for t in weights),
+               dict(self.cfg), [(dict(layer.cfg), layer.a_bar.data_ptr(), layer.p_bar.data_ptr()) for layer in self.layers])
+        slot = self._slot
+        kept = slot.lock.acquire(blocking=False)
+        try:
+            if kept and slot.key == key:
+                graph = slot.graph
             else:
-                logits = self.step(tok_buf, state)
-            token = self._sample(logits, temperature, top_k)
-            tok_buf.copy_(token[:, 0])
-            out.append(token)
-        return torch.cat(out, dim=1)
+                if kept and slot.graph is not None:
+                    slot.graph.done.synchronize()  # its buffers go back to the allocator: nothing may still read them
+                    slot.key = slot.graph = None
+                graph = _TokenGraph(self, batch, device, dtype, greedy)
+                if kept:
+                    slot.key, slot.graph = key, graph
+            try:
+                yield graph
+            finally:
+                graph.release()
+        finally:
+            if kept:
+                slot.lock.release()
 
     @staticmethod
     def _sample(logits, temperature, top_k):  # sequence_model.py:222-234

@@ -1,0 +1,74 @@
+"""The decode projections (norm, convolution step, swiglu and residual folded in) against plain float32 torch."""
+
+import importlib
+import os
+import sys
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+sys.path.insert(0, os.path.dirname(HERE))
+import kla_b200  # noqa: E402,F401
+
+pytestmark = pytest.mark.gpu
+lib = importlib.import_module("kalman-linear-attention_b200._lib")
+decode = importlib.import_module("kalman-linear-attention_b200.decode")
+
+
+def close(got, want):
+    assert got.dtype == torch.bfloat16 and got.shape == want.shape
+    torch.testing.assert_close(got.float(), want, rtol=1e-2, atol=1e-2 * want.abs().mean().item())
+
+
+def norm(x, w, eps):
+    x = x.float()
+    return (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w.float()).bfloat16().float()
+
+
+# rows around the groups of eight, K with a part of a 32-column block, N with a part of a 16-row tile and beyond one pass
+@pytest.mark.parametrize("B,N,K", [(1, 1, 8), (7, 33, 40), (8, 64, 256), (9, 130, 264), (17, 48, 1024), (33, 100, 72), (64, 4096, 512),
+                                   (3, 9500, 64)])
+def test_projection_with_norm_bias_and_residual(B, N, K):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, b, nw, res = rn(B, K + 8)[:, :K], rn(N, K) * K ** -0.5, rn(N), rn(K), rn(B, N)
+    n0 = lib.load().kla_b200_launch_count()
+    close(lib.host().project(x, w, None, None, 0.0, None), F.linear(x.float(), w.float()))
+    close(lib.host().project(x, w, b, nw, 1e-6, res), F.linear(norm(x, nw, 1e-6), w.float(), b.float()) + res.float())
+    assert lib.load().kla_b200_launch_count() - n0 == 2
+
+
+@pytest.mark.parametrize("B,H,K", [(2, 24, 40), (8, 2048, 768), (20, 40, 256), (40, 33, 512)])
+def test_swiglu_step(B, H, K):
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, nw, w12, w3 = rn(B, K), rn(K), rn(2 * H, K) * K ** -0.5, rn(K, H) * H ** -0.5
+    gate, up = F.linear(norm(x, nw, 1e-5), w12.float()).chunk(2, dim=-1)
+    close(lib.host().swiglu_step(x, nw, 1e-5, w12, None, w3, None), x.float() + F.linear((F.silu(gate) * up).bfloat16().float(), w3.float()))
+
+
+@pytest.mark.parametrize("B,d", [(1, 64), (11, 48), (64, 128)])
+def test_layer_token_in_bfloat16_follows_float32(B, d):
+    """The fused token of a bfloat16 layer against the same layer in float32, whose route is the library's GEMMs and the
+    convolution and filter kernels one by one."""
+    M, S, K = 2 * d, 16, 4
+    g = torch.Generator().manual_seed(B)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    w = {"in_proj.weight": rn(2 * M, d) * d ** -0.5, "sensor_proj.weight": rn(2 * M + 2 * S, M) * M ** -0.5,
+         "out_proj.weight": rn(d, M) * M ** -0.5, "conv.weight": rn(M, 1, K) * 0.5, "conv.bias": rn(M) * 0.1, "delta": rn(M, S) - 4,
+         "lambda_log": rn(M, S) * 0.1, "process_noise": torch.full((M, S), 0.01), "lambda_skip": torch.tensor(-1.0)}
+    w = {k: v.bfloat16().float() if k.endswith("proj.weight") else v for k, v in w.items()}
+    cfg = dict(d_state=S, discretization="ou", zero_process_noise=False, clip_value=None, obs_var_min=1e-4, obs_var_max=None,
+               value_rank="full", qk_norm=True, use_conv=True, conv_kernel_size=K, conv_activation="silu", use_gating=True,
+               gating_activation="silu", use_lambda_skip=True, return_variance=False, decode_from_prior=False)
+    f32 = decode.LayerDecoder(w, cfg).to("cuda")
+    b16 = decode.LayerDecoder({k: v.bfloat16() if k.endswith("proj.weight") else v for k, v in w.items()}, cfg).to("cuda")
+    sa, sb = f32.init_state(B, "cuda"), b16.init_state(B, "cuda", torch.bfloat16)
+    for _ in range(5):
+        x = rn(B, d).bfloat16().cuda()
+        want, got = f32.step(x.float(), sa), b16.step(x, sb)
+    torch.testing.assert_close(got.float(), want, rtol=5e-2, atol=3e-2 * want.abs().mean().item() + 1e-2)
+    torch.testing.assert_close(sb[0].float(), sa[0], rtol=2e-2, atol=2e-2)
+    torch.testing.assert_close(sb[1], sa[1], rtol=5e-2, atol=5e-2)
