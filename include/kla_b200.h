@@ -220,7 +220,8 @@ typedef struct kla_b200_slab_args {
     const float *lam0, *eta0;           /* adjoint only; both NULL = unit prior */
     kla_b200_tensor3 dy, dy_var;        /* adjoint only; dy_var.ptr may be NULL */
     float *out;                         /* [B, M, S, 8] float32 */
-    int64_t chunks, chunk_len;          /* as in kla_b200_fwd_args: lam0, eta0 and out are then per entry */
+    int64_t chunks, chunk_len;          /* as in kla_b200_fwd_args: lam0, eta0 and out are then per entry; the record no
+                                         * fold reads (forward: the last chunk's, adjoint: the first's) is not written */
 } kla_b200_slab_args;
 
 int kla_b200_slab_aggregate(const kla_b200_slab_args *args, void *stream);
@@ -271,7 +272,7 @@ int kla_b200_epilogue_bwd(const kla_b200_epilogue_bwd_args *args, void *stream);
  *      the state after the sequence is entry b*C + C-1 of lam_fin / eta_fin.
  * Backward: kla_b200_slab_aggregate (adjoint = 1, lam0 = lam_in, eta0 = eta_in),
  * kla_b200_chunk_fold (adjoint = 1) from the gradient of the returned state
- * (in_a = dlam_fin, in_b = deta_fin, [B, M, S], or both NULL), then
+ * (in_a = dlam_fin, in_b = deta_fin, [B, M, S], or both NULL; lam_in, eta_in: the chunks' start states), then
  * kla_b200_scan_bwd over the B*C entries with dlam_fin / deta_fin = the seeds
  * out_a / out_b; the gradient of the initial state is entry b*C of dlam0 / deta0.
  * The folds run in float64, one thread per (b, m, s).
@@ -282,6 +283,7 @@ typedef struct kla_b200_chunk_fold_args {
     const float *agg;         /* [B*C, M, S, 8] from kla_b200_slab_aggregate */
     const float *in_a, *in_b; /* [B, M, S] or both NULL: (lam0, eta0) / (dlam_fin, deta_fin) */
     float *out_a, *out_b;     /* [B*C, M, S]: (lam_in, eta_in) / (dlam_seed, deta_seed) */
+    const float *lam_in, *eta_in; /* adjoint: the chunks' start states [B*C, M, S]; NULL: taken from the records */
 } kla_b200_chunk_fold_args;
 
 int kla_b200_chunk_fold(const kla_b200_chunk_fold_args *args, void *stream);
@@ -417,14 +419,26 @@ typedef struct kla_b200_step_layer_args {
 int kla_b200_step_layer(const kla_b200_step_layer_args *args, void *stream);
 
 /*
+ * A block's residual sum with the RMSNorm behind it for many rows: sum = x + delta (rounded as stored), out = sum *
+ * rsqrt(mean(sum^2) + eps) * weight (src/kla/models/sequence_model.py:47-98, src/kla/layers/common.py:45-55). delta NULL:
+ * the norm of x alone, sum is not written. And the MLP's out = silu(gate) * up of gate_up [rows, 2 H] (common.py:99-122).
+ * Rows are contiguous and 16-byte aligned, D and H multiples of 8.
+ */
+int kla_b200_add_norm(int64_t rows, int64_t D, int32_t dtype, int32_t weight_dtype, const void *x, const void *delta,
+                      const void *weight, float eps, void *sum, void *out, void *stream);
+int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up, void *out, void *stream);
+
+/*
  * A projection of single-token decode with its neighbours: out = f(norm(x) W^T + bias) + residual for up to
  * KLA_B200_LINEAR_MAX_ROWS rows of bfloat16, float32 accumulation, one rounding at the store. Replaces, for one token,
  * nn.Linear with the RMSNorm before it (src/kla/layers/common.py:45-55) and what follows it: the causal convolution's
  * step on the first conv_D outputs (common.py:87-96, as kla_b200_conv_step), silu(gate) * up (common.py:99-122: weight's
  * first N/2 rows are the gate, the others up, out has N/2 columns), or the block's residual sum
- * (src/kla/models/sequence_model.py:47-98). x and weight are 16-byte aligned, K and x_stride_b multiples of 8.
+ * (src/kla/models/sequence_model.py:47-98). x and weight are 16-byte aligned, K and x_stride_b multiples of 8; x must
+ * fit shared memory (KLA_B200_LINEAR_SMEM), else KLA_B200_EUNSUPPORTED.
  */
 #define KLA_B200_LINEAR_MAX_ROWS 64
+#define KLA_B200_LINEAR_SMEM (200 * 1024) /* n rows of K + 8 bfloat16 and 1024 (n + 2) bytes must fit: n = B rounded up to 8, 16, 32, 64 */
 typedef struct kla_b200_linear_args {
     int64_t B, N, K;
     const void *x;              /* in  [B, K] */

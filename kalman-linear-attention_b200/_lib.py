@@ -32,6 +32,8 @@ SYMBOLS = (
     "kla_b200_conv_seq_bwd",
     "kla_b200_step_layer",
     "kla_b200_linear",
+    "kla_b200_add_norm",
+    "kla_b200_swiglu",
     "kla_b200_mobius_scan_fwd",
     "kla_b200_mobius_scan_bwd",
     "kla_b200_affine_scan_fwd",
@@ -157,6 +159,7 @@ class ChunkFoldArgs(Structure):
     _fields_ = [
         ("B", c_int64), ("C", c_int64), ("M", c_int64), ("S", c_int64), ("adjoint", c_int32),
         ("agg", c_void_p), ("in_a", c_void_p), ("in_b", c_void_p), ("out_a", c_void_p), ("out_b", c_void_p),
+        ("lam_in", c_void_p), ("eta_in", c_void_p),
     ]
 
 
@@ -240,7 +243,7 @@ def load() -> ctypes.CDLL:
 _host = None
 _HOST_ENTRIES = (
     "scan_fwd", "scan_bwd", "slab_aggregate", "chunk_fold", "epilogue_bwd", "step", "conv_step", "step_layer",
-    "linear", "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
+    "linear", "add_norm", "swiglu", "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
     "ckpt_bytes", "segment_scratch_bytes", "strerror",
 )
 

@@ -85,6 +85,8 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
     const int be = blockIdx.y, m_cta = blockIdx.x * MC;  // be: batch entry, what states and records are indexed by
     const ChunkSpan span = chunk_span(prm.chunk, be, prm.L);
     const int b = span.b, t_off = span.t_off, L = span.L, M = prm.M, S = prm.S;
+    // no fold reads how the last chunk acts on the state, nor how the first acts on the carry
+    if (prm.chunk.n > 1 && be % prm.chunk.n == (ADJ ? 0 : prm.chunk.n - 1)) return;
     const int NT = (L + TT - 1) / TT;
     const bool has_dyv = ADJ && prm.dyv.ptr != nullptr;
 

@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include "../../include/kla_b200.h"
+#include "kla_block.cuh"
 #include "kla_conv_bwd.cuh"
 #include "kla_decode.cuh"
 #include "kla_epilogue.cuh"
@@ -461,28 +462,38 @@ int launch_rawscan(const kla_b200_rawscan_args *a, void *stream, bool takes_stat
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
 }
 
-template <int NT, int MODE, bool NORM>
+template <int NT, int RT, int MODE, bool NORM>
 int launch_linear(const LinearParams &prm, cudaStream_t st) {
-    auto kern = kla_linear_kernel<NT, MODE, NORM>;
-    const size_t smem = kLinearRedBytes<NT, MODE> + (NORM ? linear_norm_bytes(NT, prm.K) : 0);
-    if (smem > 200 * 1024) return KLA_B200_EUNSUPPORTED;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(e);
+    auto kern = kla_linear_kernel<NT, RT, MODE, NORM>;
+    const size_t smem = kLinearRedBytes<NT, RT> + linear_x_bytes(NT, prm.K);
+    if (smem > KLA_B200_LINEAR_SMEM) return KLA_B200_EUNSUPPORTED;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, KLA_B200_LINEAR_SMEM);
+        if (e != cudaSuccess) return cuda_fail(e);
+    }
     const int n_out = MODE == kLinearSwiglu ? prm.N / 2 : prm.N;
-    // A CTA per tile up to two per SM, which is what fits; beyond (a language model's head) a CTA walks several tiles, the
-    // next one's W on its way while it adds up the last one, and normalises x once.
-    constexpr int rows = MODE == kLinearSwiglu ? 16 : 16 * kLinearTiles<NT, MODE>;
+    // A CTA per tile up to two per SM, which is what fits; beyond, a CTA walks several tiles, the next one's W on its way
+    // while it adds up the last one.
+    constexpr int rows = MODE == kLinearSwiglu ? 16 : 16 * RT;
     const int tiles = (n_out + rows - 1) / rows;
-    e = launch_dependent(kern, dim3((unsigned)(tiles < 296 ? tiles : 296)), kLinearWarps * 32, smem, st, prm);
+    const cudaError_t e = launch_dependent(kern, dim3((unsigned)(tiles < 296 ? tiles : 296)), kLinearWarps * 32, smem, st, prm);
     g_launches++;
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+// Tiles of W per CTA: one while x is small beside them or the tiles would not fill the SMs, else two, since every CTA
+// brings in all of x.
+template <int NT, int MODE, bool NORM>
+int dispatch_linear_tiles(const LinearParams &prm, cudaStream_t st) {
+    if constexpr (MODE == kLinearSwiglu) return launch_linear<NT, 2, MODE, NORM>(prm, st);
+    else if constexpr (NT < 4) return launch_linear<NT, 1, MODE, NORM>(prm, st);
+    else return prm.N > 16 * 148 ? launch_linear<NT, 2, MODE, NORM>(prm, st) : launch_linear<NT, 1, MODE, NORM>(prm, st);
 }
 template <int NT>
 int dispatch_linear(const LinearParams &prm, int mode, cudaStream_t st) {
     const bool norm = prm.norm_w != nullptr;
-    if (mode == kLinearSwiglu) return norm ? launch_linear<NT, kLinearSwiglu, true>(prm, st) : launch_linear<NT, kLinearSwiglu, false>(prm, st);
-    if (mode == kLinearConv) return norm ? launch_linear<NT, kLinearConv, true>(prm, st) : launch_linear<NT, kLinearConv, false>(prm, st);
-    return norm ? launch_linear<NT, kLinearPlain, true>(prm, st) : launch_linear<NT, kLinearPlain, false>(prm, st);
+    if (mode == kLinearSwiglu) return norm ? dispatch_linear_tiles<NT, kLinearSwiglu, true>(prm, st) : dispatch_linear_tiles<NT, kLinearSwiglu, false>(prm, st);
+    if (mode == kLinearConv) return norm ? dispatch_linear_tiles<NT, kLinearConv, true>(prm, st) : dispatch_linear_tiles<NT, kLinearConv, false>(prm, st);
+    return norm ? dispatch_linear_tiles<NT, kLinearPlain, true>(prm, st) : dispatch_linear_tiles<NT, kLinearPlain, false>(prm, st);
 }
 }  // namespace
 
@@ -720,11 +731,12 @@ int kla_b200_chunk_fold(const kla_b200_chunk_fold_args *a, void *stream) {
     if (a == nullptr || a->B < 0 || a->C < 1 || a->M < 0 || a->S < 0) return KLA_B200_EINVAL;
     if (a->S > KLA_B200_MAX_DSTATE || a->B * a->C > 65535 || a->M > (1 << 30)) return KLA_B200_EUNSUPPORTED;
     if (a->B == 0 || a->M == 0 || a->S == 0) return KLA_B200_OK;
-    if (!a->agg || !a->out_a || !a->out_b || (a->in_a == nullptr) != (a->in_b == nullptr)) return KLA_B200_EINVAL;
+    if (!a->agg || !a->out_a || !a->out_b || (a->in_a == nullptr) != (a->in_b == nullptr) || (a->lam_in == nullptr) != (a->eta_in == nullptr))
+        return KLA_B200_EINVAL;
     if (!aligned(a->agg, 16)) return KLA_B200_EALIGN;
     ChunkFoldParams prm{};
     prm.B = (int)a->B; prm.C = (int)a->C; prm.M = (int)a->M; prm.S = (int)a->S;
-    prm.agg = a->agg; prm.in_a = a->in_a; prm.in_b = a->in_b; prm.out_a = a->out_a; prm.out_b = a->out_b;
+    prm.agg = a->agg; prm.in_a = a->in_a; prm.in_b = a->in_b; prm.lam_in = a->lam_in; prm.eta_in = a->eta_in; prm.out_a = a->out_a; prm.out_b = a->out_b;
     const long long lanes = a->B * a->M * a->S;
     const unsigned blocks = (unsigned)((lanes + 127) / 128);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -857,6 +869,45 @@ int kla_b200_conv_seq_bwd(const kla_b200_conv_seq_bwd_args *a, void *stream) {
 #undef KLA_CONV_BWD_LAUNCH
     g_launches++;
     cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+
+int kla_b200_add_norm(int64_t rows, int64_t D, int32_t dtype, int32_t weight_dtype, const void *x, const void *delta, const void *weight,
+                      float eps, void *sum, void *out, void *stream) {
+    if (rows < 0 || D < 0) return KLA_B200_EINVAL;
+    if (D % 8 || D > (1 << 30) || rows > (1ll << 32)) return KLA_B200_EUNSUPPORTED;
+    if (rows == 0 || D == 0) return KLA_B200_OK;
+    if (!x || !weight || !out || (delta && !sum)) return KLA_B200_EINVAL;
+    for (const void *p : {x, delta, weight, static_cast<const void *>(sum), static_cast<const void *>(out)})
+        if (p && !aligned(p, 16)) return KLA_B200_EALIGN;
+    const AddNormParams prm{(int)rows, (int)D, x, delta, weight, sum, out, eps};
+    const unsigned grid = (unsigned)((rows + 3) / 4);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const bool b = dtype == KLA_B200_BF16, wb = weight_dtype == KLA_B200_BF16;
+    if (b && wb) kla_add_norm_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 128, 0, st>>>(prm);
+    else if (b) kla_add_norm_kernel<__nv_bfloat16, float><<<grid, 128, 0, st>>>(prm);
+    else if (wb) kla_add_norm_kernel<float, __nv_bfloat16><<<grid, 128, 0, st>>>(prm);
+    else kla_add_norm_kernel<float, float><<<grid, 128, 0, st>>>(prm);
+    g_launches++;
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+
+int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up, void *out, void *stream) {
+    if (rows < 0 || H < 0) return KLA_B200_EINVAL;
+    if (H % 8 || H > (1 << 29) || rows > (1ll << 31)) return KLA_B200_EUNSUPPORTED;
+    if (rows == 0 || H == 0) return KLA_B200_OK;
+    if (!gate_up || !out) return KLA_B200_EINVAL;
+    if (!aligned(gate_up, 16) || !aligned(out, 16)) return KLA_B200_EALIGN;
+    const long long blocks = (rows * (H / 8) + 255) / 256;
+    if (blocks > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (dtype == KLA_B200_BF16)
+        kla_swiglu_kernel<<<(unsigned)blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(gate_up), static_cast<__nv_bfloat16 *>(out), rows, (int)H);
+    else
+        kla_swiglu_kernel<<<(unsigned)blocks, 256, 0, st>>>(static_cast<const float *>(gate_up), static_cast<float *>(out), rows, (int)H);
+    g_launches++;
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
 }
 

@@ -41,7 +41,9 @@ __device__ __forceinline__ float activate_slope_fast(float x, int act) {
         const float s = rcp_approx(1.0f + __expf(-x));
         return s * fmaf(x, 1.0f - s, 1.0f);
     }
-    return activate_slope(x, act);
+    float g, slope;
+    activate_with_slope(x, act, g, slope);
+    return slope;
 }
 
 template <typename T, int VEC, int KT>

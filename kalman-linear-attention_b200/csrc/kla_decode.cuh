@@ -192,8 +192,40 @@ __global__ void __launch_bounds__(128) kla_step_layer_kernel(const StepLayerPara
     const bool row_live = bm < (long long)prm.B * M;
     const int b = row_live ? (int)(bm / M) : 0, m = row_live ? (int)(bm % M) : 0;
 
+    // a, p before the wait for the sensor projection's kernel, everything that can have been written since the launch
+    // right after it, so that the arithmetic below waits for memory once
+    const long long ms0 = (long long)m * S + j * 4, bms0 = ((long long)b * M + m) * S + j * 4;
+    // lanes wholly past the row (j * 4 >= S, e.g. S = 12 with LPC = 4) hold padding chains and touch no memory
+    const bool vec = prm.vec != 0, lane_live = row_live && j * 4 < S;
+    float lamv[4] = {1.0f, 1.0f, 1.0f, 1.0f}, etav[4] = {}, av[4] = {}, pv[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+    auto load4 = [&](float (&x)[4], const float *src) {
+        if (vec) {
+            const float4 f = *reinterpret_cast<const float4 *>(src);
+            x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (j * 4 + i < S) x[i] = src[i];
+        }
+    };
     grid_dep_launch();
-    grid_dep_wait();  // launched before the sensor projection's kernel has ended
+    if (lane_live) {
+        load4(av, prm.a + ms0);
+        load4(pv, prm.p + ms0);
+    }
+    grid_dep_wait();
+    if (lane_live) {
+        load4(lamv, prm.lam + bms0);
+        load4(etav, prm.eta + bms0);
+    }
+    T lsv = from_f32<T>(0.0f), vv = lsv, zv = lsv, gv = lsv;
+    const bool has_z = prm.skip != nullptr && prm.z != nullptr, has_gate = prm.gate != nullptr;
+    if (row_live) {
+        lsv = static_cast<const T *>(prm.ls)[(long long)b * prm.ls_sb + m];
+        vv = static_cast<const T *>(prm.v)[(long long)b * prm.v_sb + m];
+        if (has_z) zv = static_cast<const T *>(prm.z)[(long long)b * prm.z_sb + m];
+        if (has_gate) gv = static_cast<const T *>(prm.gate)[(long long)b * prm.gate_sb + m];
+    }
     // this lane's four k, q values and its share of their squared norms
     const T *kb = static_cast<const T *>(prm.k) + (long long)b * prm.k_sb;
     const T *qb = static_cast<const T *>(prm.q) + (long long)b * prm.q_sb;
@@ -232,34 +264,9 @@ __global__ void __launch_bounds__(128) kla_step_layer_kernel(const StepLayerPara
     if (row_live) {
         // observation-noise variance -> value precision, kla_layer.py:224-231
         const float lv = precision_from_log_variance(
-            to_f32<T>(static_cast<const T *>(prm.ls)[(long long)b * prm.ls_sb + m]), prm.obs_var_min, prm.obs_var_max);
-        const float vl = to_f32<T>(static_cast<const T *>(prm.v)[(long long)b * prm.v_sb + m]) * lv;
-        const long long ms0 = (long long)m * S + j * 4, bms0 = ((long long)b * M + m) * S + j * 4;
-        // lanes wholly past the row (j * 4 >= S, e.g. S = 12 with LPC = 4) hold padding chains and touch no memory
-        const bool vec = prm.vec != 0, lane_live = j * 4 < S;
-        float lamv[4], etav[4], av[4], pv[4], lo[4], eo[4];
-        if (!lane_live) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { lamv[i] = 1.0f; etav[i] = 0.0f; av[i] = 0.0f; pv[i] = 1.0f; }
-        } else if (vec) {
-            const float4 l4 = *reinterpret_cast<const float4 *>(prm.lam + bms0);
-            const float4 e4 = *reinterpret_cast<const float4 *>(prm.eta + bms0);
-            const float4 a4 = *reinterpret_cast<const float4 *>(prm.a + ms0);
-            const float4 p4 = *reinterpret_cast<const float4 *>(prm.p + ms0);
-            lamv[0] = l4.x; lamv[1] = l4.y; lamv[2] = l4.z; lamv[3] = l4.w;
-            etav[0] = e4.x; etav[1] = e4.y; etav[2] = e4.z; etav[3] = e4.w;
-            av[0] = a4.x; av[1] = a4.y; av[2] = a4.z; av[3] = a4.w;
-            pv[0] = p4.x; pv[1] = p4.y; pv[2] = p4.z; pv[3] = p4.w;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const bool in = j * 4 + i < S;
-                lamv[i] = in ? prm.lam[bms0 + i] : 1.0f;
-                etav[i] = in ? prm.eta[bms0 + i] : 0.0f;
-                av[i] = in ? prm.a[ms0 + i] : 0.0f;
-                pv[i] = in ? prm.p[ms0 + i] : 1.0f;
-            }
-        }
+            to_f32<T>(lsv), prm.obs_var_min, prm.obs_var_max);
+        const float vl = to_f32<T>(vv) * lv;
+        float lo[4], eo[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const bool in = j * 4 + i < S;
@@ -304,12 +311,9 @@ __global__ void __launch_bounds__(128) kla_step_layer_kernel(const StepLayerPara
     }
     if (row_live && j == 0) {
         // kla_layer.py:329-338: skip path, then the gate on the mean and its square on the variance
-        if (prm.skip != nullptr && prm.z != nullptr) {
-            const float sk = prm.skip[prm.skip_len > 1 ? m : 0];
-            ys = fmaf(sk, to_f32<T>(static_cast<const T *>(prm.z)[(long long)b * prm.z_sb + m]), ys);
-        }
-        if (prm.gate != nullptr) {
-            const float g = activate(to_f32<T>(static_cast<const T *>(prm.gate)[(long long)b * prm.gate_sb + m]), prm.gate_act);
+        if (has_z) ys = fmaf(prm.skip[prm.skip_len > 1 ? m : 0], to_f32<T>(zv), ys);
+        if (has_gate) {
+            const float g = activate(to_f32<T>(gv), prm.gate_act);
             ys *= g;
             yvs *= g * g;
         }

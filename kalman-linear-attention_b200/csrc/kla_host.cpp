@@ -9,6 +9,7 @@
 // which sends the wrapper to its general path with its error messages.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/utils/pybind.h>
@@ -36,6 +37,8 @@ struct Entry {
     int (*conv_step)(const kla_b200_conv_step_args *, void *) = nullptr;
     int (*step_layer)(const kla_b200_step_layer_args *, void *) = nullptr;
     int (*linear)(const kla_b200_linear_args *, void *) = nullptr;
+    int (*add_norm)(int64_t, int64_t, int32_t, int32_t, const void *, const void *, const void *, float, void *, void *, void *) = nullptr;
+    int (*swiglu)(int64_t, int64_t, int32_t, const void *, void *, void *) = nullptr;
     int (*conv_seq)(const kla_b200_conv_seq_args *, void *) = nullptr;
     int (*conv_seq_bwd)(const kla_b200_conv_seq_bwd_args *, void *) = nullptr;
     int (*rawscan[4])(const kla_b200_rawscan_args *, void *) = {};  // Moebius forward, backward, affine forward, backward
@@ -59,6 +62,8 @@ void bind(const py::dict &d) {
     take(lib.conv_step, d, "kla_b200_conv_step");
     take(lib.step_layer, d, "kla_b200_step_layer");
     take(lib.linear, d, "kla_b200_linear");
+    take(lib.add_norm, d, "kla_b200_add_norm");
+    take(lib.swiglu, d, "kla_b200_swiglu");
     take(lib.conv_seq, d, "kla_b200_conv_seq");
     take(lib.conv_seq_bwd, d, "kla_b200_conv_seq_bwd");
     take(lib.rawscan[0], d, "kla_b200_mobius_scan_fwd");
@@ -89,7 +94,12 @@ float *fp(const OptTensor &t) { return t ? fp(*t) : nullptr; }
 int32_t dt(at::ScalarType t) { return t == at::kBFloat16 ? KLA_B200_BF16 : KLA_B200_F32; }
 at::ScalarType out_type(bool bf16) { return bf16 ? at::kBFloat16 : at::kFloat; }
 void *stream_of(const Tensor &t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
-Tensor f32(const Tensor &like, at::IntArrayRef sizes) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
+// An uninitialised contiguous tensor on like's device, straight from the CUDA allocator (no dispatch).
+Tensor fresh(const Tensor &like, at::IntArrayRef sizes, at::ScalarType type) {
+    return Tensor(at::detail::empty_cuda(sizes, type, like.device(), std::nullopt));
+}
+Tensor fresh(const Tensor &like, at::IntArrayRef sizes) { return fresh(like, sizes, like.scalar_type()); }
+Tensor f32(const Tensor &like, at::IntArrayRef sizes) { return fresh(like, sizes, at::kFloat); }
 
 struct Sensors {
     bool on = false;
@@ -141,16 +151,16 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> scan_fwd(
     int64_t chunk_len) {
     const c10::cuda::CUDAGuard guard(v.device());
     const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2), E = B * chunks;
-    const auto opt = v.options().dtype(out_type(out_bf16)), bytes = v.options().dtype(at::kByte);
-    Tensor y = at::empty({B, L, M}, opt), yv = at::empty({B, L, M}, opt);
+    const auto TO = out_type(out_bf16);
+    Tensor y = fresh(v, {B, L, M}, TO), yv = fresh(v, {B, L, M}, TO);
     Tensor lam = f32(v, {E, M, S}), eta = f32(v, {E, M, S});
     OptTensor ckpt, work;
-    if (need_ckpt && L > 0) ckpt = at::empty({(int64_t)lib.ckpt_bytes(E, chunks > 1 ? chunk_len : L, M, S)}, bytes);
-    else if (segments) work = at::empty({(int64_t)lib.segment_scratch_bytes(B, M, S)}, bytes);
+    if (need_ckpt && L > 0) ckpt = fresh(v, {(int64_t)lib.ckpt_bytes(E, chunks > 1 ? chunk_len : L, M, S)}, at::kByte);
+    else if (segments) work = fresh(v, {(int64_t)lib.segment_scratch_bytes(B, M, S)}, at::kByte);
     const Sensors sen(sensors);
     kla_b200_fwd_args f{};
     f.B = B; f.L = L; f.M = M; f.S = S;
-    f.in_dtype = dt(v.scalar_type()); f.out_dtype = dt(opt.dtype().toScalarType()); f.decode_from_prior = prior;
+    f.in_dtype = dt(v.scalar_type()); f.out_dtype = dt(TO); f.decode_from_prior = prior;
     f.v = t3(v); f.lambda_v = t3(lv); f.k = t3(k); f.q = t3(q);
     f.a = fp(a); f.p = fp(p); f.lam0 = fp(lam0); f.eta0 = fp(eta0);
     f.y = t3(y); f.y_var = t3(yv); f.lam_fin = fp(lam); f.eta_fin = fp(eta);
@@ -172,7 +182,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_
     const OptTensor &deta_fin, bool prior, bool out_bf16, const SensorArg &sensors, int64_t chunks, int64_t chunk_len) {
     const c10::cuda::CUDAGuard guard(v.device());
     const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2), E = B * chunks;
-    Tensor dv = at::empty({B, L, M}, v.options()), dlv = at::empty({B, L, M}, v.options());
+    Tensor dv = fresh(v, {B, L, M}), dlv = fresh(v, {B, L, M});
     Tensor dk = f32(v, {B, L, S}), dq = f32(v, {B, L, S}), da = f32(v, {M, S}), dp = f32(v, {M, S});
     Tensor dlam0 = f32(v, {E, M, S}), deta0 = f32(v, {E, M, S});
     const Sensors sen(sensors);
@@ -211,13 +221,14 @@ Tensor slab_aggregate(const Tensor &v, const Tensor &lv, const Tensor &k, const 
 }
 
 // kla_b200_chunk_fold over aggregates [B*C, M, S, 8] -> two [B*C, M, S]
-std::tuple<Tensor, Tensor> chunk_fold(const Tensor &agg, int64_t C, const OptTensor &in_a, const OptTensor &in_b, bool adjoint) {
+std::tuple<Tensor, Tensor> chunk_fold(const Tensor &agg, int64_t C, const OptTensor &in_a, const OptTensor &in_b, const OptTensor &lam_in,
+                                      const OptTensor &eta_in, bool adjoint) {
     const c10::cuda::CUDAGuard guard(agg.device());
     const int64_t E = agg.size(0), M = agg.size(1), S = agg.size(2);
     Tensor out_a = f32(agg, {E, M, S}), out_b = f32(agg, {E, M, S});
     kla_b200_chunk_fold_args c{};
     c.B = E / C; c.C = C; c.M = M; c.S = S; c.adjoint = adjoint;
-    c.agg = fp(agg); c.in_a = fp(in_a); c.in_b = fp(in_b); c.out_a = fp(out_a); c.out_b = fp(out_b);
+    c.agg = fp(agg); c.in_a = fp(in_a); c.in_b = fp(in_b); c.lam_in = fp(lam_in); c.eta_in = fp(eta_in); c.out_a = fp(out_a); c.out_b = fp(out_b);
     check(lib.chunk_fold(&c, stream_of(agg)));
     return {out_a, out_b};
 }
@@ -228,7 +239,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor, Tensor, Tensor> scan_fwd_c
     const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const OptTensor &lam0,
     const OptTensor &eta0, bool prior, bool out_bf16, bool need_ckpt, int64_t chunks, int64_t chunk_len) {
     const Tensor agg = slab_aggregate(v, lv, k, a, p, {}, {}, {}, {}, {}, false, chunks, chunk_len);
-    auto [lam_in, eta_in] = chunk_fold(agg, chunks, lam0, eta0, false);
+    auto [lam_in, eta_in] = chunk_fold(agg, chunks, lam0, eta0, {}, {}, false);
     auto [y, yv, lam, eta, ckpt] = scan_fwd(v, lv, k, q, a, p, lam_in, eta_in, prior, out_bf16, need_ckpt, false, {}, {}, {}, {}, 0, {},
                                             {}, chunks, chunk_len);
     const int64_t B = v.size(0), M = v.size(2), S = k.size(2);
@@ -241,7 +252,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_
     const Tensor &eta_in, const OptTensor &ckpt, const Tensor &dy, const OptTensor &dyv, const OptTensor &dlam_fin,
     const OptTensor &deta_fin, bool prior, bool out_bf16, int64_t chunks, int64_t chunk_len) {
     const Tensor agg = slab_aggregate(v, lv, k, a, p, q, dy, dyv, lam_in, eta_in, prior, chunks, chunk_len);
-    auto [dlam_seed, deta_seed] = chunk_fold(agg, chunks, dlam_fin, deta_fin, true);
+    auto [dlam_seed, deta_seed] = chunk_fold(agg, chunks, dlam_fin, deta_fin, lam_in, eta_in, true);
     auto r = scan_bwd(v, lv, k, q, a, p, lam_in, eta_in, ckpt, dy, dyv, dlam_seed, deta_seed, prior, out_bf16, {}, chunks, chunk_len);
     const int64_t B = v.size(0), M = v.size(2), S = k.size(2);
     auto first = [&](const Tensor &t) { return t.view({B, chunks, M, S}).select(1, 0); };
@@ -257,15 +268,15 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> epilogue_bwd(const T
                                                                         const OptTensor &gate, const OptTensor &skip, int gate_act) {
     const c10::cuda::CUDAGuard guard(v.device());
     const int64_t B = v.size(0), L = v.size(1), M = v.size(2);
-    const auto opt = v.options().dtype(out_type(out_bf16));
-    Tensor dy = at::empty({B, L, M}, opt), dyv = at::empty({B, L, M}, opt);
+    const auto TO = out_type(out_bf16);
+    Tensor dy = fresh(v, {B, L, M}, TO), dyv = fresh(v, {B, L, M}, TO);
     OptTensor dz, dgate, dskip;
-    if (z) dz = at::empty({B, L, M}, v.options());
-    if (gate) dgate = at::empty({B, L, M}, v.options());
+    if (z) dz = fresh(v, {B, L, M});
+    if (gate) dgate = fresh(v, {B, L, M});
     if (skip) dskip = at::empty_like(*skip);
     kla_b200_epilogue_bwd_args e{};
     e.B = B; e.L = L; e.M = M;
-    e.in_dtype = dt(v.scalar_type()); e.out_dtype = dt(opt.dtype().toScalarType());
+    e.in_dtype = dt(v.scalar_type()); e.out_dtype = dt(TO);
     e.gate_activation = gate ? gate_act : KLA_B200_ACT_NONE;
     e.lambda_skip_len = skip ? (int32_t)skip->numel() : 0;
     e.dout = t3(dout); e.dout_var = t3(dout_var); e.y_raw = t3(y_raw); e.y_var_raw = t3(yv_raw);
@@ -279,7 +290,7 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> epilogue_bwd(const T
 std::tuple<Tensor, Tensor> conv_seq(const Tensor &x, const Tensor &w, const OptTensor &bias, const Tensor &state, int act) {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t B = x.size(0), L = x.size(1), D = x.size(2);
-    Tensor z = at::empty({B, L, D}, x.options()), next = at::empty_like(state);
+    Tensor z = fresh(x, {B, L, D}), next = fresh(state, state.sizes());
     kla_b200_conv_seq_args c{};
     c.B = B; c.L = L; c.D = D; c.K = w.size(1); c.dtype = dt(x.scalar_type()); c.activation = act;
     c.x = t3(x); c.weight = fp(w); c.bias = fp(bias); c.state = state.data_ptr(); c.state_out = next.data_ptr(); c.z = t3(z);
@@ -292,7 +303,7 @@ std::tuple<Tensor, Tensor, OptTensor> conv_seq_bwd(const Tensor &x, const Tensor
                                                    const Tensor &state, int act) {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t B = x.size(0), L = x.size(1), D = x.size(2), K = w.size(1);
-    Tensor dx = at::empty({B, L, D}, x.options());
+    Tensor dx = fresh(x, {B, L, D});
     Tensor sums = at::zeros({bias ? D * (K + 1) : D * K}, x.options().dtype(at::kFloat));  // dweight, then dbias
     Tensor dw = sums.narrow(0, 0, D * K).view({D, K});
     OptTensor db;
@@ -344,7 +355,7 @@ py::object step(const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor
     if (wants_grad({&v, &lv, &k, &q, &a, &p, &lam, &eta})) return py::none();
     const c10::cuda::CUDAGuard guard(v.device());
     Tensor y = f32(v, {B, M}), yv = f32(v, {B, M});
-    Tensor lo = inplace ? lam : at::empty_like(lam), eo = inplace ? eta : at::empty_like(eta);
+    Tensor lo = inplace ? lam : f32(lam, lam.sizes()), eo = inplace ? eta : f32(eta, eta.sizes());
     kla_b200_step_args s{};
     s.B = B; s.M = M; s.S = S;
     s.in_dtype = dt(T); s.out_dtype = KLA_B200_F32; s.decode_from_prior = prior;
@@ -369,12 +380,16 @@ int act_code(const py::object &name) {  // the activation's name in a config, or
 // the normalised rows must fit shared memory.
 bool few_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const OptTensor &norm_w) {
     const int64_t K = w.size(1);
+    auto fits = [K](int64_t rows) {  // KLA_B200_LINEAR_SMEM
+        int64_t n = 8;
+        while (n < rows) n *= 2;
+        return n * (K + 8) * 2 + 1024 * (n + 2) <= KLA_B200_LINEAR_SMEM;
+    };
     auto plain = [](const Tensor &t) { return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.is_cuda(); };
     return x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.size(0) >= 1 && x.size(0) <= KLA_B200_LINEAR_MAX_ROWS && x.stride(1) == 1 &&
            x.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && K % 8 == 0 && plain(w) &&
            reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0 && (!bias || plain(*bias)) &&
-           (!norm_w || (plain(*norm_w) && reinterpret_cast<uintptr_t>(norm_w->data_ptr()) % 16 == 0 &&
-                        (x.size(0) + 7) / 8 * 16 * (K + 8) <= 128 * 1024)) &&
+           (!norm_w || (plain(*norm_w) && reinterpret_cast<uintptr_t>(norm_w->data_ptr()) % 16 == 0)) && fits(x.size(0)) &&
            !wants_grad({&x, &w}) && sm100(x.device());
 }
 
@@ -387,7 +402,7 @@ struct Extra {  // what kla_b200_linear does besides the projection
 };
 
 Tensor linear_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const Extra &e) {
-    Tensor out = at::empty({x.size(0), e.swiglu ? w.size(0) / 2 : w.size(0)}, x.options());
+    Tensor out = fresh(x, {x.size(0), e.swiglu ? w.size(0) / 2 : w.size(0)});
     kla_b200_linear_args l = e.conv;
     l.B = x.size(0); l.N = w.size(0); l.K = w.size(1);
     l.x = x.data_ptr(); l.x_stride_b = x.stride(0);
@@ -405,12 +420,49 @@ Tensor rms_norm(const Tensor &x, const Tensor &w, double eps) {  // RMSNorm, src
     return (xf * at::rsqrt(xf.pow(2).mean(-1, true) + eps) * w.to(at::kFloat)).to(x.scalar_type());
 }
 
+bool vec_rows(const Tensor &t) {  // rows that 16-byte accesses can walk
+    return t.is_cuda() && t.is_contiguous() && (t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kFloat) && t.size(-1) % 8 == 0 &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+}
+
+// x + delta (x itself without delta) and its RMSNorm
+std::tuple<Tensor, Tensor> add_norm(const Tensor &x, const OptTensor &delta, const Tensor &w, double eps) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    if (!vec_rows(x) || !vec_rows(w) || (delta && (!vec_rows(*delta) || delta->scalar_type() != x.scalar_type() || delta->sizes() != x.sizes())) ||
+        wants_grad({&x, &w}) || !sm100(x.device())) {
+        const Tensor sum = delta ? x + *delta : x;
+        return {sum, rms_norm(sum, w, eps)};
+    }
+    Tensor sum = delta ? fresh(x, x.sizes()) : x, out = fresh(x, x.sizes());
+    check(lib.add_norm(x.numel() / x.size(-1), x.size(-1), dt(x.scalar_type()), dt(w.scalar_type()), x.data_ptr(),
+                       delta ? delta->data_ptr() : nullptr, w.data_ptr(), (float)eps, sum.data_ptr(), out.data_ptr(), stream_of(x)));
+    return {sum, out};
+}
+
+// silu(gate) * up of [..., 2 H] rows
+Tensor swiglu(const Tensor &gu) {
+    const c10::cuda::CUDAGuard guard(gu.device());
+    if (!vec_rows(gu) || gu.size(-1) % 16 || wants_grad({&gu}) || !sm100(gu.device())) {
+        const auto halves = gu.chunk(2, -1);
+        return at::silu(halves[0]) * halves[1];
+    }
+    auto sizes = gu.sizes().vec();
+    sizes.back() /= 2;
+    Tensor out = fresh(gu, sizes);
+    check(lib.swiglu(gu.numel() / gu.size(-1), sizes.back(), dt(gu.scalar_type()), gu.data_ptr(), out.data_ptr(), stream_of(gu)));
+    return out;
+}
+
+// A language model's head for a few rows. From this many outputs on the library's GEMM is the better read of W (50304 x 768,
+// eight rows: 8.2 us against 14), and the norm is a launch of its own.
+constexpr int64_t kWideHead = 8192;
+
 // norm (when norm_w is given), projection, residual sum (when given)
 Tensor project(const Tensor &x, const Tensor &w, const OptTensor &bias, const OptTensor &norm_w, double eps, const OptTensor &residual) {
     const c10::cuda::CUDAGuard guard(x.device());
-    if (few_rows(x, w, bias, norm_w) && (!residual || (residual->scalar_type() == at::kBFloat16 && residual->stride(-1) == 1)))
+    if (w.size(0) < kWideHead && few_rows(x, w, bias, norm_w) && (!residual || (residual->scalar_type() == at::kBFloat16 && residual->stride(-1) == 1)))
         return linear_rows(x, w, bias, Extra{norm_w, eps, residual});
-    const Tensor out = at::linear(norm_w ? rms_norm(x, *norm_w, eps) : x, w, bias);
+    const Tensor out = at::linear(norm_w ? std::get<1>(add_norm(x, {}, *norm_w, eps)) : x, w, bias);
     return residual ? *residual + out : out;
 }
 
@@ -435,8 +487,7 @@ Tensor swiglu_step(const Tensor &x, const Tensor &norm_w_, double eps, const Ten
         e.swiglu = true;
         h = linear_rows(x, w12, b12, e);
     } else {
-        const auto gu = at::linear(rms_norm(x, norm_w_, eps), w12, b12).chunk(2, -1);
-        h = at::silu(gu[0]) * gu[1];
+        h = swiglu(at::linear(std::get<1>(add_norm(x, {}, norm_w_, eps)), w12, b12));
     }
     return project(h, w3, b3, {}, 0.0, x);
 }
@@ -451,10 +502,15 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
                                       int64_t w_var, const OptTensor &norm_w, double norm_eps) {
     const c10::cuda::CUDAGuard guard(x.device());
     const Weights w{w_};
+    auto get = [&cfg](const char *name) {
+        PyObject *o = PyDict_GetItemString(cfg.ptr(), name);
+        if (o == nullptr) throw py::key_error(name);
+        return py::reinterpret_borrow<py::object>(o);
+    };
     void *stream = stream_of(x);
     const int64_t B = x.size(0), M = a_bar.size(0), S = a_bar.size(1);
     const int32_t type = dt(x.scalar_type());
-    const bool gated = cfg["use_gating"].cast<bool>();
+    const bool gated = get("use_gating").cast<bool>();
     const Tensor in_w = w.at("in_proj.weight");
     const OptTensor in_b = w.get("in_proj.bias");
     const bool fused = few_rows(x, in_w, in_b, norm_w);  // the convolution's step then rides on the projection
@@ -462,51 +518,68 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     if (fused) {
         Extra e{norm_w, norm_eps};
         if (conv_w) {
-            e.conv.conv_D = M; e.conv.conv_taps = conv_w->size(1); e.conv.conv_activation = act_code(cfg["conv_activation"]);
+            e.conv.conv_D = M; e.conv.conv_taps = conv_w->size(1); e.conv.conv_activation = act_code(get("conv_activation"));
             e.conv.conv_weight = fp(*conv_w); e.conv.conv_bias = fp(conv_b);
             e.conv.conv_state = conv_state ? conv_state->data_ptr() : nullptr;
         }
         projected = linear_rows(x, in_w, in_b, e);
     } else {
-        projected = at::linear(norm_w ? rms_norm(x, *norm_w, norm_eps) : x, in_w, in_b);
+        projected = at::linear(norm_w ? std::get<1>(add_norm(x, {}, *norm_w, norm_eps)) : x, in_w, in_b);
     }
-    Tensor z = gated ? projected.narrow(1, 0, M) : projected;
-    OptTensor gate;
-    if (gated) gate = projected.narrow(1, M, projected.size(1) - M);
+    // z and the gate are halves of the projection, the sensor signals slices of theirs: pointers, not views
+    const int64_t esz = x.element_size();
+    auto part = [esz](const Tensor &t, int64_t column) { return static_cast<char *>(t.data_ptr()) + column * esz; };
+    void *z = projected.data_ptr(), *gate = gated ? part(projected, M) : nullptr;
+    const int64_t gate_row = gated ? projected.stride(0) : 0;
+    int64_t z_row = projected.stride(0);
+    Tensor z_in = gated ? projected.narrow(1, 0, M) : projected;  // what sensor_proj reads
     if (conv_w && !fused) {
-        Tensor zc = at::empty({B, M}, x.options());
+        Tensor zc = fresh(x, {B, M});
         kla_b200_conv_step_args c{};
-        c.B = B; c.D = M; c.K = cfg["conv_kernel_size"].cast<int64_t>(); c.dtype = type;
-        c.activation = act_code(cfg["conv_activation"]);
-        c.x = z.data_ptr(); c.x_stride_b = z.stride(0); c.weight = fp(*conv_w); c.bias = fp(conv_b);
+        c.B = B; c.D = M; c.K = conv_w->size(1); c.dtype = type;
+        c.activation = act_code(get("conv_activation"));
+        c.x = z; c.x_stride_b = z_row; c.weight = fp(*conv_w); c.bias = fp(conv_b);
         c.state = conv_state ? conv_state->data_ptr() : nullptr; c.z = zc.data_ptr();
         check(lib.conv_step(&c, stream));
-        z = zc;
+        z_in = zc;
+        z = zc.data_ptr();
+        z_row = M;
     }
-    const Tensor sens = w.linear(z, "sensor_proj.weight", "sensor_proj.bias");
+    const Tensor sens = w.linear(z_in, "sensor_proj.weight", "sensor_proj.bias");
+    const int64_t row = sens.stride(0);
     // the four sensor signals, raw, as KLALayer._project_sensors splits them (src/kla/layers/kla_layer.py:199-216)
-    const bool from_conv = w_value == 0;
-    Tensor v = from_conv ? z : sens.narrow(1, 0, w_value);
-    if (!from_conv && w_.contains("value_expand.weight")) v = w.linear(v, "value_expand.weight", "value_expand.bias");
-    Tensor ls = sens.narrow(1, w_value, w_var);
-    if (w_.contains("var_expand.weight")) ls = w.linear(ls, "var_expand.weight", "var_expand.bias");
-    const int64_t at_k = (w_value + w_var), row = sens.stride(0), esz = sens.element_size();
-    char *kq = static_cast<char *>(sens.data_ptr()) + at_k * esz;
-    Tensor y = at::empty({B, M}, x.options()), yv = at::empty({B, M}, x.options());
-    const py::object vmax = cfg["obs_var_max"], clip = cfg["clip_value"];
+    void *v = z, *ls = part(sens, w_value), *kq = part(sens, w_value + w_var);
+    int64_t v_row = z_row, ls_row = row;
+    Tensor v_wide, ls_wide;  // low-rank signals, expanded
+    if (w_value != 0) {
+        v = sens.data_ptr();
+        v_row = row;
+        if (w_.contains("value_expand.weight")) {
+            v_wide = w.linear(sens.narrow(1, 0, w_value), "value_expand.weight", "value_expand.bias");
+            v = v_wide.data_ptr();
+            v_row = v_wide.stride(0);
+        }
+    }
+    if (w_.contains("var_expand.weight")) {
+        ls_wide = w.linear(sens.narrow(1, w_value, w_var), "var_expand.weight", "var_expand.bias");
+        ls = ls_wide.data_ptr();
+        ls_row = ls_wide.stride(0);
+    }
+    Tensor y = fresh(x, {B, M}), yv = fresh(x, {B, M});
+    const py::object vmax = get("obs_var_max"), clip = get("clip_value");
     kla_b200_step_layer_args s{};
     s.B = B; s.M = M; s.S = S; s.in_dtype = type; s.out_dtype = type;
-    s.decode_from_prior = cfg["decode_from_prior"].cast<bool>();
-    s.qk_norm = cfg["qk_norm"].cast<bool>();
-    s.gate_activation = gated ? act_code(cfg["gating_activation"]) : KLA_B200_ACT_NONE;
+    s.decode_from_prior = get("decode_from_prior").cast<bool>();
+    s.qk_norm = get("qk_norm").cast<bool>();
+    s.gate_activation = gated ? act_code(get("gating_activation")) : KLA_B200_ACT_NONE;
     s.lambda_skip_len = skip ? (int32_t)skip->numel() : 0;
-    s.obs_var_min = cfg["obs_var_min"].cast<float>();
+    s.obs_var_min = get("obs_var_min").cast<float>();
     s.obs_var_max = vmax.is_none() ? 0.0f : vmax.cast<float>();
     s.clip_value = clip.is_none() ? 0.0f : clip.cast<float>();
-    s.v = v.data_ptr(); s.log_sigma_v = ls.data_ptr(); s.v_stride_b = v.stride(0); s.log_sigma_v_stride_b = ls.stride(0);
-    s.k = kq; s.q = kq + S * esz; s.k_stride_b = row; s.q_stride_b = row;
-    s.z = z.data_ptr(); s.z_stride_b = z.stride(0);
-    s.gate = gate ? gate->data_ptr() : nullptr; s.gate_stride_b = gate ? gate->stride(0) : 0;
+    s.v = v; s.log_sigma_v = ls; s.v_stride_b = v_row; s.log_sigma_v_stride_b = ls_row;
+    s.k = kq; s.q = static_cast<char *>(kq) + S * esz; s.k_stride_b = row; s.q_stride_b = row;
+    s.z = z; s.z_stride_b = z_row;
+    s.gate = gate; s.gate_stride_b = gate_row;
     s.lambda_skip = fp(skip); s.a = fp(a_bar); s.p = fp(p_bar); s.lam = fp(lam); s.eta = fp(eta);
     s.y = y.data_ptr(); s.y_var = yv.data_ptr(); s.lam_out = fp(lam); s.eta_out = fp(eta);
     check(lib.step_layer(&s, stream));
@@ -522,7 +595,6 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("scan_fwd", &scan_fwd);
     m.def("scan_bwd", &scan_bwd);
     m.def("slab_aggregate", &slab_aggregate);
-    m.def("chunk_fold", &chunk_fold);
     m.def("scan_fwd_chunked", &scan_fwd_chunked);
     m.def("scan_bwd_chunked", &scan_bwd_chunked);
     m.def("epilogue_bwd", &epilogue_bwd);
@@ -531,6 +603,8 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("rawscan", &rawscan);
     m.def("step", &step);
     m.def("layer_step", &layer_step);
+    m.def("add_norm", &add_norm);
+    m.def("swiglu", &swiglu);
     m.def("project", &project);
     m.def("swiglu_step", &swiglu_step);
 }

@@ -8,12 +8,14 @@
 // With so few rows the product is a read of W, once, from HBM or L2 (2 to 17 MB per layer and projection: 0.4 to 2.6 us
 // at the measured copy rate), so the kernel is built around having enough of W in flight, not around the tensor cores:
 //   * a CTA owns 16 rows of W; its eight warps take every eighth block of 32 columns and add their partial products
-//     through shared memory, so that N/16 x 8 warps each have up to four 1 KB blocks of W in flight;
+//     through shared memory, so that N/16 x 8 warps each have up to eight 1 KB blocks of W in flight;
 //   * W goes straight from global memory into the A operand of mma.m16n8k16: which column of a block a lane holds does
 //     not matter to the sum as long as x is held the same way, so a lane takes 16 consecutive bytes of a row (two
 //     operands' worth) instead of the four-byte pieces the operand layout names;
-//   * W does not depend on the kernel before, so with programmatic dependent launch its first blocks are requested
-//     before the wait for that kernel.
+//   * W does not depend on the kernel before, so with programmatic dependent launch its first blocks, all of a warp's
+//     share up to K = 2048, are requested before the wait for that kernel;
+//   * x comes into shared memory whole, by one round of asynchronous copies: as operands fetched from L2 beside W it
+//     doubled the loads of 32 rows (B=32: 12 us for a 2064 x 2048 projection that the library does in 5).
 // Measured on B200 against the library's GEMMs, which take 4 to 5.5 us whatever the shape at these sizes:
 // @@LINEAR@@
 #pragma once
@@ -51,33 +53,21 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// 16-row tiles of W per CTA. One while x is small beside them; from 17 rows of x on two, since a CTA reads all of x for
-// every tile's worth of W (at one, 32 rows: 12 us where the library takes 5). With swiglu: the gate's tile and the up's.
-template <int NT, int MODE>
-constexpr int kLinearTiles = MODE == kLinearSwiglu || NT >= 4 ? 2 : 1;
-// blocks of W (and of x) a warp holds in flight: what the registers allow
-template <int NT, int MODE>
-constexpr int kLinearDepth = NT == 8 ? 2 : NT == 1 && kLinearTiles<NT, MODE> == 1 ? 8 : 4;
+// Blocks of W a warp holds in flight: all of K <= 2048 where the registers allow.
+template <int NT, int RT>
+constexpr int kLinearDepth = RT == 1 || NT >= 4 ? 8 : 4;
+// shared memory: partial sums of every warp, then x (normalised with NORM)
+template <int NT, int RT>
+constexpr size_t kLinearRedBytes = sizeof(float) * kLinearWarps * RT * 16 * (NT * 8 + 2);
+inline size_t linear_x_bytes(int nt, int K) { return sizeof(__nv_bfloat16) * nt * 8 * (K + 8); }
 
-// shared memory: partial sums of every warp, then (NORM) the normalised rows
-template <int NT, int MODE>
-constexpr size_t kLinearRedBytes = sizeof(float) * kLinearWarps * kLinearTiles<NT, MODE> * 16 * (NT * 8 + 2);
-inline size_t linear_norm_bytes(int nt, int K) { return sizeof(__nv_bfloat16) * nt * 8 * (K + 8); }
+__device__ __forceinline__ void cp_async_16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 
-// RMSNorm of up to four rows at once (the warp's, W rows apart), so that their loads are in flight together. The first
-// four 16-byte pieces a lane has of a row stay in registers between the two passes (K <= 1024: all of it).
-template <int W, int R>
-__device__ __forceinline__ void norm_rows(const LinearParams &prm, __nv_bfloat16 *xs, int xld, int r0, int lane) {
-    constexpr int C = 4;
-    const int chunks = prm.K / 8;
-    auto at = [&](int i, int c) { return reinterpret_cast<const uint4 *>(prm.x + (long long)(r0 + i * W) * prm.x_sb + c * 8); };
-    uint4 v[R][C];
-    float ss[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < C; ++j)
-            v[i][j] = r0 + i * W < prm.B && lane + 32 * j < chunks ? *at(i, lane + 32 * j) : make_uint4(0, 0, 0, 0);
+// RMSNorm in place of one row of x in shared memory, by one warp; nw: this lane's pieces of the norm's weights.
+template <int C>
+__device__ __forceinline__ void norm_row(uint4 *row, const uint4 (&nw)[C], const __nv_bfloat16 *norm_w, int chunks, int K, float eps, int lane) {
     auto sq = [](const uint4 &x) {
         const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162 *>(&x);
         float t = 0.0f;
@@ -88,55 +78,46 @@ __device__ __forceinline__ void norm_rows(const LinearParams &prm, __nv_bfloat16
         }
         return t;
     };
-    auto scaled = [&](uint4 x, int c, float inv) {
-        const uint4 nw = *reinterpret_cast<const uint4 *>(prm.norm_w + c * 8);
+    float ss = 0.0f;
+    for (int c = lane; c < chunks; c += 32) ss += sq(row[c]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float inv = rsqrtf(ss / (float)K + eps);
+    auto scale = [&](int c, const uint4 &w4) {
+        uint4 x = row[c];
         __nv_bfloat162 *p = reinterpret_cast<__nv_bfloat162 *>(&x);
-        const __nv_bfloat162 *q = reinterpret_cast<const __nv_bfloat162 *>(&nw);
+        const __nv_bfloat162 *q = reinterpret_cast<const __nv_bfloat162 *>(&w4);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float2 f = __bfloat1622float2(p[e]), w = __bfloat1622float2(q[e]);
             p[e] = __floats2bfloat162_rn(f.x * inv * w.x, f.y * inv * w.y);
         }
-        return x;
+        row[c] = x;
     };
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        ss[i] = 0.0f;
-#pragma unroll
-        for (int j = 0; j < C; ++j) ss[i] += sq(v[i][j]);
-        if (r0 + i * W < prm.B)
-            for (int c = lane + 32 * C; c < chunks; c += 32) ss[i] += sq(*at(i, c));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-        if (r0 + i * W >= prm.B) continue;
-        const float inv = rsqrtf(ss[i] / (float)prm.K + prm.norm_eps);
-        uint4 *dst = reinterpret_cast<uint4 *>(xs + (r0 + i * W) * xld);
-#pragma unroll
-        for (int j = 0; j < C; ++j)
-            if (lane + 32 * j < chunks) dst[lane + 32 * j] = scaled(v[i][j], lane + 32 * j, inv);
-        for (int c = lane + 32 * C; c < chunks; c += 32) dst[c] = scaled(*at(i, c), c, inv);
-    }
+    for (int j = 0; j < C; ++j)
+        if (lane + 32 * j < chunks) scale(lane + 32 * j, nw[j]);
+    for (int c = lane + 32 * C; c < chunks; c += 32) scale(c, *reinterpret_cast<const uint4 *>(norm_w + c * 8));
 }
 
-// NT: groups of eight rows of x. MODE: LinearMode. NORM: x is normalised on the way in.
-template <int NT, int MODE, bool NORM>
+// NT: groups of eight rows of x. RT: 16-row tiles of W per CTA; with swiglu the gate's and the up's. NORM: x is normalised
+// on the way in.
+template <int NT, int RT, int MODE, bool NORM>
 __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __grid_constant__ LinearParams prm) {
-    constexpr int W = kLinearWarps, RT = kLinearTiles<NT, MODE>, U = kLinearDepth<NT, MODE>, LD = NT * 8 + 2;
+    constexpr int W = kLinearWarps, U = kLinearDepth<NT, RT>, LD = NT * 8 + 2, NW = 4;
     constexpr bool GLU = MODE == kLinearSwiglu;
+    static_assert(!GLU || RT == 2, "gate and up");
     constexpr int ROWS = GLU ? 16 : 16 * RT;  // outputs per CTA
     extern __shared__ __align__(16) unsigned char smem[];
     float *red = reinterpret_cast<float *>(smem);  // [W][RT * 16][LD]
-    __nv_bfloat16 *xs = reinterpret_cast<__nv_bfloat16 *>(smem + kLinearRedBytes<NT, MODE>);
+    __nv_bfloat16 *xs = reinterpret_cast<__nv_bfloat16 *>(smem + kLinearRedBytes<NT, RT>);  // [B][K + 8]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int B = prm.B, K = prm.K, chunks = K / 8, blocks = (K + 31) / 32;
     const int n_out = GLU ? prm.N / 2 : prm.N;  // outputs per row; with swiglu W's second half is `up`
     const int row_tiles = (n_out + ROWS - 1) / ROWS;
-    const int xld = K + 8;
+    const int xld = K + 8;  // rows 16 bytes off a multiple of 128: the eight rows of a fragment meet different banks
 
-    uint4 wl[U][RT], wh[U][RT], xv[U][NT];
+    uint4 wl[U][RT], wh[U][RT];
     auto load_w = [&](int u, int tile, int kb) {
         const int ch = kb * 4 + t;
 #pragma unroll
@@ -147,29 +128,27 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
             wh[u][h] = ch < chunks && n0 + 8 < n_out ? load_once(base + 8ll * K) : make_uint4(0, 0, 0, 0);
         }
     };
-    auto load_x = [&](int u, int kb) {
-        const int ch = kb * 4 + t;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const int r = min(nt * 8 + g, B - 1);
-            xv[u][nt] = make_uint4(0, 0, 0, 0);
-            if (ch < chunks) xv[u][nt] = NORM ? *reinterpret_cast<const uint4 *>(xs + r * xld + ch * 8)
-                                              : *reinterpret_cast<const uint4 *>(prm.x + (long long)r * prm.x_sb + ch * 8);
-        }
-    };
     grid_dep_launch();
 #pragma unroll
     for (int u = 0; u < U; ++u) load_w(u, blockIdx.x, warp + u * W);
+    uint4 nw[NW];
+    if (NORM) {
+#pragma unroll
+        for (int j = 0; j < NW; ++j)
+            if (lane + 32 * j < chunks) nw[j] = *reinterpret_cast<const uint4 *>(prm.norm_w + (lane + 32 * j) * 8);
+    }
     grid_dep_wait();  // everything below may read what the kernel before wrote
 
+    // all of x into shared memory, one round of asynchronous copies; a warp takes whole rows
+    for (int r = warp; r < B; r += W)
+        for (int c = lane; c < chunks; c += 32) cp_async_16(xs + r * xld + c * 8, prm.x + (long long)r * prm.x_sb + c * 8);
+    cp_async_wait_all();
     if (NORM) {
-        constexpr int R = NT < 4 ? NT : 4;
-#pragma unroll
-        for (int r0 = 0; r0 < NT; r0 += R) norm_rows<W, R>(prm, xs, xld, warp + r0 * W, lane);
-        __syncthreads();
+        __syncwarp();
+        for (int r = warp; r < B; r += W)
+            norm_row<NW>(reinterpret_cast<uint4 *>(xs + r * xld), nw, prm.norm_w, chunks, K, prm.norm_eps, lane);
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) load_x(u, warp + u * W);
+    __syncthreads();
 
     for (int tile = blockIdx.x; tile < row_tiles; tile += gridDim.x) {
         float acc[RT][NT][4] = {};
@@ -177,21 +156,20 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
             const bool last = kb0 + W * U >= blocks;  // of this tile: what follows is the next tile's beginning
 #pragma unroll
             for (int u = 0; u < U; ++u) {
+                const int ch = (kb0 + u * W) * 4 + t;
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
+                for (int nt = 0; nt < NT; ++nt) {
+                    uint4 x = make_uint4(0, 0, 0, 0);
+                    if (ch < chunks) x = *reinterpret_cast<const uint4 *>(xs + min(nt * 8 + g, B - 1) * xld + ch * 8);
 #pragma unroll
                     for (int h = 0; h < RT; ++h) {
-                        mma_16816(acc[h][nt], wl[u][h].x, wh[u][h].x, wl[u][h].y, wh[u][h].y, xv[u][nt].x, xv[u][nt].y);
-                        mma_16816(acc[h][nt], wl[u][h].z, wh[u][h].z, wl[u][h].w, wh[u][h].w, xv[u][nt].z, xv[u][nt].w);
+                        mma_16816(acc[h][nt], wl[u][h].x, wh[u][h].x, wl[u][h].y, wh[u][h].y, x.x, x.y);
+                        mma_16816(acc[h][nt], wl[u][h].z, wh[u][h].z, wl[u][h].w, wh[u][h].w, x.z, x.w);
                     }
-                // the registers just read take what comes U blocks later
-                if (!last) {
-                    load_w(u, tile, kb0 + (U + u) * W);
-                    load_x(u, kb0 + (U + u) * W);
-                } else if (tile + (int)gridDim.x < row_tiles) {
-                    load_w(u, tile + gridDim.x, warp + u * W);
-                    if (blocks > W * U) load_x(u, warp + u * W);  // else they are there already
                 }
+                // the registers just read take what comes U blocks later
+                if (!last) load_w(u, tile, kb0 + (U + u) * W);
+                else if (tile + (int)gridDim.x < row_tiles) load_w(u, tile + gridDim.x, warp + u * W);
             }
         }
 #pragma unroll

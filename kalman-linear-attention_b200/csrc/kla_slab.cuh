@@ -17,13 +17,15 @@ namespace kla {
 //
 //   forward  in:  agg [B*C, M, S, 8] (MODE 0 records), lam0/eta0 [B, M, S] or nullptr
 //            out: lam_in, eta_in [B*C, M, S], the state before each chunk's first step
-//   adjoint  in:  agg [B*C, M, S, 8] (MODE 1 records), dlam_fin/deta_fin [B, M, S] or nullptr
+//   adjoint  in:  agg [B*C, M, S, 8] (MODE 1 records), dlam_fin/deta_fin [B, M, S] or nullptr, lam_in/eta_in as above
+//                 or nullptr: with them the first chunk needs no record (the state it ends in is the second's start)
 //            out: dlam_seed, deta_seed [B*C, M, S]: passed to the backward kernel as the gradient
 //                 of each chunk's returned state, they make it start from the right carry
 struct ChunkFoldParams {
     int B, C, M, S;
     const float *agg;
     const float *in_a, *in_b;
+    const float *lam_in, *eta_in;  // adjoint: [B*C, M, S] start states
     float *out_a, *out_b;
 };
 
@@ -44,7 +46,8 @@ __global__ void __launch_bounds__(128) kla_chunk_fold_kernel(const ChunkFoldPara
     };
     float4 lo[kAhead], hi[kAhead];  // slot i: the i-th record from here in the order of the fold
     auto fetch_nth = [&](int n, float4 &l, float4 &h) {  // record number n in that order (nothing past the last)
-        if (n < C) fetch(ADJ ? C - 1 - n : n, l, h);
+        l = h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (n < (ADJ && (prm.lam_in == nullptr || C == 1) ? C : C - 1)) fetch(ADJ ? C - 1 - n : n, l, h);
     };
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) fetch_nth(i, lo[i], hi[i]);
@@ -87,7 +90,11 @@ __global__ void __launch_bounds__(128) kla_chunk_fold_kernel(const ChunkFoldPara
                 const float4 l = lo[i], h = hi[i];
                 fetch_nth(n + kAhead, lo[i], hi[i]);
                 const long long o = (b * C + (C - 1 - n)) * lanes + ms;
-                const double P_end = h.y, mean_end = h.z;  // record: K00 K01 K11 b0 | b1 P_end mean_end
+                double P_end = h.y, mean_end = h.z;  // record: K00 K01 K11 b0 | b1 P_end mean_end
+                if (n == C - 1 && n > 0 && prm.lam_in != nullptr) {
+                    P_end = 1.0 / (double)prm.lam_in[o + lanes];
+                    mean_end = (double)prm.eta_in[o + lanes] * P_end;
+                }
                 const double deta = cm * P_end;
                 prm.out_b[o] = (float)deta;
                 prm.out_a[o] = (float)(-(cP * P_end * P_end + mean_end * deta));

@@ -293,20 +293,22 @@ class ModelDecoder:
         return [layer.init_state(batch, device, dtype) for layer in self.layers]
 
     def _norm(self, x, name):  # RMSNorm, src/kla/layers/common.py:45-55
-        xf = x.float()
-        xf = xf * torch.rsqrt(xf.pow(2).mean(dim=-1, keepdim=True) + self.cfg["norm_eps"])
-        return (xf * self.w[name + ".weight"].float()).to(x.dtype)
+        return self._add_norm(x, None, name)[1]
+
+    def _add_norm(self, x, delta, name):
+        """``x + delta`` (``x`` itself when ``delta`` is None) and its norm."""
+        return _lib.host().add_norm(x, delta, self.w[name + ".weight"], self.cfg["norm_eps"])
 
     def _mlp(self, i, x):  # src/kla/layers/common.py:99-122
         pre = f"blocks.{i}.mlp."
         if self.cfg["mlp"] == "swiglu":
-            gate, up = F.linear(x, self.w[pre + "w12.weight"], self.w.get(pre + "w12.bias")).chunk(2, dim=-1)
-            return F.linear(F.silu(gate) * up, self.w[pre + "w3.weight"], self.w.get(pre + "w3.bias"))
+            h = _lib.host().swiglu(F.linear(x, self.w[pre + "w12.weight"], self.w.get(pre + "w12.bias")))
+            return F.linear(h, self.w[pre + "w3.weight"], self.w.get(pre + "w3.bias"))
         return F.linear(F.gelu(F.linear(x, self.w[pre + "w1.weight"], self.w.get(pre + "w1.bias"))),
                         self.w[pre + "w2.weight"], self.w.get(pre + "w2.bias"))
 
-    def _head(self, x):
-        return self._cap(F.linear(self._norm(x, "norm_f"), self.w["lm_head.weight"]))
+    def _head(self, x, branch):
+        return self._cap(F.linear(self._add_norm(x, branch, "norm_f")[1], self.w["lm_head.weight"]))
 
     def _cap(self, logits):
         cap = self.cfg["logit_softcap"]
@@ -328,14 +330,18 @@ class ModelDecoder:
         return x
 
     def _prompt_blocks(self, x, state):
+        """A prompt through the blocks, each residual sum together with the norm behind it. Returns the sum and the last
+        branch, still to be added (``_add_norm`` with the final norm, or of the position that is needed)."""
+        branch = None
         for i, layer in enumerate(self.layers):
-            mixed = layer.prefill(self._norm(x, f"blocks.{i}.mixer_norm"), state[i])[0]
-            if isinstance(mixed, tuple):  # a layer that returns variances: the mean path (sequence_model.py:85-86)
-                mixed = mixed[0]
-            x = x + mixed
+            x, h = self._add_norm(x, branch, f"blocks.{i}.mixer_norm")
+            branch = layer.prefill(h, state[i])[0]
+            if isinstance(branch, tuple):  # a layer that returns variances: the mean path (sequence_model.py:85-86)
+                branch = branch[0]
             if self.cfg["mlp"] != "none":
-                x = x + self._mlp(i, self._norm(x, f"blocks.{i}.mlp_norm"))
-        return x
+                x, h = self._add_norm(x, branch, f"blocks.{i}.mlp_norm")
+                branch = self._mlp(i, h)
+        return x, branch
 
     @torch.no_grad()
     def prefill(self, input_ids: torch.Tensor, state=None):
@@ -343,7 +349,7 @@ class ModelDecoder:
         x = F.embedding(input_ids, self.w["embedding.weight"])
         if state is None:
             state = self.init_state(x.shape[0], x.device, x.dtype)
-        return self._head(self._prompt_blocks(x, state)), state
+        return self._head(*self._prompt_blocks(x, state)), state
 
     @torch.no_grad()
     def step(self, token: torch.Tensor, state):
@@ -363,8 +369,9 @@ class ModelDecoder:
         graph_ctx = self._token_graph(B, x.device, x.dtype, greedy) if use_graph and max_new_tokens > 1 else contextlib.nullcontext()
         with graph_ctx as graph:
             state = graph.reset() if graph is not None else self.init_state(B, x.device, x.dtype)
-            last = self._prompt_blocks(x, state)[:, -1]  # the prompt's other logits are not needed
-            token = self._sample(self._head(last), temperature, top_k)
+            # the head sees the last position: the prompt's other logits are not needed
+            last = (None if t is None else t[:, -1].contiguous() for t in self._prompt_blocks(x, state))
+            token = self._sample(self._head(*last), temperature, top_k)
             if max_new_tokens <= 1:
                 return torch.cat((input_ids, token), dim=1)
             out = torch.empty(B, P + max_new_tokens, device=x.device, dtype=input_ids.dtype)

@@ -142,8 +142,7 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
     The kernels put one CTA on every 32 / 16 / 8 ... channels (d_state 16 / 32 / 64 ...) of every batch element.
     When that grid leaves most of the GPU empty, the sequence is cut into C chunks that run as B*C batch entries;
     building the chunks' start states costs about 0.7x of a forward + backward pass on top, so chunking is only
-    chosen when the plain grid fills less than a third of the resident CTA slots; then up to 16 chunks, enough
-    for about four waves of CTAs. Chunks keep at least 64 steps and are equally long where the count divides L, else
+    chosen when the plain grid fills less than a third of the resident CTA slots; then up to 16 chunks. Chunks keep at least 64 steps and are equally long where the count divides L, else
     a multiple of 16 steps with a shorter last one (:func:`_chunk_len`). ``requested`` (or the environment variable
     KLA_B200_TIME_CHUNKS) overrides the choice; it is lowered to the nearest usable divisor of L."""
     import os
@@ -158,8 +157,13 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
     if requested is None:
         if ctas == 0 or 3 * ctas > _RESIDENT_CTAS:
             return 1
-        # measured on B200 (T=4096, M=1024): several waves of short chunks beat one wave of long ones, up to 16 chunks
-        want = min(16, (4 * _RESIDENT_CTAS) // ctas)
+        # Whole rounds of the resident slots: enough chunks for one, more rounds while chunks are longer than about 256
+        # steps, which evens out the last one. Measured on B200, forward / training step in us: B=1 L=1536 M=1536
+        # (48 CTAs) 3 chunks 79 / 233, 4 91 / 287, 6 69 / 208, 8 73 / 227, 16 74 / 235, uncut 108 / 380; B=1 L=8192 M=2048
+        # (64 CTAs) 4 chunks 431 / 1367, 16 355 / 1154.
+        rounds = 1
+        while (want := min(16, rounds * _RESIDENT_CTAS // ctas)) < 16 and L > 288 * want:
+            rounds += 1
     else:
         want = max(1, int(requested))
     want = min(want, max(1, L // _MIN_CHUNK_STEPS), max(1, 65535 // max(B, 1)))

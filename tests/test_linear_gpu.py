@@ -29,7 +29,7 @@ def norm(x, w, eps):
 
 # rows around the groups of eight, K with a part of a 32-column block, N with a part of a 16-row tile and beyond one pass
 @pytest.mark.parametrize("B,N,K", [(1, 1, 8), (7, 33, 40), (8, 64, 256), (9, 130, 264), (17, 48, 1024), (33, 100, 72), (64, 4096, 512),
-                                   (3, 9500, 64)])
+                                   (3, 8000, 64)])
 def test_projection_with_norm_bias_and_residual(B, N, K):
     g = torch.Generator(device="cuda").manual_seed(N)
     rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
@@ -72,3 +72,21 @@ def test_layer_token_in_bfloat16_follows_float32(B, d):
     torch.testing.assert_close(got.float(), want, rtol=5e-2, atol=3e-2 * want.abs().mean().item() + 1e-2)
     torch.testing.assert_close(sb[0].float(), sa[0], rtol=2e-2, atol=2e-2)
     torch.testing.assert_close(sb[1], sa[1], rtol=5e-2, atol=5e-2)
+
+
+# a row within the registers, across them, and one that does not divide into vectors
+@pytest.mark.parametrize("rows,D", [(1, 8), (5, 768), (33, 1032), (7, 4096), (4, 36)])
+@pytest.mark.parametrize("dtype,wtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+def test_residual_sum_norm_and_gate(rows, D, dtype, wtype):
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, d, w = rn(2, rows, D).to(dtype), rn(2, rows, D).to(dtype), rn(D).to(wtype)
+    tol = dict(rtol=1e-2, atol=1e-2) if dtype == torch.bfloat16 else dict(rtol=2e-6, atol=2e-6)
+    for delta in (None, d):
+        s, out = lib.host().add_norm(x, delta, w, 1e-6)
+        want = x if delta is None else x + d
+        assert torch.equal(s, want)
+        ref = want.double() * torch.rsqrt(want.double().pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+        torch.testing.assert_close(out.double(), ref, **tol)
+    a, b = x.double().chunk(2, dim=-1)
+    torch.testing.assert_close(lib.host().swiglu(x).double(), F.silu(a) * b, **tol)
