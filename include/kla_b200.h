@@ -437,8 +437,8 @@ int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up,
  * (src/kla/models/sequence_model.py:47-98). x and weight are 16-byte aligned, K and x_stride_b multiples of 8; x must
  * fit shared memory (KLA_B200_LINEAR_SMEM), else KLA_B200_EUNSUPPORTED.
  */
-#define KLA_B200_LINEAR_MAX_ROWS 64
-#define KLA_B200_LINEAR_SMEM (200 * 1024) /* n rows of K + 8 bfloat16 and 1024 (n + 2) bytes must fit: n = B rounded up to 8, 16, 32, 64 */
+#define KLA_B200_LINEAR_MAX_ROWS 32
+#define KLA_B200_LINEAR_SMEM (200 * 1024) /* n rows of K + 8 bfloat16 and 1024 (n + 2) bytes must fit: n = B rounded up to 8, 16, 32 */
 typedef struct kla_b200_linear_args {
     int64_t B, N, K;
     const void *x;              /* in  [B, K] */

@@ -405,12 +405,17 @@ int dispatch_step(int din, int dout, bool prior, int lpc, const StepParams &prm,
 }
 template <typename T, typename TO, int LPC, bool PRIOR>
 int launch_step_layer(const StepLayerParams &prm, cudaStream_t st) {
-    const long long threads = (long long)prm.B * prm.M * LPC;
-    if ((threads + 127) / 128 > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;  // grid.x limit
-    const unsigned blocks = (unsigned)((threads + 127) / 128);
-    const cudaError_t e = launch_dependent(kla_step_layer_kernel<T, TO, LPC, PRIOR>, dim3(blocks), 128, 0, st, prm);
-    g_launches++;
-    return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+    auto go = [&](auto kern, int channels) -> int {
+        const long long blocks = (long long)prm.B * ((prm.M + channels - 1) / channels);
+        if (blocks > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;  // grid.x limit
+        const cudaError_t e = launch_dependent(kern, dim3((unsigned)blocks), 128, 0, st, prm);
+        g_launches++;
+        return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+    };
+    // Four channels per thread once that still leaves every SM two CTAs; below, the CTAs' latency is the time.
+    if ((long long)prm.B * prm.M >= 296ll * kStepLayerChannels<LPC, 4>)
+        return go(kla_step_layer_kernel<T, TO, LPC, PRIOR, 4>, kStepLayerChannels<LPC, 4>);
+    return go(kla_step_layer_kernel<T, TO, LPC, PRIOR, 1>, kStepLayerChannels<LPC, 1>);
 }
 int dispatch_step_layer(int din, int dout, bool prior, int lpc, const StepLayerParams &prm, cudaStream_t st) {
     KLA_DISPATCH(launch_step_layer, din, dout, prior, lpc, prm, st);
@@ -465,7 +470,7 @@ int launch_rawscan(const kla_b200_rawscan_args *a, void *stream, bool takes_stat
 template <int NT, int RT, int MODE, bool NORM>
 int launch_linear(const LinearParams &prm, cudaStream_t st) {
     auto kern = kla_linear_kernel<NT, RT, MODE, NORM>;
-    const size_t smem = kLinearRedBytes<NT, RT> + linear_x_bytes(NT, prm.K);
+    const size_t smem = kLinearRedBytes<NT, RT> + linear_x_bytes(kLinearStaged<NT, NORM>, NT, prm.K);
     if (smem > KLA_B200_LINEAR_SMEM) return KLA_B200_EUNSUPPORTED;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, KLA_B200_LINEAR_SMEM);
@@ -936,8 +941,7 @@ int kla_b200_linear(const kla_b200_linear_args *a, void *stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (a->B <= 8) return dispatch_linear<1>(prm, mode, st);
     if (a->B <= 16) return dispatch_linear<2>(prm, mode, st);
-    if (a->B <= 32) return dispatch_linear<4>(prm, mode, st);
-    return dispatch_linear<8>(prm, mode, st);
+    return dispatch_linear<4>(prm, mode, st);
 }
 
 int kla_b200_step_layer(const kla_b200_step_layer_args *a, void *stream) {

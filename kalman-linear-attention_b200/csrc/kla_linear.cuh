@@ -14,10 +14,13 @@
 //     operands' worth) instead of the four-byte pieces the operand layout names;
 //   * W does not depend on the kernel before, so with programmatic dependent launch its first blocks, all of a warp's
 //     share up to K = 2048, are requested before the wait for that kernel;
-//   * x comes into shared memory whole, by one round of asynchronous copies: as operands fetched from L2 beside W it
-//     doubled the loads of 32 rows (B=32: 12 us for a 2064 x 2048 projection that the library does in 5).
-// Measured on B200 against the library's GEMMs, which take 4 to 5.5 us whatever the shape at these sizes:
-// @@LINEAR@@
+// Measured on B200 in a CUDA graph, us per projection, against the library's GEMM alone (rows x columns of W):
+//   B=8   3072 x 768 4.2 (3.7), with the norm 4.4; 3104 x 1536 5.9 (5.4); 768 x 1536 3.4 (4.4); 768 x 2048 3.6 (5.2)
+//   B=16  4096 x 1024 3.9 (3.6); 4128 x 2048 5.6 (5.5); 1024 x 2048 4.6 (5.9)
+//   B=32  4096 x 1024 5.3 (3.5); 4128 x 2048 8.1 (5.6); 1024 x 2048 5.4 (4.9)
+// What bounds it is latency: about 3 us of launch, one round trip for x, the sum over warps and the store. Beyond 16 rows
+// the library's kernels are the faster ones on the device, but a call costs the host 10 us against 4, so a token issued
+// eagerly still takes less (layer step B=32 d_model 1024: 28.9 us eager and 27.7 us in a graph; 85 us as library calls).
 #pragma once
 
 #include "kla_common.cuh"
@@ -40,7 +43,6 @@ struct LinearParams {
 
 enum LinearMode { kLinearPlain = 0, kLinearSwiglu = 1, kLinearConv = 2 };
 constexpr int kLinearWarps = 8;    // warps per CTA = ways the columns are split
-constexpr int kLinearMaxRows = 64;
 
 __device__ __forceinline__ uint4 load_once(const void *p) {  // read-only, used once: not kept in L1
     uint4 v;
@@ -53,13 +55,18 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Blocks of W a warp holds in flight: all of K <= 2048 where the registers allow.
+// Where x is read from. Up to eight rows, and where it is normalised, from shared memory; more rows as they are straight
+// into the operands, a piece beside each block of W: staging them cost every CTA 64 KB of copies before its first product
+// (B=32, 4096 x 1024: 7.2 against 4.5 us).
+template <int NT, bool NORM>
+constexpr bool kLinearStaged = NORM || NT == 1;
+// Blocks of W (and, unstaged, of x) a warp holds in flight: all of K <= 2048 where the registers allow.
 template <int NT, int RT>
-constexpr int kLinearDepth = RT == 1 || NT >= 4 ? 8 : 4;
+constexpr int kLinearDepth = NT == 1 && RT == 1 ? 8 : 4;
 // shared memory: partial sums of every warp, then x (normalised with NORM)
 template <int NT, int RT>
 constexpr size_t kLinearRedBytes = sizeof(float) * kLinearWarps * RT * 16 * (NT * 8 + 2);
-inline size_t linear_x_bytes(int nt, int K) { return sizeof(__nv_bfloat16) * nt * 8 * (K + 8); }
+inline size_t linear_x_bytes(bool staged, int nt, int K) { return staged ? sizeof(__nv_bfloat16) * nt * 8 * (K + 8) : 0; }
 
 __device__ __forceinline__ void cp_async_16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -106,6 +113,7 @@ template <int NT, int RT, int MODE, bool NORM>
 __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __grid_constant__ LinearParams prm) {
     constexpr int W = kLinearWarps, U = kLinearDepth<NT, RT>, LD = NT * 8 + 2, NW = 4;
     constexpr bool GLU = MODE == kLinearSwiglu;
+    constexpr bool STAGED = kLinearStaged<NT, NORM>;
     static_assert(!GLU || RT == 2, "gate and up");
     constexpr int ROWS = GLU ? 16 : 16 * RT;  // outputs per CTA
     extern __shared__ __align__(16) unsigned char smem[];
@@ -117,7 +125,7 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
     const int row_tiles = (n_out + ROWS - 1) / ROWS;
     const int xld = K + 8;  // rows 16 bytes off a multiple of 128: the eight rows of a fragment meet different banks
 
-    uint4 wl[U][RT], wh[U][RT];
+    uint4 wl[U][RT], wh[U][RT], xv[STAGED ? 1 : U][NT];
     auto load_w = [&](int u, int tile, int kb) {
         const int ch = kb * 4 + t;
 #pragma unroll
@@ -126,6 +134,16 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
             const __nv_bfloat16 *base = prm.w + (long long)((GLU ? h * n_out : 0) + n0) * K + ch * 8;
             wl[u][h] = ch < chunks && n0 < n_out ? load_once(base) : make_uint4(0, 0, 0, 0);
             wh[u][h] = ch < chunks && n0 + 8 < n_out ? load_once(base + 8ll * K) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    auto load_x = [&](uint4 (&x)[NT], int kb) {
+        const int ch = kb * 4 + t;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const int r = min(nt * 8 + g, B - 1);
+            x[nt] = make_uint4(0, 0, 0, 0);
+            if (ch < chunks) x[nt] = STAGED ? *reinterpret_cast<const uint4 *>(xs + r * xld + ch * 8)
+                                            : *reinterpret_cast<const uint4 *>(prm.x + (long long)r * prm.x_sb + ch * 8);
         }
     };
     grid_dep_launch();
@@ -139,16 +157,20 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
     }
     grid_dep_wait();  // everything below may read what the kernel before wrote
 
-    // all of x into shared memory, one round of asynchronous copies; a warp takes whole rows
-    for (int r = warp; r < B; r += W)
-        for (int c = lane; c < chunks; c += 32) cp_async_16(xs + r * xld + c * 8, prm.x + (long long)r * prm.x_sb + c * 8);
-    cp_async_wait_all();
-    if (NORM) {
-        __syncwarp();
+    if constexpr (STAGED) {  // all of x, one round of asynchronous copies; a warp takes whole rows
         for (int r = warp; r < B; r += W)
-            norm_row<NW>(reinterpret_cast<uint4 *>(xs + r * xld), nw, prm.norm_w, chunks, K, prm.norm_eps, lane);
+            for (int c = lane; c < chunks; c += 32) cp_async_16(xs + r * xld + c * 8, prm.x + (long long)r * prm.x_sb + c * 8);
+        cp_async_wait_all();
+        if (NORM) {
+            __syncwarp();
+            for (int r = warp; r < B; r += W)
+                norm_row<NW>(reinterpret_cast<uint4 *>(xs + r * xld), nw, prm.norm_w, chunks, K, prm.norm_eps, lane);
+        }
+        __syncthreads();
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) load_x(xv[u], warp + u * W);
     }
-    __syncthreads();
 
     for (int tile = blockIdx.x; tile < row_tiles; tile += gridDim.x) {
         float acc[RT][NT][4] = {};
@@ -156,20 +178,23 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
             const bool last = kb0 + W * U >= blocks;  // of this tile: what follows is the next tile's beginning
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int ch = (kb0 + u * W) * 4 + t;
+                uint4 (&x)[NT] = xv[STAGED ? 0 : u];
+                if constexpr (STAGED) load_x(x, kb0 + u * W);
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    uint4 x = make_uint4(0, 0, 0, 0);
-                    if (ch < chunks) x = *reinterpret_cast<const uint4 *>(xs + min(nt * 8 + g, B - 1) * xld + ch * 8);
+                for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                     for (int h = 0; h < RT; ++h) {
-                        mma_16816(acc[h][nt], wl[u][h].x, wh[u][h].x, wl[u][h].y, wh[u][h].y, x.x, x.y);
-                        mma_16816(acc[h][nt], wl[u][h].z, wh[u][h].z, wl[u][h].w, wh[u][h].w, x.z, x.w);
+                        mma_16816(acc[h][nt], wl[u][h].x, wh[u][h].x, wl[u][h].y, wh[u][h].y, x[nt].x, x[nt].y);
+                        mma_16816(acc[h][nt], wl[u][h].z, wh[u][h].z, wl[u][h].w, wh[u][h].w, x[nt].z, x[nt].w);
                     }
-                }
                 // the registers just read take what comes U blocks later
-                if (!last) load_w(u, tile, kb0 + (U + u) * W);
-                else if (tile + (int)gridDim.x < row_tiles) load_w(u, tile + gridDim.x, warp + u * W);
+                if (!last) {
+                    load_w(u, tile, kb0 + (U + u) * W);
+                    if constexpr (!STAGED) load_x(x, kb0 + (U + u) * W);
+                } else if (tile + (int)gridDim.x < row_tiles) {
+                    load_w(u, tile + gridDim.x, warp + u * W);
+                    if constexpr (!STAGED) load_x(x, warp + u * W);
+                }
             }
         }
 #pragma unroll
