@@ -424,6 +424,9 @@ int dispatch_step_layer(int din, int dout, bool prior, int lpc, const StepLayerP
 }  // namespace
 
 namespace {
+template <class Op, bool WIDE>
+int launch_rawscan_as(const kla_b200_rawscan_args *a, void *stream);
+
 template <class Op>
 int launch_rawscan(const kla_b200_rawscan_args *a, void *stream, bool takes_state0, bool gives_dstate0) {
     if (a == nullptr || a->B < 0 || a->L < 0 || a->N < 0) return KLA_B200_EINVAL;
@@ -438,6 +441,15 @@ int launch_rawscan(const kla_b200_rawscan_args *a, void *stream, bool takes_stat
         if (!aligned(a->out[k], sizeof(float))) return KLA_B200_EALIGN;
     }
     if (a->B == 0 || a->N == 0) return KLA_B200_OK;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
+    if (Op::NIN >= 6 && (a->N + kRawLC - 1) / kRawLC * a->B <= sms) return launch_rawscan_as<Op, false>(a, stream);
+    return launch_rawscan_as<Op, true>(a, stream);
+}
+
+template <class Op, bool WIDE>
+int launch_rawscan_as(const kla_b200_rawscan_args *a, void *stream) {
+    constexpr int kRawTT = RawTile<Op, WIDE>::TT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RawParams prm{};
     prm.B = (int)a->B; prm.L = (int)a->L; prm.N = (int)a->N;
@@ -457,11 +469,11 @@ int launch_rawscan(const kla_b200_rawscan_args *a, void *stream, bool takes_stat
     prm.use_tma = tma;
     if (int rc = wait_ctl(&prm.wait)) return rc;
     prm.wait.skip_tile = -1;  // the hook is for the fused scan kernels
-    auto kern = kla_rawscan_kernel<Op>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RawSmem<Op>::kTotal);
+    auto kern = kla_rawscan_kernel<Op, WIDE>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RawSmem<Op, WIDE>::kTotal);
     if (e != cudaSuccess) return cuda_fail(e);
     dim3 grid((unsigned)((a->N + kRawLC - 1) / kRawLC), (unsigned)a->B);
-    kern<<<grid, kRawLC + 32, RawSmem<Op>::kTotal, st>>>(prm);
+    kern<<<grid, kRawLC + 32, RawSmem<Op, WIDE>::kTotal, st>>>(prm);
     g_launches++;
     e = cudaGetLastError();
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
@@ -826,12 +838,15 @@ int kla_b200_conv_seq(const kla_b200_conv_seq_args *a, void *stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define KLA_CONV_LAUNCH(KERNEL, T)                                                    \
     do {                                                                              \
-        if (a->K <= 4) {                                                              \
-            if (pair) KERNEL<T, 2, 4><<<grid, 128, 0, st>>>(prm);                     \
-            else KERNEL<T, 1, 4><<<grid, 128, 0, st>>>(prm);                          \
+        if (a->K == 4 && a->activation == KLA_B200_ACT_SILU) {                        \
+            if (pair) KERNEL<T, 2, 4, true><<<grid, 128, 0, st>>>(prm);               \
+            else KERNEL<T, 1, 4, true><<<grid, 128, 0, st>>>(prm);                    \
+        } else if (a->K <= 4) {                                                       \
+            if (pair) KERNEL<T, 2, 4, false><<<grid, 128, 0, st>>>(prm);              \
+            else KERNEL<T, 1, 4, false><<<grid, 128, 0, st>>>(prm);                   \
         } else {                                                                      \
-            if (pair) KERNEL<T, 2, kConvMaxTaps><<<grid, 128, 0, st>>>(prm);          \
-            else KERNEL<T, 1, kConvMaxTaps><<<grid, 128, 0, st>>>(prm);               \
+            if (pair) KERNEL<T, 2, kConvMaxTaps, false><<<grid, 128, 0, st>>>(prm);   \
+            else KERNEL<T, 1, kConvMaxTaps, false><<<grid, 128, 0, st>>>(prm);        \
         }                                                                             \
     } while (0)
     if (a->dtype == KLA_B200_F32) KLA_CONV_LAUNCH(kla_conv_seq_kernel, float);
@@ -860,14 +875,16 @@ int kla_b200_conv_seq_bwd(const kla_b200_conv_seq_bwd_args *a, void *stream) {
     prm.B = (int)a->B; prm.L = (int)a->L; prm.D = (int)a->D; prm.K = (int)a->K;
     prm.x = t3(a->x); prm.dz = t3(a->dz); prm.dx = t3(a->dx); prm.w = a->weight; prm.bias = a->bias;
     prm.state = a->state; prm.dw = a->dweight; prm.dbias = a->dbias; prm.act = a->activation;
-    // one channel per thread: with two, the backward's five register windows cost more in occupancy than the wider
-    // accesses give back (0.35 against 0.22 ms at B=16, L=2048, D=1536, bfloat16)
+    // One channel per thread: with two, the backward's register windows cost in occupancy what the wider accesses give
+    // back (B=16 L=2048 D=1536 bfloat16 152 against 156 us for the layer's default, 215 against 350 us for other taps).
     dim3 grid((unsigned)((a->D + 127) / 128), (unsigned)chunks, (unsigned)a->B);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define KLA_CONV_BWD_LAUNCH(T)                                                                  \
     do {                                                                                        \
-        if (a->K <= 4) kla_conv_seq_bwd_kernel<T, 1, 4><<<grid, 128, 0, st>>>(prm);             \
-        else kla_conv_seq_bwd_kernel<T, 1, kConvMaxTaps><<<grid, 128, 0, st>>>(prm);            \
+        if (a->K == 4 && a->activation == KLA_B200_ACT_SILU)                                    \
+            kla_conv_seq_bwd_kernel<T, 1, 4, true><<<grid, 128, 0, st>>>(prm);                 \
+        else if (a->K <= 4) kla_conv_seq_bwd_kernel<T, 1, 4, false><<<grid, 128, 0, st>>>(prm); \
+        else kla_conv_seq_bwd_kernel<T, 1, kConvMaxTaps, false><<<grid, 128, 0, st>>>(prm);     \
     } while (0)
     if (a->dtype == KLA_B200_F32) KLA_CONV_BWD_LAUNCH(float);
     else KLA_CONV_BWD_LAUNCH(__nv_bfloat16);

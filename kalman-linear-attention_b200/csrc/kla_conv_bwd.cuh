@@ -46,12 +46,14 @@ __device__ __forceinline__ float activate_slope_fast(float x, int act) {
     return slope;
 }
 
-template <typename T, int VEC, int KT>
+// EXACT as in kla_conv_seq_kernel.
+template <typename T, int VEC, int KT, bool EXACT>
 __global__ void __launch_bounds__(128) kla_conv_seq_bwd_kernel(const ConvSeqBwdParams prm) {
     const int d = (blockIdx.x * blockDim.x + threadIdx.x) * VEC, b = blockIdx.z;
     const int t0 = blockIdx.y * kConvBwdChunk;
     if (d >= prm.D) return;
-    const int K = prm.K, L = prm.L;
+    const int K = EXACT ? KT : prm.K, L = prm.L;
+    const int act = EXACT ? (int)kActSilu : prm.act;
     const T *xb = static_cast<const T *>(prm.x.ptr) + (long long)b * prm.x.sb + d;
     const T *gb = static_cast<const T *>(prm.dz.ptr) + (long long)b * prm.dz.sb + d;
     T *ob = static_cast<T *>(prm.dx.ptr) + (long long)b * prm.dx.sb + d;
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(128) kla_conv_seq_bwd_kernel(const ConvSeqBwdP
 #pragma unroll
         for (int i = 0; i < MAXT; ++i) {
             wl[i][e] = i < K ? prm.w[(long long)(d + e) * K + i] : 0.0f;
-            wr[i][e] = i >= lead ? prm.w[(long long)(d + e) * K + (i - lead)] : 0.0f;
+            wr[i][e] = EXACT ? wl[i][e] : i >= lead ? prm.w[(long long)(d + e) * K + (i - lead)] : 0.0f;
             dwin[i][e] = accw[i][e] = 0.0f;
             xw[i][e] = 0.0f;
             if (i > lead) {  // the K-1 inputs before t0, one place further back than in the loop, which shifts first
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(128) kla_conv_seq_bwd_kernel(const ConvSeqBwdP
                         float pre = bias[e];
 #pragma unroll
                         for (int i = 0; i < MAXT; ++i) pre = fmaf(wr[i][e], xw[i][e], pre);
-                        dpre = gin[u][e] * activate_slope_fast(pre, prm.act);
+                        dpre = gin[u][e] * activate_slope_fast(pre, act);
                         if (FULL || t < t1) {  // the sums over t belong to the chunk that owns t
                             accb[e] += dpre;
 #pragma unroll

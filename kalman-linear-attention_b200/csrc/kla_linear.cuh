@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
     constexpr bool STAGED = kLinearStaged<NT, NORM>;
     static_assert(!GLU || RT == 2, "gate and up");
     constexpr int ROWS = GLU ? 16 : 16 * RT;  // outputs per CTA
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     float *red = reinterpret_cast<float *>(smem);  // [W][RT * 16][LD]
     __nv_bfloat16 *xs = reinterpret_cast<__nv_bfloat16 *>(smem + kLinearRedBytes<NT, RT>);  // [B][K + 8]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;

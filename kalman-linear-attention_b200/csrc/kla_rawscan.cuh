@@ -25,7 +25,6 @@
 namespace kla {
 
 constexpr int kRawLC = 128;   // lanes per CTA (= compute threads)
-constexpr int kRawTT = 8;     // steps per tile
 constexpr int kRawNSO = 3;    // output tiles in the store ring
 constexpr int kRawMaxIn = 6, kRawMaxOut = 4;
 
@@ -60,7 +59,7 @@ constexpr float kRawDenMin = 1e-12f;  // floor on the Moebius denominator, tiled
 // step(x, prev, y): x = this step's inputs, prev = the HALO input at t-1 (the
 // initial state at t = 0).
 struct MobiusFwd {  // in: A B C D   out: lam
-    static constexpr int NIN = 4, NOUT = 1, HALO = -1, NSI = 2;
+    static constexpr int NIN = 4, NOUT = 1, HALO = -1;
     static constexpr bool REV = false;
     static constexpr float kPrior = 1.0f;  // lam0 when none is given, tiled_mobius_scan.py:303-305
     float lam;
@@ -73,7 +72,7 @@ struct MobiusFwd {  // in: A B C D   out: lam
     __device__ float finish() const { return 0.0f; }
 };
 struct AffineFwd {  // in: alpha r   out: eta
-    static constexpr int NIN = 2, NOUT = 1, HALO = -1, NSI = 3;
+    static constexpr int NIN = 2, NOUT = 1, HALO = -1;
     static constexpr bool REV = false;
     static constexpr float kPrior = 0.0f;  // eta_{-1} = 0
     float eta;
@@ -88,7 +87,7 @@ struct AffineFwd {  // in: alpha r   out: eta
 // den = C lam' + D and gain = (AD - BC)/den^2, nu_t = dlam_t + gain_{t+1} nu_{t+1},
 // dA = nu lam'/den, dB = nu/den, dC = -nu lam lam'/den, dD = -nu lam/den, dlam0 = gain_0 nu_0.
 struct MobiusBwd {  // in: A B C D lam dlam   out: dA dB dC dD
-    static constexpr int NIN = 6, NOUT = 4, HALO = 4, NSI = 2;
+    static constexpr int NIN = 6, NOUT = 4, HALO = 4;
     static constexpr bool REV = true;
     static constexpr float kPrior = 1.0f;
     float c;
@@ -108,7 +107,7 @@ struct MobiusBwd {  // in: A B C D lam dlam   out: dA dB dC dD
 // Adjoint of the affine scan (tiled_mobius_scan.py:289-296): mu_t = deta_t + alpha_{t+1} mu_{t+1},
 // dalpha = mu eta', dr = mu.
 struct AffineBwd {  // in: alpha eta deta   out: dalpha dr
-    static constexpr int NIN = 3, NOUT = 2, HALO = 1, NSI = 2;
+    static constexpr int NIN = 3, NOUT = 2, HALO = 1;
     static constexpr bool REV = true;
     static constexpr float kPrior = 0.0f;
     float c;
@@ -122,19 +121,33 @@ struct AffineBwd {  // in: alpha eta deta   out: dalpha dr
     __device__ float finish() const { return c; }
 };
 
-template <class Op>
-struct RawSmem {
-    static constexpr size_t kBars = 128;
-    static constexpr size_t kInTile = sizeof(float) * (kRawTT + 1) * kRawLC;  // one extra row for the halo
-    static constexpr size_t kOutTile = sizeof(float) * kRawTT * kRawLC;
-    static constexpr size_t kIn = Op::NIN * kInTile, kOut = Op::NOUT * kOutTile;
-    static constexpr size_t kTotal = kBars + Op::NSI * kIn + kRawNSO * kOut;
+// Tile shape of a recurrence: TT steps, NSI input tiles in flight. WIDE: two CTAs share an SM (the usual case), so their
+// shared memory may take half of it; otherwise one has it to itself. Measured on B200, TB/s of the tensors, at B=2 L=4096
+// N=16384 / B=1 L=4096 N=8192 (64 CTAs), 8-step tiles with 2-3 stages first: Moebius forward 5.5 / 1.7, 16 steps 6.8 / 2.3;
+// affine forward 5.5 / 1.7, 16 steps 6.0 / 2.2 (2 stages), 8 steps with 5 stages 6.6 / 1.8; affine backward 5.3 / 1.8,
+// 16 steps 6.5 / 2.5. The Moebius backward's ten tensors leave room for two CTAs at 8 steps and two stages only (6.3;
+// 16 steps 4.8), but alone on their SMs 16 steps are better (2.0 against 2.3): with few CTAs the hand-over of a tile, about
+// a third of a microsecond, is what counts.
+template <class Op, bool WIDE>
+struct RawTile {
+    static constexpr int TT = Op::NIN >= 6 && WIDE ? 8 : 16;
+    static constexpr int NSI = Op::NIN == 2 ? 4 : 2;
 };
 
-template <class Op>
+template <class Op, bool WIDE>
+struct RawSmem {
+    static constexpr int kTT = RawTile<Op, WIDE>::TT, kNSI = RawTile<Op, WIDE>::NSI;
+    static constexpr size_t kBars = 128;
+    static constexpr size_t kInTile = sizeof(float) * (kTT + 1) * kRawLC;  // one extra row for the halo
+    static constexpr size_t kOutTile = sizeof(float) * kTT * kRawLC;
+    static constexpr size_t kIn = Op::NIN * kInTile, kOut = Op::NOUT * kOutTile;
+    static constexpr size_t kTotal = kBars + kNSI * kIn + kRawNSO * kOut;
+};
+
+template <class Op, bool WIDE>
 __global__ void __launch_bounds__(kRawLC + 32) kla_rawscan_kernel(const __grid_constant__ RawParams prm) {
-    using Sm = RawSmem<Op>;
-    constexpr int LC = kRawLC, TT = kRawTT, NSI = Op::NSI, NSO = kRawNSO, NIN = Op::NIN, NOUT = Op::NOUT;
+    using Sm = RawSmem<Op, WIDE>;
+    constexpr int LC = kRawLC, TT = Sm::kTT, NSI = Sm::kNSI, NSO = kRawNSO, NIN = Op::NIN, NOUT = Op::NOUT;
     constexpr int NCW = LC / 32;  // compute warps
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *full_in = reinterpret_cast<uint64_t *>(smem);  // [NSI]

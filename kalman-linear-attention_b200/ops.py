@@ -437,11 +437,21 @@ def kla_scan_b200(
         gate_act = epi.get("gate_activation", "silu")
         if gate_act not in ("silu", "gelu", "relu"):
             raise ValueError("gate_activation must be 'silu', 'gelu' or 'relu'")
+        if not _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip):
+            if skip is not None:
+                epi["lambda_skip"] = skip.float().reshape(-1).contiguous()
+            y, y_var, lam_fin, eta_fin, _ = _launch_fwd(
+                v, lambda_v, k, q, a, p, lam0, eta0, bool(decode_from_prior), out_dtype, False, log_variance, epi)
+            return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)
         y, y_var, lam_fin, eta_fin = _KLAScanEpilogueB200.apply(
             v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip, bool(decode_from_prior),
             out_dtype, log_variance, gate_act)
         return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)
     return _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, decode_from_prior, out_dtype, log_variance, time_chunks)
+
+
+def _wants_grad(*tensors) -> bool:
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
 def _check_log_variance(log_variance):
@@ -459,6 +469,15 @@ def _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, log_varianc
     chunks = pick_time_chunks(B, L, M, k.shape[2], time_chunks) if L > 0 and log_variance is None else 1
     if chunks > 1 and time_chunks is not None and not all(_chunkable(t, B, L) for t in (v, lambda_v, k, q)):
         chunks = 1  # an explicit count is taken for sequences that lie back to back
+    if not _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0):  # inference: no autograd node, no checkpoints
+        if chunks > 1:
+            y, y_var, lam_fin, eta_fin, *_ = _lib.host().scan_fwd_chunked(
+                v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype == torch.bfloat16, False, chunks,
+                _chunk_len(L, chunks))
+        else:
+            y, y_var, lam_fin, eta_fin, _ = _launch_fwd(
+                v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype, False, log_variance)
+        return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)
     y, y_var, lam_fin, eta_fin = _KLAScanB200.apply(
         v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype, log_variance, chunks)
     return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)

@@ -58,3 +58,27 @@ def test_chunks_cover_every_length():
             c = ops.pick_time_chunks(B, L, M, 16)
             n = ops._chunk_len(L, c)
             assert (c - 1) * n < L <= c * n and (c == 1 or n >= 64), (L, c, n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,L,M,S", [(1, 1, 4, 1), (2, 15, 9, 16), (1, 16, 3, 12), (3, 17, 33, 4), (1, 70, 130, 16), (80, 33, 20, 16)])
+def test_raw_scans_around_their_tiles(B, L, M, S):
+    """Both tile shapes of the raw scans (the last case has more CTAs than SMs) against a float64 loop and autograd."""
+    g = torch.Generator(device="cuda").manual_seed(L)
+    rn = lambda *s: torch.rand(*s, generator=g, device="cuda") + 0.2
+    ins = [rn(B, L, M, S).requires_grad_() for _ in range(6)]
+    lam0 = rn(B, M, S).requires_grad_()
+    ref = [t.detach().double().requires_grad_() for t in (*ins, lam0)]
+    lam, eta, r_lam, r_eta = ref[6], torch.zeros_like(ref[6]), [], []
+    for t in range(L):
+        a, b, c, d, al, r = (x[:, t] for x in ref[:6])
+        lam, eta = (a * lam + b) / (c * lam + d), al * eta + r
+        r_lam.append(lam)
+        r_eta.append(eta)
+    outs = [kla_b200.mobius_scan_b200(*ins[:4], lam0), kla_b200.affine_scan_b200(*ins[4:])]
+    refs = [torch.stack(r_lam, 1), torch.stack(r_eta, 1)]
+    w = [rn(B, L, M, S), rn(B, L, M, S)]
+    grads = torch.autograd.grad(outs, [*ins, lam0], w)
+    r_grads = torch.autograd.grad(refs, ref, [x.double() for x in w])
+    for got, want in zip((*outs, *grads), (*refs, *r_grads)):
+        torch.testing.assert_close(got.double(), want, rtol=2e-5, atol=2e-5 * want.abs().mean().item())
