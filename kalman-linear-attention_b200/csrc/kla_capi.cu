@@ -897,7 +897,7 @@ int kla_b200_conv_seq_bwd(const kla_b200_conv_seq_bwd_args *a, void *stream) {
 int kla_b200_add_norm(int64_t rows, int64_t D, int32_t dtype, int32_t weight_dtype, const void *x, const void *delta, const void *weight,
                       float eps, void *sum, void *out, void *stream) {
     if (rows < 0 || D < 0) return KLA_B200_EINVAL;
-    if (D % 8 || D > (1 << 30) || rows > (1ll << 32)) return KLA_B200_EUNSUPPORTED;
+    if (D % 8 || D > (1 << 30) || rows > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;
     if (rows == 0 || D == 0) return KLA_B200_OK;
     if (!x || !weight || !out || (delta && !sum)) return KLA_B200_EINVAL;
     for (const void *p : {x, delta, weight, static_cast<const void *>(sum), static_cast<const void *>(out)})
