@@ -428,6 +428,10 @@ int kla_b200_add_norm(int64_t rows, int64_t D, int32_t dtype, int32_t weight_dty
                       const void *weight, float eps, void *sum, void *out, void *stream);
 int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up, void *out, void *stream);
 
+/* out[r] = index of the first largest of x[r, 0 .. n-1] (a NaN counts as the largest), n >= 1: the greedy choice of a token
+ * (src/kla/models/sequence_model.py:222-225). */
+int kla_b200_argmax(int64_t rows, int64_t n, int32_t dtype, const void *x, int64_t row_stride, int64_t *out, void *stream);
+
 /*
  * A projection of single-token decode with its neighbours: out = f(norm(x) W^T + bias) + residual for up to
  * KLA_B200_LINEAR_MAX_ROWS rows of bfloat16, float32 accumulation, one rounding at the store. Replaces, for one token,

@@ -933,6 +933,21 @@ int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up,
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
 }
 
+int kla_b200_argmax(int64_t rows, int64_t n, int32_t dtype, const void *x, int64_t row_stride, int64_t *out, void *stream) {
+    if (rows < 0 || n < 1 || row_stride < 0) return KLA_B200_EINVAL;
+    if (n > (1 << 30) || rows > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;
+    if (rows == 0) return KLA_B200_OK;
+    if (!x || !out) return KLA_B200_EINVAL;
+    if (!aligned(x, dtype == KLA_B200_BF16 ? 2 : 4) || !aligned(out, 8)) return KLA_B200_EALIGN;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    long long *o = reinterpret_cast<long long *>(out);
+    if (dtype == KLA_B200_BF16) kla_argmax_kernel<<<(unsigned)rows, 1024, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), row_stride, (int)n, o);
+    else kla_argmax_kernel<<<(unsigned)rows, 1024, 0, st>>>(static_cast<const float *>(x), row_stride, (int)n, o);
+    g_launches++;
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+
 int kla_b200_linear(const kla_b200_linear_args *a, void *stream) {
     if (a == nullptr || a->B < 0 || a->N < 0 || a->K < 0) return KLA_B200_EINVAL;
     if (a->B > KLA_B200_LINEAR_MAX_ROWS || a->N > (1 << 30) || a->K > (1 << 20) || a->K % 8 || a->x_stride_b % 8) return KLA_B200_EUNSUPPORTED;

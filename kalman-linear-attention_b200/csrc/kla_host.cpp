@@ -39,6 +39,7 @@ struct Entry {
     int (*linear)(const kla_b200_linear_args *, void *) = nullptr;
     int (*add_norm)(int64_t, int64_t, int32_t, int32_t, const void *, const void *, const void *, float, void *, void *, void *) = nullptr;
     int (*swiglu)(int64_t, int64_t, int32_t, const void *, void *, void *) = nullptr;
+    int (*argmax)(int64_t, int64_t, int32_t, const void *, int64_t, int64_t *, void *) = nullptr;
     int (*conv_seq)(const kla_b200_conv_seq_args *, void *) = nullptr;
     int (*conv_seq_bwd)(const kla_b200_conv_seq_bwd_args *, void *) = nullptr;
     int (*rawscan[4])(const kla_b200_rawscan_args *, void *) = {};  // Moebius forward, backward, affine forward, backward
@@ -64,6 +65,7 @@ void bind(const py::dict &d) {
     take(lib.linear, d, "kla_b200_linear");
     take(lib.add_norm, d, "kla_b200_add_norm");
     take(lib.swiglu, d, "kla_b200_swiglu");
+    take(lib.argmax, d, "kla_b200_argmax");
     take(lib.conv_seq, d, "kla_b200_conv_seq");
     take(lib.conv_seq_bwd, d, "kla_b200_conv_seq_bwd");
     take(lib.rawscan[0], d, "kla_b200_mobius_scan_fwd");
@@ -453,6 +455,16 @@ Tensor swiglu(const Tensor &gu) {
     return out;
 }
 
+// out[...] (int64) = argmax of x[..., n] over its last dimension; returns out
+Tensor argmax(const Tensor &x, Tensor out) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto T = x.scalar_type();
+    if (x.dim() != 2 || x.size(1) < 1 || x.stride(1) != 1 || !x.is_cuda() || (T != at::kFloat && T != at::kBFloat16) || !sm100(x.device()))
+        return out.copy_(x.argmax(-1));
+    check(lib.argmax(x.size(0), x.size(1), dt(T), x.data_ptr(), x.stride(0), out.data_ptr<int64_t>(), stream_of(x)));
+    return out;
+}
+
 // A language model's head for a few rows. From this many outputs on the library's GEMM is the better read of W (50304 x 768,
 // eight rows: 8.2 us against 14), and the norm is a launch of its own.
 constexpr int64_t kWideHead = 8192;
@@ -605,6 +617,7 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("layer_step", &layer_step);
     m.def("add_norm", &add_norm);
     m.def("swiglu", &swiglu);
+    m.def("argmax", &argmax);
     m.def("project", &project);
     m.def("swiglu_step", &swiglu_step);
 }

@@ -197,14 +197,23 @@ class _TokenGraph:
         self.done = None  # recorded behind the last use
         side = torch.cuda.Stream(device)
         side.wait_stream(torch.cuda.current_stream(device))
-        with torch.cuda.stream(side):  # libraries set themselves up outside the capture
-            dec.step(self.token, self.state).argmax(dim=-1)
-        torch.cuda.current_stream(device).wait_stream(side)
         self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph):
-            self.logits = dec.step(self.token, self.state)
-            if greedy:
-                self.token.copy_(self.logits.argmax(dim=-1))
+        with torch.cuda.stream(side):
+            self._token(dec, greedy)  # libraries set themselves up outside the capture
+            # captured by hand: torch.cuda.graph collects garbage and empties the allocator's cache first, which every
+            # allocation after it then pays for; thread-local, so that other threads may go on allocating
+            self.graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                self.logits = self._token(dec, greedy)
+            finally:
+                self.graph.capture_end()
+        torch.cuda.current_stream(device).wait_stream(side)
+
+    def _token(self, dec, greedy):
+        logits = dec.step(self.token, self.state)
+        if greedy:
+            _lib.host().argmax(logits, self.token)
+        return logits
 
     def reset(self):
         """The prior state, ordered behind whatever used the buffers last."""
@@ -417,7 +426,7 @@ class ModelDecoder:
     @staticmethod
     def _sample(logits, temperature, top_k):  # sequence_model.py:222-234
         if temperature <= 0:
-            return logits.argmax(dim=-1, keepdim=True)
+            return _lib.host().argmax(logits, torch.empty(logits.shape[:-1], device=logits.device, dtype=torch.long)).unsqueeze(-1)
         logits = logits / temperature
         if top_k is not None:
             kth = torch.topk(logits, top_k, dim=-1).values[..., -1, None]

@@ -90,3 +90,15 @@ def test_residual_sum_norm_and_gate(rows, D, dtype, wtype):
         torch.testing.assert_close(out.double(), ref, **tol)
     a, b = x.double().chunk(2, dim=-1)
     torch.testing.assert_close(lib.host().swiglu(x).double(), F.silu(a) * b, **tol)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1), (3, 7), (8, 50304), (5, 8200), (2, 1023)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_greedy_choice(rows, n, dtype):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(rows, n, generator=g, device="cuda").to(dtype)  # bfloat16: the largest value is often there twice
+    got = lib.host().argmax(x, torch.empty(rows, device="cuda", dtype=torch.long))
+    first = (x == x.max(dim=-1, keepdim=True).values).long().argmax(dim=-1)
+    assert torch.equal(got, first)
+    x[-1, n // 2:] = float("nan")
+    assert lib.host().argmax(x, got)[-1] == n // 2
