@@ -58,6 +58,8 @@
 // before the previous step's arithmetic and unrolling the whole tile gave 1.20 -> 1.17 ms.
 #pragma once
 
+#include <type_traits>
+
 #include "kla_fwd.cuh"
 
 namespace kla {
@@ -138,11 +140,20 @@ struct BwdShape {
 template <typename T, typename TO, int SPAD, int TT>
 struct BwdSmem {
     using Sh = BwdShape<SPAD>;
+    // bfloat16 tiles are widened once by the loader, from a ring of raw tiles into the stages: by the eight lanes and two
+    // groups that read each value the conversions were a tenth of a CTA's instructions (B=8 L=4096 M=1024 S=16: 1.27 ms
+    // where float32 takes 1.15). At four states the wider stages would leave room for one CTA per SM instead of two.
+    static constexpr bool kWiden = sizeof(T) == 2 && SPAD >= 8;
+    using TV = std::conditional_t<kWiden, float, T>;   // v, lambda_v as staged
+    using TD = std::conditional_t<kWiden, float, TO>;  // dy, dyvar as staged
+    static constexpr int kRawTiles = 2;
+    static constexpr size_t kRawI = ((sizeof(T) * TT * Sh::kMC + 127) / 128) * 128, kRawO = ((sizeof(TO) * TT * Sh::kMC + 127) / 128) * 128;
+    static constexpr size_t kRaw = kWiden ? 2 * kRawI + 2 * kRawO : 0;
     static constexpr size_t kBars = 128;
-    static constexpr size_t kTileI = ((sizeof(T) * TT * Sh::kMC + 127) / 128) * 128;   // v or lambda_v
-    static constexpr size_t kTileO = ((sizeof(TO) * TT * Sh::kMC + 127) / 128) * 128;  // dy or dyvar
+    static constexpr size_t kTileI = ((sizeof(TV) * TT * Sh::kMC + 127) / 128) * 128;  // v or lambda_v
+    static constexpr size_t kTileO = ((sizeof(TD) * TT * Sh::kMC + 127) / 128) * 128;  // dy or dyvar
     static constexpr size_t kKq = sizeof(float4) * TT * SPAD;                          // (k, k, q, q) per (t, s)
-    static constexpr size_t kLamF = sizeof(T) == 4 ? 0 : ((sizeof(float) * TT * Sh::kMC + 127) / 128) * 128;  // as in FwdSmem
+    static constexpr size_t kLamF = sizeof(TV) == 4 ? 0 : ((sizeof(float) * TT * Sh::kMC + 127) / 128) * 128;  // as in FwdSmem
     static constexpr size_t kIn = 2 * kTileI + 2 * kTileO + kKq + kLamF;
     // Trajectory: a row of one float4 (P', n' of two channels) per compute thread for every (step, state). Rows are
     // padded by 64 bytes, so that helper lanes reading the same column of two neighbouring rows meet different banks.
@@ -150,7 +161,7 @@ struct BwdSmem {
     static constexpr size_t kTraj = sizeof(float4) * TT * Sh::kSPT * kRow;  // one of two
     static constexpr size_t kPost = sizeof(float4) * Sh::kSPT * kRow;       // state after the last step
     static constexpr size_t kRawKq = SPAD <= 16 ? 0 : 2 * ((sizeof(T) * TT * SPAD + 127) / 128) * 128;  // k and q of a tile as they are in memory
-    static constexpr size_t kTotal = kBars + kBwdStages * kIn + 2 * kTraj + kPost + 2 * kRawKq;
+    static constexpr size_t kTotal = kBars + kBwdStages * kIn + 2 * kTraj + kPost + 2 * kRawKq + kRawTiles * kRaw;
 };
 
 constexpr int kBwdThreads = 384;  // reverse, replay and helper groups of four warps each
@@ -186,24 +197,27 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
     uint64_t *traj_full = empty_in + NS;                     // [2]   replay -> reverse: trajectory of a tile written
     uint64_t *part_full = traj_full + 2;                     // [2]   reverse -> summing helpers: partial sums written
     uint64_t *buf_empty = part_full + 2;                     // [2]   summing helpers -> replay: buffer reusable
-    static_assert((2 * NS + 6) * sizeof(uint64_t) <= Sm::kBars, "barriers fit their slot");
+    uint64_t *raw_full = buf_empty + 2;                      // [kRawTiles] bfloat16 tiles loaded, not yet widened
+    static_assert((2 * NS + 6 + Sm::kRawTiles) * sizeof(uint64_t) <= Sm::kBars, "barriers fit their slot");
+    using TV = typename Sm::TV;
+    using TD = typename Sm::TD;
     unsigned char *in_base = smem + Sm::kBars;
     unsigned char *traj_base = in_base + NS * Sm::kIn;
     unsigned char *raw_base = traj_base + 2 * Sm::kTraj + Sm::kPost;  // two tiles of k, q as they are in memory
     float4 *post = reinterpret_cast<float4 *>(traj_base + 2 * Sm::kTraj);                                // [SPT][ROW]
     auto trajbuf = [&](int bf) { return reinterpret_cast<float4 *>(traj_base + bf * Sm::kTraj); };      // [TT*SPT][ROW]
-    auto vstage = [&](int s) { return reinterpret_cast<T *>(in_base + s * Sm::kIn); };
-    auto lstage = [&](int s) { return reinterpret_cast<T *>(in_base + s * Sm::kIn + Sm::kTileI); };
-    auto dystage = [&](int s) { return reinterpret_cast<TO *>(in_base + s * Sm::kIn + 2 * Sm::kTileI); };
-    auto dyvstage = [&](int s) { return reinterpret_cast<TO *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + Sm::kTileO); };
+    auto vstage = [&](int s) { return reinterpret_cast<TV *>(in_base + s * Sm::kIn); };
+    auto lstage = [&](int s) { return reinterpret_cast<TV *>(in_base + s * Sm::kIn + Sm::kTileI); };
+    auto dystage = [&](int s) { return reinterpret_cast<TD *>(in_base + s * Sm::kIn + 2 * Sm::kTileI); };
+    auto dyvstage = [&](int s) { return reinterpret_cast<TD *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + Sm::kTileO); };
     auto kqstage = [&](int s) { return reinterpret_cast<float4 *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + 2 * Sm::kTileO); };
     // the precision tile the kernel computes with: float32 where lambda_v is float32 or formed from log-variances
     auto lfstage = [&](int s) {
         return reinterpret_cast<float *>(in_base + s * Sm::kIn +
-                                         (sizeof(T) == 4 ? Sm::kTileI : 2 * Sm::kTileI + 2 * Sm::kTileO + Sm::kKq));
+                                         (sizeof(TV) == 4 ? Sm::kTileI : 2 * Sm::kTileI + 2 * Sm::kTileO + Sm::kKq));
     };
     auto lam_pair = [&](int s, int at) {
-        if constexpr (sizeof(T) == 4 || LOGV) return load_pair(lfstage(s) + at);
+        if constexpr (sizeof(TV) == 4 || LOGV) return load_pair(lfstage(s) + at);
         else return load_pair(lstage(s) + at);
     };
 
@@ -228,9 +242,10 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
-            mbar_init(&full_in[s], stage_arrivals(prm.use_tma, kProducers));
+            mbar_init(&full_in[s], Sm::kWiden ? kProducers : stage_arrivals(prm.use_tma, kProducers));
             mbar_init(&empty_in[s], kStageUsers);
         }
+        for (int r = 0; r < Sm::kRawTiles; ++r) mbar_init(&raw_full[r], prm.use_tma ? 1 : stage_arrivals(false, kProducers));
         for (int bf = 0; bf < 2; ++bf) {
             mbar_init(&traj_full[bf], NW);
             mbar_init(&part_full[bf], NW);
@@ -294,16 +309,16 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 const int n = min(TT, L - tile * TT);
                 if (!mbar_wait(prm.wait, &full_in[s], (ti / NS) & 1, 11)) break;
                 if (LOGV) {  // this warp's channels of the tile: log-variance -> precision, float32
-                    const T *raw = lstage(s) + cwarp * CPW;
+                    const TV *raw = lstage(s) + cwarp * CPW;
                     float *lf = lfstage(s) + cwarp * CPW;
                     for (int e = lane; e < TT * CPW; e += 32) {
                         const int at = (e / CPW) * MC + e % CPW;
-                        lf[at] = precision_from_log_variance_fast(to_f32<T>(raw[at]), prm.obs_var_min, prm.obs_var_max);
+                        lf[at] = precision_from_log_variance_fast(to_f32<TV>(raw[at]), prm.obs_var_min, prm.obs_var_max);
                     }
                     fence_proxy_async();  // these plain stores are ordered before the bulk copy that refills the stage
                     __syncwarp();
                 }
-                const T *vrow = vstage(s) + cw;
+                const TV *vrow = vstage(s) + cw;
                 const float4 *kqrow = kqstage(s) + j;
                 float4 *traj = trajbuf(bf) + ctid;
                 float2 P[SPT], nm[SPT];
@@ -370,9 +385,9 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 const int n = min(TT, L - tile * TT);
                 if (!mbar_wait(prm.wait, &traj_full[bf], (ti / 2) & 1, 17)) break;
                 if (!mbar_wait(prm.wait, &full_in[s], (ti / NS) & 1, 18)) break;
-                const T *vrow = vstage(s) + cw;
-                const TO *dyrow = dystage(s) + cw;
-                const TO *dyvrow = dyvstage(s) + cw;
+                const TV *vrow = vstage(s) + cw;
+                const TD *dyrow = dystage(s) + cw;
+                const TD *dyvrow = dyvstage(s) + cw;
                 const float4 *kqrow = kqstage(s) + j;
                 const float4 *traj = trajbuf(bf) + ctid;
                 float2 *parts = reinterpret_cast<float2 *>(trajbuf(bf)) + cwarp * 64 + lane;
@@ -573,7 +588,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
         const int htid = tid - 2 * NTC;
         const int hlane = htid & 31;
         constexpr uint32_t kBytesI = sizeof(T) * TT * MC, kBytesO = sizeof(TO) * TT * MC;
-        int produced = 0;
+        int produced = 0, raw_issued = 0;
         bool ok = true;
 
         if (htid < kProducers) {
@@ -586,7 +601,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
             const TO *dyvb = has_dyv ? static_cast<const TO *>(prm.dyv.ptr) + (long long)b * prm.dyv.sb + (long long)t_off * prm.dyv.st : nullptr;
             if (!has_dyv) {  // dyvar absent: its stage buffers stay zero for the whole kernel
                 for (int s = 0; s < NS; ++s)
-                    for (int idx = htid; idx < TT * MC; idx += kProducers) dyvstage(s)[idx] = from_f32<TO>(0.0f);
+                    for (int idx = htid; idx < TT * MC; idx += kProducers) dyvstage(s)[idx] = from_f32<TD>(0.0f);
             }
             // (k, q) of the next tile are on their way while the current one is handed over, so the loader never sits on a
             // global-memory latency: in registers up to 16 states, by per-thread asynchronous copies into shared memory
@@ -610,52 +625,107 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 stage_tile<T, TT, SPAD, kProducers>(raw(bf, 0), kb, prm.k.st, t0, L, 0, S, htid);
                 stage_tile<T, TT, SPAD, kProducers>(raw(bf, 1), qb, prm.q.st, t0, L, 0, S, htid);
             };
+            // the four activation tiles from step t0 on into T / TO buffers; with TMA one thread arrives on `bar` with their bytes
+            auto load_tiles = [&](int t0, auto *v, auto *lv, auto *dy, auto *dyv, uint64_t *bar) {
+                if (prm.use_tma) {
+                    if (htid == 0) {
+                        mbar_arrive_expect_tx(bar, 2 * kBytesI + (has_dyv ? 2 : 1) * kBytesO);
+                        tma_load_3d(v, &prm.tm_v, m_cta, t_off + t0, b, bar);
+                        tma_load_3d(lv, &prm.tm_lv, m_cta, t_off + t0, b, bar);
+                        tma_load_3d(dy, &prm.tm_dy, m_cta, t_off + t0, b, bar);
+                        if (has_dyv) tma_load_3d(dyv, &prm.tm_dyv, m_cta, t_off + t0, b, bar);
+                    }
+                } else {
+                    stage_tile<T, TT, MC, kProducers>(v, vb, prm.v.st, t0, L, m_cta, M, htid);
+                    stage_tile<T, TT, MC, kProducers>(lv, lb, prm.lv.st, t0, L, m_cta, M, htid);
+                    stage_tile<TO, TT, MC, kProducers>(dy, dyb, prm.dy.st, t0, L, m_cta, M, htid);
+                    if (has_dyv) stage_tile<TO, TT, MC, kProducers>(dyv, dyvb, prm.dyv.st, t0, L, m_cta, M, htid);
+                }
+            };
+            // bfloat16: tile number i of the walk (v, lambda_v, dy, dy_var as which = 0 .. 3) in the raw ring, its fetch, and the
+            // widening of one of its tensors
+            constexpr int NR = Sm::kRawTiles;
+            unsigned char *tiles_base = raw_base + 2 * Sm::kRawKq;
+            auto rawtile = [&](int i, int which) {
+                return reinterpret_cast<T *>(tiles_base + (i % NR) * Sm::kRaw +
+                                             (which < 2 ? which * Sm::kRawI : 2 * Sm::kRawI + (which - 2) * Sm::kRawO));
+            };
+            auto fetch_tiles = [&](int i) {
+                if constexpr (Sm::kWiden) {
+                    uint64_t *bar = &raw_full[i % NR];
+                    load_tiles((NT - 1 - i) * TT, rawtile(i, 0), rawtile(i, 1), reinterpret_cast<TO *>(rawtile(i, 2)),
+                               reinterpret_cast<TO *>(rawtile(i, 3)), bar);
+                    if (!prm.use_tma) {
+                        stage_arrive(bar);
+                        mbar_arrive(bar);
+                    }
+                    raw_issued = i + 1;
+                }
+            };
+            auto widen = [&](const auto *src, float *dst) {
+                if constexpr (sizeof(*src) == 2) {
+#pragma unroll 1
+                    for (int c = htid; c < TT * MC / 8; c += kProducers) {
+                        const uint4 x = reinterpret_cast<const uint4 *>(src)[c];
+                        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&x);
+                        const float2 f0 = __bfloat1622float2(h[0]), f1 = __bfloat1622float2(h[1]), f2 = __bfloat1622float2(h[2]),
+                                     f3 = __bfloat1622float2(h[3]);
+                        reinterpret_cast<float4 *>(dst)[2 * c] = make_float4(f0.x, f0.y, f1.x, f1.y);
+                        reinterpret_cast<float4 *>(dst)[2 * c + 1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int c = htid; c < TT * MC / 4; c += kProducers) reinterpret_cast<float4 *>(dst)[c] = reinterpret_cast<const float4 *>(src)[c];
+                }
+            };
             if (NT > 0) {
                 if (kInRegs) load_kq((NT - 1) * TT);
                 else fetch_kq((NT - 1) * TT, 0);
             }
-            for (int it = 0; it < NT; ++it) {
-                const int tile = NT - 1 - it, s = it % NS, t0 = tile * TT;
-                // the stage is free once the compute groups and the summing helpers are done with it
-                if (it >= NS && !mbar_wait(prm.wait, &empty_in[s], (it / NS - 1) & 1, 13, 100)) { ok = false; break; }
-                if (!kInRegs) {
-                    cp_async_wait_all();  // k, q of this tile, asked for a tile ago
-                    __syncwarp();
-                }
-                if (prm.use_tma) {
-                    if (htid == 0) {
-                        mbar_arrive_expect_tx(&full_in[s], 2 * kBytesI + (has_dyv ? 2 : 1) * kBytesO);
-                        tma_load_3d(vstage(s), &prm.tm_v, m_cta, t_off + t0, b, &full_in[s]);
-                        tma_load_3d(lstage(s), &prm.tm_lv, m_cta, t_off + t0, b, &full_in[s]);
-                        tma_load_3d(dystage(s), &prm.tm_dy, m_cta, t_off + t0, b, &full_in[s]);
-                        if (has_dyv) tma_load_3d(dyvstage(s), &prm.tm_dyv, m_cta, t_off + t0, b, &full_in[s]);
+            // (widening, the walk begins NR turns early with nothing but the fetches of the first raw tiles)
+#pragma unroll 1
+            for (int it = Sm::kWiden ? -NR : 0; it < NT; ++it) {
+                if (!Sm::kWiden || it >= 0) {
+                    const int tile = NT - 1 - it, s = it % NS, t0 = tile * TT;
+                    // the stage is free once the compute groups and the summing helpers are done with it
+                    if (it >= NS && !mbar_wait(prm.wait, &empty_in[s], (it / NS - 1) & 1, 13, 100)) { ok = false; break; }
+                    if (!kInRegs) {
+                        cp_async_wait_all();  // k, q of this tile, asked for a tile ago
+                        __syncwarp();
                     }
-                } else {
-                    stage_tile<T, TT, MC, kProducers>(vstage(s), vb, prm.v.st, t0, L, m_cta, M, htid);
-                    stage_tile<T, TT, MC, kProducers>(lstage(s), lb, prm.lv.st, t0, L, m_cta, M, htid);
-                    stage_tile<TO, TT, MC, kProducers>(dystage(s), dyb, prm.dy.st, t0, L, m_cta, M, htid);
-                    if (has_dyv)
-                        stage_tile<TO, TT, MC, kProducers>(dyvstage(s), dyvb, prm.dyv.st, t0, L, m_cta, M, htid);
-                }
-                if (!prm.use_tma) stage_arrive(&full_in[s]);
-                float4 *kq = kqstage(s);
-                if (kInRegs) {
+                    if constexpr (Sm::kWiden) {
+                        if (!mbar_wait(prm.wait, &raw_full[it % NR], (it / NR) & 1, 16)) { ok = false; break; }
+                        widen(rawtile(it, 0), vstage(s));
+                        widen(rawtile(it, 1), lstage(s));
+                        widen(reinterpret_cast<const TO *>(rawtile(it, 2)), dystage(s));
+                        if (has_dyv) widen(reinterpret_cast<const TO *>(rawtile(it, 3)), dyvstage(s));
+                    } else {
+                        load_tiles(t0, vstage(s), lstage(s), dystage(s), dyvstage(s), &full_in[s]);
+                        if (!prm.use_tma) stage_arrive(&full_in[s]);
+                    }
+                    float4 *kq = kqstage(s);
+                    if (kInRegs) {
 #pragma unroll
-                    for (int e = 0; e < (kInRegs ? KQP : 0); ++e) kq[htid + e * kProducers] = make_float4(kr[e], kr[e], qr[e], qr[e]);
-                    if (tile > 0) load_kq(t0 - TT);
-                } else {
-                    if (tile > 0) fetch_kq(t0 - TT, (it + 1) & 1);
-                    const T *rk = raw(it & 1, 0), *rq = raw(it & 1, 1);
+                        for (int e = 0; e < (kInRegs ? KQP : 0); ++e) kq[htid + e * kProducers] = make_float4(kr[e], kr[e], qr[e], qr[e]);
+                        if (tile > 0) load_kq(t0 - TT);
+                    } else {
+                        if (tile > 0) fetch_kq(t0 - TT, (it + 1) & 1);
+                        const T *rk = raw(it & 1, 0), *rq = raw(it & 1, 1);
 #pragma unroll 8
-                    for (int idx = htid; idx < TT * SPAD; idx += kProducers) {
-                        const float k = to_f32<T>(rk[idx]), q = to_f32<T>(rq[idx]);
-                        kq[idx] = make_float4(k, k, q, q);
+                        for (int idx = htid; idx < TT * SPAD; idx += kProducers) {
+                            const float k = to_f32<T>(rk[idx]), q = to_f32<T>(rq[idx]);
+                            kq[idx] = make_float4(k, k, q, q);
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
+                    // (test hook, as in the forward: the wait for tile skip_tile runs out)
+                    if ((Sm::kWiden || !(prm.use_tma && htid == 0)) && !(it == prm.wait.skip_tile && htid == 1)) mbar_arrive(&full_in[s]);
+                    produced = it + 1;
                 }
-                // (test hook, as in the forward: the wait for tile skip_tile runs out)
-                if (!(prm.use_tma && htid == 0) && !(it == prm.wait.skip_tile && htid == 1)) mbar_arrive(&full_in[s]);
-                produced = it + 1;
+                if constexpr (Sm::kWiden) {
+                    __syncwarp();  // the raw tile has been read
+                    if (it + NR < NT) fetch_tiles(it + NR);
+                }
             }
         } else {
             // ---- summing helpers: finish the sums of each processed tile
@@ -665,7 +735,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
             for (int jt = 0; jt < NT; ++jt) {
                 const int tile = NT - 1 - jt, s = jt % NS, t0 = tile * TT, bf = jt & 1;
                 const int n = min(TT, L - t0);
-                const T *vt = vstage(s);
+                const TV *vt = vstage(s);
                 const float2 *parts = reinterpret_cast<const float2 *>(trajbuf(bf));
                 if (!mbar_wait(prm.wait, &part_full[bf], (jt / 2) & 1, 14, 100)) break;
                 // dk, dq: add the CTA's channels. A unit is two neighbouring states of one step (the shares of lanes
@@ -755,7 +825,11 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
         }
         if (!ok) cp_async_wait_all();
         if (!ok && prm.use_tma && htid == 0) {
-            for (int t = max(0, produced - NS); t < produced; ++t) mbar_wait(prm.wait, &full_in[t % NS], (t / NS) & 1, 15);
+            if (Sm::kWiden)
+                for (int t = max(0, raw_issued - Sm::kRawTiles); t < raw_issued; ++t)
+                    mbar_wait(prm.wait, &raw_full[t % Sm::kRawTiles], (t / Sm::kRawTiles) & 1, 15);
+            else
+                for (int t = max(0, produced - NS); t < produced; ++t) mbar_wait(prm.wait, &full_in[t % NS], (t / NS) & 1, 15);
         }
     }
 }
