@@ -309,14 +309,9 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 const int n = min(TT, L - tile * TT);
                 if (!mbar_wait(prm.wait, &full_in[s], (ti / NS) & 1, 11)) break;
                 if (LOGV) {  // this warp's channels of the tile: log-variance -> precision, float32
-                    const TV *raw = lstage(s) + cwarp * CPW;
-                    float *lf = lfstage(s) + cwarp * CPW;
-                    for (int e = lane; e < TT * CPW; e += 32) {
-                        const int at = (e / CPW) * MC + e % CPW;
-                        lf[at] = precision_from_log_variance_fast(to_f32<TV>(raw[at]), prm.obs_var_min, prm.obs_var_max);
-                    }
-                    fence_proxy_async();  // these plain stores are ordered before the bulk copy that refills the stage
-                    __syncwarp();
+                    precisions_from_tile<TV, TT, MC, CPW>(lstage(s) + cwarp * CPW, lfstage(s) + cwarp * CPW, prm.obs_var_min,
+                                                          prm.obs_var_max, lane);
+                    __syncwarp();  // (in place where the stage is a bulk copy's: the loader's fence orders the two)
                 }
                 const TV *vrow = vstage(s) + cw;
                 const float4 *kqrow = kqstage(s) + j;
@@ -629,6 +624,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
             auto load_tiles = [&](int t0, auto *v, auto *lv, auto *dy, auto *dyv, uint64_t *bar) {
                 if (prm.use_tma) {
                     if (htid == 0) {
+                        if (LOGV && !Sm::kWiden) fence_proxy_async();  // the replay overwrote the log-variances in place
                         mbar_arrive_expect_tx(bar, 2 * kBytesI + (has_dyv ? 2 : 1) * kBytesO);
                         tma_load_3d(v, &prm.tm_v, m_cta, t_off + t0, b, bar);
                         tma_load_3d(lv, &prm.tm_lv, m_cta, t_off + t0, b, bar);

@@ -713,31 +713,45 @@ int kla_b200_epilogue_bwd(const kla_b200_epilogue_bwd_args *a, void *stream) {
     if (has_skip) { prm.z = t3(a->z); prm.dz = t3(a->dz); prm.skip = a->lambda_skip; prm.skip_len = a->lambda_skip_len; prm.dskip = a->dlambda_skip; }
     if (has_gate) { prm.gate = t3(a->gate); prm.dgate = t3(a->dgate); prm.gate_act = a->gate_activation; }
     prm.dy = t3(a->dy); prm.dy_var = t3(a->dy_var);
-    // four channels per thread when every tensor can be read and written as 4-element vectors
-    auto vec_ok = [&](const kla_b200_tensor3 &t, size_t sz) {
-        return t.ptr == nullptr || (aligned(t.ptr, 4 * sz) && t.stride_b % 4 == 0 && t.stride_t % 4 == 0);
+    // four channels per thread when every tensor can be read and written as 4-element vectors, eight when they are all
+    // bfloat16 and 8-element ones
+    auto vec_ok = [&](const kla_b200_tensor3 &t, size_t sz, int n) {
+        return t.ptr == nullptr || (aligned(t.ptr, n * sz) && t.stride_b % n == 0 && t.stride_t % n == 0);
     };
-    const bool vec = a->M % 4 == 0 && vec_ok(a->dout, osz) && vec_ok(a->dout_var, osz) && vec_ok(a->dy, osz) &&
-                     vec_ok(a->dy_var, osz) && (!has_gate || (vec_ok(a->gate, esz) && vec_ok(a->dgate, esz) &&
-                     vec_ok(a->y_raw, osz) && vec_ok(a->y_var_raw, osz))) && (!has_skip || (vec_ok(a->z, esz) && vec_ok(a->dz, esz)));
-    const int per = vec ? 4 : 1;
-    dim3 grid((unsigned)((a->M + 128 * per - 1) / (128 * per)), (unsigned)row_blocks, (unsigned)a->B);
-#define KLA_EPI_LAUNCH(T, TO)                                                                                   \
-    do {                                                                                                        \
-        if (vec) {                                                                                              \
-            if (has_skip && has_gate) kla_epilogue_bwd_kernel<T, TO, 4, true, true><<<grid, 128, 0, st>>>(prm);  \
-            else if (has_skip) kla_epilogue_bwd_kernel<T, TO, 4, true, false><<<grid, 128, 0, st>>>(prm);        \
-            else kla_epilogue_bwd_kernel<T, TO, 4, false, true><<<grid, 128, 0, st>>>(prm);                      \
-        } else {                                                                                                \
-            if (has_skip && has_gate) kla_epilogue_bwd_kernel<T, TO, 1, true, true><<<grid, 128, 0, st>>>(prm);  \
-            else if (has_skip) kla_epilogue_bwd_kernel<T, TO, 1, true, false><<<grid, 128, 0, st>>>(prm);        \
-            else kla_epilogue_bwd_kernel<T, TO, 1, false, true><<<grid, 128, 0, st>>>(prm);                      \
-        }                                                                                                       \
+    auto all_ok = [&](int n) {
+        return a->M % n == 0 && vec_ok(a->dout, osz, n) && vec_ok(a->dout_var, osz, n) && vec_ok(a->dy, osz, n) &&
+               vec_ok(a->dy_var, osz, n) && (!has_gate || (vec_ok(a->gate, esz, n) && vec_ok(a->dgate, esz, n) &&
+               vec_ok(a->y_raw, osz, n) && vec_ok(a->y_var_raw, osz, n))) && (!has_skip || (vec_ok(a->z, esz, n) && vec_ok(a->dz, esz, n)));
+    };
+    const int per = osz == 2 && all_ok(8) ? 8 : all_ok(4) ? 4 : 1;
+    // few rows per CTA until many of them would still give every SM four CTAs
+    const int64_t columns = (a->M + 128 * per - 1) / (128 * per);
+    const bool few = columns * a->B * row_blocks < 4 * 148;
+    const int rows = few ? kEpiFewRows : kEpiRows;
+    dim3 grid((unsigned)columns, (unsigned)((a->L + rows - 1) / rows), (unsigned)a->B);
+#define KLA_EPI_ROWS(T, TO, VEC, Z, G)                                                                   \
+    do {                                                                                                 \
+        if (few) kla_epilogue_bwd_kernel<T, TO, VEC, kEpiFewRows, Z, G><<<grid, 128, 0, st>>>(prm);       \
+        else kla_epilogue_bwd_kernel<T, TO, VEC, kEpiRows, Z, G><<<grid, 128, 0, st>>>(prm);              \
+    } while (0)
+#define KLA_EPI_HALVES(T, TO, VEC)                                \
+    do {                                                          \
+        if (has_skip && has_gate) KLA_EPI_ROWS(T, TO, VEC, true, true); \
+        else if (has_skip) KLA_EPI_ROWS(T, TO, VEC, true, false); \
+        else KLA_EPI_ROWS(T, TO, VEC, false, true);               \
+    } while (0)
+#define KLA_EPI_LAUNCH(T, TO)                   \
+    do {                                        \
+        if (per == 4) KLA_EPI_HALVES(T, TO, 4); \
+        else KLA_EPI_HALVES(T, TO, 1);          \
     } while (0)
     if (!has_skip && !has_gate) return KLA_B200_EINVAL;  // nothing to differentiate
     if (a->in_dtype == KLA_B200_F32) KLA_EPI_LAUNCH(float, float);
     else if (a->out_dtype == KLA_B200_F32) KLA_EPI_LAUNCH(__nv_bfloat16, float);
+    else if (per == 8) KLA_EPI_HALVES(__nv_bfloat16, __nv_bfloat16, 8);
     else KLA_EPI_LAUNCH(__nv_bfloat16, __nv_bfloat16);
+#undef KLA_EPI_HALVES
+#undef KLA_EPI_ROWS
 #undef KLA_EPI_LAUNCH
     g_launches++;
     e = cudaGetLastError();

@@ -293,6 +293,27 @@ __device__ __forceinline__ float from_f32<float>(float x) { return x; }
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 
+// A warp's columns of a [TT x MC] tile of log-variances -> float32 precisions (raw and lam point at its first column, and
+// may be the same memory). All of a lane's elements are read before the first is stored: one after the other, each behind
+// the stores before it, they cost the scan kernels 700 cycles a tile.
+template <typename T, int TT, int MC, int CPW>
+__device__ __forceinline__ void precisions_from_tile(const T *raw, float *lam, float vmin, float vmax, int lane) {
+    constexpr int N = TT * CPW, PER = (N + 31) / 32;
+    float x[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = lane + 32 * i;
+        x[i] = N % 32 == 0 || e < N ? to_f32<T>(raw[(e / CPW) * MC + e % CPW]) : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) x[i] = precision_from_log_variance_fast(x[i], vmin, vmax);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = lane + 32 * i;
+        if (N % 32 == 0 || e < N) lam[(e / CPW) * MC + e % CPW] = x[i];
+    }
+}
+
 // ---------------------------------------------------------------- mbarrier + TMA
 //
 // Producer/consumer hand-off between helper and compute warps uses mbarrier

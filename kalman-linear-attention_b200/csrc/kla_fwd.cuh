@@ -91,7 +91,7 @@ struct FwdSmem {
 // SEG: sequences cut into segments (FwdParams::seg, SegCtl). Again a separate instantiation: the unsegmented kernel
 // then carries none of that code (with it, one CTA per SM ran 3 % slower).
 template <typename T, typename TO, int SPT, int LPC, int CH, int NW, int NH, int TT, bool PRIOR, bool EPI, bool SEG>
-__global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC <= 8 ? 3 : 1) kla_fwd_kernel(const __grid_constant__ FwdParams prm) {
+__global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI ? 4 : LPC <= 8 ? 3 : 1) kla_fwd_kernel(const __grid_constant__ FwdParams prm) {
     using Sh = ScanShape<SPT, LPC, CH, NW, NH, TT>;
     using Sm = FwdSmem<T, SPT, LPC, CH, NW, NH, TT>;
     constexpr int SPAD = Sh::kSPad, MC = Sh::kMC, MCP = Sh::kMCP;
@@ -99,10 +99,11 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
     constexpr int HP = SPT / 2;  // pairs of states per thread
     static_assert(SPT % 2 == 0, "states are processed in pairs");
     // helper warps split by task: the first NH/2 load and stage inputs, the others sum and store outputs
-    // With the epilogue the drainers carry the heavier load (activation, skip, second store): three drainer warps
-    // and one loader warp there, where that keeps a drainer thread on one channel pair from tile to tile.
+    // With the epilogue the drainers carry the heavier load (activation, skip, second store): one loader warp and three
+    // drainers there, where that keeps a drainer thread on one channel pair from tile to tile. With six helpers (a CTA alone
+    // on its SM, see the launcher) two load and four drain.
     constexpr bool kWideDrain = EPI && NH == 4 && (3 * 32) % (MC / 2) == 0;
-    constexpr int kProducers = kWideDrain ? 32 : (NH / 2) * 32, kDrainers = Sh::kHelpers - kProducers;
+    constexpr int kProducers = kWideDrain ? 32 : NH == 6 ? 64 : (NH / 2) * 32, kDrainers = Sh::kHelpers - kProducers;
     static_assert(NH >= 2, "one loading and one storing helper warp at least");
     static_assert(TT % kCkptInterval == 0, "checkpoints fall on fixed steps of a tile");
 
@@ -334,14 +335,9 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
             const int t0 = tile * TT;
             if (!mbar_wait(prm.wait, &full_in[s], (tile / NS) & 1, 1)) break;
             if (pro) {  // this warp's channels of the tile: log-variance -> precision, float32
-                const T *raw = lstage(s) + warp * Sh::kCPW;
-                float *lf = lfstage(s) + warp * Sh::kCPW;
-                for (int e = lane; e < TT * Sh::kCPW; e += 32) {
-                    const int at = (e / Sh::kCPW) * MC + e % Sh::kCPW;
-                    lf[at] = precision_from_log_variance_fast(to_f32<T>(raw[at]), prm.obs_var_min, prm.obs_var_max);
-                }
-                fence_proxy_async();  // these plain stores are ordered before the bulk copy that refills the stage
-                __syncwarp();
+                precisions_from_tile<T, TT, MC, Sh::kCPW>(lstage(s) + warp * Sh::kCPW, lfstage(s) + warp * Sh::kCPW,
+                                                          prm.obs_var_min, prm.obs_var_max, lane);
+                __syncwarp();  // (float32: in place, ordered before the bulk copy that refills the stage by the loader's fence)
             }
             if (tile >= NO && !mbar_wait(prm.wait, &empty_out[o], (tile / NO - 1) & 1, 2)) break;
             if (ck != nullptr) store_ckpt();
@@ -443,6 +439,9 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 ? 1 : !EPI ? 4 : LPC 
                 if (it >= NS && !mbar_wait(prm.wait, &empty_in[s], (it / NS - 1) & 1, 3, 100)) { ok = false; break; }
                 if (prm.use_tma) {
                     if (htid == 0) {
+                        // float32 log-variances were overwritten in place by the compute warps; as a fence of theirs it held
+                        // up every tile (bfloat16 needs none: its precisions have a buffer no bulk copy writes)
+                        if (sizeof(T) == 4 && pro) fence_proxy_async();
                         mbar_arrive_expect_tx(&full_in[s], 2 * kTileBytes);
                         tma_load_3d(vstage(s), &prm.tm_v, m_cta, t_off + t0, b, &full_in[s]);
                         tma_load_3d(lstage(s), &prm.tm_lv, m_cta, t_off + t0, b, &full_in[s]);

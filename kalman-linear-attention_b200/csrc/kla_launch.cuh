@@ -18,6 +18,7 @@ constexpr int kNW = KLA_NW;            // compute warps per CTA
 #define KLA_NH 4
 #endif
 constexpr int kNH = KLA_NH;            // helper warps per CTA
+constexpr int kEpiNH = 6;             // ... of the forward with epilogue where every CTA has an SM to itself
 constexpr int kTT = 16;                // steps per tile of the forward (two checkpoints)
 constexpr int kBwdTT = kCkptInterval;  // steps per tile of the backward
 #ifndef KLA_SPT
