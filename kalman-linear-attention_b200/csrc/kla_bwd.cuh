@@ -49,7 +49,7 @@
 // on; the state its walk starts from needs no hand-over, the replay group computes it from the checkpoints.
 //
 // Measured on B200 at T=4096, M=1024, S=16, float32, against the kernel with one channel per thread and scalar
-// arithmetic: B=8 1.42 -> 1.17 ms, B=4 0.88 -> 0.71 ms, B=16 2.59 -> 2.16 ms; 46 instead of 66 warp instructions per 32
+// arithmetic: B=8 1.42 -> 1.15 ms, B=4 0.88 -> 0.69 ms, B=16 2.59 -> 2.13 ms; 43.5 instead of 66 warp instructions per 32
 // lane-steps. What bounds it is the FP32 pipe's register reads: 30 pair operations per two chains and step in the
 // reverse walk and 8 in the replay, 12 and 2 of them three-operand FMAs at 3.75 cycles (kla_common.cuh), add up to about
 // 235 of the 291 cycles a scheduler spends on a warp's step. Not limits: shared memory (the trajectory through tensor
