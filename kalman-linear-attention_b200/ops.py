@@ -155,7 +155,14 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
     mc = 4 * (32 // lpc)
     ctas = B * ((M + mc - 1) // mc)
     if requested is None:
-        if ctas == 0 or 3 * ctas > _RESIDENT_CTAS:
+        # Not below 640 steps, where the uncut kernels are done before three launches are (B=1 L=300 M=512: 27 us against
+        # 36 to 52 cut, training 163 against 220 to 275). From about 90 CTAs on cutting breaks even, and only for long
+        # sequences (96 CTAs: L=900 66 / 234 uncut, 77 / 246 cut; L=2048 143 / 499 and 148 / 491; L=4096 280 / 985 and
+        # 273 / 906), or for rows that TMA cannot read, which a CTA stages too slowly (B=3 L=1537 M=1001 training 540 and
+        # 451).
+        if ctas == 0 or 3 * ctas > _RESIDENT_CTAS or L < 640:
+            return 1
+        if 10 * ctas > 3 * _RESIDENT_CTAS and L < 2048 and M % 4 == 0:
             return 1
         # Whole rounds of the resident slots: enough chunks for one, more rounds while chunks are longer than about 256
         # steps, which evens out the last one. Measured on B200, forward / training step in us: B=1 L=1536 M=1536
@@ -164,6 +171,8 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
         rounds = 1
         while (want := min(16, rounds * _RESIDENT_CTAS // ctas)) < 16 and L > 288 * want:
             rounds += 1
+        if L % want:  # equal chunks where a neighbouring count gives them
+            want = next((c for c in (want + 1, want - 1) if 1 < c <= 16 and L % c == 0), want)
     else:
         want = max(1, int(requested))
     want = min(want, max(1, L // _MIN_CHUNK_STEPS), max(1, 65535 // max(B, 1)))

@@ -26,8 +26,9 @@ def _rel(got, ref):
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,L,M,S,dtype", [
     (1, 1037, 33, 16, torch.float32),    # 16 chunks of 80 steps, the last one 77 short; odd channels
-    (2, 129, 1001, 16, torch.float32),   # two chunks, 80 + 49
-    (1, 65, 7, 16, torch.float32),       # one chunk of 64 steps would leave a step over
+    (2, 641, 40, 16, torch.float32),     # chunks of 80 steps and one of a single step
+    (1, 700, 7, 16, torch.bfloat16),     # 7 channels in bfloat16, the last chunk short
+    (2, 129, 1001, 16, torch.float32),   # too short to cut
     (3, 200, 35, 16, torch.bfloat16),    # bfloat16 rows off every 4-byte boundary
     (2, 77, 34, 24, torch.bfloat16),     # even bfloat16 rows, padded states
     (2, 150, 19, 40, torch.float32),     # k, q of wide states, S not a power of two
