@@ -428,6 +428,11 @@ int kla_b200_add_norm(int64_t rows, int64_t D, int32_t dtype, int32_t weight_dty
                       const void *weight, float eps, void *sum, void *out, void *stream);
 int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up, void *out, void *stream);
 
+/* k and q [B, L, S] l2-normalised over S (x / max(|x|, 1e-12)) and, with clip > 0, clamped to [-clip, clip]
+ * (src/kla/layers/kla_layer.py:217-222), into contiguous tensors of the same type. */
+int kla_b200_qk_norm(int64_t B, int64_t L, int64_t S, int32_t dtype, kla_b200_tensor3 k, kla_b200_tensor3 q, float clip, void *k_out,
+                     void *q_out, void *stream);
+
 /* out[r] = index of the first largest of x[r, 0 .. n-1] (a NaN counts as the largest), n >= 1: the greedy choice of a token
  * (src/kla/models/sequence_model.py:222-225). */
 int kla_b200_argmax(int64_t rows, int64_t n, int32_t dtype, const void *x, int64_t row_stride, int64_t *out, void *stream);

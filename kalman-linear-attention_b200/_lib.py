@@ -35,6 +35,7 @@ SYMBOLS = (
     "kla_b200_add_norm",
     "kla_b200_swiglu",
     "kla_b200_argmax",
+    "kla_b200_qk_norm",
     "kla_b200_mobius_scan_fwd",
     "kla_b200_mobius_scan_bwd",
     "kla_b200_affine_scan_fwd",
@@ -244,7 +245,7 @@ def load() -> ctypes.CDLL:
 _host = None
 _HOST_ENTRIES = (
     "scan_fwd", "scan_bwd", "slab_aggregate", "chunk_fold", "epilogue_bwd", "step", "conv_step", "step_layer",
-    "linear", "add_norm", "swiglu", "argmax", "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
+    "linear", "add_norm", "swiglu", "argmax", "qk_norm", "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
     "ckpt_bytes", "segment_scratch_bytes", "strerror",
 )
 

@@ -108,6 +108,44 @@ __global__ void __launch_bounds__(128) kla_add_norm_kernel(const __grid_constant
     }
 }
 
+// The keys and queries of a prompt, l2-normalised over their states and clipped (src/kla/layers/kla_layer.py:217-222;
+// common.py:25-27): one warp per (batch element, step), k in its lower and q in its upper half. As tensor operations six
+// launches and 22 us at B=4 L=8192 S=16.
+struct QkNormParams {
+    int B, L, S;
+    Tensor3 k, q;  // [B, L, S]
+    void *ko, *qo; // [B, L, S] contiguous
+    float clip;    // 0: none
+};
+
+template <typename T>
+__global__ void __launch_bounds__(128) kla_qk_norm_kernel(const __grid_constant__ QkNormParams prm) {
+    const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (row >= (long long)prm.B * prm.L) return;  // whole warps
+    const int b = (int)(row / prm.L), t = (int)(row % prm.L), S = prm.S;
+    const int half = (threadIdx.x >> 4) & 1, lane = threadIdx.x & 15;
+    const Tensor3 &in = half ? prm.q : prm.k;
+    const T *x = static_cast<const T *>(in.ptr) + (long long)b * in.sb + (long long)t * in.st;
+    T *o = static_cast<T *>(half ? prm.qo : prm.ko) + row * S;
+    float v[8], ss = 0.0f;  // S <= 128
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int s = lane + 16 * i;
+        v[i] = s < S ? to_f32<T>(x[s]) : 0.0f;
+        ss = fmaf(v[i], v[i], ss);
+    }
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+    const float n = fmaxf(sqrtf(ss), 1e-12f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int s = lane + 16 * i;
+        float y = v[i] / n;
+        if (prm.clip > 0.0f) y = fminf(fmaxf(y, -prm.clip), prm.clip);
+        if (s < S) o[s] = from_f32<T>(y);
+    }
+}
+
 // Index of the first largest value of each row (a NaN counts as the largest): a CTA per row, each thread a strided share.
 // The reduction of a [8, 50304] bfloat16 head took 14 us as a tensor operation.
 template <typename T>

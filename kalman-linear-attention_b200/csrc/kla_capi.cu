@@ -947,6 +947,26 @@ int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up,
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
 }
 
+int kla_b200_qk_norm(int64_t B, int64_t L, int64_t S, int32_t dtype, kla_b200_tensor3 k, kla_b200_tensor3 q, float clip, void *k_out,
+                     void *q_out, void *stream) {
+    int rc = check_common(B, L, 1, S, dtype, dtype);
+    if (rc) return rc;
+    if (B == 0 || L == 0 || S == 0) return KLA_B200_OK;
+    const size_t esz = dtype == KLA_B200_F32 ? 4 : 2;
+    if (!k_out || !q_out) return KLA_B200_EINVAL;
+    if ((rc = check_t3(k, esz, true)) || (rc = check_t3(q, esz, true))) return rc;
+    if (!aligned(k_out, esz) || !aligned(q_out, esz)) return KLA_B200_EALIGN;
+    const long long blocks = (B * L + 3) / 4;
+    if (blocks > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;
+    const QkNormParams prm{(int)B, (int)L, (int)S, t3(k), t3(q), k_out, q_out, clip};
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (dtype == KLA_B200_BF16) kla_qk_norm_kernel<__nv_bfloat16><<<(unsigned)blocks, 128, 0, st>>>(prm);
+    else kla_qk_norm_kernel<float><<<(unsigned)blocks, 128, 0, st>>>(prm);
+    g_launches++;
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
+}
+
 int kla_b200_argmax(int64_t rows, int64_t n, int32_t dtype, const void *x, int64_t row_stride, int64_t *out, void *stream) {
     if (rows < 0 || n < 1 || row_stride < 0) return KLA_B200_EINVAL;
     if (n > (1 << 30) || rows > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;

@@ -39,6 +39,7 @@ struct Entry {
     int (*linear)(const kla_b200_linear_args *, void *) = nullptr;
     int (*add_norm)(int64_t, int64_t, int32_t, int32_t, const void *, const void *, const void *, float, void *, void *, void *) = nullptr;
     int (*swiglu)(int64_t, int64_t, int32_t, const void *, void *, void *) = nullptr;
+    int (*qk_norm)(int64_t, int64_t, int64_t, int32_t, kla_b200_tensor3, kla_b200_tensor3, float, void *, void *, void *) = nullptr;
     int (*argmax)(int64_t, int64_t, int32_t, const void *, int64_t, int64_t *, void *) = nullptr;
     int (*conv_seq)(const kla_b200_conv_seq_args *, void *) = nullptr;
     int (*conv_seq_bwd)(const kla_b200_conv_seq_bwd_args *, void *) = nullptr;
@@ -65,6 +66,7 @@ void bind(const py::dict &d) {
     take(lib.linear, d, "kla_b200_linear");
     take(lib.add_norm, d, "kla_b200_add_norm");
     take(lib.swiglu, d, "kla_b200_swiglu");
+    take(lib.qk_norm, d, "kla_b200_qk_norm");
     take(lib.argmax, d, "kla_b200_argmax");
     take(lib.conv_seq, d, "kla_b200_conv_seq");
     take(lib.conv_seq_bwd, d, "kla_b200_conv_seq_bwd");
@@ -455,6 +457,23 @@ Tensor swiglu(const Tensor &gu) {
     return out;
 }
 
+// k, q [B, L, S] l2-normalised over S, then clamped to [-clip, clip] when clip > 0
+std::tuple<Tensor, Tensor> qk_norm(const Tensor &k, const Tensor &q, double clip) {
+    const c10::cuda::CUDAGuard guard(k.device());
+    const auto T = k.scalar_type();
+    if (!k.is_cuda() || (T != at::kFloat && T != at::kBFloat16) || q.scalar_type() != T || k.dim() != 3 || q.sizes() != k.sizes() ||
+        !rows_ok(k) || !rows_ok(q) || k.size(2) > KLA_B200_MAX_DSTATE || !sm100(k.device())) {
+        auto one = [clip](const Tensor &x) {
+            const Tensor y = x / x.norm(2, -1, true).clamp_min(1e-12);
+            return clip > 0.0 ? y.clamp(-clip, clip) : y;
+        };
+        return {one(k), one(q)};
+    }
+    Tensor ko = fresh(k, k.sizes()), qo = fresh(q, q.sizes());
+    check(lib.qk_norm(k.size(0), k.size(1), k.size(2), dt(T), t3(k), t3(q), (float)clip, ko.data_ptr(), qo.data_ptr(), stream_of(k)));
+    return {ko, qo};
+}
+
 // out[...] (int64) = argmax of x[..., n] over its last dimension; returns out
 Tensor argmax(const Tensor &x, Tensor out) {
     const c10::cuda::CUDAGuard guard(x.device());
@@ -618,6 +637,7 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("add_norm", &add_norm);
     m.def("swiglu", &swiglu);
     m.def("argmax", &argmax);
+    m.def("qk_norm", &qk_norm);
     m.def("project", &project);
     m.def("swiglu_step", &swiglu_step);
 }

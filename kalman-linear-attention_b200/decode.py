@@ -142,11 +142,11 @@ class LayerDecoder:
             conv_state.copy_(new_window)
             z = zc
         v, ls, k, q = self._sensors(z, self._linear(z, "sensor_proj"))
-        if cfg["qk_norm"]:  # [B, L, S]: small next to the [B, L, M] tensors, left to torch
-            k = k / k.norm(dim=-1, keepdim=True).clamp_min(1e-12)
-            q = q / q.norm(dim=-1, keepdim=True).clamp_min(1e-12)
-        if cfg["clip_value"] is not None:
-            k, q = k.clamp(-cfg["clip_value"], cfg["clip_value"]), q.clamp(-cfg["clip_value"], cfg["clip_value"])
+        clip = cfg["clip_value"]
+        if cfg["qk_norm"]:
+            k, q = _lib.host().qk_norm(k, q, clip or 0.0)
+        if clip is not None and (clip == 0 or not cfg["qk_norm"]):
+            k, q = k.clamp(-clip, clip), q.clamp(-clip, clip)
         epi = {}
         if self.skip is not None:
             epi.update(z=z, lambda_skip=self.skip)

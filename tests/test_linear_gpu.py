@@ -102,3 +102,17 @@ def test_greedy_choice(rows, n, dtype):
     assert torch.equal(got, first)
     x[-1, n // 2:] = float("nan")
     assert lib.host().argmax(x, got)[-1] == n // 2
+
+
+@pytest.mark.parametrize("B,L,S,clip", [(1, 1, 1, 0.0), (2, 5, 16, 0.0), (1, 3, 17, 0.3), (3, 2, 100, 0.05), (1, 4, 128, 0.0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_keys_and_queries_are_normalised_and_clipped(B, L, S, clip, dtype):
+    g = torch.Generator(device="cuda").manual_seed(S)
+    wide = torch.randn(B, L, 2 * S + 3, generator=g, device="cuda").to(dtype)  # slices of a projection
+    k, q = wide[..., 1:1 + S], wide[..., S + 2:2 * S + 2]
+    k[0, 0] = 0
+    tol = dict(rtol=1e-2, atol=1e-3) if dtype == torch.bfloat16 else dict(rtol=1e-6, atol=1e-7)
+    for got, x in zip(lib.host().qk_norm(k, q, clip), (k, q)):
+        want = x.double() / x.double().norm(dim=-1, keepdim=True).clamp_min(1e-12)
+        assert got.dtype == dtype and got.is_contiguous()
+        torch.testing.assert_close(got.double(), want.clamp(-clip, clip) if clip else want, **tol)
