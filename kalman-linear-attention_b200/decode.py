@@ -254,12 +254,12 @@ class ModelDecoder:
     reference's ``SequenceModel.forward`` with a state and ``SequenceModel.generate``
     (src/kla/models/sequence_model.py:150-173, 200-220).
 
-    A block is ``x += mixer(norm(x))`` then ``x += mlp(norm(x))`` (sequence_model.py:47-98). The mixers run
-    through :class:`LayerDecoder` (two fused kernels per layer and token, the scan kernels for the prompt); the
-    norms, the channel MLPs, the embedding and the LM head are a handful of library calls each and stay torch
-    operations. One decoded token is a fixed sequence of launches over state that is updated in place, so
-    ``generate`` captures it once in a CUDA graph and replays it: a token then costs no host work but one replay,
-    where the reference's loop issues several hundred small launches per token from Python.
+    A block is ``x += mixer(norm(x))`` then ``x += mlp(norm(x))`` (sequence_model.py:47-98). For one token of up to 32
+    sequences in bfloat16 that is six kernels: the projections with norm, convolution step, gate and residual sum folded
+    in, and the filter step. For a prompt the projections are library GEMMs and what stands between them one kernel each.
+    One decoded token is a fixed sequence of launches over state that is updated in place, so ``generate`` captures it in
+    a CUDA graph, which it keeps for calls with the same batch, types and weights, and replays it: a token then costs no
+    host work but one replay, where the reference's loop issues several hundred small launches per token from Python.
 
     Built from plain tensors (``SequenceModel.state_dict()``) and plain config dicts; ``from_model`` reads them
     off a reference model. The reference package is not needed at run time."""
