@@ -2,10 +2,11 @@
 
 The reference layer's decode route (``KLALayer.forward`` with a state and ``L == 1``,
 src/kla/layers/kla_layer.py:295-345) is three projections with elementwise work between
-them. ``LayerDecoder.step`` keeps the projections as library GEMMs and runs the rest as two
-kernels: ``kla_b200_conv_step`` (``CausalConv1d`` advanced by one token,
-src/kla/layers/common.py:87-96) and ``kla_b200_step_layer`` (sensor post-processing, the
-filter step, skip path and gate; kla_layer.py:199-231, 277-293, 329-338).
+them. ``LayerDecoder.step`` runs them as ``kla_b200_linear`` for up to 32 bfloat16 rows, the
+first with the step of ``CausalConv1d`` (src/kla/layers/common.py:87-96) inside, and as library
+GEMMs around ``kla_b200_conv_step`` otherwise; between the second and the third stands
+``kla_b200_step_layer`` (sensor post-processing, the filter step, skip path and gate;
+kla_layer.py:199-231, 277-293, 329-338).
 
 A decoder is built from plain tensors and a plain config dict, so it does not need the
 reference package at run time; ``LayerDecoder.from_layer`` reads both off a reference
