@@ -381,20 +381,23 @@ int act_code(const py::object &name) {  // the activation's name in a config, or
 }
 
 // Whether kla_b200_linear takes the projection: a few bfloat16 rows, nothing to differentiate, vectors aligned; with a norm
-// the normalised rows must fit shared memory.
+// the normalised rows must fit shared memory. The kernel is given pointers, so whatever does not agree in shape or device
+// is left to the tensor operations, which raise their own errors.
 bool few_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const OptTensor &norm_w) {
-    const int64_t K = w.size(1);
+    if (x.dim() != 2 || w.dim() != 2 || !x.is_cuda()) return false;
+    const int64_t N = w.size(0), K = w.size(1);
     auto fits = [K](int64_t rows) {  // KLA_B200_LINEAR_SMEM
         int64_t n = 8;
         while (n < rows) n *= 2;
         return n * (K + 8) * 2 + 1024 * (n + 2) <= KLA_B200_LINEAR_SMEM;
     };
-    auto plain = [](const Tensor &t) { return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.is_cuda(); };
-    return x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.size(0) >= 1 && x.size(0) <= KLA_B200_LINEAR_MAX_ROWS && x.stride(1) == 1 &&
-           x.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && K % 8 == 0 && plain(w) &&
-           reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0 && (!bias || plain(*bias)) &&
-           (!norm_w || (plain(*norm_w) && reinterpret_cast<uintptr_t>(norm_w->data_ptr()) % 16 == 0)) && fits(x.size(0)) &&
-           !wants_grad({&x, &w}) && sm100(x.device());
+    auto plain = [&x](const Tensor &t) { return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.device() == x.device(); };
+    auto vector = [&plain](const OptTensor &t, int64_t n) { return !t || (plain(*t) && t->dim() == 1 && t->size(0) == n); };
+    return x.scalar_type() == at::kBFloat16 && x.size(0) >= 1 && x.size(0) <= KLA_B200_LINEAR_MAX_ROWS && x.size(1) == K && K >= 8 &&
+           x.stride(1) == 1 && x.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && K % 8 == 0 && plain(w) &&
+           reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0 && vector(bias, N) && vector(norm_w, K) &&
+           (!norm_w || reinterpret_cast<uintptr_t>(norm_w->data_ptr()) % 16 == 0) && fits(x.size(0)) &&
+           !wants_grad({&x, &w, bias ? &*bias : &x, norm_w ? &*norm_w : &x}) && sm100(x.device());
 }
 
 struct Extra {  // what kla_b200_linear does besides the projection
@@ -424,16 +427,17 @@ Tensor rms_norm(const Tensor &x, const Tensor &w, double eps) {  // RMSNorm, src
     return (xf * at::rsqrt(xf.pow(2).mean(-1, true) + eps) * w.to(at::kFloat)).to(x.scalar_type());
 }
 
-bool vec_rows(const Tensor &t) {  // rows that 16-byte accesses can walk
-    return t.is_cuda() && t.is_contiguous() && (t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kFloat) && t.size(-1) % 8 == 0 &&
+bool vec_rows(const Tensor &t) {  // rows, at least one, that 16-byte accesses can walk
+    return t.is_cuda() && t.dim() >= 1 && t.numel() > 0 && t.is_contiguous() && (t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kFloat) && t.size(-1) % 8 == 0 &&
            reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
 }
 
 // x + delta (x itself without delta) and its RMSNorm
 std::tuple<Tensor, Tensor> add_norm(const Tensor &x, const OptTensor &delta, const Tensor &w, double eps) {
     const c10::cuda::CUDAGuard guard(x.device());
-    if (!vec_rows(x) || !vec_rows(w) || (delta && (!vec_rows(*delta) || delta->scalar_type() != x.scalar_type() || delta->sizes() != x.sizes())) ||
-        wants_grad({&x, &w}) || !sm100(x.device())) {
+    if (!vec_rows(x) || !vec_rows(w) || w.dim() != 1 || w.size(0) != x.size(-1) || w.device() != x.device() ||
+        (delta && (!vec_rows(*delta) || delta->scalar_type() != x.scalar_type() || delta->sizes() != x.sizes() || delta->device() != x.device())) ||
+        wants_grad({&x, &w, delta ? &*delta : &x}) || !sm100(x.device())) {
         const Tensor sum = delta ? x + *delta : x;
         return {sum, rms_norm(sum, w, eps)};
     }
@@ -491,7 +495,12 @@ constexpr int64_t kWideHead = 8192;
 // norm (when norm_w is given), projection, residual sum (when given)
 Tensor project(const Tensor &x, const Tensor &w, const OptTensor &bias, const OptTensor &norm_w, double eps, const OptTensor &residual) {
     const c10::cuda::CUDAGuard guard(x.device());
-    if (w.size(0) < kWideHead && few_rows(x, w, bias, norm_w) && (!residual || (residual->scalar_type() == at::kBFloat16 && residual->stride(-1) == 1)))
+    auto sums = [&] {  // the residual is one the kernel can add
+        return !residual || (residual->scalar_type() == at::kBFloat16 && residual->dim() == 2 && residual->size(0) == x.size(0) &&
+                             residual->size(1) == w.size(0) && residual->stride(1) == 1 && residual->device() == x.device() &&
+                             !wants_grad({&*residual}));
+    };
+    if (w.size(0) < kWideHead && few_rows(x, w, bias, norm_w) && sums())
         return linear_rows(x, w, bias, Extra{norm_w, eps, residual});
     const Tensor out = at::linear(norm_w ? std::get<1>(add_norm(x, {}, *norm_w, eps)) : x, w, bias);
     return residual ? *residual + out : out;

@@ -116,3 +116,35 @@ def test_keys_and_queries_are_normalised_and_clipped(B, L, S, clip, dtype):
         want = x.double() / x.double().norm(dim=-1, keepdim=True).clamp_min(1e-12)
         assert got.dtype == dtype and got.is_contiguous()
         torch.testing.assert_close(got.double(), want.clamp(-clip, clip) if clip else want, **tol)
+
+
+def test_shapes_that_do_not_agree_raise_or_broadcast_as_tensor_operations_do():
+    """The kernels are given pointers: a row shorter than the weights' is for the tensor operations to refuse."""
+    rn = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    host, B, N, K = lib.host(), 4, 48, 64
+    w, norm_w, res = rn(N, K), rn(K), rn(B, N)
+    for x in (rn(B, K - 8), rn(B, K + 8), rn(B, 8)):
+        with pytest.raises(RuntimeError):
+            host.project(x, w, None, None, 0.0, None)
+        with pytest.raises(RuntimeError):
+            host.project(x, w, None, norm_w, 1e-6, None)
+        with pytest.raises(RuntimeError):
+            host.swiglu_step(x, norm_w, 1e-6, w, None, rn(K, N // 2), None)
+    x = rn(B, K)
+    for bad in (dict(bias=rn(N - 8)), dict(norm=rn(K // 2)), dict(res=rn(B, N - 8)), dict(res=rn(B - 1, N)), dict(bias=rn(N).cpu()),
+                dict(norm=rn(K).cpu())):
+        with pytest.raises(RuntimeError):
+            host.project(x, w, bad.get("bias"), bad.get("norm"), 1e-6, bad.get("res"))
+    with pytest.raises(RuntimeError):  # the MLP's output is narrower than what it is added to
+        host.swiglu_step(x, norm_w, 1e-6, w, None, rn(K - 8, N // 2), None)
+    for wrong in (rn(K - 8), rn(2 * K)):
+        with pytest.raises(RuntimeError):
+            host.add_norm(x, None, wrong, 1e-6)
+    with pytest.raises(RuntimeError):
+        host.add_norm(x, rn(B, K - 8), norm_w, 1e-6)
+    # one value for all columns, one row for all rows: broadcast
+    one = rn(1)
+    close(host.add_norm(x, None, one, 1e-6)[1], norm(x, one, 1e-6))
+    close(host.project(x, w, None, None, 0.0, res[:1]), F.linear(x.float(), w.float()) + res[:1].float())
+    assert host.add_norm(rn(0, K), None, norm_w, 1e-6)[1].shape == (0, K) and host.swiglu(rn(0, K)).shape == (0, K // 2)
+    assert host.add_norm(rn(B, 0), None, rn(0), 1e-6)[1].shape == (B, 0) and host.swiglu(rn(B, 0)).shape == (B, 0)
