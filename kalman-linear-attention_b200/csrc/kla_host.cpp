@@ -91,6 +91,20 @@ void check(int rc) {
     throw std::runtime_error("kla_b200: " + msg);
 }
 
+// Tensors the kernels would read or write past their end, or as another type.
+void require(bool ok, const char *what) {
+    if (!ok) throw py::value_error(std::string("kla_b200: ") + what);
+}
+void require_type(const Tensor &t) {
+    const auto T = t.scalar_type();
+    if (T == at::kFloat || T == at::kBFloat16) return;
+    PyErr_SetString(PyExc_NotImplementedError, (std::string("The b200 kernels take float32 or bfloat16 activations, not ") + c10::toString(T) + ".").c_str());
+    throw py::error_already_set();
+}
+bool is(const Tensor &t, const at::Device &dev, at::ScalarType type, at::IntArrayRef sizes) {
+    return t.device() == dev && t.scalar_type() == type && t.sizes() == sizes && t.is_contiguous();
+}
+
 kla_b200_tensor3 t3(const Tensor &t) { return kla_b200_tensor3{t.data_ptr(), t.stride(0), t.stride(1)}; }
 kla_b200_tensor3 t3(const OptTensor &t) { return t ? t3(*t) : kla_b200_tensor3{nullptr, 0, 0}; }
 float *fp(const Tensor &t) { return static_cast<float *>(t.data_ptr()); }
@@ -293,7 +307,12 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> epilogue_bwd(const T
 // kla_b200_conv_seq -> z, the window after the sequence
 std::tuple<Tensor, Tensor> conv_seq(const Tensor &x, const Tensor &w, const OptTensor &bias, const Tensor &state, int act) {
     const c10::cuda::CUDAGuard guard(x.device());
+    require_type(x);
+    require(x.dim() == 3 && w.dim() == 2 && w.size(0) == x.size(2) && w.size(1) >= 1, "the convolution takes x [B, L, D] and weights [D, K]");
     const int64_t B = x.size(0), L = x.size(1), D = x.size(2);
+    require(rows_ok(x) && is(w, x.device(), at::kFloat, w.sizes()) && (!bias || is(*bias, x.device(), at::kFloat, {D})) &&
+                is(state, x.device(), x.scalar_type(), {B, D, w.size(1) - 1}),
+            "the convolution's window must be [B, D, K - 1] of x's type, its weights float32, all contiguous and on one device");
     Tensor z = fresh(x, {B, L, D}), next = fresh(state, state.sizes());
     kla_b200_conv_seq_args c{};
     c.B = B; c.L = L; c.D = D; c.K = w.size(1); c.dtype = dt(x.scalar_type()); c.activation = act;
@@ -548,11 +567,26 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
         return py::reinterpret_borrow<py::object>(o);
     };
     void *stream = stream_of(x);
+    require_type(x);
+    require(x.dim() == 2 && a_bar.dim() == 2, "a token is [B, d_model]");
+    const auto dev = x.device();
     const int64_t B = x.size(0), M = a_bar.size(0), S = a_bar.size(1);
     const int32_t type = dt(x.scalar_type());
     const bool gated = get("use_gating").cast<bool>();
+    for (const Tensor *t : {&lam, &eta}) require(is(*t, dev, at::kFloat, {B, M, S}), "the filter state must be contiguous float32 [B, M, S] on x's device");
+    for (const Tensor *t : {&a_bar, &p_bar}) require(is(*t, dev, at::kFloat, {M, S}), "a_bar and p_bar must be contiguous float32 [M, S] on x's device");
+    require(!skip || is(*skip, dev, at::kFloat, {skip->numel() == 1 ? 1 : M}), "the skip weights must be one float32 value or one per channel, on x's device");
+    if (conv_w) {
+        require(conv_w->dim() == 2 && is(*conv_w, dev, at::kFloat, {M, conv_w->size(1)}) && (!conv_b || is(*conv_b, dev, at::kFloat, {M})),
+                "the convolution's weights must be contiguous float32 [M, K] and [M] on x's device");
+        require(conv_state ? is(*conv_state, dev, x.scalar_type(), {B, M, conv_w->size(1) - 1}) : conv_w->size(1) == 1,
+                "the convolution's window must be contiguous [B, M, K - 1] of x's type on its device");
+    }
     const Tensor in_w = w.at("in_proj.weight");
     const OptTensor in_b = w.get("in_proj.bias");
+    const Tensor sensor_w = w.at("sensor_proj.weight");
+    require(in_w.dim() == 2 && in_w.size(0) == (gated ? 2 * M : M), "in_proj must have one output per channel, two with a gate");
+    require(sensor_w.dim() == 2 && sensor_w.size(0) == w_value + w_var + 2 * S, "sensor_proj must have one output per sensor signal");
     const bool fused = few_rows(x, in_w, in_b, norm_w);  // the convolution's step then rides on the projection
     Tensor projected;
     if (fused) {
@@ -585,7 +619,7 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
         z = zc.data_ptr();
         z_row = M;
     }
-    const Tensor sens = w.linear(z_in, "sensor_proj.weight", "sensor_proj.bias");
+    const Tensor sens = project(z_in, sensor_w, w.get("sensor_proj.bias"), {}, 0.0, {});
     const int64_t row = sens.stride(0);
     // the four sensor signals, raw, as KLALayer._project_sensors splits them (src/kla/layers/kla_layer.py:199-216)
     void *v = z, *ls = part(sens, w_value), *kq = part(sens, w_value + w_var);
@@ -599,12 +633,14 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
             v = v_wide.data_ptr();
             v_row = v_wide.stride(0);
         }
+        require((v_wide.defined() ? v_wide.size(1) : w_value) == M, "there must be one value per channel");
     }
     if (w_.contains("var_expand.weight")) {
         ls_wide = w.linear(sens.narrow(1, w_value, w_var), "var_expand.weight", "var_expand.bias");
         ls = ls_wide.data_ptr();
         ls_row = ls_wide.stride(0);
     }
+    require((ls_wide.defined() ? ls_wide.size(1) : w_var) == M, "there must be one log-variance per channel");
     Tensor y = fresh(x, {B, M}), yv = fresh(x, {B, M});
     const py::object vmax = get("obs_var_max"), clip = get("clip_value");
     kla_b200_step_layer_args s{};

@@ -52,6 +52,11 @@ def discretize(weights: dict, config: dict):
     return a_bar.contiguous(), p_bar.contiguous()
 
 
+def _require_cuda(x: torch.Tensor) -> None:
+    if not x.is_cuda:
+        raise NotImplementedError("The b200 decode kernels need CUDA tensors; use the reference layer on this device.")
+
+
 class LayerDecoder:
     def __init__(self, weights: dict, config: dict):
         missing = [k for k in CONFIG_KEYS if k not in config]
@@ -128,8 +133,7 @@ class LayerDecoder:
         convolution runs in ``kla_b200_conv_seq``; the scan runs with the sensor prologue and the skip/gate epilogue inside
         (``kla_scan_b200(log_variance=, epilogue=)``). Returns ``(out, state)`` -- or ``((out, out_var),
         state)`` -- with ``state`` ready for ``step``."""
-        if not x.is_cuda:
-            raise NotImplementedError("The b200 kernels need CUDA tensors; use the reference layer on this device.")
+        _require_cuda(x)
         cfg, M = self.cfg, self.M
         B, L, _ = x.shape
         if state is None:
@@ -176,10 +180,7 @@ class LayerDecoder:
     def step(self, x: torch.Tensor, state):
         """One token. ``x``: [B, d_model]; ``state``: the tuple of ``init_state``, updated in place.
         Returns ``out`` [B, d_model], or ``(out, out_var)`` when the config returns variances."""
-        if not x.is_cuda:
-            raise NotImplementedError("The b200 decode kernels need CUDA tensors; use the reference layer on this device.")
-        if x.dtype not in (torch.float32, torch.bfloat16):
-            raise NotImplementedError(f"The b200 decode kernels take float32 or bfloat16 activations, not {x.dtype}.")
+        _require_cuda(x)
         conv_state, lam, eta = state
         out, y_var = _lib.host().layer_step(self.w, self.cfg, x, conv_state, lam, eta, self.a_bar, self.p_bar, self.skip,
                                             self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var, None, 0.0)
@@ -327,6 +328,7 @@ class ModelDecoder:
     def _step_blocks(self, x, state):
         """One token through the blocks: norm, mixer and residual sum of a block are the layer's step with the norm folded
         into its first projection and the sum into its last; the MLP likewise."""
+        _require_cuda(x)
         host, w, eps = _lib.host(), self.w, self.cfg["norm_eps"]
         for i, layer in enumerate(self.layers):
             pre = f"blocks.{i}."
@@ -342,6 +344,7 @@ class ModelDecoder:
     def _prompt_blocks(self, x, state):
         """A prompt through the blocks, each residual sum together with the norm behind it. Returns the sum and the last
         branch, still to be added (``_add_norm`` with the final norm, or of the position that is needed)."""
+        _require_cuda(x)
         branch = None
         for i, layer in enumerate(self.layers):
             x, h = self._add_norm(x, branch, f"blocks.{i}.mixer_norm")
@@ -374,6 +377,7 @@ class ModelDecoder:
         recurrent state. ``temperature <= 0`` is greedy. With ``use_graph`` the per-token work of all layers is
         one CUDA graph replay; sampling happens between replays, on the device."""
         x = F.embedding(input_ids, self.w["embedding.weight"])
+        _require_cuda(x)
         B, P = input_ids.shape
         greedy = temperature <= 0
         graph_ctx = self._token_graph(B, x.device, x.dtype, greedy) if use_graph and max_new_tokens > 1 else contextlib.nullcontext()

@@ -56,6 +56,36 @@ def test_cpu_tensors_are_refused():
         kla_b200.LayerDecoder(weights, {"d_state": 8})
 
 
+def tiny_model(d=32, M=64, S=16, layers=1, vocab=24, dtype=torch.float32):
+    """A ``ModelDecoder`` of random weights: swiglu MLP, the layers' default configuration."""
+    g = torch.Generator().manual_seed(d)
+    rn = lambda *s, scale=1.0: torch.randn(*s, generator=g) * scale
+    cfg = dict(d_state=S, discretization="ou", zero_process_noise=False, clip_value=None, obs_var_min=1e-4, obs_var_max=None,
+               value_rank="full", qk_norm=True, use_conv=True, conv_kernel_size=4, conv_activation="silu", use_gating=True,
+               gating_activation="silu", use_lambda_skip=True, return_variance=False, decode_from_prior=False)
+    w = {"embedding.weight": rn(vocab, d).to(dtype), "lm_head.weight": rn(vocab, d, scale=d ** -0.5).to(dtype),
+         "norm_f.weight": torch.ones(d, dtype=dtype)}
+    for i in range(layers):
+        b, m = f"blocks.{i}.", f"blocks.{i}.mixer."
+        w.update({m + "in_proj.weight": rn(2 * M, d, scale=d ** -0.5).to(dtype),
+                  m + "sensor_proj.weight": rn(2 * M + 2 * S, M, scale=M ** -0.5).to(dtype),
+                  m + "out_proj.weight": rn(d, M, scale=M ** -0.5).to(dtype), m + "conv.weight": rn(M, 1, 4, scale=0.5),
+                  m + "conv.bias": rn(M, scale=0.1), m + "delta": rn(M, S) - 4, m + "lambda_log": rn(M, S, scale=0.1),
+                  m + "process_noise": torch.full((M, S), 0.01), m + "lambda_skip": torch.tensor(-1.0),
+                  b + "mixer_norm.weight": torch.ones(d, dtype=dtype), b + "mlp_norm.weight": torch.ones(d, dtype=dtype),
+                  b + "mlp.w12.weight": rn(4 * d, d, scale=d ** -0.5).to(dtype), b + "mlp.w3.weight": rn(d, 2 * d, scale=(2 * d) ** -0.5).to(dtype)})
+    return kla_b200.ModelDecoder(w, [cfg] * layers, dict(n_layers=layers, norm_eps=1e-6, mlp="swiglu", logit_softcap=None))
+
+
+def test_a_model_on_the_cpu_is_refused_not_served():
+    dec = tiny_model()
+    ids = torch.zeros(2, 3, dtype=torch.long)
+    for call in (lambda: dec.prefill(ids), lambda: dec.step(ids[:, 0], dec.init_state(2, "cpu")), lambda: dec.generate(ids, 4),
+                 lambda: dec.generate(ids, 1), lambda: dec.generate(ids, 4, use_graph=False)):
+        with pytest.raises(NotImplementedError, match="CUDA"):
+            call()
+
+
 @needs_ref
 def test_from_layer_reads_a_reference_layer():
     sys.path.insert(0, REF_SRC)
@@ -233,3 +263,38 @@ def test_causal_conv_bf16_tracks_float32():
         outs[dt] = [z.float().detach()] + [t.float() for t in torch.autograd.grad(z, [x, weight, bias], dz.to(dt))]
     for a_, b_ in zip(outs[torch.bfloat16], outs[torch.float32]):
         assert ((a_ - b_).abs().max() / (b_.abs().max() + 1e-6)).item() < 2e-2
+
+
+# ------------------------------------------------------------ what the kernels are not given
+
+@pytest.mark.gpu
+def test_types_without_a_kernel_are_refused():
+    layer = import_module("kalman-linear-attention_b200.layer")
+    for dtype in (torch.float16, torch.float64):
+        dec = tiny_model(dtype=dtype).to("cuda")
+        ids = torch.zeros(2, 3, dtype=torch.long, device="cuda")
+        for call in (lambda: dec.step(ids[:, 0], dec.init_state(2, "cuda", dtype)), lambda: dec.prefill(ids), lambda: dec.generate(ids, 3),
+                     lambda: dec.layers[0].step(torch.zeros(2, 32, device="cuda", dtype=dtype), dec.layers[0].init_state(2, "cuda", dtype)),
+                     lambda: layer.causal_conv_b200(torch.zeros(1, 8, 32, device="cuda", dtype=dtype), torch.zeros(32, 1, 4, device="cuda"), None)):
+            with pytest.raises(NotImplementedError, match="float32 or bfloat16"):
+                call()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_state_that_does_not_fit_the_token_is_refused(dtype):
+    dec = tiny_model(dtype=dtype).to("cuda").layers[0]
+    M, S, B = dec.M, dec.S, 3
+    x = torch.zeros(B, 32, device="cuda", dtype=dtype)
+    good = dec.init_state(B, "cuda", dtype)
+    dec.step(x, good)
+    conv, lam, eta = good
+    other = torch.bfloat16 if dtype == torch.float32 else torch.float32
+    wide = torch.ones(B, 2, M, S, device="cuda")
+    for bad in (dec.init_state(B - 1, "cuda", dtype), (conv.to(other), lam, eta), (conv[..., :2], lam, eta), (None, lam, eta),
+                (conv, lam.double(), eta), (conv, wide[:, 0], eta), (conv, lam, eta[:, :-1].contiguous()), (conv, lam.cpu(), eta)):
+        with pytest.raises(ValueError):
+            dec.step(x, bad)
+    dec.w = dict(dec.w, **{"in_proj.weight": dec.w["in_proj.weight"][:M]})
+    with pytest.raises(ValueError, match="in_proj"):
+        dec.step(x, good)
