@@ -598,8 +598,9 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
         }
         projected = linear_rows(x, in_w, in_b, e);
     } else {
-        projected = at::linear(norm_w ? std::get<1>(add_norm(x, {}, *norm_w, norm_eps)) : x, in_w, in_b);
+        projected = at::linear(norm_w ? std::get<1>(add_norm(x, {}, *norm_w, norm_eps)) : x, in_w, in_b).to(x.scalar_type());
     }
+    // The kernels read x's type; under autocast the projections come in another.
     // z and the gate are halves of the projection, the sensor signals slices of theirs: pointers, not views
     const int64_t esz = x.element_size();
     auto part = [esz](const Tensor &t, int64_t column) { return static_cast<char *>(t.data_ptr()) + column * esz; };
@@ -619,7 +620,7 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
         z = zc.data_ptr();
         z_row = M;
     }
-    const Tensor sens = project(z_in, sensor_w, w.get("sensor_proj.bias"), {}, 0.0, {});
+    const Tensor sens = project(z_in, sensor_w, w.get("sensor_proj.bias"), {}, 0.0, {}).to(x.scalar_type());
     const int64_t row = sens.stride(0);
     // the four sensor signals, raw, as KLALayer._project_sensors splits them (src/kla/layers/kla_layer.py:199-216)
     void *v = z, *ls = part(sens, w_value), *kq = part(sens, w_value + w_var);
@@ -629,14 +630,14 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
         v = sens.data_ptr();
         v_row = row;
         if (w_.contains("value_expand.weight")) {
-            v_wide = w.linear(sens.narrow(1, 0, w_value), "value_expand.weight", "value_expand.bias");
+            v_wide = w.linear(sens.narrow(1, 0, w_value), "value_expand.weight", "value_expand.bias").to(x.scalar_type());
             v = v_wide.data_ptr();
             v_row = v_wide.stride(0);
         }
         require((v_wide.defined() ? v_wide.size(1) : w_value) == M, "there must be one value per channel");
     }
     if (w_.contains("var_expand.weight")) {
-        ls_wide = w.linear(sens.narrow(1, w_value, w_var), "var_expand.weight", "var_expand.bias");
+        ls_wide = w.linear(sens.narrow(1, w_value, w_var), "var_expand.weight", "var_expand.bias").to(x.scalar_type());
         ls = ls_wide.data_ptr();
         ls_row = ls_wide.stride(0);
     }

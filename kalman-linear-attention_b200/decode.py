@@ -143,7 +143,8 @@ class LayerDecoder:
         z, gate = (projected[..., :M], projected[..., M:]) if cfg["use_gating"] else (projected, None)
         if cfg["use_conv"]:
             # the causal convolution over the prompt, in place of cat + transpose + conv1d + activation + transpose
-            zc, new_window = _lib.host().conv_seq(z, self.conv_w, self.conv_b, conv_state, _lib.ACT[cfg["conv_activation"]])
+            zc, new_window = _lib.host().conv_seq(z, self.conv_w, self.conv_b, conv_state.to(z.dtype).contiguous(),
+                                                  _lib.ACT[cfg["conv_activation"]])  # z: autocast's type, if it is on
             conv_state.copy_(new_window)
             z = zc
         v, ls, k, q = self._sensors(z, self._linear(z, "sensor_proj"))

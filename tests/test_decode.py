@@ -298,3 +298,21 @@ def test_a_state_that_does_not_fit_the_token_is_refused(dtype):
     dec.w = dict(dec.w, **{"in_proj.weight": dec.w["in_proj.weight"][:M]})
     with pytest.raises(ValueError, match="in_proj"):
         dec.step(x, good)
+
+
+@pytest.mark.gpu
+def test_decode_under_autocast_follows_float32():
+    """Autocast gives float32 activations bfloat16 projections. Each of a layer's three rounds its operands and its result
+    (2^-9 of their size); what is between them does not enlarge that, so 3e-2 of the output's size covers it."""
+    dec = tiny_model(d=64, M=128).to("cuda").layers[0]
+    g = torch.Generator().manual_seed(3)
+    prompt, x = torch.randn(2, 20, 64, generator=g).cuda(), torch.randn(2, 64, generator=g).cuda()
+    want, state = dec.prefill(prompt)
+    want_step = dec.step(x, state)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        got, state_a = dec.prefill(prompt)
+        got_step = dec.step(x, state_a)
+    assert [t.dtype for t in state_a] == [t.dtype for t in state]
+    for a, b in ((got, want), (got_step, want_step)):
+        assert (a.float() - b).abs().max() <= 3e-2 * b.abs().max()
+    torch.testing.assert_close(state_a[0], state[0], rtol=2e-2, atol=2e-2 * state[0].abs().mean().item())
