@@ -1098,8 +1098,9 @@ int kla_b200_scan_fwd_static(const kla_b200_fwd_args *args, void *stream, const 
     *ckpt = nullptr;
     int rc = check_common(args->B, args->L, args->M, args->S, args->in_dtype, args->out_dtype);
     if (rc) return rc;
-    if (kla_b200_ckpt_bytes(args->B, args->L, args->M, args->S) > (size_t)KLA_B200_STATIC_CKPT_BYTES)
-        return KLA_B200_ETOOBIG;
+    ChunkCtl chunk;  // a cut sequence keeps checkpoints per chunk, more of them than the uncut one
+    if ((rc = check_chunks(args->B, args->L, args->chunks, args->chunk_len, &chunk))) return rc;
+    if (kla_b200_ckpt_bytes(args->B * chunk.n, chunk.len, args->M, args->S) > (size_t)KLA_B200_STATIC_CKPT_BYTES) return KLA_B200_ETOOBIG;
     void *scratch = nullptr;
     if ((rc = static_ckpt_address(&scratch))) return rc;
     kla_b200_fwd_args a = *args;

@@ -129,6 +129,14 @@ def test_sizes_that_overflow_are_refused_not_wrapped(L):
     out = ctypes.c_void_p()
     assert lib.kla_b200_scan_fwd_static(ctypes.byref(a), None, ctypes.byref(out)) == 5  # too big for the built-in scratch
     assert out.value is None
+    # a sequence cut into chunks keeps a checkpoint per chunk and eight steps: chunks of one step need eight times the
+    # 30 MB the uncut sequence does
+    a = L.FwdArgs(B=1, L=3840, M=512, S=16)
+    assert lib.kla_b200_ckpt_bytes(1, 3840, 512, 16) < L.STATIC_CKPT_BYTES < lib.kla_b200_ckpt_bytes(3840, 1, 512, 16)
+    a.chunks, a.chunk_len = 3840, 1
+    assert lib.kla_b200_scan_fwd_static(ctypes.byref(a), None, ctypes.byref(out)) == 5 and out.value is None
+    a.chunks, a.chunk_len = 3, 100  # chunks that do not cover the sequence
+    assert lib.kla_b200_scan_fwd_static(ctypes.byref(a), None, ctypes.byref(out)) == 1 and out.value is None
     # a decode step whose grid would not fit 31 bits is refused instead of running a truncated grid
     big = dict(B=65535, M=1 << 30, S=128, in_dtype=0, out_dtype=0)
     s_args = L.StepArgs(v=ptr, lambda_v=ptr, k=ptr, q=ptr, a=ptr, p=ptr, lam=ptr, eta=ptr, y=ptr, y_var=ptr,
