@@ -414,6 +414,7 @@ typedef struct kla_b200_step_layer_args {
     const float *lam, *eta;       /* [B, M, S] */
     void *y, *y_var;              /* [B, M] contiguous */
     float *lam_out, *eta_out;     /* [B, M, S]; may alias lam, eta */
+    int32_t weights_ready;        /* as in kla_b200_linear_args, of a and p */
 } kla_b200_step_layer_args;
 
 int kla_b200_step_layer(const kla_b200_step_layer_args *args, void *stream);
@@ -464,6 +465,9 @@ typedef struct kla_b200_linear_args {
     int32_t conv_activation;    /* KLA_B200_ACT_* */
     const float *conv_weight, *conv_bias; /* [conv_D, conv_taps]; [conv_D] or NULL */
     void *conv_state;           /* in/out [B, conv_D, conv_taps-1] bfloat16 contiguous */
+    int32_t weights_ready;      /* nonzero: the kernel in front on this stream was started after everything that wrote weight
+                                 * and norm_weight had ended, and writes neither: they may be read before it has ended
+                                 * (programmatic dependent launch). 0: nothing is read before. */
 } kla_b200_linear_args;
 
 int kla_b200_linear(const kla_b200_linear_args *args, void *stream);

@@ -93,7 +93,7 @@ class StepLayerArgs(Structure):
         ("k", c_void_p), ("q", c_void_p), ("k_stride_b", c_int64), ("q_stride_b", c_int64),
         ("z", c_void_p), ("gate", c_void_p), ("z_stride_b", c_int64), ("gate_stride_b", c_int64),
         ("lambda_skip", c_void_p), ("a", c_void_p), ("p", c_void_p), ("lam", c_void_p), ("eta", c_void_p),
-        ("y", c_void_p), ("y_var", c_void_p), ("lam_out", c_void_p), ("eta_out", c_void_p),
+        ("y", c_void_p), ("y_var", c_void_p), ("lam_out", c_void_p), ("eta_out", c_void_p), ("weights_ready", c_int32),
     ]
 
 

@@ -1003,6 +1003,7 @@ int kla_b200_linear(const kla_b200_linear_args *a, void *stream) {
         prm.D = (int)a->conv_D; prm.taps = (int)a->conv_taps; prm.conv_act = a->conv_activation;
         prm.conv_w = a->conv_weight; prm.conv_b = a->conv_bias; prm.conv_state = static_cast<__nv_bfloat16 *>(a->conv_state);
     }
+    prm.weights_ready = a->weights_ready;
     const int mode = a->swiglu ? kLinearSwiglu : a->conv_D ? kLinearConv : kLinearPlain;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (a->B <= 8) return dispatch_linear<1>(prm, mode, st);
@@ -1035,6 +1036,7 @@ int kla_b200_step_layer(const kla_b200_step_layer_args *a, void *stream) {
     prm.lam_out = a->lam_out; prm.eta_out = a->eta_out; prm.y = a->y; prm.yv = a->y_var;
     prm.skip = a->lambda_skip_len != 0 ? a->lambda_skip : nullptr; prm.skip_len = a->lambda_skip_len;
     prm.obs_var_min = a->obs_var_min; prm.obs_var_max = a->obs_var_max; prm.clip = a->clip_value;
+    prm.weights_ready = a->weights_ready;
     prm.qk_norm = a->qk_norm; prm.gate_act = a->gate_activation;
     prm.vec = a->S % 4 == 0 && aligned(a->lam, 16) && aligned(a->eta, 16) && aligned(a->a, 16) && aligned(a->p, 16) &&
               aligned(a->lam_out, 16) && aligned(a->eta_out, 16);

@@ -191,6 +191,7 @@ struct StepLayerParams {
     float obs_var_min, obs_var_max, clip;  // obs_var_max <= 0: none; clip <= 0: none
     int qk_norm, gate_act;
     int vec;  // as StepParams::vec
+    int weights_ready;  // a and p may be read before the kernel in front has ended
 };
 
 // A thread holds four consecutive states of NCH channels of one batch element, LPC adjacent lanes a channel; a CTA covers
@@ -220,8 +221,9 @@ __global__ void __launch_bounds__(128) kla_step_layer_kernel(const __grid_consta
                 if (j * 4 + i < S) x[i] = src[i];
         }
     };
-    // a, p before the wait for the sensor projection's kernel, everything that can have been written since the launch
-    // right after it, so that the arithmetic below waits for memory once
+    // a, p before the wait for the sensor projection's kernel where they are ready, everything that can have been written
+    // since the launch right after it, so that the arithmetic below waits for memory once
+    if (!prm.weights_ready) grid_dep_wait();
     grid_dep_launch();
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {

@@ -1,4 +1,4 @@
-// Linear layers of single-token decode: y[B, N] = x[B, K] W[N, K]^T for up to 64 rows of bfloat16, with what stands
+// Linear layers of single-token decode: y[B, N] = x[B, K] W[N, K]^T for up to 32 rows of bfloat16, with what stands
 // before and after the projection in a decode step folded in:
 //
 //   before  RMSNorm of x (src/kla/layers/common.py:45-55);
@@ -12,8 +12,9 @@
 //   * W goes straight from global memory into the A operand of mma.m16n8k16: which column of a block a lane holds does
 //     not matter to the sum as long as x is held the same way, so a lane takes 16 consecutive bytes of a row (two
 //     operands' worth) instead of the four-byte pieces the operand layout names;
-//   * W does not depend on the kernel before, so with programmatic dependent launch its first blocks, all of a warp's
-//     share up to K = 2048, are requested before the wait for that kernel;
+//   * where W does not depend on the kernel before (the caller says so), its first blocks are requested before the wait for
+//     that kernel (programmatic dependent launch): all of a warp's share up to K = 2048 for up to eight rows, up to 1024 for
+//     more rows and for swiglu;
 // Measured on B200 in a CUDA graph, us per projection, against the library's GEMM alone (rows x columns of W):
 //   B=8   3072 x 768 4.2 (3.7), with the norm 4.4; 3104 x 1536 5.9 (5.4); 768 x 1536 3.4 (4.4); 768 x 2048 3.6 (5.2)
 //   B=16  4096 x 1024 3.9 (3.6); 4128 x 2048 5.6 (5.5); 1024 x 2048 4.6 (5.9)
@@ -29,6 +30,7 @@ namespace kla {
 
 struct LinearParams {
     int B, N, K;
+    int weights_ready;  // W and norm_w may be read before the kernel in front has ended
     const __nv_bfloat16 *x, *w, *bias;  // [B, K] with row stride, [N, K], [N] or nullptr
     long long x_sb, out_sb, res_sb;
     __nv_bfloat16 *out;
@@ -60,7 +62,8 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 // (B=32, 4096 x 1024: 7.2 against 4.5 us).
 template <int NT, bool NORM>
 constexpr bool kLinearStaged = NORM || NT == 1;
-// Blocks of W (and, unstaged, of x) a warp holds in flight: all of K <= 2048 where the registers allow.
+// Blocks of W (and, unstaged, of x) a warp holds in flight: its share of K <= 2048, or <= 1024 where the registers allow no
+// more.
 template <int NT, int RT>
 constexpr int kLinearDepth = NT == 1 && RT == 1 ? 8 : 4;
 // shared memory: partial sums of every warp, then x (normalised with NORM)
@@ -146,6 +149,7 @@ __global__ void __launch_bounds__(kLinearWarps * 32) kla_linear_kernel(const __g
                                             : *reinterpret_cast<const uint4 *>(prm.x + (long long)r * prm.x_sb + ch * 8);
         }
     };
+    if (!prm.weights_ready) grid_dep_wait();  // before the launch: the next kernel's weights are then ready too
     grid_dep_launch();
 #pragma unroll
     for (int u = 0; u < U; ++u) load_w(u, blockIdx.x, warp + u * W);

@@ -316,3 +316,26 @@ def test_decode_under_autocast_follows_float32():
     for a, b in ((got, want), (got_step, want_step)):
         assert (a.float() - b).abs().max() <= 3e-2 * b.abs().max()
     torch.testing.assert_close(state_a[0], state[0], rtol=2e-2, atol=2e-2 * state[0].abs().mean().item())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("use_conv", [True, False])
+def test_a_layer_uses_the_weights_the_kernel_in_front_of_it_writes(use_conv):
+    """The decode projections let their successor start before they have stored anything. Here one of them produces the
+    weights of the layer whose token comes next."""
+    lib = import_module("kalman-linear-attention_b200._lib")
+    dec = tiny_model(dtype=torch.bfloat16).to("cuda").layers[0]
+    if not use_conv:
+        dec.cfg["use_conv"], dec.conv_w, dec.conv_b = False, None, None
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, source = rn(4, 32), rn(128, 8192) * 8192 ** -0.5
+    in_shape = dec.w["in_proj.weight"].shape
+    for _ in range(20):
+        seed = rn(32, 8192)
+        torch.cuda.synchronize()
+        made = lib.host().project(seed, source, None, None, 0.0, None)  # [32, 128]
+        dec.w = dict(dec.w, **{"in_proj.weight": made.view(in_shape)})
+        got = dec.step(x, dec.init_state(4, "cuda", torch.bfloat16))
+        torch.cuda.synchronize()
+        assert torch.equal(got, dec.step(x, dec.init_state(4, "cuda", torch.bfloat16)))
