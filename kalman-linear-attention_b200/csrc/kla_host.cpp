@@ -674,6 +674,22 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     return {project(y, w.at("out_proj.weight"), w.get("out_proj.bias"), {}, 0.0, norm_w ? OptTensor(x) : OptTensor()), yv};
 }
 
+// What a captured step would read: address, type and layout of each tensor. 220 of them take 18 us, as Python tuples 1000.
+py::bytes stamp(const std::vector<OptTensor> &ts) {
+    std::vector<int64_t> v;
+    v.reserve(ts.size() * 8);
+    for (const OptTensor &t : ts) {
+        if (!t) {
+            v.push_back(-1);
+            continue;
+        }
+        v.insert(v.end(), {(int64_t)reinterpret_cast<uintptr_t>(t->data_ptr()), (int64_t)t->scalar_type(), (int64_t)t->device().index(), t->dim()});
+        v.insert(v.end(), t->sizes().begin(), t->sizes().end());
+        v.insert(v.end(), t->strides().begin(), t->strides().end());
+    }
+    return py::bytes(reinterpret_cast<const char *>(v.data()), v.size() * sizeof(int64_t));
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_kla_host, m) {
@@ -700,4 +716,5 @@ PYBIND11_MODULE(_kla_host, m) {
         return project(x, w, bias, norm_w, eps, residual);
     });
     m.def("swiglu_step", &swiglu_step);
+    m.def("stamp", &stamp);
 }

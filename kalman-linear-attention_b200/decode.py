@@ -406,9 +406,12 @@ class ModelDecoder:
     @contextlib.contextmanager
     def _token_graph(self, batch: int, device, dtype, greedy: bool):
         """The captured decode step for this batch: the kept one when it fits and is free, else a new one."""
-        weights = [t for d in (self.w, *(layer.w for layer in self.layers)) for t in d.values()]
-        key = (batch, device, dtype, greedy, torch.is_autocast_enabled("cuda"), tuple(t.data_ptr() for t in weights),
-               dict(self.cfg), [(dict(layer.cfg), layer.a_bar.data_ptr(), layer.p_bar.data_ptr()) for layer in self.layers])
+        own = [t for name, t in self.w.items() if ".mixer." not in name]
+        layers = [t for layer in self.layers
+                  for t in (*layer.w.values(), layer.a_bar, layer.p_bar, layer.skip, layer.conv_w, getattr(layer, "conv_b", None))]
+        key = (batch, device, dtype, greedy, torch.is_autocast_enabled("cuda"), torch.get_autocast_dtype("cuda"),
+               torch.is_inference_mode_enabled(), _lib.host().stamp(own + layers), dict(self.cfg),
+               [(dict(layer.cfg), layer.w_value, layer.w_var) for layer in self.layers])
         slot = self._slot
         kept = slot.lock.acquire(blocking=False)
         try:

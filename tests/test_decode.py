@@ -86,6 +86,51 @@ def test_a_model_on_the_cpu_is_refused_not_served():
             call()
 
 
+def test_a_kept_decode_step_covers_everything_it_reads(monkeypatch):
+    """The captured step is taken again only for the tensors, layouts, settings and modes it was captured with."""
+    made = []
+
+    class Graph:
+        def __init__(self, *args):
+            made.append(args)
+            self.done = self
+
+        release = synchronize = lambda self: None
+
+    monkeypatch.setattr(decode, "_TokenGraph", Graph)
+    dec = tiny_model(layers=2)
+
+    def captures(call=lambda: None):
+        n = len(made)
+        call()
+        for _ in range(2):
+            with dec._token_graph(2, torch.device("cpu"), torch.float32, True):
+                pass
+        return len(made) - n
+
+    assert captures() == 1 and captures() == 0
+    kept = []  # a freed tensor's address could come back with its successor
+
+    def replace(get, put, name):
+        kept.append(get(name))
+        put(name, kept[-1].clone())
+
+    for layer in dec.layers:
+        for name in ("a_bar", "p_bar", "skip", "conv_w", "conv_b"):
+            assert captures(lambda: replace(layer.__getattribute__, layer.__setattr__, name)) == 1, name
+        for name in ("in_proj.weight", "sensor_proj.weight", "out_proj.weight"):
+            assert captures(lambda: replace(layer.w.__getitem__, layer.w.__setitem__, name)) == 1, name
+    for name in [n for n in dec.w if ".mixer." not in n]:
+        assert captures(lambda: replace(dec.w.__getitem__, dec.w.__setitem__, name)) == 1, name
+    w = dec.w["lm_head.weight"]
+    assert captures(lambda: dec.w.update({"lm_head.weight": w[:-1]})) == 1  # the same address, another shape
+    assert captures(lambda: dec.cfg.update(norm_eps=1e-5)) == 1
+    assert captures(lambda: dec.layers[1].cfg.update(obs_var_min=1e-3)) == 1
+    with torch.inference_mode():  # tensors made in this mode cannot be written outside it
+        assert captures() == 1
+    assert captures() == 1
+
+
 @needs_ref
 def test_from_layer_reads_a_reference_layer():
     sys.path.insert(0, REF_SRC)
