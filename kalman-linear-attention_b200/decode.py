@@ -389,7 +389,7 @@ class ModelDecoder:
             token = self._sample(self._head(*last), temperature, top_k)
             if max_new_tokens <= 1:
                 return torch.cat((input_ids, token), dim=1)
-            out = torch.empty(B, P + max_new_tokens, device=x.device, dtype=input_ids.dtype)
+            out = torch.empty(B, P + max_new_tokens, device=x.device, dtype=torch.promote_types(input_ids.dtype, torch.long))
             out[:, :P] = input_ids
             out[:, P] = token[:, 0]
             tok_buf = token[:, 0].clone() if graph is None else graph.token.copy_(token[:, 0])

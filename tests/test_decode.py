@@ -384,3 +384,14 @@ def test_a_layer_uses_the_weights_the_kernel_in_front_of_it_writes(use_conv):
         got = dec.step(x, dec.init_state(4, "cuda", torch.bfloat16))
         torch.cuda.synchronize()
         assert torch.equal(got, dec.step(x, dec.init_state(4, "cuda", torch.bfloat16)))
+
+
+@pytest.mark.gpu
+def test_generated_ids_are_int64_for_any_count():
+    dec = tiny_model().to("cuda")
+    ids = torch.tensor([[1, 2, 3], [4, 5, 6]], device="cuda")
+    want = dec.generate(ids, 5)
+    for dtype in (torch.int32, torch.int64):
+        for new in (1, 5):
+            got = dec.generate(ids.to(dtype), new)
+            assert got.dtype == torch.int64 and torch.equal(got, want[:, :3 + new])
