@@ -198,6 +198,7 @@ class _TokenGraph:
         self.state = dec.init_state(batch, device, dtype)
         self.token = torch.zeros(batch, device=device, dtype=torch.long)
         self.done = None  # recorded behind the last use
+        self.stream = torch.cuda.current_stream(device)  # whose memory the buffers are
         side = torch.cuda.Stream(device)
         side.wait_stream(torch.cuda.current_stream(device))
         self.graph = torch.cuda.CUDAGraph()
@@ -219,9 +220,14 @@ class _TokenGraph:
         return logits
 
     def reset(self):
-        """The prior state, ordered behind whatever used the buffers last."""
+        """The prior state, ordered behind whatever used the buffers last. They are memory of the stream that captured the
+        step: another stream that uses them says so to the allocator."""
+        stream = torch.cuda.current_stream(self.token.device)
         if self.done is not None:
-            torch.cuda.current_stream(self.token.device).wait_event(self.done)
+            stream.wait_event(self.done)
+        if stream != self.stream:
+            for t in (self.token, *(t for layer in self.state for t in layer if t is not None)):
+                t.record_stream(stream)
         for conv, lam, eta in self.state:
             if conv is not None:
                 conv.zero_()

@@ -395,3 +395,23 @@ def test_generated_ids_are_int64_for_any_count():
         for new in (1, 5):
             got = dec.generate(ids.to(dtype), new)
             assert got.dtype == torch.int64 and torch.equal(got, want[:, :3 + new])
+
+
+@pytest.mark.gpu
+def test_a_kept_step_on_another_stream_keeps_its_buffers_until_it_is_done():
+    """The kept step's buffers belong to the stream of the call that captured it. A later call replays it on another
+    stream; the decoder is dropped while that stream still has it all to do, and the first stream asks for memory."""
+    dec = tiny_model(d=64, M=256, layers=2).to("cuda")
+    ids = torch.arange(12, device="cuda").view(2, 6)
+    want = dec.generate(ids, 24)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(40_000_000)  # 20 ms
+        got = dec.generate(ids, 24)
+    shapes = {t.shape for layer in dec._slot.graph.state for t in layer} | {dec._slot.graph.token.shape}
+    weights = [dec.w, *(dict(layer.__dict__) for layer in dec.layers)]  # the caller's to keep
+    del dec
+    taken = [torch.full(s, 1e9, device="cuda") for s in shapes for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and taken and weights
