@@ -136,12 +136,13 @@ __global__ void __launch_bounds__(128) kla_qk_norm_kernel(const __grid_constant_
     }
 #pragma unroll
     for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-    const float n = fmaxf(sqrtf(ss), 1e-12f);
+    float n = sqrtf(ss);
+    if (n < 1e-12f) n = 1e-12f;  // as the clamps of the tensor operations, these let a NaN through
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int s = lane + 16 * i;
         float y = v[i] / n;
-        if (prm.clip > 0.0f) y = fminf(fmaxf(y, -prm.clip), prm.clip);
+        if (prm.clip > 0.0f) y = y < -prm.clip ? -prm.clip : y > prm.clip ? prm.clip : y;
         if (s < S) o[s] = from_f32<T>(y);
     }
 }

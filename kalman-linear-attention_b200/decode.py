@@ -150,8 +150,8 @@ class LayerDecoder:
         v, ls, k, q = self._sensors(z, self._linear(z, "sensor_proj"))
         clip = cfg["clip_value"]
         if cfg["qk_norm"]:
-            k, q = _lib.host().qk_norm(k, q, clip or 0.0)
-        if clip is not None and (clip == 0 or not cfg["qk_norm"]):
+            k, q = _lib.host().qk_norm(k, q, max(clip or 0.0, 0.0))
+        if clip is not None and (clip <= 0 or not cfg["qk_norm"]):
             k, q = k.clamp(-clip, clip), q.clamp(-clip, clip)
         epi = {}
         if self.skip is not None:

@@ -118,6 +118,17 @@ def test_keys_and_queries_are_normalised_and_clipped(B, L, S, clip, dtype):
         torch.testing.assert_close(got.double(), want.clamp(-clip, clip) if clip else want, **tol)
 
 
+@pytest.mark.parametrize("clip", [0.0, 0.3])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_keys_that_are_not_finite_stay_so(clip, dtype):
+    x = torch.randn(1, 5, 20, device="cuda").to(dtype)
+    x[0, 1, 3], x[0, 2, 19], x[0, 3, 0] = float("nan"), float("inf"), float("-inf")
+    want = x.double() / x.double().norm(dim=-1, keepdim=True).clamp_min(1e-12)
+    want = want.clamp(-clip, clip) if clip else want
+    for got in lib.host().qk_norm(x, x, clip):
+        torch.testing.assert_close(got.double(), want, rtol=1e-2, atol=1e-3, equal_nan=True)
+
+
 def test_shapes_that_do_not_agree_raise_or_broadcast_as_tensor_operations_do():
     """The kernels are given pointers: a row shorter than the weights' is for the tensor operations to refuse."""
     rn = lambda *s: torch.randn(*s, device="cuda").bfloat16()
