@@ -20,6 +20,7 @@ import sys
 from typing import NamedTuple, Optional
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from ._lib import MAX_DSTATE
@@ -460,7 +461,11 @@ def kla_scan_b200(
 
 
 def _wants_grad(*tensors) -> bool:
-    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+    """Whether the call needs the autograd function: for a backward, or to refuse forward-mode tangents, which it has no
+    rule for (a plain launch would drop them)."""
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors):
+        return True
+    return forward_ad._current_level >= 0 and any(t is not None and forward_ad.unpack_dual(t).tangent is not None for t in tensors)
 
 
 def _check_log_variance(log_variance):

@@ -141,6 +141,21 @@ def test_wrapper_widens_and_validates(oracle_launches):
     torch.testing.assert_close(y1, y2)
 
 
+def test_forward_mode_tangents_are_refused_not_dropped(oracle_launches):
+    from torch.autograd import forward_ad
+
+    ins = _t(load_golden("backends"))
+    extras = (dict(), dict(epilogue=dict(gate=torch.ones_like(ins[0]))), dict(initial_state=kla_b200.init_state(2, 16, 8)))
+    with forward_ad.dual_level():
+        dual = [forward_ad.make_dual(ins[0], torch.ones_like(ins[0])), *ins[1:]]
+        for extra in extras:
+            for grad in (torch.enable_grad, torch.no_grad):
+                with grad(), pytest.raises((NotImplementedError, RuntimeError), match="jvp|forward"):
+                    kla_b200.kla_scan_b200(*dual, **extra)
+        y, _, _ = kla_b200.kla_scan_b200(*ins)  # no tangents: served inside a level too
+    torch.testing.assert_close(y, kla_b200.kla_scan_b200(*ins)[0])
+
+
 # ------------------------------------------------ plugging into the reference
 
 needs_ref = pytest.mark.skipif(not os.path.isdir(REF_SRC), reason="reference package not present")
