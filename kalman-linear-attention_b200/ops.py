@@ -137,8 +137,20 @@ def _chunkable(t: Optional[torch.Tensor], B: int, L: int) -> bool:
     return t is None or B == 1 or t.stride(0) == L * t.stride(1)
 
 
-def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = None) -> int:
-    """Number of time chunks for the time-parallel scan. 1 = the plain lane-serial kernels.
+def _row_bytes(tensors) -> int:
+    """Largest power of two, up to 16, that every row of the [B, L, M] tensors starts on. TMA reads rows of 16."""
+    n = 16
+    for t in tensors:
+        e = t.element_size()
+        for x in (t.data_ptr(), t.stride(0) * e if t.shape[0] > 1 else 0, t.stride(1) * e if t.shape[1] > 1 else 0):
+            while x % n:
+                n //= 2
+    return n
+
+
+def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = None, tensors=(), training: bool = False) -> int:
+    """Number of time chunks for the time-parallel scan. 1 = the plain lane-serial kernels. ``tensors``: the activations,
+    for the alignment of their rows; ``training``: a backward follows.
 
     The kernels put one CTA on every 32 / 16 / 8 ... channels (d_state 16 / 32 / 64 ...) of every batch element.
     When that grid leaves most of the GPU empty, the sequence is cut into C chunks that run as B*C batch entries;
@@ -159,12 +171,18 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
         # Not below 640 steps, where the uncut kernels are done before three launches are (B=1 L=300 M=512: 27 us against
         # 36 to 52 cut, training 163 against 220 to 275). From about 90 CTAs on cutting breaks even, and only for long
         # sequences (96 CTAs: L=900 66 / 234 uncut, 77 / 246 cut; L=2048 143 / 499 and 148 / 491; L=4096 280 / 985 and
-        # 273 / 906), or for rows that TMA cannot read, which a CTA stages too slowly (B=3 L=1537 M=1001 training 540 and
-        # 451).
+        # 273 / 906). Rows that TMA cannot read are staged too slowly by one CTA of a backward: training gains from 640
+        # steps on, inference only where they are not even 4-byte aligned and from 900 steps on. At 94 and 96 CTAs (B, M = 3,
+        # 1001; 1, 2981; 6, 497; 2, 1473, all within 3 %), forward / training, uncut and cut: float32 L=641 52 / 229 and
+        # 68 / 220, L=1537 116 / 523 and 133 / 450, L=1999 151 / 673 and 161 / 548; bfloat16 rows of 8 bytes (M = 1004, 3004,
+        # 500, 1476) 52 / 270 and 72 / 241, 117 / 645 and 139 / 510, 151 / 840 and 168 / 628; odd ones 79 / 517 and 98 / 407,
+        # 181 / 1780 and 165 / 1140, 234 / 2420 and 210 / 1495.
         if ctas == 0 or 3 * ctas > _RESIDENT_CTAS or L < 640:
             return 1
-        if 10 * ctas > 3 * _RESIDENT_CTAS and L < 2048 and M % 4 == 0:
-            return 1
+        if 10 * ctas > 3 * _RESIDENT_CTAS and L < 2048:
+            row = _row_bytes(tensors)
+            if row == 16 or not (training or (row < 4 and L >= 900)):
+                return 1
         # Whole rounds of the resident slots: enough chunks for one, more rounds while chunks are longer than about 256
         # steps, which evens out the last one. Measured on B200, forward / training step in us: B=1 L=1536 M=1536
         # (48 CTAs) 3 chunks 79 / 233, 4 91 / 287, 6 69 / 208, 8 73 / 227, 16 74 / 235, uncut 108 / 380; B=1 L=8192 M=2048
@@ -480,10 +498,11 @@ def _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, log_varianc
     """The scan of canonical arguments, without an epilogue."""
     log_variance = _check_log_variance(log_variance)
     B, L, M = v.shape
-    chunks = pick_time_chunks(B, L, M, k.shape[2], time_chunks) if L > 0 and log_variance is None else 1
+    training = _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0)
+    chunks = pick_time_chunks(B, L, M, k.shape[2], time_chunks, (v, lambda_v), training) if L > 0 and log_variance is None else 1
     if chunks > 1 and time_chunks is not None and not all(_chunkable(t, B, L) for t in (v, lambda_v, k, q)):
         chunks = 1  # an explicit count is taken for sequences that lie back to back
-    if not _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0):  # inference: no autograd node, no checkpoints
+    if not training:  # inference: no autograd node, no checkpoints
         if chunks > 1:
             y, y_var, lam_fin, eta_fin, *_ = _lib.host().scan_fwd_chunked(
                 v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype == torch.bfloat16, False, chunks,

@@ -61,6 +61,26 @@ def test_chunks_cover_every_length():
             assert (c - 1) * n < L <= c * n and (c == 1 or n >= 64), (L, c, n)
 
 
+def test_chunks_near_one_cta_per_sm_follow_what_tma_can_read():
+    """At 89 to 98 CTAs and below 2048 steps a sequence is cut only where its rows are staged without TMA."""
+    pick = lambda B, L, M, dtype, training, stride=0, offset=0: ops.pick_time_chunks(
+        B, L, M, 16, None, [torch.empty(B * L * (M + stride) + offset, dtype=dtype)[offset:].view(B, L, M + stride)[..., :M]] * 2, training)
+    f32, bf16 = torch.float32, torch.bfloat16
+    for B, M in ((3, 1024), (1, 3008), (6, 512)):  # rows of 16 bytes in both types
+        for dtype in (f32, bf16):
+            for L in (640, 1537, 2047):
+                assert pick(B, L, M, dtype, True) == pick(B, L, M, dtype, False) == 1
+        assert pick(B, 2048, M, f32, True) > 1 and pick(B, 2048, M, f32, False) > 1
+    for B, M in ((3, 1004), (1, 3004), (6, 500)):  # in float32 only
+        assert pick(B, 1537, M, f32, True) == 1 and pick(B, 1537, M, bf16, True) > 1 and pick(B, 1537, M, bf16, False) == 1
+    for B, M in ((3, 1001), (1, 2981), (6, 497)):  # in neither
+        assert pick(B, 700, M, f32, True) > 1 and pick(B, 1537, M, f32, False) == 1
+        assert pick(B, 700, M, bf16, True) > 1 and pick(B, 700, M, bf16, False) == 1 and pick(B, 1537, M, bf16, False) > 1
+    assert pick(3, 1537, 1024, f32, True, stride=2) > 1 and pick(3, 1537, 1024, f32, True, stride=4) == 1  # slices of wider rows
+    assert pick(3, 1537, 1024, f32, True, offset=1) > 1 and pick(3, 1537, 1001, f32, True, stride=23) == 1
+    assert pick(1, 639, 3000, bf16, True) == 1 and ops.pick_time_chunks(3, 1537, 1024, 16) == 1
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,L,M,S", [(1, 1, 4, 1), (2, 15, 9, 16), (1, 16, 3, 12), (3, 17, 33, 4), (1, 70, 130, 16), (80, 33, 20, 16)])
 def test_raw_scans_around_their_tiles(B, L, M, S):
