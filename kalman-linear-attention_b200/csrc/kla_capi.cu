@@ -271,11 +271,7 @@ int plan_segments_for(int64_t ctas, int64_t L, bool backward, int sms, int force
 int plan_segments(int64_t ctas, int64_t L, bool backward, int *seg_len) {
     const char *env = getenv("KLA_B200_SEGMENTS");  // read per launch: the tests switch it within one process
     const int forced = env != nullptr ? atoi(env) : -1;
-    int dev = 0, sms = 0;
-    if (forced < 0 && (cudaGetDevice(&dev) != cudaSuccess ||
-                       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
-        sms = 0;
-    return plan_segments_for(ctas, L, backward, sms, forced, seg_len);
+    return plan_segments_for(ctas, L, backward, forced < 0 ? device_sms() : 0, forced, seg_len);
 }
 
 // Fill prm.seg for one direction; its ticket and done words go on the list of what to clear before the launch. The working memory is the bytes behind the
@@ -413,7 +409,7 @@ int launch_step_layer(const StepLayerParams &prm, cudaStream_t st) {
         return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
     };
     // Four channels per thread once that still leaves every SM two CTAs; below, the CTAs' latency is the time.
-    if ((long long)prm.B * prm.M >= 296ll * kStepLayerChannels<LPC, 4>)
+    if ((long long)prm.B * prm.M >= 2ll * device_sms() * kStepLayerChannels<LPC, 4>)
         return go(kla_step_layer_kernel<T, TO, LPC, PRIOR, 4>, kStepLayerChannels<LPC, 4>);
     return go(kla_step_layer_kernel<T, TO, LPC, PRIOR, 1>, kStepLayerChannels<LPC, 1>);
 }
@@ -441,9 +437,7 @@ int launch_rawscan(const kla_b200_rawscan_args *a, void *stream, bool takes_stat
         if (!aligned(a->out[k], sizeof(float))) return KLA_B200_EALIGN;
     }
     if (a->B == 0 || a->N == 0) return KLA_B200_OK;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
-    if (Op::NIN >= 6 && (a->N + kRawLC - 1) / kRawLC * a->B <= sms) return launch_rawscan_as<Op, false>(a, stream);
+    if (Op::NIN >= 6 && (a->N + kRawLC - 1) / kRawLC * a->B <= device_sms()) return launch_rawscan_as<Op, false>(a, stream);
     return launch_rawscan_as<Op, true>(a, stream);
 }
 
@@ -492,8 +486,8 @@ int launch_linear(const LinearParams &prm, cudaStream_t st) {
     // A CTA per tile up to two per SM, which is what fits; beyond, a CTA walks several tiles, the next one's W on its way
     // while it adds up the last one.
     constexpr int rows = MODE == kLinearSwiglu ? 16 : 16 * RT;
-    const int tiles = (n_out + rows - 1) / rows;
-    const cudaError_t e = launch_dependent(kern, dim3((unsigned)(tiles < 296 ? tiles : 296)), kLinearWarps * 32, smem, st, prm);
+    const int tiles = (n_out + rows - 1) / rows, most = 2 * device_sms();
+    const cudaError_t e = launch_dependent(kern, dim3((unsigned)(tiles < most ? tiles : most)), kLinearWarps * 32, smem, st, prm);
     g_launches++;
     return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
 }
@@ -503,7 +497,7 @@ template <int NT, int MODE, bool NORM>
 int dispatch_linear_tiles(const LinearParams &prm, cudaStream_t st) {
     if constexpr (MODE == kLinearSwiglu) return launch_linear<NT, 2, MODE, NORM>(prm, st);
     else if constexpr (NT < 4) return launch_linear<NT, 1, MODE, NORM>(prm, st);
-    else return prm.N > 16 * 148 ? launch_linear<NT, 2, MODE, NORM>(prm, st) : launch_linear<NT, 1, MODE, NORM>(prm, st);
+    else return prm.N > 16 * device_sms() ? launch_linear<NT, 2, MODE, NORM>(prm, st) : launch_linear<NT, 1, MODE, NORM>(prm, st);
 }
 template <int NT>
 int dispatch_linear(const LinearParams &prm, int mode, cudaStream_t st) {
@@ -726,7 +720,7 @@ int kla_b200_epilogue_bwd(const kla_b200_epilogue_bwd_args *a, void *stream) {
     const int per = osz == 2 && all_ok(8) ? 8 : all_ok(4) ? 4 : 1;
     // few rows per CTA until many of them would still give every SM four CTAs
     const int64_t columns = (a->M + 128 * per - 1) / (128 * per);
-    const bool few = columns * a->B * row_blocks < 4 * 148;
+    const bool few = columns * a->B * row_blocks < 4 * device_sms();
     const int rows = few ? kEpiFewRows : kEpiRows;
     dim3 grid((unsigned)columns, (unsigned)((a->L + rows - 1) / rows), (unsigned)a->B);
 #define KLA_EPI_ROWS(T, TO, VEC, Z, G)                                                                   \

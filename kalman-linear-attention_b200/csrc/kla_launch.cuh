@@ -30,6 +30,13 @@ constexpr int kSPT = KLA_SPT;          // states per thread
 #endif
 constexpr int kCH = KLA_CH;            // channels per thread
 
+// SMs of the current device; those of a whole B200 where the runtime does not say (the launch will then say why)
+inline int device_sms() {
+    int dev = 0, sms = 0;
+    const bool ok = cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+    return ok && sms > 0 ? sms : 148;
+}
+
 // channels per CTA of the scan kernels for a given number of lanes per channel
 inline int scan_channels_per_cta(int lpc) { return kNW * (32 / lpc) * kCH; }
 

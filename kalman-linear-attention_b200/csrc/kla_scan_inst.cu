@@ -17,13 +17,13 @@ cudaError_t launch_fwd(const FwdParams &prm, cudaStream_t st) {
     // The epilogue's tile passes set the pace of a CTA that has an SM to itself, where two more helper warps take them off
     // it (B=2 L=8192 M=2048 bfloat16: 0.85 -> 0.64 ms, 0.56 without epilogue); with more CTAs per SM they would only
     // compete with the recurrence for issue slots (B=4: 0.97 -> 1.01 ms).
-    const bool alone = (unsigned long long)grid.x * grid.y <= 148;
+    const bool alone = prm.epilogue && (long long)grid.x * grid.y <= device_sms();
     auto kern = prm.epilogue ? (seg ? kla_fwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kTT, PRIOR, true, true>
                                 : alone ? kla_fwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kEpiNH, kTT, PRIOR, true, false>
                                         : kla_fwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kTT, PRIOR, true, false>)
                              : (seg ? kla_fwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kTT, PRIOR, false, true>
                                     : kla_fwd_kernel<T, TO, kSPT, LPC, kCH, kNW, kNH, kTT, PRIOR, false, false>);
-    const int helpers = prm.epilogue && !seg && alone ? kEpiNH : kNH;
+    const int helpers = !seg && alone ? kEpiNH : kNH;
     const size_t smem = prm.epilogue ? Sm::kTotal : Sm::kPlain;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sm::kTotal);
     if (e != cudaSuccess) return e;
