@@ -11,6 +11,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/GradMode.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/utils/pybind.h>
 
@@ -419,6 +420,20 @@ bool few_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const Opt
            !wants_grad({&x, &w, bias ? &*bias : &x, norm_w ? &*norm_w : &x}) && sm100(x.device());
 }
 
+// Whether a projection that few_rows() takes is faster so than as the library's GEMM with the norm, gate and sum as kernels
+// of their own. Up to 16 rows always. Beyond, a CTA brings in (and normalises) four groups of eight rows and keeps half as
+// much of W in flight; the library's kernels win as rows x N x K grows. Measured in a CUDA graph, W from HBM, us, kernel
+// against library (plain; gate and up with norm and the projection behind; norm with the convolution's step):
+//    51 M  24 rows 2080 x 1024 3.4 / 4.3                    75 M  24 rows 4096 x 768 14.8 / 15.8
+//    68 M  32 rows 2080 x 1024 3.5 / 4.3                    75 M  32 rows 3072 x 768 9.2 / 8.9
+//    67 M  32 rows 1024 x 2048 5.3 / 6.0                    95 M  17 rows 5440 x 1024 23.2 / 18.9
+//    81 M  17 rows 3104 x 1536 6.5 / 5.4                   100 M  24 rows 4096 x 1024 10.8 / 9.9
+//    89 M  32 rows 1024 x 2720 9.0 / 8.2                   101 M  32 rows 4096 x 768 16.3 / 15.9
+//   144 M  17 rows 4128 x 2048 7.6 / 6.4                   134 M  32 rows 4096 x 1024 12.5 / 9.9
+bool kernel_pays(int64_t rows, int64_t N, int64_t K) { return rows <= 16 || rows * N * K <= 80'000'000; }
+// Who runs a projection that few_rows() takes: whoever is faster, or what the caller says.
+enum class By { size, kernel, library };
+
 struct Extra {  // what kla_b200_linear does besides the projection
     const OptTensor &norm_w;
     double norm_eps = 0.0;
@@ -509,20 +524,33 @@ Tensor argmax(const Tensor &x, Tensor out) {
     return out;
 }
 
-// A language model's head for a few rows. From this many outputs on the library's GEMM is the better read of W (50304 x 768,
-// eight rows: 8.2 us against 14), and the norm is a launch of its own.
-constexpr int64_t kWideHead = 8192;
+// A language model's head (a norm in front, no sum behind): from how many outputs on the library's GEMM and the
+// norm as a launch of its own are the better read of W. Measured as above, W from HBM, us, kernel / library at one and eight
+// rows: K=128 N=4096 2.7 3.9 / 4.1 4.2, N=8192 4.1 5.3 / 4.4 4.8; K=256 N=8192 4.5 5.6 / 5.5 5.7, N=16384 7.9 9.1 / 6.1 6.3;
+// K=512 N=8192 4.8 6.1 / 6.7 6.8, N=16384 8.4 9.8 / 7.8 7.9; K=768 N=16384 8.7 10.3 / 9.6 9.7, N=32000 14.6 16.0 / 13.7 13.9;
+// K=1024 N=16384 9.4 10.8 / 11.4 11.6, N=50304 23.8 25.5 / 25.7 26.3. At 32 rows the library wins from 4096 outputs on at
+// every K (K=256 7.6 / 5.3, K=1024 12.5 / 8.3).
+int64_t widest_head(int64_t rows, int64_t K) { return rows <= 16 ? 12 * K + 4096 : 2048; }
+
+// From so many outputs on any other projection is the library's too, at eight rows: 8192 x 1024 7.3 / 5.7, 8224 x 4096
+// 15.4 / 13.5, 16384 x 2048 15.0 / 13.6; below, 4128 x 2048 7.0 / 8.0, 4096 x 8192 21.4 / 20.9.
+constexpr int64_t kWidePlain = 8192;
 
 // norm (when norm_w is given), projection, residual sum (when given)
 Tensor project(const Tensor &x, const Tensor &w, const OptTensor &bias, const OptTensor &norm_w, double eps, const OptTensor &residual,
-               bool weights_ready = true) {
+               bool weights_ready = true, By by = By::size) {
     const c10::cuda::CUDAGuard guard(x.device());
     auto sums = [&] {  // the residual is one the kernel can add
         return !residual || (residual->scalar_type() == at::kBFloat16 && residual->dim() == 2 && residual->size(0) == x.size(0) &&
                              residual->size(1) == w.size(0) && residual->stride(1) == 1 && residual->device() == x.device() &&
                              !wants_grad({&*residual}));
     };
-    if (w.size(0) < kWideHead && few_rows(x, w, bias, norm_w) && sums())
+    const bool head = norm_w && !residual;
+    auto pays = [&] {
+        const int64_t rows = x.size(0), N = w.size(0), K = w.size(1);
+        return head ? N <= widest_head(rows, K) : N < kWidePlain && kernel_pays(rows, N, K);
+    };
+    if (by != By::library && few_rows(x, w, bias, norm_w) && (by == By::kernel || pays()) && sums())
         return linear_rows(x, w, bias, Extra{norm_w, eps, residual}, weights_ready);
     const Tensor out = at::linear(norm_w ? std::get<1>(add_norm(x, {}, *norm_w, eps)) : x, w, bias);
     return residual ? *residual + out : out;
@@ -535,8 +563,8 @@ struct Weights {  // a layer's weights by name; what a dict does not hold is abs
         const PyObject *o = PyDict_GetItemString(d.ptr(), name);
         return o ? OptTensor(py::handle(const_cast<PyObject *>(o)).cast<Tensor>()) : OptTensor();
     }
-    Tensor linear(const Tensor &x, const char *w, const char *b, bool weights_ready) const {
-        return project(x, at(w), get(b), {}, 0.0, {}, weights_ready);
+    Tensor linear(const Tensor &x, const char *w, const char *b, bool weights_ready, By by) const {
+        return project(x, at(w), get(b), {}, 0.0, {}, weights_ready, by);
     }
 };
 
@@ -546,7 +574,7 @@ Tensor swiglu_step(const Tensor &x, const Tensor &norm_w_, double eps, const Ten
     const c10::cuda::CUDAGuard guard(x.device());
     const OptTensor norm_w = norm_w_;
     Tensor h;
-    if (few_rows(x, w12, b12, norm_w) && w12.size(0) % 2 == 0) {
+    if (few_rows(x, w12, b12, norm_w) && w12.size(0) % 2 == 0 && kernel_pays(x.size(0), w12.size(0), w12.size(1))) {
         Extra e{norm_w, eps};
         e.swiglu = true;
         h = linear_rows(x, w12, b12, e, true);
@@ -593,7 +621,23 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     const bool in_model = norm_w.has_value();  // other kernels of the token, or the embedding's, are in front
     require(in_w.dim() == 2 && in_w.size(0) == (gated ? 2 * M : M), "in_proj must have one output per channel, two with a gate");
     require(sensor_w.dim() == 2 && sensor_w.size(0) == w_value + w_var + 2 * S, "sensor_proj must have one output per sensor signal");
-    const bool fused = few_rows(x, in_w, in_b, norm_w);  // the convolution's step then rides on the projection
+    // A lone layer issued call by call is bound by the host, where the library's calls cost 7 us more each (B=17 d_model 768:
+    // 23.0 us a token, 26.5 with one of them); in a graph its three GEMMs win together where the widest does (d_model 768, B=17
+    // 21.9 against 19.0, B=32 28.6 and 21.8; d_model 1024, B=32 27.6 and 24.3; but d_model 512, B=32 15.7 and 16.6).
+    By by = By::size;
+    if (!in_model) {
+        by = By::kernel;
+        if (!kernel_pays(B, sensor_w.size(0), sensor_w.size(1)) &&
+            c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+            by = By::library;
+            // The eager tokens before the capture did not use the library: it may have to set itself up now, which the other
+            // capture modes would not let it.
+            const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+            at::cuda::getCurrentCUDABlasHandle();
+        }
+    }
+    // with the kernel the convolution's step rides on the first projection
+    const bool fused = by != By::library && few_rows(x, in_w, in_b, norm_w) && (by == By::kernel || kernel_pays(B, in_w.size(0), in_w.size(1)));
     Tensor projected;
     if (fused) {
         Extra e{norm_w, norm_eps};
@@ -615,7 +659,8 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     int64_t z_row = projected.stride(0);
     Tensor z_in = gated ? projected.narrow(1, 0, M) : projected;  // what sensor_proj reads
     // What runs in front of a lone layer may write its weights, and may let its successor start before it has (these kernels
-    // do): the first kernel of the token reads its weights only after it (B=32 d_model 1024: 30.8 against 30.7 us a token).
+    // do): the first kernel of the token reads its weights only after it (B=32 d_model 1024, tokens back to back: 28.9 against
+    // 28.2 us).
     bool weights_ready = fused || in_model;
     if (conv_w && !fused) {
         Tensor zc = fresh(x, {B, M});
@@ -630,7 +675,7 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
         z_row = M;
         weights_ready = true;
     }
-    const Tensor sens = project(z_in, sensor_w, w.get("sensor_proj.bias"), {}, 0.0, {}, weights_ready).to(x.scalar_type());
+    const Tensor sens = project(z_in, sensor_w, w.get("sensor_proj.bias"), {}, 0.0, {}, weights_ready, by).to(x.scalar_type());
     const int64_t row = sens.stride(0);
     // the four sensor signals, raw, as KLALayer._project_sensors splits them (src/kla/layers/kla_layer.py:199-216)
     void *v = z, *ls = part(sens, w_value), *kq = part(sens, w_value + w_var);
@@ -640,14 +685,14 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
         v = sens.data_ptr();
         v_row = row;
         if (w_.contains("value_expand.weight")) {
-            v_wide = w.linear(sens.narrow(1, 0, w_value), "value_expand.weight", "value_expand.bias", weights_ready).to(x.scalar_type());
+            v_wide = w.linear(sens.narrow(1, 0, w_value), "value_expand.weight", "value_expand.bias", weights_ready, by).to(x.scalar_type());
             v = v_wide.data_ptr();
             v_row = v_wide.stride(0);
         }
         require((v_wide.defined() ? v_wide.size(1) : w_value) == M, "there must be one value per channel");
     }
     if (w_.contains("var_expand.weight")) {
-        ls_wide = w.linear(sens.narrow(1, w_value, w_var), "var_expand.weight", "var_expand.bias", weights_ready).to(x.scalar_type());
+        ls_wide = w.linear(sens.narrow(1, w_value, w_var), "var_expand.weight", "var_expand.bias", weights_ready, by).to(x.scalar_type());
         ls = ls_wide.data_ptr();
         ls_row = ls_wide.stride(0);
     }
@@ -671,7 +716,7 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     s.y = y.data_ptr(); s.y_var = yv.data_ptr(); s.lam_out = fp(lam); s.eta_out = fp(eta);
     s.weights_ready = weights_ready;
     check(lib.step_layer(&s, stream));
-    return {project(y, w.at("out_proj.weight"), w.get("out_proj.bias"), {}, 0.0, norm_w ? OptTensor(x) : OptTensor()), yv};
+    return {project(y, w.at("out_proj.weight"), w.get("out_proj.bias"), {}, 0.0, norm_w ? OptTensor(x) : OptTensor(), true, by), yv};
 }
 
 // What a captured step would read: address, type and layout of each tensor. 220 of them take 18 us, as Python tuples 1000.

@@ -20,8 +20,9 @@
 //   B=16  4096 x 1024 3.9 (3.6); 4128 x 2048 5.6 (5.5); 1024 x 2048 4.6 (5.9)
 //   B=32  4096 x 1024 5.3 (3.5); 4128 x 2048 8.1 (5.6); 1024 x 2048 5.4 (4.9)
 // What bounds it is latency: about 3 us of launch, one round trip for x, the sum over warps and the store. Beyond 16 rows
-// the library's kernels are the faster ones on the device, but a call costs the host 10 us against 4, so a token issued
-// eagerly still takes less (layer step B=32 d_model 1024: 28.9 us eager and 27.7 us in a graph; 85 us as library calls).
+// the library's kernels are the faster ones where a projection is large (kernel_pays in kla_host.cpp draws the line), but a
+// call costs the host 11 us against 4, so a lone layer's token issued eagerly takes less with these (B=32 d_model 1024:
+// 29 us against 41; in a graph 27.6 against 24.4, and a captured one therefore takes the library's).
 #pragma once
 
 #include "kla_common.cuh"

@@ -2,8 +2,8 @@
 
 The reference layer's decode route (``KLALayer.forward`` with a state and ``L == 1``,
 src/kla/layers/kla_layer.py:295-345) is three projections with elementwise work between
-them. ``LayerDecoder.step`` runs them as ``kla_b200_linear`` for up to 32 bfloat16 rows, the
-first with the step of ``CausalConv1d`` (src/kla/layers/common.py:87-96) inside, and as library
+them. ``LayerDecoder.step`` runs them as ``kla_b200_linear`` for up to 32 bfloat16 rows (large
+layers of more than 16 rows only outside a graph capture), the first with the step of ``CausalConv1d`` (src/kla/layers/common.py:87-96) inside, and as library
 GEMMs around ``kla_b200_conv_step`` otherwise; between the second and the third stands
 ``kla_b200_step_layer`` (sensor post-processing, the filter step, skip path and gate;
 kla_layer.py:199-231, 277-293, 329-338).
@@ -263,9 +263,9 @@ class ModelDecoder:
     reference's ``SequenceModel.forward`` with a state and ``SequenceModel.generate``
     (src/kla/models/sequence_model.py:150-173, 200-220).
 
-    A block is ``x += mixer(norm(x))`` then ``x += mlp(norm(x))`` (sequence_model.py:47-98). For one token of up to 32
+    A block is ``x += mixer(norm(x))`` then ``x += mlp(norm(x))`` (sequence_model.py:47-98). For one token of up to 16
     sequences in bfloat16 that is six kernels: the projections with norm, convolution step, gate and residual sum folded
-    in, and the filter step. For a prompt the projections are library GEMMs and what stands between them one kernel each.
+    in, and the filter step. For up to 32 sequences large projections are library GEMMs. For a prompt the projections are library GEMMs and what stands between them one kernel each.
     One decoded token is a fixed sequence of launches over state that is updated in place, so ``generate`` captures it in
     a CUDA graph, which it keeps for calls with the same batch, types and weights, and replays it: a token then costs no
     host work but one replay, where the reference's loop issues several hundred small launches per token from Python.

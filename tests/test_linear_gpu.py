@@ -40,6 +40,25 @@ def test_projection_with_norm_bias_and_residual(B, N, K):
     assert lib.load().kla_b200_launch_count() - n0 == 2
 
 
+# both sides of the line between the kernel and the library's GEMM beyond 16 rows (80 M multiply-adds), and of a head's
+@pytest.mark.parametrize("B,N,K,launches", [(16, 4128, 2048, 1), (17, 4128, 1136, 1), (17, 4128, 1144, 0), (32, 2496, 1000, 1), (32, 2504, 1000, 0)])
+def test_large_projections_beyond_sixteen_rows_go_to_the_library(B, N, K, launches):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, b = rn(B, K), rn(N, K) * K ** -0.5, rn(N)
+    n0 = lib.load().kla_b200_launch_count()
+    close(lib.host().project(x, w, b, None, 0.0, None), F.linear(x.float(), w.float(), b.float()))
+    assert lib.load().kla_b200_launch_count() - n0 == launches
+
+
+@pytest.mark.parametrize("B,N,K", [(8, 4864, 64), (8, 4872, 64), (17, 2048, 64), (17, 2056, 64)])
+def test_heads_on_both_sides_of_the_line(B, N, K):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, nw = rn(B, K), rn(N, K) * K ** -0.5, rn(K)
+    close(lib.host().project(x, w, None, nw, 1e-6, None), F.linear(norm(x, nw, 1e-6), w.float()))
+
+
 @pytest.mark.parametrize("B,H,K", [(2, 24, 40), (8, 2048, 768), (20, 40, 256), (32, 33, 512)])
 def test_swiglu_step(B, H, K):
     g = torch.Generator(device="cuda").manual_seed(H)
@@ -72,6 +91,41 @@ def test_layer_token_in_bfloat16_follows_float32(B, d):
     torch.testing.assert_close(got.float(), want, rtol=5e-2, atol=3e-2 * want.abs().mean().item() + 1e-2)
     torch.testing.assert_close(sb[0].float(), sa[0], rtol=2e-2, atol=2e-2)
     torch.testing.assert_close(sb[1], sa[1], rtol=5e-2, atol=5e-2)
+
+
+def test_a_captured_token_of_a_large_layer_follows_the_eager_one():
+    """Between 17 and 32 rows a large layer's projections are the library's while a graph is captured. Both routes round
+    the same float32 sums once; a sum that falls on the other side changes a result by 2^-8 of it."""
+    B, d, S, K = 24, 768, 16, 4
+    M = 2 * d
+    g = torch.Generator(device="cuda").manual_seed(0)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    w = {"in_proj.weight": (rn(2 * M, d) * d ** -0.5).bfloat16(), "sensor_proj.weight": (rn(2 * M + 2 * S, M) * M ** -0.5).bfloat16(),
+         "out_proj.weight": (rn(d, M) * M ** -0.5).bfloat16(), "conv.weight": rn(M, 1, K) * 0.5, "conv.bias": rn(M) * 0.1,
+         "delta": rn(M, S) - 4, "lambda_log": rn(M, S) * 0.1, "process_noise": torch.full((M, S), 0.01, device="cuda"),
+         "lambda_skip": torch.tensor(-1.0, device="cuda")}
+    cfg = dict(d_state=S, discretization="ou", zero_process_noise=False, clip_value=None, obs_var_min=1e-4, obs_var_max=None,
+               value_rank="full", qk_norm=True, use_conv=True, conv_kernel_size=K, conv_activation="silu", use_gating=True,
+               gating_activation="silu", use_lambda_skip=True, return_variance=False, decode_from_prior=False)
+    dec, x = decode.LayerDecoder(w, cfg), rn(B, d).bfloat16()
+    eager, state = dec.init_state(B, "cuda", torch.bfloat16), dec.init_state(B, "cuda", torch.bfloat16)
+    launched = []
+
+    def token(st):
+        n0 = lib.load().kla_b200_launch_count()
+        out = dec.step(x, st)
+        launched.append(lib.load().kla_b200_launch_count() - n0)
+        return out
+
+    want = token(eager)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = token(state)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert launched == [4, 2]
+    for a, b in ((got, want), *zip(state, eager)):
+        assert (a.float() - b.float()).norm() <= 2 ** -7 * b.float().norm()
 
 
 # a row within the registers, across them, and one that does not divide into vectors
