@@ -97,6 +97,16 @@ class StepLayerArgs(Structure):
     ]
 
 
+class LinearArgs(Structure):
+    _fields_ = [
+        ("B", c_int64), ("N", c_int64), ("K", c_int64),
+        ("x", c_void_p), ("x_stride_b", c_int64), ("weight", c_void_p), ("bias", c_void_p), ("out", c_void_p), ("out_stride_b", c_int64),
+        ("norm_weight", c_void_p), ("norm_eps", c_float), ("swiglu", c_int32), ("residual", c_void_p), ("residual_stride_b", c_int64),
+        ("conv_D", c_int64), ("conv_taps", c_int64), ("conv_activation", c_int32),
+        ("conv_weight", c_void_p), ("conv_bias", c_void_p), ("conv_state", c_void_p), ("weights_ready", c_int32),
+    ]
+
+
 class RawScanArgs(Structure):
     _fields_ = [
         ("B", c_int64), ("L", c_int64), ("N", c_int64),
@@ -228,6 +238,14 @@ def load() -> ctypes.CDLL:
     lib.kla_b200_conv_seq_bwd.argtypes = [POINTER(ConvSeqBwdArgs), c_void_p]
     lib.kla_b200_step_layer.restype = c_int
     lib.kla_b200_step_layer.argtypes = [POINTER(StepLayerArgs), c_void_p]
+    lib.kla_b200_linear.restype = c_int
+    lib.kla_b200_linear.argtypes = [POINTER(LinearArgs), c_void_p]
+    lib.kla_b200_add_norm.restype = c_int
+    lib.kla_b200_add_norm.argtypes = [c_int64, c_int64, c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p]
+    lib.kla_b200_swiglu.restype = c_int
+    lib.kla_b200_swiglu.argtypes = [c_int64, c_int64, c_int32, c_void_p, c_void_p, c_void_p]
+    lib.kla_b200_argmax.restype = c_int
+    lib.kla_b200_argmax.argtypes = [c_int64, c_int64, c_int32, c_void_p, c_int64, c_void_p, c_void_p]
     lib.kla_b200_step.restype = c_int
     lib.kla_b200_step.argtypes = [POINTER(StepArgs), c_void_p]
     lib.kla_b200_strerror.restype = c_char_p

@@ -109,11 +109,12 @@ int lpc_for(int64_t S) {
     return lpc;  // 1..32 for S <= 128
 }
 
+bool known_type(int32_t dtype) { return dtype == KLA_B200_F32 || dtype == KLA_B200_BF16; }
+
 int check_common(int64_t B, int64_t L, int64_t M, int64_t S, int32_t in_dtype, int32_t out_dtype) {
     if (B < 0 || L < 0 || M < 0 || S < 0) return KLA_B200_EINVAL;
     if (S > KLA_B200_MAX_DSTATE) return KLA_B200_EUNSUPPORTED;
-    if (in_dtype != KLA_B200_F32 && in_dtype != KLA_B200_BF16) return KLA_B200_EUNSUPPORTED;
-    if (out_dtype != KLA_B200_F32 && out_dtype != KLA_B200_BF16) return KLA_B200_EUNSUPPORTED;
+    if (!known_type(in_dtype) || !known_type(out_dtype)) return KLA_B200_EUNSUPPORTED;
     if (in_dtype == KLA_B200_F32 && out_dtype == KLA_B200_BF16) return KLA_B200_EUNSUPPORTED;
     if (B > 65535 || L > (1 << 30) || M > (1 << 30)) return KLA_B200_EUNSUPPORTED;
     return KLA_B200_OK;
@@ -905,7 +906,7 @@ int kla_b200_conv_seq_bwd(const kla_b200_conv_seq_bwd_args *a, void *stream) {
 int kla_b200_add_norm(int64_t rows, int64_t D, int32_t dtype, int32_t weight_dtype, const void *x, const void *delta, const void *weight,
                       float eps, void *sum, void *out, void *stream) {
     if (rows < 0 || D < 0) return KLA_B200_EINVAL;
-    if (D % 8 || D > (1 << 30) || rows > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;
+    if (D % 8 || D > (1 << 30) || rows > 0x7fffffffll || !known_type(dtype) || !known_type(weight_dtype)) return KLA_B200_EUNSUPPORTED;
     if (rows == 0 || D == 0) return KLA_B200_OK;
     if (!x || !weight || !out || (delta && !sum)) return KLA_B200_EINVAL;
     for (const void *p : {x, delta, weight, static_cast<const void *>(sum), static_cast<const void *>(out)})
@@ -925,7 +926,7 @@ int kla_b200_add_norm(int64_t rows, int64_t D, int32_t dtype, int32_t weight_dty
 
 int kla_b200_swiglu(int64_t rows, int64_t H, int32_t dtype, const void *gate_up, void *out, void *stream) {
     if (rows < 0 || H < 0) return KLA_B200_EINVAL;
-    if (H % 8 || H > (1 << 29) || rows > (1ll << 31)) return KLA_B200_EUNSUPPORTED;
+    if (H % 8 || H > (1 << 29) || rows > (1ll << 31) || !known_type(dtype)) return KLA_B200_EUNSUPPORTED;
     if (rows == 0 || H == 0) return KLA_B200_OK;
     if (!gate_up || !out) return KLA_B200_EINVAL;
     if (!aligned(gate_up, 16) || !aligned(out, 16)) return KLA_B200_EALIGN;
@@ -963,7 +964,7 @@ int kla_b200_qk_norm(int64_t B, int64_t L, int64_t S, int32_t dtype, kla_b200_te
 
 int kla_b200_argmax(int64_t rows, int64_t n, int32_t dtype, const void *x, int64_t row_stride, int64_t *out, void *stream) {
     if (rows < 0 || n < 1 || row_stride < 0) return KLA_B200_EINVAL;
-    if (n > (1 << 30) || rows > 0x7fffffffll) return KLA_B200_EUNSUPPORTED;
+    if (n > (1 << 30) || rows > 0x7fffffffll || !known_type(dtype)) return KLA_B200_EUNSUPPORTED;
     if (rows == 0) return KLA_B200_OK;
     if (!x || !out) return KLA_B200_EINVAL;
     if (!aligned(x, dtype == KLA_B200_BF16 ? 2 : 4) || !aligned(out, 8)) return KLA_B200_EALIGN;
@@ -980,8 +981,11 @@ int kla_b200_linear(const kla_b200_linear_args *a, void *stream) {
     if (a == nullptr || a->B < 0 || a->N < 0 || a->K < 0) return KLA_B200_EINVAL;
     if (a->B > KLA_B200_LINEAR_MAX_ROWS || a->N > (1 << 30) || a->K > (1 << 20) || a->K % 8 || a->x_stride_b % 8) return KLA_B200_EUNSUPPORTED;
     if (a->B == 0 || a->N == 0) return KLA_B200_OK;
-    if (a->K == 0 || !a->x || !a->weight || !a->out || a->x_stride_b < 0 || a->out_stride_b < 0) return KLA_B200_EINVAL;
-    if (!aligned(a->x, 16) || !aligned(a->weight, 16) || (a->norm_weight && !aligned(a->norm_weight, 16)) || !aligned(a->out, 2)) return KLA_B200_EALIGN;
+    if (a->K == 0 || !a->x || !a->weight || !a->out || a->x_stride_b < 0 || a->out_stride_b < 0 || a->residual_stride_b < 0) return KLA_B200_EINVAL;
+    for (const void *p : {a->x, a->weight, a->norm_weight})
+        if (p && !aligned(p, 16)) return KLA_B200_EALIGN;
+    for (const void *p : {a->bias, a->residual, static_cast<const void *>(a->out), static_cast<const void *>(a->conv_state)})
+        if (p && !aligned(p, 2)) return KLA_B200_EALIGN;
     if (a->swiglu && (a->N % 2 || a->conv_D)) return KLA_B200_EINVAL;
     LinearParams prm{};
     prm.B = (int)a->B; prm.N = (int)a->N; prm.K = (int)a->K;

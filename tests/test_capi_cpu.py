@@ -117,6 +117,33 @@ def test_new_entry_points_reject_bad_arguments_without_cuda(L):
     assert lib.kla_b200_launch_count() == 0
 
 
+def test_decode_entry_points_reject_bad_arguments_without_cuda(L):
+    lib = L.load()
+    buf = (ctypes.c_float * 4096)()
+    at = (ctypes.addressof(buf) + 63) // 64 * 64
+
+    def linear(**kw):
+        args = dict(B=2, N=16, K=16, x=at, x_stride_b=16, weight=at, out=at, out_stride_b=16)
+        return lib.kla_b200_linear(ctypes.byref(L.LinearArgs(**{**args, **kw})), None)
+
+    assert lib.kla_b200_linear(None, None) == 1
+    assert linear(B=0) == 0 and linear(N=0) == 0
+    for bad in (dict(K=0), dict(x=None), dict(weight=None), dict(out=None), dict(B=-1), dict(x_stride_b=-8), dict(residual=at, residual_stride_b=-1),
+                dict(swiglu=1, N=17), dict(swiglu=1, conv_D=8), dict(conv_D=8, conv_taps=4), dict(conv_D=8, conv_taps=1, conv_weight=at, conv_activation=9)):
+        assert linear(**bad) == 1, bad
+    for bad in (dict(B=33), dict(K=20), dict(x_stride_b=20), dict(conv_D=17, conv_taps=1), dict(conv_D=8, conv_taps=9)):
+        assert linear(**bad) == 2, bad
+    assert linear(B=8, K=1 << 14, norm_weight=at) == 2  # eight normalised rows of that length do not fit shared memory
+    for name, off in (("x", 8), ("weight", 2), ("norm_weight", 8), ("out", 1), ("bias", 1), ("residual", 1), ("conv_state", 1)):
+        assert linear(**{name: at + off}) == 4, name
+    for dtype in (-1, 2, 7):
+        assert lib.kla_b200_add_norm(1, 8, dtype, 0, at, None, at, 1e-6, at, at, None) == 2
+        assert lib.kla_b200_add_norm(1, 8, 0, dtype, at, None, at, 1e-6, at, at, None) == 2
+        assert lib.kla_b200_swiglu(1, 8, dtype, at, at, None) == 2
+        assert lib.kla_b200_argmax(1, 8, dtype, at, 8, at, None) == 2
+    assert lib.kla_b200_launch_count() == 0
+
+
 def test_sizes_that_overflow_are_refused_not_wrapped(L):
     lib = L.load()
     size_max = ctypes.c_size_t(-1).value

@@ -40,6 +40,21 @@ def test_projection_with_norm_bias_and_residual(B, N, K):
     assert lib.load().kla_b200_launch_count() - n0 == 2
 
 
+@pytest.mark.parametrize("B,H,K", [(3, 24, 40), (12, 40, 256), (32, 33, 512)])
+def test_gate_and_up_of_rows_taken_as_they_are(B, H, K):
+    """The C entry's swiglu without a norm in front, which the wrappers do not use."""
+    import ctypes
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, b, out = rn(B, K), rn(2 * H, K) * K ** -0.5, rn(2 * H), torch.empty(B, H, device="cuda", dtype=torch.bfloat16)
+    lib.check(lib.load().kla_b200_linear(ctypes.byref(lib.LinearArgs(
+        B=B, N=2 * H, K=K, x=x.data_ptr(), x_stride_b=K, weight=w.data_ptr(), bias=b.data_ptr(), out=out.data_ptr(), out_stride_b=H, swiglu=1)),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    gate, up = F.linear(x.float(), w.float(), b.float()).chunk(2, dim=-1)
+    close(out, F.silu(gate) * up)
+
+
 # both sides of the line between the kernel and the library's GEMM beyond 16 rows (80 M multiply-adds), and of a head's
 @pytest.mark.parametrize("B,N,K,launches", [(16, 4128, 2048, 1), (17, 4128, 1136, 1), (17, 4128, 1144, 0), (32, 2496, 1000, 1), (32, 2504, 1000, 0)])
 def test_large_projections_beyond_sixteen_rows_go_to_the_library(B, N, K, launches):
