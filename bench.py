@@ -458,7 +458,7 @@ def run_b200(args):
                          "peak_source": peak_src, "algorithmic_bytes": bwd_bytes, "ms": bwd_ms,
                          "nominal_peak_gbs": 8000.0, "frac_of_nominal": ach_bwd / 8000.0,
                          "note": "not HBM-bound at d_state=16: 43.5 warp-instructions per 32 lane-steps against 24.8 KB per "
-                                 "token; bound by the FP32 pipe's register reads (ncu: issue slots 58 % busy, FP32 pipe 63 %; the "
+                                 "token; bound by the FP32 pipe's register reads (ncu: issue slots 56 % busy, FP32 pipe 58 %; the "
                                  "256 sequences run as 16 segments each, handed from CTA to CTA)"},
             "roofline_fwd": {"bound": "hbm", "kernel": "kla_fwd_kernel", "achieved": ach_fwd, "peak": peak,
                              "unit": "GB/s", "frac": ach_fwd / peak, "traffic": NCU_TRAFFIC["kla_fwd_kernel"] * B / 8 if "kla_fwd_kernel" in NCU_TRAFFIC else None,
@@ -1017,10 +1017,13 @@ def run_decode_layer(args):
         y = y * F.silu(gate)
         return F.linear(y, dec.w["out_proj.weight"])
 
+    lib = __import__("importlib").import_module("kalman-linear-attention_b200._lib")
+
     def graph_of(step_fn):
         st = dec.init_state(B, dev, dt)
         step_fn(xs[0], st)
         torch.cuda.synchronize()
+        n0 = lib.load().kla_b200_launch_count()
         s = torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(s):
@@ -1029,7 +1032,7 @@ def run_decode_layer(args):
                 for t in range(NTOK):
                     out = step_fn(xs[t], st)
         torch.cuda.current_stream().wait_stream(s)
-        return gr, out
+        return gr, out, lib.load().kla_b200_launch_count() - n0
 
     def time_graph(gr):
         for _ in range(max(args.warmup, 3)):
@@ -1043,11 +1046,8 @@ def run_decode_layer(args):
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) * 1e3 / (args.steps * NTOK)
 
-    lib = __import__("importlib").import_module("kalman-linear-attention_b200._lib")
-    n0 = lib.load().kla_b200_launch_count()
-    g_fused, out_f = graph_of(dec.step)
-    launches_per_pass = lib.load().kla_b200_launch_count() - n0 - 2
-    g_eager, out_e = graph_of(eager_step)
+    g_fused, out_f, launches_per_pass = graph_of(dec.step)
+    g_eager, out_e, _ = graph_of(eager_step)
     us_f, us_e = time_graph(g_fused), time_graph(g_eager)
     # bytes a token must move besides the three GEMMs: state (lam, eta, conv window) read + write, a, p, activations
     esz = 2
