@@ -15,10 +15,12 @@
 //   * where W does not depend on the kernel before (the caller says so), its first blocks are requested before the wait for
 //     that kernel (programmatic dependent launch): all of a warp's share up to K = 2048 for up to eight rows, up to 1024 for
 //     more rows and for swiglu;
-// Measured on B200 in a CUDA graph, us per projection, against the library's GEMM alone (rows x columns of W):
-//   B=8   3072 x 768 4.2 (3.7), with the norm 4.4; 3104 x 1536 5.9 (5.4); 768 x 1536 3.4 (4.4); 768 x 2048 3.6 (5.2)
-//   B=16  4096 x 1024 3.9 (3.6); 4128 x 2048 5.6 (5.5); 1024 x 2048 4.6 (5.9)
-//   B=32  4096 x 1024 5.3 (3.5); 4128 x 2048 8.1 (5.6); 1024 x 2048 5.4 (4.9)
+// Measured on B200 in a CUDA graph, W in L2, us per projection, against the library's GEMM with what the kernel folds in as
+// launches of their own:
+//   B=8   3072 x 768 4.2 (4.7), with the norm 4.8 (7.2); 3104 x 1536 4.7 (6.7); 768 x 1536 3.6 (5.2); 768 x 2048 with the
+//         residual 4.2 (7.2)
+//   B=16  4096 x 1024 3.6 (4.2), with the norm 6.7 (7.2); 4128 x 2048 6.2 (5.2), W from HBM 5.7 (6.3); 1024 x 2048 3.8 (6.7)
+//   B=32  4096 x 1024 4.8 (4.2), with the norm 10.4 (7.3); 4128 x 2048 8.3 (5.7); 1024 x 2048 5.2 (6.2)
 // What bounds it is latency: about 3 us of launch, one round trip for x, the sum over warps and the store. Beyond 16 rows
 // the library's kernels are the faster ones where a projection is large (kernel_pays in kla_host.cpp draws the line), but a
 // call costs the host 11 us against 4, so a lone layer's token issued eagerly takes less with these (B=32 d_model 1024:

@@ -2,6 +2,7 @@
 
 import importlib
 import os
+import subprocess
 import sys
 
 import pytest
@@ -146,6 +147,36 @@ def test_a_captured_token_of_a_large_layer_follows_the_eager_one():
     assert launched == [4, 2]
     for a, b in ((got, want), *zip(state, eager)):
         assert (a.float() - b.float()).norm() <= 2 ** -7 * b.float().norm()
+
+
+def test_a_large_layer_is_captured_before_the_library_has_run():
+    """In a process whose tokens so far were all kernels of this package, the capture itself sets the library up."""
+    code = """
+import importlib, sys
+import torch
+sys.path.insert(0, %r)
+import kla_b200
+B, d, S = 24, 768, 16
+M = 2 * d
+rn = lambda *s: torch.randn(*s, device="cuda")
+w = {"in_proj.weight": (rn(2 * M, d) * d ** -0.5).bfloat16(), "sensor_proj.weight": (rn(2 * M + 2 * S, M) * M ** -0.5).bfloat16(),
+     "out_proj.weight": (rn(d, M) * M ** -0.5).bfloat16(), "delta": rn(M, S) - 4, "lambda_log": rn(M, S) * 0.1,
+     "process_noise": torch.full((M, S), 0.01, device="cuda")}
+cfg = dict(d_state=S, discretization="ou", zero_process_noise=False, clip_value=None, obs_var_min=1e-4, obs_var_max=None,
+           value_rank="full", qk_norm=True, use_conv=False, conv_kernel_size=4, conv_activation="silu", use_gating=True,
+           gating_activation="silu", use_lambda_skip=False, return_variance=False, decode_from_prior=False)
+dec, x = kla_b200.LayerDecoder(w, cfg), rn(B, d).bfloat16()
+a, b = dec.init_state(B, "cuda", torch.bfloat16), dec.init_state(B, "cuda", torch.bfloat16)
+want = dec.step(x, a)
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    got = dec.step(x, b)
+g.replay()
+torch.cuda.synchronize()
+assert (got.float() - want.float()).norm() <= 2 ** -7 * want.float().norm()
+""" % os.path.dirname(HERE)
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
 
 
 # a row within the registers, across them, and one that does not divide into vectors
