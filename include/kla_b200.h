@@ -473,6 +473,49 @@ typedef struct kla_b200_linear_args {
 int kla_b200_linear(const kla_b200_linear_args *args, void *stream);
 
 /*
+ * One token of up to KLA_B200_TOKEN_MAX_ROWS rows of bfloat16 through a stack of KLA blocks, or through one lone layer, in one
+ * launch: per layer what kla_b200_linear (in_proj with the convolution's step), kla_b200_linear (sensor_proj),
+ * kla_b200_step_layer and kla_b200_linear (out_proj) do, then, with mlp, the swiglu MLP's two projections, with the norms and
+ * residual sums of a block where norm_weight is given (src/kla/layers/kla_layer.py:295-345,
+ * src/kla/models/sequence_model.py:47-98). Results are those of these calls to the bit. Every projection's weight is
+ * [N, K] contiguous, 16-byte aligned, K a multiple of 8; all of v, log-variance, k, q come straight from sensor_proj.
+ * work: kla_b200_token_work_bytes, all zero before the first launch that uses it and from then on used by launches with the same
+ * B, d, mlp and per layer M, S, hidden, gated and w_value only, one at a time (it holds tagged words that a launch tells from
+ * those of the launches before). The launch is a cooperative grid of one CTA per SM.
+ */
+#define KLA_B200_TOKEN_MAX_ROWS 8
+#define KLA_B200_TOKEN_MAX_LAYERS 32
+typedef struct kla_b200_token_layer {
+    const void *in_weight, *in_bias;          /* [M or 2 M (gated), d]; biases: bfloat16 [N] or NULL, all of them */
+    const void *sensor_weight, *sensor_bias;  /* [w_value + M + 2 S, M] */
+    const void *out_weight, *out_bias;        /* [d, M] */
+    const void *w12, *b12, *w3, *b3;          /* [2 hidden, d], [d, hidden]; with mlp */
+    const void *norm_weight, *mlp_norm_weight; /* bfloat16 [d]; norm_weight NULL: neither norm nor residual sum */
+    const float *conv_weight, *conv_bias;     /* [M, conv_taps], [M] or NULL; conv_weight NULL: no convolution */
+    void *conv_state;                         /* in/out [B, M, conv_taps - 1] bfloat16 */
+    const float *a, *p, *lambda_skip;         /* [M, S]; [lambda_skip_len] or NULL */
+    float *lam, *eta;                         /* in/out [B, M, S] */
+    int64_t M, S, hidden, conv_taps;
+    int32_t gated, w_value;                   /* w_value: M, or 0 where the value is the convolution's output */
+    int32_t conv_activation, gate_activation, lambda_skip_len, qk_norm, decode_from_prior;
+    float obs_var_min, obs_var_max, clip_value;
+} kla_b200_token_layer;
+typedef struct kla_b200_token_args {
+    int64_t B, d, layers;
+    int32_t mlp;                 /* every layer is followed by a swiglu MLP; needs norm weights */
+    float norm_eps;
+    const void *x;               /* in  [B, d] bfloat16, 16-byte aligned, row stride a multiple of 8 */
+    int64_t x_stride_b;
+    void *out;                   /* out [B, d] contiguous */
+    void *y_var;                 /* out [B, M] gated variance of a lone layer, or NULL */
+    void *work;
+    const kla_b200_token_layer *layer;
+} kla_b200_token_args;
+
+size_t kla_b200_token_work_bytes(const kla_b200_token_args *args); /* 0: kla_b200_token refuses these sizes */
+int kla_b200_token(const kla_b200_token_args *args, void *stream);
+
+/*
  * Raw scan pair over materialised coefficients. Replaces the reference's
  * tiled_mobius_scan(A, B, C, D, lam0) and tiled_affine_scan(alpha, r)
  * (src/kla/ops/kernels/triton/tiled_mobius_scan.py:301-311) and their exact

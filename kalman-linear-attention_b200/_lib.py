@@ -32,6 +32,8 @@ SYMBOLS = (
     "kla_b200_conv_seq_bwd",
     "kla_b200_step_layer",
     "kla_b200_linear",
+    "kla_b200_token_work_bytes",
+    "kla_b200_token",
     "kla_b200_add_norm",
     "kla_b200_swiglu",
     "kla_b200_argmax",
@@ -104,6 +106,26 @@ class LinearArgs(Structure):
         ("norm_weight", c_void_p), ("norm_eps", c_float), ("swiglu", c_int32), ("residual", c_void_p), ("residual_stride_b", c_int64),
         ("conv_D", c_int64), ("conv_taps", c_int64), ("conv_activation", c_int32),
         ("conv_weight", c_void_p), ("conv_bias", c_void_p), ("conv_state", c_void_p), ("weights_ready", c_int32),
+    ]
+
+
+class TokenLayer(Structure):
+    _fields_ = [
+        *((n, c_void_p) for n in (
+            "in_weight", "in_bias", "sensor_weight", "sensor_bias", "out_weight", "out_bias", "w12", "b12", "w3", "b3", "norm_weight",
+            "mlp_norm_weight", "conv_weight", "conv_bias", "conv_state", "a", "p", "lambda_skip", "lam", "eta")),
+        ("M", c_int64), ("S", c_int64), ("hidden", c_int64), ("conv_taps", c_int64),
+        *((n, c_int32) for n in (
+            "gated", "w_value", "conv_activation", "gate_activation", "lambda_skip_len", "qk_norm", "decode_from_prior")),
+        ("obs_var_min", c_float), ("obs_var_max", c_float), ("clip_value", c_float),
+    ]
+
+
+class TokenArgs(Structure):
+    _fields_ = [
+        ("B", c_int64), ("d", c_int64), ("layers", c_int64), ("mlp", c_int32), ("norm_eps", c_float),
+        ("x", c_void_p), ("x_stride_b", c_int64), ("out", c_void_p), ("y_var", c_void_p), ("work", c_void_p),
+        ("layer", POINTER(TokenLayer)),
     ]
 
 
@@ -240,6 +262,10 @@ def load() -> ctypes.CDLL:
     lib.kla_b200_step_layer.argtypes = [POINTER(StepLayerArgs), c_void_p]
     lib.kla_b200_linear.restype = c_int
     lib.kla_b200_linear.argtypes = [POINTER(LinearArgs), c_void_p]
+    lib.kla_b200_token_work_bytes.restype = c_size_t
+    lib.kla_b200_token_work_bytes.argtypes = [POINTER(TokenArgs)]
+    lib.kla_b200_token.restype = c_int
+    lib.kla_b200_token.argtypes = [POINTER(TokenArgs), c_void_p]
     lib.kla_b200_add_norm.restype = c_int
     lib.kla_b200_add_norm.argtypes = [c_int64, c_int64, c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p]
     lib.kla_b200_swiglu.restype = c_int
@@ -263,7 +289,7 @@ def load() -> ctypes.CDLL:
 _host = None
 _HOST_ENTRIES = (
     "scan_fwd", "scan_bwd", "slab_aggregate", "chunk_fold", "epilogue_bwd", "step", "conv_step", "step_layer",
-    "linear", "add_norm", "swiglu", "argmax", "qk_norm", "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
+    "linear", "token_work_bytes", "token", "add_norm", "swiglu", "argmax", "qk_norm", "conv_seq", "conv_seq_bwd", "mobius_scan_fwd", "mobius_scan_bwd", "affine_scan_fwd", "affine_scan_bwd",
     "ckpt_bytes", "segment_scratch_bytes", "strerror",
 )
 

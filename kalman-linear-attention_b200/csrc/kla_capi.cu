@@ -16,6 +16,7 @@
 #include "kla_rawscan.cuh"
 #include "kla_slab.cuh"
 #include "kla_step.cuh"
+#include "kla_token.cuh"
 
 // The device's status word (kla_b200_device_status). Kernels get its device address in their
 // parameters (WaitCtl::status): in host code the name below is only a handle.
@@ -506,6 +507,132 @@ int dispatch_linear(const LinearParams &prm, int mode, cudaStream_t st) {
     if (mode == kLinearSwiglu) return norm ? dispatch_linear_tiles<NT, kLinearSwiglu, true>(prm, st) : dispatch_linear_tiles<NT, kLinearSwiglu, false>(prm, st);
     if (mode == kLinearConv) return norm ? dispatch_linear_tiles<NT, kLinearConv, true>(prm, st) : dispatch_linear_tiles<NT, kLinearConv, false>(prm, st);
     return norm ? dispatch_linear_tiles<NT, kLinearPlain, true>(prm, st) : dispatch_linear_tiles<NT, kLinearPlain, false>(prm, st);
+}
+
+// Where the words between the phases of a token lie in its working memory.
+struct TokenWork {
+    size_t proj, sens, y, xa, xb, h, total;
+};
+TokenWork token_work(const kla_b200_token_args *a) {
+    int64_t proj = 0, sens = 0, y = 0, h = 0;
+    for (int64_t i = 0; i < a->layers; ++i) {
+        const kla_b200_token_layer &l = a->layer[i];
+        const int64_t p = (l.gated ? 2 : 1) * l.M, s = l.w_value + l.M + 2 * l.S;
+        proj = p > proj ? p : proj;
+        sens = s > sens ? s : sens;
+        y = l.M > y ? l.M : y;
+        h = l.hidden > h ? l.hidden : h;
+    }
+    TokenWork w{};
+    size_t at = kTokHeader;
+    auto place = [&](int64_t columns) {
+        const size_t here = at;
+        at += ((size_t)a->B * columns * sizeof(uint32_t) + 255) / 256 * 256;
+        return here;
+    };
+    w.proj = place(proj); w.sens = place(sens); w.y = place(y); w.xa = place(a->d); w.xb = place(a->d); w.h = place(a->mlp ? h : 0);
+    w.total = at;
+    return w;
+}
+
+int64_t token_widest(const kla_b200_token_args *a) {  // columns of the widest projection, whose x has to fit shared memory
+    int64_t K = a->d;
+    for (int64_t i = 0; i < a->layers; ++i) {
+        K = a->layer[i].M > K ? a->layer[i].M : K;
+        if (a->mlp && a->layer[i].hidden > K) K = a->layer[i].hidden;
+    }
+    return K;
+}
+
+int check_token(const kla_b200_token_args *a) {
+    if (a == nullptr || a->B < 0 || a->d < 0 || a->layers < 0 || (a->layers > 0 && !a->layer)) return KLA_B200_EINVAL;
+    if (a->B > KLA_B200_TOKEN_MAX_ROWS || a->layers > KLA_B200_TOKEN_MAX_LAYERS || a->d % 8 || a->d > (1 << 20)) return KLA_B200_EUNSUPPORTED;
+    for (int64_t i = 0; i < a->layers; ++i) {
+        const kla_b200_token_layer &l = a->layer[i];
+        if (l.M < 0 || l.S < 0 || l.hidden < 0 || l.w_value < 0 || l.lambda_skip_len < 0) return KLA_B200_EINVAL;
+        if (l.M % 8 || l.M > (1 << 18) || l.S > KLA_B200_MAX_DSTATE || (a->mlp && (l.hidden % 8 || l.hidden > (1 << 18)))) return KLA_B200_EUNSUPPORTED;
+        if (l.M == 0 || l.S == 0 || (l.w_value != 0 && l.w_value != l.M) || (a->mlp && (l.hidden == 0 || !l.norm_weight))) return KLA_B200_EINVAL;
+        if (l.conv_weight && (l.conv_taps < 1 || l.conv_taps > KLA_B200_MAX_CONV_TAPS)) return KLA_B200_EUNSUPPORTED;
+        if (l.conv_activation < KLA_B200_ACT_SILU || l.conv_activation > KLA_B200_ACT_NONE || l.gate_activation < KLA_B200_ACT_SILU ||
+            l.gate_activation > KLA_B200_ACT_NONE)
+            return KLA_B200_EINVAL;
+        if (l.lambda_skip_len != 0 && l.lambda_skip_len != 1 && l.lambda_skip_len != l.M) return KLA_B200_EINVAL;
+    }
+    const int widest = (int)token_widest(a);
+    return token_ring(widest) ? KLA_B200_OK : KLA_B200_EUNSUPPORTED;
+}
+
+template <int LAYERS>
+int launch_token(const kla_b200_token_args *a, cudaStream_t st) {
+    using bf16 = __nv_bfloat16;
+    TokenParams<LAYERS> prm{};
+    const int B = (int)a->B, d = (int)a->d, G = device_sms();
+    const bool mlp = a->mlp != 0;
+    const TokenWork w = token_work(a);
+    auto words = [&](size_t offset) { return reinterpret_cast<uint32_t *>(static_cast<char *>(a->work) + offset); };
+    uint32_t *xa = words(w.xa), *xb = words(w.xb), *h = words(w.h);
+    prm.B = B; prm.layers = (int)a->layers; prm.phases = mlp ? 5 : 3; prm.norm_eps = a->norm_eps;
+    prm.out_var = static_cast<bf16 *>(a->y_var);
+    prm.proj = words(w.proj); prm.sens = words(w.sens); prm.y = words(w.y); prm.sync = words(0);
+    if (int rc = wait_ctl(&prm.wait)) return rc;
+    for (int i = 0; i < prm.layers; ++i) {
+        const kla_b200_token_layer &l = a->layer[i];
+        TokenLayer &t = prm.layer[i];
+        const int M = (int)l.M, S = (int)l.S, hidden = (int)l.hidden, N_in = (l.gated ? 2 : 1) * M, N_sensor = l.w_value + M + 2 * S;
+        const bool first = i == 0, last = i + 1 == prm.layers;
+        auto phase = [&](int k, const void *weight, const void *bias, const void *norm, int N, int K, const void *src, int64_t src_sb, void *dst, int dst_sb) {
+            TokenPhase &p = t.ph[k];
+            p.w = static_cast<const bf16 *>(weight); p.bias = static_cast<const bf16 *>(bias); p.norm_w = static_cast<const bf16 *>(norm);
+            p.src = src; p.src_sb = src_sb; p.dst = dst; p.dst_sb = dst_sb; p.N = N; p.K = K;
+            const int octs = (N + 7) / 8;
+            p.oct_q = octs / G; p.oct_r = octs % G;
+        };
+        // x: what the layer starts from, words of the layer before (their last projection's outputs)
+        const void *x = first ? a->x : mlp ? xb : xa;
+        const int64_t x_sb = first ? a->x_stride_b : d;
+        void *mixed = last && !mlp ? a->out : xa, *sum = last ? a->out : xb;
+        phase(kTokIn, l.in_weight, l.in_bias, l.norm_weight, N_in, d, x, x_sb, prm.proj, N_in);
+        phase(kTokSensor, l.sensor_weight, l.sensor_bias, nullptr, N_sensor, M, prm.proj, N_in, prm.sens, N_sensor);
+        phase(kTokOut, l.out_weight, l.out_bias, nullptr, d, M, prm.y, M, mixed, d);
+        t.ph[kTokIn].plain_src = first;
+        t.ph[kTokOut].plain_dst = last && !mlp;
+        if (l.norm_weight) { t.ph[kTokOut].res = x; t.ph[kTokOut].res_sb = x_sb; t.ph[kTokOut].plain_res = first; }
+        if (mlp) {
+            phase(kTokGateUp, l.w12, l.b12, l.mlp_norm_weight, hidden, d, xa, d, h, hidden);
+            phase(kTokDown, l.w3, l.b3, nullptr, d, hidden, h, hidden, sum, d);
+            t.ph[kTokDown].res = xa; t.ph[kTokDown].res_sb = d; t.ph[kTokDown].plain_dst = last;
+        }
+        t.conv_w = l.conv_weight; t.conv_b = l.conv_bias; t.conv_state = static_cast<bf16 *>(l.conv_state);
+        t.a = l.a; t.p = l.p; t.skip = l.lambda_skip_len ? l.lambda_skip : nullptr; t.lam = l.lam; t.eta = l.eta;
+        t.M = M; t.S = S; t.taps = (int)l.conv_taps; t.conv_act = l.conv_activation;
+        t.gate_act = l.gate_activation; t.gated = l.gated != 0; t.skip_len = l.lambda_skip_len; t.w_value = l.w_value;
+        t.qk_norm = l.qk_norm; t.prior = l.decode_from_prior;
+        t.vec = S % 4 == 0 && aligned(l.a, 16) && aligned(l.p, 16) && aligned(l.lam, 16) && aligned(l.eta, 16);
+        t.lpc = 1;
+        while (4 * t.lpc < S) t.lpc *= 2;
+        const int channels = 32 / t.lpc;
+        t.blocks = (M + channels - 1) / channels;
+        t.unit_q = B * t.blocks / (G * kTokWarps); t.unit_r = B * t.blocks % (G * kTokWarps);
+        t.obs_var_min = l.obs_var_min; t.obs_var_max = l.obs_var_max; t.clip = l.clip_value;
+    }
+    prm.ring = token_ring((int)token_widest(a));
+    const size_t smem = token_smem((int)token_widest(a), prm.ring);
+    auto kern = kla_token_kernel<LAYERS>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;  // CTAs wait for one another's words
+    attr.val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)G);
+    cfg.blockDim = dim3(kTokThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, prm);
+    g_launches++;
+    return e == cudaSuccess ? KLA_B200_OK : cuda_fail(e);
 }
 }  // namespace
 
@@ -1007,6 +1134,30 @@ int kla_b200_linear(const kla_b200_linear_args *a, void *stream) {
     if (a->B <= 8) return dispatch_linear<1>(prm, mode, st);
     if (a->B <= 16) return dispatch_linear<2>(prm, mode, st);
     return dispatch_linear<4>(prm, mode, st);
+}
+
+size_t kla_b200_token_work_bytes(const kla_b200_token_args *a) { return check_token(a) == KLA_B200_OK ? token_work(a).total : 0; }
+
+int kla_b200_token(const kla_b200_token_args *a, void *stream) {
+    if (int rc = check_token(a)) return rc;
+    if (a->B == 0 || a->d == 0 || a->layers == 0) return KLA_B200_OK;
+    if (!a->x || !a->out || !a->work || a->x_stride_b < 0 || (a->y_var && a->layers != 1)) return KLA_B200_EINVAL;
+    if (a->x_stride_b % 8) return KLA_B200_EUNSUPPORTED;
+    if (!aligned(a->x, 16) || !aligned(a->out, 16) || !aligned(a->work, 256) || !aligned(a->y_var, 2)) return KLA_B200_EALIGN;
+    for (int64_t i = 0; i < a->layers; ++i) {
+        const kla_b200_token_layer &l = a->layer[i];
+        if (!l.in_weight || !l.sensor_weight || !l.out_weight || !l.a || !l.p || !l.lam || !l.eta) return KLA_B200_EINVAL;
+        if ((a->mlp && (!l.w12 || !l.w3 || !l.mlp_norm_weight)) || (l.conv_weight && l.conv_taps > 1 && !l.conv_state) || (l.lambda_skip_len && !l.lambda_skip))
+            return KLA_B200_EINVAL;
+        for (const void *p : {l.in_weight, l.sensor_weight, l.out_weight, l.norm_weight, a->mlp ? l.w12 : nullptr, a->mlp ? l.w3 : nullptr, a->mlp ? l.mlp_norm_weight : nullptr})
+            if (p && !aligned(p, 16)) return KLA_B200_EALIGN;
+        for (const void *p : {l.in_bias, l.sensor_bias, l.out_bias, l.b12, l.b3, static_cast<const void *>(l.conv_state)})
+            if (p && !aligned(p, 2)) return KLA_B200_EALIGN;
+        for (const float *p : {l.conv_weight, l.conv_bias, l.a, l.p, l.lambda_skip, static_cast<const float *>(l.lam), static_cast<const float *>(l.eta)})
+            if (p && !aligned(p, 4)) return KLA_B200_EALIGN;
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return a->layers == 1 ? launch_token<1>(a, st) : launch_token<KLA_B200_TOKEN_MAX_LAYERS>(a, st);
 }
 
 int kla_b200_step_layer(const kla_b200_step_layer_args *a, void *stream) {

@@ -179,6 +179,24 @@ __global__ void __launch_bounds__(128) kla_conv_seq_kernel(const ConvSeqParams p
     }
 }
 
+// One state of one channel by one token, in the reference's information form and with its floors
+// (src/kla/ops/kla_ops.py:310-327); lv: the value's precision, vl: value times precision.
+__device__ __forceinline__ void filter_step(float a, float p_raw, float lam0, float eta0, float lv, float vl, float k, bool prior, float &lam,
+                                            float &eta, float &mean, float &var) {
+    const float p = fmaxf(p_raw, kPMin);                // kla_ops.py:316
+    const float a2 = fmaxf(a * a, kEps);                // :317
+    const float phi = fmaxf(lv * k * k, kEps);          // :310-312
+    const float inv = 1.0f / fmaxf(a2 + p * lam0, kEps);  // :319
+    lam = lam0 * inv + phi;                             // :320
+    eta = (a * inv) * eta0 + vl * k;                    // :321
+    var = 1.0f / fmaxf(lam, kEps);                      // :323
+    mean = eta * var;                                   // :324
+    if (prior) {                                        // :325-327
+        mean = a * mean;
+        var = a2 * var + p;
+    }
+}
+
 struct StepLayerParams {
     int B, M, S;
     const void *v, *ls, *k, *q, *z, *gate;  // z, gate may be nullptr
@@ -297,19 +315,8 @@ __global__ void __launch_bounds__(128) kla_step_layer_kernel(const __grid_consta
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const bool in = j * 4 + i < S;
-            const float a = av[c][i];
-            const float p = fmaxf(pv[c][i], kPMin);                     // kla_ops.py:316
-            const float a2 = fmaxf(a * a, kEps);                        // :317
-            const float phi = fmaxf(lv * kv[i] * kv[i], kEps);          // :310-312
-            const float inv = 1.0f / fmaxf(a2 + p * lamv[c][i], kEps);  // :319
-            const float lam = lamv[c][i] * inv + phi;                   // :320
-            const float eta = (a * inv) * etav[c][i] + vl * kv[i];      // :321
-            float var = 1.0f / fmaxf(lam, kEps);                        // :323
-            float mean = eta * var;                                     // :324
-            if (PRIOR) {                                                // :325-327
-                mean = a * mean;
-                var = a2 * var + p;
-            }
+            float lam, eta, mean, var;
+            filter_step(av[c][i], pv[c][i], lamv[c][i], etav[c][i], lv, vl, kv[i], PRIOR, lam, eta, mean, var);
             if (in) {
                 ys = fmaf(mean, qv[i], ys);                             // :329
                 yvs = fmaf(var, qv[i] * qv[i], yvs);                    // :330

@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <algorithm>
 #include <optional>
 #include <string>
 #include <tuple>
@@ -38,6 +39,8 @@ struct Entry {
     int (*conv_step)(const kla_b200_conv_step_args *, void *) = nullptr;
     int (*step_layer)(const kla_b200_step_layer_args *, void *) = nullptr;
     int (*linear)(const kla_b200_linear_args *, void *) = nullptr;
+    size_t (*token_work_bytes)(const kla_b200_token_args *) = nullptr;
+    int (*token)(const kla_b200_token_args *, void *) = nullptr;
     int (*add_norm)(int64_t, int64_t, int32_t, int32_t, const void *, const void *, const void *, float, void *, void *, void *) = nullptr;
     int (*swiglu)(int64_t, int64_t, int32_t, const void *, void *, void *) = nullptr;
     int (*qk_norm)(int64_t, int64_t, int64_t, int32_t, kla_b200_tensor3, kla_b200_tensor3, float, void *, void *, void *) = nullptr;
@@ -65,6 +68,8 @@ void bind(const py::dict &d) {
     take(lib.conv_step, d, "kla_b200_conv_step");
     take(lib.step_layer, d, "kla_b200_step_layer");
     take(lib.linear, d, "kla_b200_linear");
+    take(lib.token_work_bytes, d, "kla_b200_token_work_bytes");
+    take(lib.token, d, "kla_b200_token");
     take(lib.add_norm, d, "kla_b200_add_norm");
     take(lib.swiglu, d, "kla_b200_swiglu");
     take(lib.qk_norm, d, "kla_b200_qk_norm");
@@ -431,6 +436,18 @@ bool few_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const Opt
 //    89 M  32 rows 1024 x 2720 9.0 / 8.2                   101 M  32 rows 4096 x 768 16.3 / 15.9
 //   144 M  17 rows 4128 x 2048 7.6 / 6.4                   134 M  32 rows 4096 x 1024 12.5 / 9.9
 bool kernel_pays(int64_t rows, int64_t N, int64_t K) { return rows <= 16 || rows * N * K <= 80'000'000; }
+// Rows up to which a token is one kernel. Blocks of a model, in a graph, us, one kernel / separate ones: 12 layers d_model 768
+// 8 rows 270 / 328, 1 row 248 / 264, d_model 128 8 rows 199 / 211, d_model 1024 4 rows 314 / 354; 4 layers d_model 2048 8 rows
+// 244 / 256. (Two groups of eight rows, as the kernel was tried: 12 layers d_model 768 16 rows 377 / 371.)
+constexpr int64_t kTokenRows = KLA_B200_TOKEN_MAX_ROWS;
+// A lone layer's token is one kernel only where it is issued call by call, four launches costing the host 21 us whatever the
+// sizes, and where the kernel takes less than that. us, one kernel / separate ones, eager: 8 rows d_model 256 14.4 / 20.6, 768
+// 17.9 / 20.2, 1024 18.7 / 20.7, 2048 40.8 / 39.6; with 32 states 768 21.0 / 21.9, 1024 22.6 / 20.7. Captured, where the kernel's
+// working memory is cleared with every replay, the separate ones win: 8 rows d_model 256 16.4 / 14.3, 1024 20.5 / 19.8.
+bool lone_token_pays(int64_t B, int64_t d, int64_t M, int64_t S) {
+    return 3 * M * d + 2 * M * (M + S) <= 16'000'000 && B * M * S <= 400'000 &&
+           c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
+}
 // Who runs a projection that few_rows() takes: whoever is faster, or what the caller says.
 enum class By { size, kernel, library };
 
@@ -584,6 +601,180 @@ Tensor swiglu_step(const Tensor &x, const Tensor &norm_w_, double eps, const Ten
     return project(h, w3, b3, {}, 0.0, x);
 }
 
+// ------------------------------------------------------------------------------------------ a token as one kernel
+
+py::object entry(const py::dict &d, const char *name) {
+    PyObject *o = PyDict_GetItemString(d.ptr(), name);
+    if (o == nullptr) throw py::key_error(name);
+    return py::reinterpret_borrow<py::object>(o);
+}
+
+// A layer as ModelDecoder and LayerDecoder hand it over: weights and config by name, what was made of them, its state.
+struct LayerArgs {
+    const py::dict &w, &cfg;
+    const OptTensor &conv_state;
+    const Tensor &lam, &eta, &a_bar, &p_bar;
+    const OptTensor &skip, &conv_w, &conv_b;
+    int64_t w_value, w_var;
+};
+
+// Whether kla_b200_token takes the layer for tokens like x; fills l if so. Checks what the kernels are given pointers for, as
+// layer_step and few_rows do for the separate ones: whatever does not fit is theirs, with their errors.
+bool token_layer(const Tensor &x, const LayerArgs &a, const OptTensor &norm_w, kla_b200_token_layer &l) {
+    if (a.a_bar.dim() != 2 || a.w.contains("value_expand.weight") || a.w.contains("var_expand.weight")) return false;
+    const auto dev = x.device();
+    const int64_t B = x.size(0), d = x.size(1), M = a.a_bar.size(0), S = a.a_bar.size(1);
+    const Weights w{a.w};
+    const bool gated = entry(a.cfg, "use_gating").cast<bool>();
+    if ((a.w_value != 0 && a.w_value != M) || a.w_var != M || M < 8 || M % 8 || S < 1 || S > KLA_B200_MAX_DSTATE) return false;
+    if (!is(a.lam, dev, at::kFloat, {B, M, S}) || !is(a.eta, dev, at::kFloat, {B, M, S}) || !is(a.a_bar, dev, at::kFloat, {M, S}) ||
+        !is(a.p_bar, dev, at::kFloat, {M, S}))
+        return false;
+    if (a.skip && !is(*a.skip, dev, at::kFloat, {a.skip->numel() == 1 ? 1 : M})) return false;
+    if (a.conv_w) {
+        if (a.conv_w->dim() != 2 || a.conv_w->size(1) < 1 || a.conv_w->size(1) > KLA_B200_MAX_CONV_TAPS ||
+            !is(*a.conv_w, dev, at::kFloat, {M, a.conv_w->size(1)}) || (a.conv_b && !is(*a.conv_b, dev, at::kFloat, {M})))
+            return false;
+        if (a.conv_state ? !is(*a.conv_state, dev, at::kBFloat16, {B, M, a.conv_w->size(1) - 1}) : a.conv_w->size(1) != 1) return false;
+    }
+    auto matrix = [&](const char *name, const char *bias_name, int64_t N, int64_t K, const void *&p, const void *&bias) {
+        const OptTensor t = w.get(name), b = w.get(bias_name);
+        auto plain = [&](const Tensor &u) { return u.scalar_type() == at::kBFloat16 && u.device() == dev && u.is_contiguous(); };
+        if (!t || !plain(*t) || t->dim() != 2 || t->size(0) != N || t->size(1) != K || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16) return false;
+        if (b && (!plain(*b) || b->dim() != 1 || b->size(0) != N)) return false;
+        if (wants_grad({&*t, b ? &*b : &*t})) return false;
+        p = t->data_ptr();
+        bias = b ? b->data_ptr() : nullptr;
+        return true;
+    };
+    if (!matrix("in_proj.weight", "in_proj.bias", gated ? 2 * M : M, d, l.in_weight, l.in_bias) ||
+        !matrix("sensor_proj.weight", "sensor_proj.bias", a.w_value + a.w_var + 2 * S, M, l.sensor_weight, l.sensor_bias) ||
+        !matrix("out_proj.weight", "out_proj.bias", d, M, l.out_weight, l.out_bias))
+        return false;
+    if (norm_w) {
+        if (!few_rows(x, w.at("in_proj.weight"), {}, norm_w)) return false;
+        l.norm_weight = norm_w->data_ptr();
+    }
+    if (a.conv_w) {
+        l.conv_weight = fp(*a.conv_w); l.conv_bias = fp(a.conv_b); l.conv_taps = a.conv_w->size(1);
+        l.conv_state = a.conv_state ? a.conv_state->data_ptr() : nullptr;
+        l.conv_activation = act_code(entry(a.cfg, "conv_activation"));
+    }
+    const py::object vmax = entry(a.cfg, "obs_var_max"), clip = entry(a.cfg, "clip_value");
+    l.a = fp(a.a_bar); l.p = fp(a.p_bar); l.lambda_skip = fp(a.skip); l.lambda_skip_len = a.skip ? (int32_t)a.skip->numel() : 0;
+    l.lam = fp(a.lam); l.eta = fp(a.eta);
+    l.M = M; l.S = S; l.gated = gated; l.w_value = (int32_t)a.w_value;
+    l.gate_activation = gated ? act_code(entry(a.cfg, "gating_activation")) : KLA_B200_ACT_NONE;
+    l.qk_norm = entry(a.cfg, "qk_norm").cast<bool>(); l.decode_from_prior = entry(a.cfg, "decode_from_prior").cast<bool>();
+    l.obs_var_min = entry(a.cfg, "obs_var_min").cast<float>();
+    l.obs_var_max = vmax.is_none() ? 0.0f : vmax.cast<float>();
+    l.clip_value = clip.is_none() ? 0.0f : clip.cast<float>();
+    return true;
+}
+
+// What a token's working memory is good for: launches of one kind.
+using TokenKind = std::vector<int64_t>;
+TokenKind token_kind(const kla_b200_token_args &t) {
+    TokenKind k{t.B, t.d, t.mlp};
+    for (int64_t i = 0; i < t.layers; ++i) {
+        const kla_b200_token_layer &l = t.layer[i];
+        k.insert(k.end(), {l.M, l.S, l.hidden, l.gated, l.w_value});
+    }
+    return k;
+}
+
+// Zeroed working memory for launches of a kind. Launches of one stream follow one another and share it, those of another
+// stream have their own: kept by stream (its id is never given to another one) and kind, the last kMost of up to kLargest
+// bytes. While a graph is captured it belongs to the graph, whose replays follow one another, and is cleared at its beginning.
+Tensor token_work(const Tensor &like, const kla_b200_token_args &t, int64_t bytes) {
+    constexpr size_t kMost = 32;
+    constexpr int64_t kLargest = 4 << 20;
+    struct Kept {
+        int device;
+        unsigned long long stream;
+        TokenKind kind;
+        Tensor work;
+    };
+    // under the interpreter's lock; never destroyed: at exit the CUDA context goes first
+    static auto &kept = *new std::vector<Kept>();
+    const int device = like.device().index();
+    unsigned long long id = 0;
+    auto zeros = [&] { return at::zeros({bytes}, like.options().dtype(at::kByte).requires_grad(false)); };
+    if (bytes > kLargest || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None ||
+        cudaStreamGetId(at::cuda::getCurrentCUDAStream(device).stream(), &id) != cudaSuccess)
+        return zeros();
+    TokenKind kind = token_kind(t);
+    for (const Kept &k : kept)
+        if (k.device == device && k.stream == id && k.kind == kind) return k.work;
+    if (kept.size() >= kMost) kept.erase(kept.begin());  // back to the allocator, in the order of the stream that used it
+    kept.push_back(Kept{device, id, std::move(kind), zeros()});
+    return kept.back().work;
+}
+
+// Runs the layers filled in by token_layer -> [B, d], or nothing where a projection's x does not fit the kernel. works: zeroed
+// working memory of the caller's, one per KLA_B200_TOKEN_MAX_LAYERS layers; empty: filled with new ones, for the caller to keep.
+OptTensor run_token(const Tensor &x, const std::vector<kla_b200_token_layer> &layers, bool mlp, double eps, const OptTensor &y_var,
+                    std::optional<py::list> works) {
+    std::vector<kla_b200_token_args> runs;
+    std::vector<int64_t> bytes;
+    for (size_t first = 0; first < layers.size(); first += KLA_B200_TOKEN_MAX_LAYERS) {
+        kla_b200_token_args t{};
+        t.B = x.size(0); t.d = x.size(1); t.layers = (int64_t)std::min(layers.size() - first, (size_t)KLA_B200_TOKEN_MAX_LAYERS);
+        t.mlp = mlp; t.norm_eps = (float)eps;
+        t.layer = layers.data() + first;
+        bytes.push_back((int64_t)lib.token_work_bytes(&t));
+        if (bytes.back() == 0) return {};
+        runs.push_back(t);
+    }
+    Tensor in = x;
+    for (size_t i = 0; i < runs.size(); ++i) {
+        kla_b200_token_args &t = runs[i];
+        if (works && works->size() <= i) works->append(at::zeros({bytes[i]}, x.options().dtype(at::kByte).requires_grad(false)));
+        const Tensor work = works ? (*works)[i].cast<Tensor>() : token_work(x, t, bytes[i]);
+        require(work.device() == x.device() && work.nbytes() >= (size_t)bytes[i], "a token's working memory belongs to another kind of token");
+        Tensor out = fresh(x, {t.B, t.d});
+        t.x = in.data_ptr(); t.x_stride_b = in.stride(0);
+        t.out = out.data_ptr(); t.y_var = y_var ? y_var->data_ptr() : nullptr;
+        t.work = work.data_ptr();
+        check(lib.token(&t, stream_of(x)));
+        in = out;
+    }
+    return in;
+}
+
+// A row count, type and layout of x that kla_b200_token takes.
+bool token_rows(const Tensor &x, int64_t most) {
+    return x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.size(0) >= 1 && x.size(0) <= most && x.size(1) >= 8 &&
+           x.size(1) % 8 == 0 && x.stride(1) == 1 && x.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 &&
+           !wants_grad({&x}) && sm100(x.device());
+}
+
+// One token through all blocks of a model, or None where a block or the rows are not ones kla_b200_token takes. blocks: per
+// block (weights, config, conv window, lam, eta, a_bar, p_bar, skip, conv weights, conv bias, w_value, w_var, norm weight) and,
+// with a swiglu MLP behind the mixer, (norm weight, w12, bias, w3, bias).
+using BlockArgs = std::tuple<py::dict, py::dict, OptTensor, Tensor, Tensor, Tensor, Tensor, OptTensor, OptTensor, OptTensor, int64_t, int64_t, Tensor>;
+using MlpArgs = std::tuple<Tensor, Tensor, OptTensor, Tensor, OptTensor>;
+py::object model_token(const Tensor &x, const std::vector<BlockArgs> &blocks, const std::vector<MlpArgs> &mlps, double eps, std::optional<py::list> works) {
+    if (!token_rows(x, kTokenRows) || blocks.empty() || (!mlps.empty() && mlps.size() != blocks.size())) return py::none();
+    const c10::cuda::CUDAGuard guard(x.device());
+    std::vector<kla_b200_token_layer> layers(blocks.size());
+    for (size_t i = 0; i < blocks.size(); ++i) {
+        const auto &[w, cfg, conv_state, lam, eta, a_bar, p_bar, skip, conv_w, conv_b, w_value, w_var, norm_w] = blocks[i];
+        if (!token_layer(x, LayerArgs{w, cfg, conv_state, lam, eta, a_bar, p_bar, skip, conv_w, conv_b, w_value, w_var}, norm_w, layers[i])) return py::none();
+        if (mlps.empty()) continue;
+        const auto &[mlp_norm, w12, b12, w3, b3] = mlps[i];
+        const int64_t hidden = w12.dim() == 2 ? w12.size(0) / 2 : 0;
+        if (!few_rows(x, w12, b12, mlp_norm) || w12.size(0) != 2 * hidden || hidden < 8 || hidden % 8) return py::none();
+        if (w3.dim() != 2 || w3.size(0) != x.size(1) || w3.size(1) != hidden || w3.scalar_type() != at::kBFloat16 || !w3.is_contiguous() || w3.device() != x.device() ||
+            reinterpret_cast<uintptr_t>(w3.data_ptr()) % 16 || wants_grad({&w3}) ||
+            (b3 && (b3->scalar_type() != at::kBFloat16 || !b3->is_contiguous() || b3->dim() != 1 || b3->size(0) != w3.size(0) || b3->device() != x.device() || wants_grad({&*b3}))))
+            return py::none();
+        layers[i].mlp_norm_weight = mlp_norm.data_ptr(); layers[i].w12 = w12.data_ptr(); layers[i].b12 = b12 ? b12->data_ptr() : nullptr;
+        layers[i].w3 = w3.data_ptr(); layers[i].b3 = b3 ? b3->data_ptr() : nullptr; layers[i].hidden = hidden;
+    }
+    return py::cast(run_token(x, layers, !mlps.empty(), eps, {}, works));
+}
+
 // One token of a layer (LayerDecoder.step), with the block's norm before it and its residual sum after it when norm_w is given
 // (ModelDecoder): three projections, the convolution's step and the fused filter step. conv_state
 // (absent without a convolution), lam and eta are updated in place. Returns the layer's output and the gated variance, which
@@ -621,6 +812,13 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     const bool in_model = norm_w.has_value();  // other kernels of the token, or the embedding's, are in front
     require(in_w.dim() == 2 && in_w.size(0) == (gated ? 2 * M : M), "in_proj must have one output per channel, two with a gate");
     require(sensor_w.dim() == 2 && sensor_w.size(0) == w_value + w_var + 2 * S, "sensor_proj must have one output per sensor signal");
+    if (!in_model && token_rows(x, kTokenRows) && lone_token_pays(B, x.size(1), M, S)) {
+        std::vector<kla_b200_token_layer> one(1);
+        if (token_layer(x, LayerArgs{w_, cfg, conv_state, lam, eta, a_bar, p_bar, skip, conv_w, conv_b, w_value, w_var}, {}, one[0])) {
+            const Tensor yv = fresh(x, {B, M});
+            if (const OptTensor out = run_token(x, one, false, 0.0, yv, {})) return {*out, yv};
+        }
+    }
     // A lone layer issued call by call is bound by the host, where the library's calls cost 7 us more each (B=17 d_model 768:
     // 23.0 us a token, 26.5 with one of them); in a graph its three GEMMs win together where the widest does (d_model 768, B=17
     // 21.9 against 19.0, B=32 28.6 and 21.8; d_model 1024, B=32 27.6 and 24.3; but d_model 512, B=32 15.7 and 16.6).
@@ -752,6 +950,7 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("rawscan", &rawscan);
     m.def("step", &step);
     m.def("layer_step", &layer_step);
+    m.def("model_token", &model_token);
     m.def("add_norm", &add_norm);
     m.def("swiglu", &swiglu);
     m.def("argmax", &argmax);

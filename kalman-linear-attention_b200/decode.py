@@ -2,7 +2,8 @@
 
 The reference layer's decode route (``KLALayer.forward`` with a state and ``L == 1``,
 src/kla/layers/kla_layer.py:295-345) is three projections with elementwise work between
-them. ``LayerDecoder.step`` runs them as ``kla_b200_linear`` for up to 32 bfloat16 rows (large
+them. ``LayerDecoder.step`` runs a small layer's token of up to eight bfloat16 rows, issued outside a graph capture, as one kernel
+(``kla_b200_token``), the projections as ``kla_b200_linear`` for up to 32 bfloat16 rows (large
 layers of more than 16 rows only outside a graph capture), the first with the step of ``CausalConv1d`` (src/kla/layers/common.py:87-96) inside, and as library
 GEMMs around ``kla_b200_conv_step`` otherwise; between the second and the third stands
 ``kla_b200_step_layer`` (sensor post-processing, the filter step, skip path and gate;
@@ -197,6 +198,7 @@ class _TokenGraph:
     def __init__(self, dec: "ModelDecoder", batch: int, device, dtype, greedy: bool):
         self.state = dec.init_state(batch, device, dtype)
         self.token = torch.zeros(batch, device=device, dtype=torch.long)
+        self.work = []  # of the kernel that a whole token is, made by its first run here; replays follow one another
         self.done = None  # recorded behind the last use
         self.stream = torch.cuda.current_stream(device)  # whose memory the buffers are
         side = torch.cuda.Stream(device)
@@ -214,7 +216,7 @@ class _TokenGraph:
         torch.cuda.current_stream(device).wait_stream(side)
 
     def _token(self, dec, greedy):
-        logits = dec.step(self.token, self.state)
+        logits = dec._token_logits(self.token, self.state, self.work)
         if greedy:
             _lib.host().argmax(logits, self.token)
         return logits
@@ -226,7 +228,7 @@ class _TokenGraph:
         if self.done is not None:
             stream.wait_event(self.done)
         if stream != self.stream:
-            for t in (self.token, *(t for layer in self.state for t in layer if t is not None)):
+            for t in (self.token, *self.work, *(t for layer in self.state for t in layer if t is not None)):
                 t.record_stream(stream)
         for conv, lam, eta in self.state:
             if conv is not None:
@@ -263,9 +265,9 @@ class ModelDecoder:
     reference's ``SequenceModel.forward`` with a state and ``SequenceModel.generate``
     (src/kla/models/sequence_model.py:150-173, 200-220).
 
-    A block is ``x += mixer(norm(x))`` then ``x += mlp(norm(x))`` (sequence_model.py:47-98). For one token of up to 16
-    sequences in bfloat16 that is six kernels: the projections with norm, convolution step, gate and residual sum folded
-    in, and the filter step. For up to 32 sequences large projections are library GEMMs. For a prompt the projections are library GEMMs and what stands between them one kernel each.
+    A block is ``x += mixer(norm(x))`` then ``x += mlp(norm(x))`` (sequence_model.py:47-98). For one token of up to eight
+    sequences in bfloat16 all blocks are one kernel (``kla_b200_token``), for up to 16 a block is six: the projections with norm,
+    convolution step, gate and residual sum folded in, and the filter step. For up to 32 sequences large projections are library GEMMs. For a prompt the projections are library GEMMs and what stands between them one kernel each.
     One decoded token is a fixed sequence of launches over state that is updated in place, so ``generate`` captures it in
     a CUDA graph, which it keeps for calls with the same batch, types and weights, and replays it: a token then costs no
     host work but one replay, where the reference's loop issues several hundred small launches per token from Python.
@@ -332,19 +334,29 @@ class ModelDecoder:
         cap = self.cfg["logit_softcap"]
         return logits if cap is None else cap * torch.tanh(logits / cap)
 
-    def _step_blocks(self, x, state):
-        """One token through the blocks: norm, mixer and residual sum of a block are the layer's step with the norm folded
-        into its first projection and the sum into its last; the MLP likewise."""
+    def _step_blocks(self, x, state, work=None):
+        """One token through the blocks: of up to eight sequences in bfloat16 all of them as one kernel (``work``: a list of
+        its working memory where the caller keeps it); otherwise norm, mixer and residual sum of a block are the layer's step with
+        the norm folded into its first projection and the sum into its last, and the MLP likewise."""
         _require_cuda(x)
-        host, w, eps = _lib.host(), self.w, self.cfg["norm_eps"]
+        host, w, eps, mlp = _lib.host(), self.w, self.cfg["norm_eps"], self.cfg["mlp"]
+        if mlp in ("swiglu", "none") and x.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
+            blocks = [(m.w, m.cfg, *st, m.a_bar, m.p_bar, m.skip, m.conv_w, getattr(m, "conv_b", None), m.w_value, m.w_var,
+                       w[f"blocks.{i}.mixer_norm.weight"]) for i, (m, st) in enumerate(zip(self.layers, state))]
+            mlps = [] if mlp == "none" else [
+                (w[f"blocks.{i}.mlp_norm.weight"], w[f"blocks.{i}.mlp.w12.weight"], w.get(f"blocks.{i}.mlp.w12.bias"),
+                 w[f"blocks.{i}.mlp.w3.weight"], w.get(f"blocks.{i}.mlp.w3.bias")) for i in range(len(self.layers))]
+            y = host.model_token(x, blocks, mlps, eps, work)
+            if y is not None:
+                return y
         for i, layer in enumerate(self.layers):
             pre = f"blocks.{i}."
             x = layer.block_step(x, state[i], w[pre + "mixer_norm.weight"], eps)
-            if self.cfg["mlp"] == "swiglu":
+            if mlp == "swiglu":
                 m = pre + "mlp."
                 x = host.swiglu_step(x, w[pre + "mlp_norm.weight"], eps, w[m + "w12.weight"], w.get(m + "w12.bias"),
                                      w[m + "w3.weight"], w.get(m + "w3.bias"))
-            elif self.cfg["mlp"] != "none":
+            elif mlp != "none":
                 x = x + self._mlp(i, self._norm(x, pre + "mlp_norm"))
         return x
 
@@ -374,7 +386,10 @@ class ModelDecoder:
     @torch.no_grad()
     def step(self, token: torch.Tensor, state):
         """One token per sequence: ``token`` [B] -> logits [B, vocab]; ``state`` is updated in place."""
-        x = self._step_blocks(F.embedding(token, self.w["embedding.weight"]), state)
+        return self._token_logits(token, state)
+
+    def _token_logits(self, token, state, work=None):
+        x = self._step_blocks(F.embedding(token, self.w["embedding.weight"]), state, work)
         return self._cap(_lib.host().project(x, self.w["lm_head.weight"], None, self.w["norm_f.weight"], self.cfg["norm_eps"], None))
 
     @torch.no_grad()

@@ -216,3 +216,27 @@ def test_segment_plan(L):
     assert plan(4, 16, True, forced=4) == (1, 16)
     n, length = plan(320, 1 << 20, True)
     assert n == 8 and length % 16 == 0 and n * length >= 1 << 20
+
+
+def test_token_entry_point_rejects_bad_arguments_without_cuda(L):
+    lib = L.load()
+    layer = L.TokenLayer(M=16, S=4, w_value=16, conv_activation=3, gate_activation=3)
+
+    def call(layer=layer, **kw):
+        a = L.TokenArgs(**dict(dict(B=1, d=16, layers=1, layer=ctypes.pointer(layer) if layer else None), **kw))
+        return lib.kla_b200_token(ctypes.byref(a), None), lib.kla_b200_token_work_bytes(ctypes.byref(a))
+
+    other = lambda **kw: L.TokenLayer(**dict(dict(M=16, S=4, w_value=16, conv_activation=3, gate_activation=3), **kw))
+    assert lib.kla_b200_token(None, None) == 1 and lib.kla_b200_token_work_bytes(None) == 0
+    assert call(B=0) == (0, 256) and call()[0] == 1 and call()[1] > 256  # nothing to do; NULL tensors
+    for refused in (call(B=9), call(layers=33), call(d=12), call(other(M=12)), call(other(S=129)), call(d=1 << 16), call(other(conv_weight=16, conv_taps=9))):
+        assert refused == (2, 0)
+    for invalid in (call(None), call(B=-1), call(other(M=0)), call(other(S=0)), call(other(w_value=8)), call(mlp=1),
+                    call(other(gate_activation=7)), call(other(lambda_skip_len=3))):
+        assert invalid == (1, 0)
+    one = dict(x=256, out=256, work=256)
+    full = dict(in_weight=256, sensor_weight=256, out_weight=256, a=256, p=256, lam=256, eta=256)
+    assert call(other(**full), **dict(one, x_stride_b=4))[0] == 2
+    assert call(other(**full), **dict(one, x=8))[0] == 4 and call(other(**full), **dict(one, work=128))[0] == 4
+    assert call(other(**dict(full, in_weight=8)), **one)[0] == 4 and call(other(**dict(full, lam=2)), **one)[0] == 4
+    assert call(other(**dict(full, lam=None)), **one)[0] == 1 and call(other(**dict(full, conv_weight=256, conv_taps=4)), **one)[0] == 1
