@@ -9,25 +9,41 @@
 //       x' = (1 + p phi) x + a2 phi w,   w' = p x + a2 w,   z' = r w' + a z,
 //   (the variance-form step of kla_common.cuh multiplied through by its
 //   denominator), so a stretch of steps is the product of its step matrices:
-//   7 numbers (m00 m01 / m10 m11 / m20 m21 m22), rescaled every other step --
-//   a common factor does not change P or mean. This is the reference's
-//   trace-normalised 2x2 Moebius product (src/kla/ops/kla_ops.py:76-116)
-//   extended by the row that carries the mean, which lets one pass serve both
-//   recurrences instead of two dependent ones (kla_ops.py:248, 274-280).
+//   7 numbers (m00 m01 / m10 m11 / m20 m21 m22); a common factor does not change
+//   P or mean. This is the reference's trace-normalised 2x2 Moebius product
+//   (src/kla/ops/kla_ops.py:76-116) extended by the row that carries the mean,
+//   which lets one pass serve both recurrences instead of two dependent ones
+//   (kla_ops.py:248, 274-280). The product is not formed as one. What a stretch
+//   does to a state (P0, m0) is what it would do to a state known exactly at 0,
+//   the filter itself run from (C, b) = (0, 0), and how the knowledge of m0 that
+//   the stretch's observations carry changes that:
+//       P = C + A^2 P0 / (1 + J P0),   mean = b + A (m0 + eta P0) / (1 + J P0),
+//   with A' = a A g, J' = J + phi (a A) A', eta' = eta + A' (r - phi a b), g the
+//   gain of the run from 0. That is 15 pair operations a step where the matrices
+//   take 18.5 with their rescaling, five numbers that stay in range by themselves,
+//   and the record is (1, J / C, C J + A^2 / b, b J + A eta, A) over 1 + J.
 //
 // * adjoint. With the forward trajectory fixed, the backward carries obey
 //   c_{t-1} = J_t (c_t + e_t), J_t = [[a2 g^2, a2 g (r - phi mean_t)], [0, a g]],
 //   e_t = (dyvar q^2, dy q): affine, upper triangular. Walking FORWARD in time,
 //   K_t = J_1 ... J_t and b = sum_t K_t e_t give the carry that leaves the
 //   stretch at its first step as K c_in + b (5 numbers). It needs the stretch's
-//   true initial state, i.e. it runs after the forward fold.
+//   true initial state, i.e. it runs after the forward fold. With a2 = a^2 and
+//   r - phi mean_t = g (r - phi a mean_{t-1}) the diagonal is one product,
+//   K00 = K11^2, and K01 = K11 R with R' = R + K11' (r - phi a mean): 19 pair
+//   operations a step instead of 25. (a2's floor of 1e-12, which binds where
+//   |a| < 1e-6, is left out of K00: 1e-12 of the carry at the most.)
+//
+// Both walks keep -a, -a2 and -p as their constants and -Pp, -1/d as they go:
+// every product then has the sign the next sum needs, since a pair instruction
+// has no operand negation.
 //
 // Kernel shape: as the scan kernels. NW compute warps, each thread owning SPT
 // states of one channel as pairs (paired fp32 instructions), and one loader warp
 // that brings tiles of TT steps in: v, lambda_v (and dy, dy_var) as TMA tiles
-// signalled on mbarriers, k (and q) regrouped by owning lane. The forward
-// aggregate has no reciprocal on its dependent path, so one warp per scheduler
-// already runs at the arithmetic rate. Nothing is written but the final record.
+// signalled on mbarriers, k (and q) regrouped by owning lane. Nothing is written but the final record.
+// Measured on B200, B=2 L=1024 M=1024 S=16 in 16 chunks, float32, against the form with matrices: forward 29.7 -> 27.3 us,
+// adjoint 39.8 -> 34.3; bound by the FP32 pipe (17.7 of the 27.3 us) and by the start of CTAs of two tiles each.
 #pragma once
 
 #include "kla_common.cuh"
@@ -104,18 +120,22 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
         const int j = lane % LPC, cl = lane / LPC;
         const int cw = warp * CLS + cl;  // this thread's channel, CTA-relative
         const int m = m_cta + cw;
-        float2 ca[HP], ca2[HP], cp[HP];
-        // forward: m00 m01 m10 m11 m20 m21 m22; adjoint: K00 K01 K11 b0 b1 P mean
-        float2 A[7][HP];
+        float2 na[HP], na2[HP], np[HP];  // negated constants
+        // forward: A, b, C, -J, eta; adjoint: K11, R, b0, b1, P, mean
+        constexpr int NA = ADJ ? 6 : 5;
+        float2 A[NA][HP];
 #pragma unroll
         for (int i = 0; i < SPT; ++i) {
             const int s = i * LPC + j;
             const bool live = (m < M) && (s < S);
             const float av = live ? prm.a[(long long)m * S + s] : 0.0f;
             const float pv = live ? prm.p[(long long)m * S + s] : 1.0f;
-            pair_el(ca, i) = av;
-            pair_el(ca2, i) = live ? fmaxf(av * av, kEps) : 0.0f;
-            pair_el(cp, i) = fmaxf(pv, kPMin);
+            pair_el(na, i) = -av;
+            pair_el(na2, i) = live ? -fmaxf(av * av, kEps) : 0.0f;
+            pair_el(np, i) = -fmaxf(pv, kPMin);
+            pair_el(A[0], i) = 1.0f;
+#pragma unroll
+            for (int e = 1; e < NA; ++e) pair_el(A[e], i) = 0.0f;
             if (ADJ) {
                 float lam = 1.0f, eta = 0.0f;
                 if (live && prm.lam0 != nullptr) {
@@ -123,17 +143,12 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
                     eta = prm.eta0[((long long)be * M + m) * S + s];
                 }
                 const float P0 = 1.0f / fmaxf(lam, kLamMin);
-                pair_el(A[0], i) = 1.0f; pair_el(A[1], i) = 0.0f; pair_el(A[2], i) = 1.0f;
-                pair_el(A[3], i) = 0.0f; pair_el(A[4], i) = 0.0f;
-                pair_el(A[5], i) = P0; pair_el(A[6], i) = eta * P0;
-            } else {
-                pair_el(A[0], i) = 1.0f; pair_el(A[1], i) = 0.0f; pair_el(A[2], i) = 0.0f; pair_el(A[3], i) = 1.0f;
-                pair_el(A[4], i) = 0.0f; pair_el(A[5], i) = 0.0f; pair_el(A[6], i) = 1.0f;
+                pair_el(A[NA - 2], i) = P0;
+                pair_el(A[NA - 1], i) = eta * P0;
             }
         }
 
-        auto step = [&](const T *vrow, const T *lrow, const TO *dyrow, const TO *dyvrow, const float *kqrow, int tt,
-                        bool rescale) {
+        auto step = [&](const T *vrow, const T *lrow, const TO *dyrow, const TO *dyvrow, const float *kqrow, int tt) {
             const float2 lv = dup2(to_f32<T>(lrow[tt * MC])), vv = dup2(to_f32<T>(vrow[tt * MC]));
             const float *row = kqrow + tt * NK * SPAD;
             float2 kk[HP], qq[HP];
@@ -153,53 +168,37 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
                     if (ADJ) qq[h] = *reinterpret_cast<const float2 *>(row + SPT + 2 * h);
                 }
             }
-            if constexpr (!ADJ) {
+            float dyf = 0.0f, dyvf = 0.0f;
+            if constexpr (ADJ) {
+                dyf = to_f32<TO>(dyrow[tt * MC]);
+                dyvf = to_f32<TO>(dyvrow[tt * MC]);
+            }
+            constexpr int iP = ADJ ? 4 : 2, iM = ADJ ? 5 : 1;  // variance and mean of the run
+            float2 nPp[HP], ng[HP], r[HP], phi[HP];
 #pragma unroll
-                for (int h = 0; h < HP; ++h) {
-                    float2 phi, r;
-                    chain_inputs2(lv, vv, kk[h], phi, r);
-                    // the step as two shears: w' = p x + a2 w, then x' = x + phi w' (= (1 + p phi) x + a2 phi w)
-                    const float2 n10 = fma2(ca2[h], A[2][h], mul2(cp[h], A[0][h]));
-                    const float2 n11 = fma2(ca2[h], A[3][h], mul2(cp[h], A[1][h]));
-                    const float2 n00 = fma2(phi, n10, A[0][h]), n01 = fma2(phi, n11, A[1][h]);
-                    A[4][h] = fma2(r, n10, mul2(ca[h], A[4][h]));
-                    A[5][h] = fma2(r, n11, mul2(ca[h], A[5][h]));
-                    A[6][h] = mul2(ca[h], A[6][h]);
-                    A[0][h] = n00; A[1][h] = n01; A[2][h] = n10; A[3][h] = n11;
-                    if (rescale) {  // a common factor leaves P = w/x and mean = z/x unchanged
-                        const float2 sc = rcp_approx2(add2(n00, n01));
+            for (int h = 0; h < HP; ++h) {
+                chain_inputs2(lv, vv, kk[h], phi[h], r[h]);
+                nPp[h] = fma2(na2[h], A[iP][h], np[h]);
+                ng[h] = fma2(phi[h], nPp[h], make_float2(-1.0f, -1.0f));
+            }
 #pragma unroll
-                        for (int e = 0; e < 7; ++e) A[e][h] = mul2(A[e][h], sc);
-                    }
-                }
-            } else {
-                const float dyf = to_f32<TO>(dyrow[tt * MC]), dyvf = to_f32<TO>(dyvrow[tt * MC]);
-                float2 Pp[HP], g[HP], r[HP], phi[HP];
+            for (int h = 0; h < HP; ++h) ng[h] = rcp_approx2(ng[h]);
 #pragma unroll
-                for (int h = 0; h < HP; ++h) {
-                    chain_inputs2(lv, vv, kk[h], phi[h], r[h]);
-                    g[h] = chain_denominator2(A[5][h], phi[h], ca2[h], cp[h], Pp[h]);
-                }
-#pragma unroll
-                for (int h = 0; h < HP; ++h) g[h] = rcp_approx2(g[h]);
-#pragma unroll
-                for (int h = 0; h < HP; ++h) {
-                    chain_update2(A[5][h], A[6][h], Pp[h], g[h], r[h], ca[h]);  // P_t, mean_t
-                    const float2 a2g = mul2(ca2[h], g[h]);
-                    const float2 j00 = mul2(a2g, g[h]);
-                    const float2 j01 = mul2(a2g, fma2(neg2(phi[h]), A[6][h], r[h]));
-                    const float2 j11 = mul2(ca[h], g[h]);
-                    float2 e0 = mul2(dup2(dyvf), mul2(qq[h], qq[h])), e1 = mul2(dup2(dyf), qq[h]);
-                    if (PRIOR) {
-                        e0 = mul2(e0, ca2[h]);
-                        e1 = mul2(e1, ca[h]);
-                    }
-                    const float2 K00 = mul2(A[0][h], j00);
-                    const float2 K01 = fma2(A[0][h], j01, mul2(A[1][h], j11));
-                    const float2 K11 = mul2(A[2][h], j11);
-                    A[0][h] = K00; A[1][h] = K01; A[2][h] = K11;
-                    A[3][h] = fma2(K00, e0, fma2(K01, e1, A[3][h]));
-                    A[4][h] = fma2(K11, e1, A[4][h]);
+            for (int h = 0; h < HP; ++h) {
+                const float2 nam = mul2(na[h], A[iM][h]), t = fma2(phi[h], nam, r[h]), naA = mul2(na[h], A[0][h]);
+                A[iP][h] = mul2(nPp[h], ng[h]);
+                A[iM][h] = mul2(ng[h], fma2(nPp[h], r[h], nam));
+                A[0][h] = mul2(naA, ng[h]);
+                if constexpr (!ADJ) {
+                    A[3][h] = fma2(mul2(phi[h], naA), A[0][h], A[3][h]);
+                    A[4][h] = fma2(A[0][h], t, A[4][h]);
+                } else {
+                    A[1][h] = fma2(A[0][h], t, A[1][h]);
+                    float2 kq = mul2(A[0][h], qq[h]);
+                    if (PRIOR) kq = neg2(mul2(kq, na[h]));
+                    const float2 f = mul2(kq, dup2(dyf));
+                    A[2][h] = fma2(A[1][h], f, fma2(mul2(kq, dup2(dyvf)), kq, A[2][h]));
+                    A[3][h] = add2(A[3][h], f);
                 }
             }
         };
@@ -214,10 +213,10 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
 #pragma unroll 1
                 for (int t4 = 0; t4 < TT; t4 += 4) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) step(vrow, lrow, dyrow, dyvrow, kqrow, t4 + u, (u & 1) != 0);
+                    for (int u = 0; u < 4; ++u) step(vrow, lrow, dyrow, dyvrow, kqrow, t4 + u);
                 }
             } else {
-                for (int tt = 0; t0 + tt < L; ++tt) step(vrow, lrow, dyrow, dyvrow, kqrow, tt, (tt & 1) != 0);
+                for (int tt = 0; t0 + tt < L; ++tt) step(vrow, lrow, dyrow, dyvrow, kqrow, tt);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_in[s]);
@@ -228,8 +227,17 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
             const int s = i * LPC + j;
             if (m < M && s < S) {
                 float4 *o = reinterpret_cast<float4 *>(prm.out + (((long long)be * M + m) * S + s) * 8);
-                o[0] = make_float4(pair_el(A[0], i), pair_el(A[1], i), pair_el(A[2], i), pair_el(A[3], i));
-                o[1] = make_float4(pair_el(A[4], i), pair_el(A[5], i), pair_el(A[6], i), 0.0f);
+                float x[NA];
+#pragma unroll
+                for (int e = 0; e < NA; ++e) x[e] = pair_el(A[e], i);
+                if constexpr (!ADJ) {
+                    const float J = -x[3], sc = 1.0f / (1.0f + J);  // m00 + m01 = 1: folds of many records stay in range
+                    o[0] = make_float4(sc, J * sc, x[2] * sc, fmaf(x[0], x[0], x[2] * J) * sc);
+                    o[1] = make_float4(x[1] * sc, fmaf(x[0], x[4], x[1] * J) * sc, x[0] * sc, 0.0f);
+                } else {
+                    o[0] = make_float4(x[0] * x[0], x[0] * x[1], x[0], x[2]);
+                    o[1] = make_float4(x[3], x[4], x[5], 0.0f);
+                }
             }
         }
     } else {
