@@ -166,16 +166,6 @@ struct BwdSmem {
 
 constexpr int kBwdThreads = 384;  // reverse, replay and helper groups of four warps each
 
-// two neighbouring activations as a pair of floats
-__device__ __forceinline__ float2 load_pair(const float *p) { return *reinterpret_cast<const float2 *>(p); }
-__device__ __forceinline__ float2 load_pair(const __nv_bfloat16 *p) {
-    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p));
-}
-__device__ __forceinline__ void store_pair(float *p, float x, float y) { *reinterpret_cast<float2 *>(p) = make_float2(x, y); }
-__device__ __forceinline__ void store_pair(__nv_bfloat16 *p, float x, float y) {
-    *reinterpret_cast<__nv_bfloat162 *>(p) = __floats2bfloat162_rn(x, y);
-}
-
 // LOGV: lambda_v arrives as a log-variance (BwdParams::lv_log_sigma). A separate instantiation, so that the plain
 // kernel does not carry that code.
 // SEG: sequences cut into segments (BwdParams::seg, SegCtl), also a separate instantiation.

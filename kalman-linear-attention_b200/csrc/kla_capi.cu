@@ -701,6 +701,8 @@ int kla_b200_scan_fwd(const kla_b200_fwd_args *a, void *stream) {
             if (a->y_raw.ptr != nullptr) {
                 if ((rc = check_t3(a->y_raw, osz, true)) || (rc = check_t3(a->y_var_raw, osz, true))) return rc;
                 prm.y_raw = t3(a->y_raw); prm.yv_raw = t3(a->y_var_raw);
+                prm.vec_raw = osz == 4 ? vec2_ok<float>(a->y_raw) && vec2_ok<float>(a->y_var_raw)
+                                       : vec2_ok<__nv_bfloat16>(a->y_raw) && vec2_ok<__nv_bfloat16>(a->y_var_raw);
             }
             if (has_skip && ((a->lambda_skip_len != 1 && a->lambda_skip_len != a->M) || !a->lambda_skip || !a->z.ptr))
                 return KLA_B200_EINVAL;

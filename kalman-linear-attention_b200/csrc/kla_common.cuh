@@ -293,6 +293,16 @@ __device__ __forceinline__ float from_f32<float>(float x) { return x; }
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 
+// two neighbouring activations as a pair of floats
+__device__ __forceinline__ float2 load_pair(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+__device__ __forceinline__ float2 load_pair(const __nv_bfloat16 *p) {
+    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p));
+}
+__device__ __forceinline__ void store_pair(float *p, float x, float y) { *reinterpret_cast<float2 *>(p) = make_float2(x, y); }
+__device__ __forceinline__ void store_pair(__nv_bfloat16 *p, float x, float y) {
+    *reinterpret_cast<__nv_bfloat162 *>(p) = __floats2bfloat162_rn(x, y);
+}
+
 // A warp's columns of a [TT x MC] tile of log-variances -> float32 precisions (raw and lam point at its first column, and
 // may be the same memory). All of a lane's elements are read before the first is stored: one after the other, each behind
 // the stores before it, they cost the scan kernels 700 cycles a tile.
@@ -459,8 +469,8 @@ __device__ __forceinline__ void stage_tile(T *smem, const T *base, long long st,
 // Sum the per-lane-group partials of one tile over the LPC lane groups and
 // write two [rows x MC] output tiles. part: [TT][LPC][MCP] float2 in shared
 // memory. Each thread handles pairs of channels, so consecutive lanes read
-// consecutive 16-byte words. FIN maps (sum.x, sum.y, tt, channel) to the two
-// output values. vec0/vec1: 2-element vector stores are legal for that output.
+// consecutive 16-byte words. FIN makes the output values (x, y)
+// of a pair's two channels (the second may be none) from their sums. vec0/vec1: 2-element vector stores are legal for that output.
 template <typename TO, int LPC, int MC, int MCP, int TT, int NTHR, typename Fin>
 __device__ __forceinline__ void output_pass(const float2 *part, TO *o0, long long st0, int vec0, TO *o1,
                                             long long st1, int vec1, int nrows, int m0, int M, int tid, Fin fin) {
@@ -475,12 +485,12 @@ __device__ __forceinline__ void output_pass(const float2 *part, TO *o0, long lon
             const float4 x = *reinterpret_cast<const float4 *>(part + (tt * LPC + jj) * MCP + c);
             ax += x.x; ay += x.y; bx += x.z; by += x.w;
         }
-        float r0[2], r1[2];
-        fin(make_float2(ax, ay), tt, c, r0[0], r1[0]);
-        fin(make_float2(bx, by), tt, c + 1, r0[1], r1[1]);
+        const bool full = m0 + c + 1 < M;
+        float2 f0 = make_float2(ax, ay), f1 = make_float2(bx, by);
+        fin(f0, f1, tt, c, full);
+        const float r0[2] = {f0.x, f1.x}, r1[2] = {f0.y, f1.y};
         TO *p0 = o0 + (long long)tt * st0 + m0 + c;
         TO *p1 = o1 + (long long)tt * st1 + m0 + c;
-        const bool full = m0 + c + 1 < M;
         if (full && vec0) {
             if constexpr (sizeof(TO) == 4) {
                 *reinterpret_cast<float2 *>(p0) = make_float2(r0[0], r0[1]);

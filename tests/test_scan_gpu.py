@@ -608,3 +608,31 @@ def test_forward_without_checkpoints_is_segmented_too(kb, monkeypatch):
     torch.cuda.synchronize()
     lib.check_status()
     assert torch.equal(y1, y0) and torch.equal(yv1, yv0) and torch.equal(st1.lam, st0.lam) and torch.equal(st1.eta, st0.eta)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 31, 34, 65])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_training_epilogue_keeps_raw_outputs_at_any_width(M, dtype):
+    """The raw outputs that the epilogue's adjoint reads are stored as pairs of channels where the rows allow it, one by one
+    otherwise. The gate's gradient is made of them: 2 g' (y dy + 2 g y_var dy_var), each factor rounded to the activations' type
+    once on either path (2^-8 of it for bfloat16, 6e-8 for float32; four of them and float32's own sums)."""
+    import kla_b200
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    B, L, S = 2, 37, 16
+    v, z, gate, dy, dyv = (rn(B, L, M).to(dtype) for _ in range(5))
+    lv = F.softplus(rn(B, L, M)).reciprocal().to(dtype)
+    k, q = (F.normalize(rn(B, L, S), dim=-1).to(dtype) for _ in range(2))
+    a, p, skip = torch.sigmoid(rn(M, S)), F.softplus(rn(M, S)), rn(M)
+    gate.requires_grad_(True)
+    epi = dict(z=z, lambda_skip=skip, gate=gate, gate_activation="silu")
+    y, y_var, _ = kla_b200.kla_scan_b200(v, lv, k, q, a, p, out_dtype=dtype, epilogue=epi)
+    got, = torch.autograd.grad([y, y_var], [gate], [dy, dyv])
+    with torch.no_grad():
+        y0, yv0, _ = kla_b200.kla_scan_b200(v, lv, k, q, a, p, out_dtype=dtype)
+    gf = gate.detach().float().requires_grad_(True)
+    s = F.silu(gf)
+    want, = torch.autograd.grad([(y0.float() + skip * z.float()) * s, yv0.float() * s * s], [gf], [dy.float(), dyv.float()])
+    assert (got.float() - want).norm() <= (4 * 2 ** -8 if dtype == torch.bfloat16 else 1e-5) * want.norm()
