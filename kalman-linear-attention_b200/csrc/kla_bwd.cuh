@@ -49,13 +49,14 @@
 // on; the state its walk starts from needs no hand-over, the replay group computes it from the checkpoints.
 //
 // Measured on B200 at T=4096, M=1024, S=16, float32, against the kernel with one channel per thread and scalar
-// arithmetic: B=8 1.42 -> 1.15 ms, B=4 0.88 -> 0.69 ms, B=16 2.59 -> 2.13 ms; 43.5 instead of 66 warp instructions per 32
-// lane-steps. What bounds it is the FP32 pipe's register reads: 30 pair operations per two chains and step in the
+// arithmetic: B=8 1.42 -> 1.13 ms, B=4 0.88 -> 0.69 ms, B=16 2.59 -> 2.13 ms; 43.5 instead of 66 warp instructions per 32
+// lane-steps. What bounds it is the FP32 pipe's register reads: 29 pair operations per two chains and step in the
 // reverse walk and 8 in the replay, 12 and 2 of them three-operand FMAs at 3.75 cycles (kla_common.cuh), add up to about
 // 235 of the 291 cycles a scheduler spends on a warp's step. Not limits: shared memory (the trajectory through tensor
 // memory, a third less shared-memory traffic, takes the same 1.17 ms), the helpers (1.12 ms without their sums), the
 // replay (1.08 ms without its arithmetic). Scalar FMAs in place of the pair FMAs: 1.25 ms. Fetching a step's inputs
-// before the previous step's arithmetic and unrolling the whole tile gave 1.20 -> 1.17 ms.
+// before the previous step's arithmetic and unrolling the whole tile gave 1.20 -> 1.17 ms; shares of dk, dq summed as halves
+// and doubled once per CTA 1.144 -> 1.132.
 #pragma once
 
 #include <type_traits>
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                 // P, nm: the state after the step on entry, before it on return; nxt, gn: fetched and formed for step un
                 auto reverse_step = [&](int u, const StepIn &in, const float2 (&g)[SPT], int un, StepIn &nxt, float2 (&gn)[SPT]) {
                     fetch(nxt, un);
-                    const float2 nlv = neg2(in.lv), lv2 = add2(in.lv, in.lv), vl = mul2(in.v, in.lv);
+                    const float2 nlv = neg2(in.lv), hv = mul2(in.v, dup2(0.5f)), hdy = mul2(in.dy, dup2(0.5f));
                     float2 D, E, share[SPT];
 #pragma unroll
                     for (int i = 0; i < SPT; ++i) {
@@ -457,18 +458,18 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                             naccA[i] = fma2(mob, nm[i], naccA[i]);
                             naccA2[i] = fma2(nvob, P[i], naccA2[i]);
                             naccP[i] = add2(naccP[i], nvob);
-                            dq = fma2(add2(qd, qd), fma2(ca2[i], P[i], cp[i]), mul2(in.dy, mul2(ca[i], nm[i])));
+                            dq = fma2(qd, fma2(ca2[i], P[i], cp[i]), mul2(hdy, mul2(ca[i], nm[i])));
                         } else {
                             mbar = fma2(in.dy, q, cm[i]);
                             nPbar = fma2(qd, q, ncP[i]);
-                            dq = fma2(add2(qd, qd), P[i], mul2(in.dy, nm[i]));
+                            dq = fma2(qd, P[i], mul2(hdy, nm[i]));
                         }
                         const float2 phibar = mul2(P[i], fma2(mbar, nm[i], mul2(nPbar, P[i])));
                         const float2 rbar = mul2(P[i], mbar);
                         const float2 ubar = mul2(mbar, g[i]);
                         const float2 nPpbar = mul2(g[i], fma2(mbar, nw, mul2(nPbar, g[i])));
                         const float2 z = mul2(phibar, k);
-                        const float2 dk = fma2(z, lv2, mul2(rbar, vl));
+                        const float2 dk = mul2(in.lv, fma2(rbar, hv, z));
                         D = i == 0 ? mul2(rbar, k) : fma2(rbar, k, D);
                         E = i == 0 ? mul2(z, k) : fma2(z, k, E);
                         cm[i] = mul2(ubar, ca[i]);
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                         naccP[i] = add2(naccP[i], nPpbar);
                         P[i] = in.P[i];
                         nm[i] = in.nm[i];
-                        share[i] = make_float2(dk.x + dk.y, dq.x + dq.y);  // this thread's dk, -dq for (t, s)
+                        share[i] = make_float2(dk.x + dk.y, dq.x + dq.y);  // half of this thread's dk, -dq for (t, s)
                     }
                     gain(gn, nxt, P);
                     // parked where the warp's own trajectory slots of this step were: row (u, i) of the warp is 64 float2s,
@@ -739,17 +740,19 @@ __global__ void __launch_bounds__(kBwdThreads, 2) kla_bwd_kernel(const __grid_co
                             x0 = add2(x0, make_float2(x.x, x.y));
                             x1 = add2(x1, make_float2(x.z, x.w));
                         }
+                    x0 = mul2(x0, make_float2(2.0f, -2.0f));  // the shares are halves of dk and -dq
+                    x1 = mul2(x1, make_float2(2.0f, -2.0f));
                     if (st < S && u < n) {
                         const long long at = ((long long)b * prm.L + t_off + t0 + u) * S + st;
                         if (prm.vec_dkq) {
                             atomicAdd(reinterpret_cast<float2 *>(prm.dk + at), make_float2(x0.x, x1.x));
-                            atomicAdd(reinterpret_cast<float2 *>(prm.dq + at), make_float2(-x0.y, -x1.y));
+                            atomicAdd(reinterpret_cast<float2 *>(prm.dq + at), make_float2(x0.y, x1.y));
                         } else {
                             atomicAdd(prm.dk + at, x0.x);
-                            atomicAdd(prm.dq + at, -x0.y);
+                            atomicAdd(prm.dq + at, x0.y);
                             if (st + 1 < S) {
                                 atomicAdd(prm.dk + at + 1, x1.x);
-                                atomicAdd(prm.dq + at + 1, -x1.y);
+                                atomicAdd(prm.dq + at + 1, x1.y);
                             }
                         }
                     }

@@ -617,6 +617,8 @@ def test_training_epilogue_keeps_raw_outputs_at_any_width(M, dtype):
     """The raw outputs that the epilogue's adjoint reads are stored as pairs of channels where the rows allow it, one by one
     otherwise. The gate's gradient is made of them: 2 g' (y dy + 2 g y_var dy_var), each factor rounded to the activations' type
     once on either path (2^-8 of it for bfloat16, 6e-8 for float32; four of them and float32's own sums)."""
+    import torch.nn.functional as F
+
     import kla_b200
 
     g = torch.Generator(device="cuda").manual_seed(M)
