@@ -92,7 +92,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
     auto lstage = [&](int s) { return reinterpret_cast<T *>(in_base + s * Sm::kIn + Sm::kTileI); };
     auto dystage = [&](int s) { return reinterpret_cast<TO *>(in_base + s * Sm::kIn + 2 * Sm::kTileI); };
     auto dyvstage = [&](int s) { return reinterpret_cast<TO *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + Sm::kTileO); };
-    // k (and q) of a step, grouped by owning lane: [TT][LPC][NK][SPT] floats, state s = i * LPC + j at [j][.][i]
+    // k (and q) of a step, grouped by owning lane: [TT][NK][LPC][SPT] floats, state s = i * LPC + j at [.][j][i]
     auto kqstage = [&](int s) {
         return reinterpret_cast<float *>(in_base + s * Sm::kIn + 2 * Sm::kTileI + (ADJ ? 2 * Sm::kTileO : 0));
     };
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
                 kk[0] = make_float2(k4.x, k4.y);
                 kk[1] = make_float2(k4.z, k4.w);
                 if (ADJ) {
-                    const float4 q4 = *reinterpret_cast<const float4 *>(row + SPT);
+                    const float4 q4 = *reinterpret_cast<const float4 *>(row + SPAD);
                     qq[0] = make_float2(q4.x, q4.y);
                     qq[1] = make_float2(q4.z, q4.w);
                 }
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
 #pragma unroll
                 for (int h = 0; h < HP; ++h) {
                     kk[h] = *reinterpret_cast<const float2 *>(row + 2 * h);
-                    if (ADJ) qq[h] = *reinterpret_cast<const float2 *>(row + SPT + 2 * h);
+                    if (ADJ) qq[h] = *reinterpret_cast<const float2 *>(row + SPAD + 2 * h);
                 }
             }
             float dyf = 0.0f, dyvf = 0.0f;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
             if (!mbar_wait(prm.wait, &full_in[s], (tile / NS) & 1, 31)) break;
             const T *vrow = vstage(s) + cw, *lrow = lstage(s) + cw;
             const TO *dyrow = dystage(s) + cw, *dyvrow = dyvstage(s) + cw;
-            const float *kqrow = kqstage(s) + j * NK * SPT;
+            const float *kqrow = kqstage(s) + j * SPT;
             if (t0 + TT <= L) {
 #pragma unroll 1
                 for (int t4 = 0; t4 < TT; t4 += 4) {
@@ -294,9 +294,9 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
             for (int e = 0; e < KQP; ++e) {
                 const int idx = lane + e * 32, row = idx / SPAD, sidx = idx % SPAD;
                 if (idx < TT * SPAD) {
-                    float *dst = kq + row * NK * SPAD + (sidx % LPC) * NK * SPT + sidx / LPC;
+                    float *dst = kq + row * NK * SPAD + (sidx % LPC) * SPT + sidx / LPC;
                     dst[0] = kr[e];
-                    if (ADJ) dst[SPT] = qr[e];
+                    if (ADJ) dst[SPAD] = qr[e];
                 }
             }
             if (it + 1 < NT) load_kq(t0 + TT);

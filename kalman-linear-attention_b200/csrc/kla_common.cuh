@@ -466,6 +466,11 @@ __device__ __forceinline__ void stage_tile(T *smem, const T *base, long long st,
     }
 }
 
+// Rows of the partial-sum buffers of lanes eight apart meet the same banks. From 16 lanes per channel on, where they store at
+// the same time, the upper ones therefore hold the two channels of a pair the other way round.
+template <int LPC>
+__device__ __forceinline__ int swapped_channels(int j) { return LPC > 8 ? (j >> 3) & 1 : 0; }
+
 // Sum the per-lane-group partials of one tile over the LPC lane groups and
 // write two [rows x MC] output tiles. part: [TT][LPC][MCP] float2 in shared
 // memory. Each thread handles pairs of channels, so consecutive lanes read
@@ -483,7 +488,11 @@ __device__ __forceinline__ void output_pass(const float2 *part, TO *o0, long lon
 #pragma unroll
         for (int jj = 0; jj < LPC; ++jj) {
             const float4 x = *reinterpret_cast<const float4 *>(part + (tt * LPC + jj) * MCP + c);
-            ax += x.x; ay += x.y; bx += x.z; by += x.w;
+            if (swapped_channels<LPC>(jj)) {
+                ax += x.z; ay += x.w; bx += x.x; by += x.y;
+            } else {
+                ax += x.x; ay += x.y; bx += x.z; by += x.w;
+            }
         }
         const bool full = m0 + c + 1 < M;
         float2 f0 = make_float2(ax, ay), f1 = make_float2(bx, by);

@@ -125,7 +125,9 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI
     auto gstage = [&](int e) { return reinterpret_cast<T *>(epi_base + e * Sm::kEpi + Sm::kTile); };
     auto vstage = [&](int s) { return reinterpret_cast<T *>(in_base + s * Sm::kIn); };
     auto lstage = [&](int s) { return reinterpret_cast<T *>(in_base + s * Sm::kIn + Sm::kTile); };
-    // (k, q) of a step, grouped by owning lane: [TT][LPC][2][SPT] floats, state s = i * LPC + j at [j][.][i]
+    // k and q of a step, grouped by owning lane: [TT][2][LPC][SPT] floats, state s = i * LPC + j at [.][j][i]. (With k and q of a
+    // lane side by side, lanes four apart met the same banks from eight lanes per channel on, and half the shared-memory cycles
+    // that bounded the kernel at S = 64 were conflicts: B=4 L=2048 M=512 float32 312 -> 280 us, with swapped_channels().)
     auto kqstage = [&](int s) { return reinterpret_cast<float *>(in_base + s * Sm::kIn + 2 * Sm::kTile); };
     auto lfstage = [&](int s) {
         return reinterpret_cast<float *>(in_base + s * Sm::kIn + (sizeof(T) == 4 ? Sm::kTile : 2 * Sm::kTile + Sm::kKq));
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI
             const float *row = kqrow + tt * 2 * SPAD;
             if constexpr (SPT == 4) {
                 const float4 kk = *reinterpret_cast<const float4 *>(row);
-                const float4 qq = *reinterpret_cast<const float4 *>(row + SPT);
+                const float4 qq = *reinterpret_cast<const float4 *>(row + SPAD);
                 in.k[0] = make_float2(kk.x, kk.y);
                 in.k[1] = make_float2(kk.z, kk.w);
                 in.q[0] = make_float2(qq.x, qq.y);
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI
 #pragma unroll
                 for (int h = 0; h < HP; ++h) {
                     in.k[h] = *reinterpret_cast<const float2 *>(row + 2 * h);
-                    in.q[h] = *reinterpret_cast<const float2 *>(row + SPT + 2 * h);
+                    in.q[h] = *reinterpret_cast<const float2 *>(row + SPAD + 2 * h);
                 }
             }
         };
@@ -344,8 +346,8 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI
             const T *lrow = lstage(s) + cw;
             const float *lfrow = lfstage(s) + cw;
             const T *vrow = vstage(s) + cw;
-            const float *kqrow = kqstage(s) + j * 2 * SPT;
-            float2 *yrow = ystage(o) + j * MCP + cw;
+            const float *kqrow = kqstage(s) + j * SPT;
+            float2 *yrow = ystage(o) + j * MCP + (cw ^ swapped_channels<LPC>(j));
             StepIn in;
             StepPre pr, prn;
             fetch(in, lrow, lfrow, vrow, kqrow, 0);
@@ -455,9 +457,9 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI
                 for (int e = 0; e < KQP; ++e) {
                     const int idx = htid + e * kProducers, row = idx / SPAD, sidx = idx % SPAD;
                     if (idx < TT * SPAD) {
-                        float *dst = kq + row * 2 * SPAD + (sidx % LPC) * 2 * SPT + sidx / LPC;
+                        float *dst = kq + row * 2 * SPAD + (sidx % LPC) * SPT + sidx / LPC;
                         dst[0] = kr[e];
-                        dst[SPT] = qr[e];
+                        dst[SPAD] = qr[e];
                     }
                 }
                 if (it + 1 < NT) load_kq(t0 + TT);
