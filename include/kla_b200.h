@@ -112,6 +112,8 @@ typedef struct kla_b200_fwd_args {
      * state of its own. lam0, eta0, lam_fin, eta_fin then hold [B*chunks, M, S] (entry b*chunks + c is chunk c of batch
      * element b) and ckpt is kla_b200_ckpt_bytes(B*chunks, chunk_len, M, S) bytes. 0 or 1: sequences are whole. */
     int64_t chunks, chunk_len;
+    /* with chunks > 1: lam_fin, eta_fin hold [B, M, S], the state after each sequence, not after each of its chunks */
+    int32_t sequence_state;
 } kla_b200_fwd_args;
 
 /* Bytes of the scratch the forward writes for the backward: the filter state
@@ -222,6 +224,9 @@ typedef struct kla_b200_slab_args {
     float *out;                         /* [B, M, S, 8] float32 */
     int64_t chunks, chunk_len;          /* as in kla_b200_fwd_args: lam0, eta0 and out are then per entry; the record no
                                          * fold reads (forward: the last chunk's, adjoint: the first's) is not written */
+    /* as in kla_b200_fwd_args */
+    int32_t lambda_v_is_log_variance;
+    float obs_var_min, obs_var_max;
 } kla_b200_slab_args;
 
 int kla_b200_slab_aggregate(const kla_b200_slab_args *args, void *stream);

@@ -149,6 +149,7 @@ class FwdArgs(Structure):
         ("z", Tensor3), ("gate", Tensor3), ("lambda_skip", c_void_p),
         ("lambda_skip_len", c_int32), ("gate_activation", c_int32),
         ("y_raw", Tensor3), ("y_var_raw", Tensor3), ("work", c_void_p), ("chunks", c_int64), ("chunk_len", c_int64),
+        ("sequence_state", c_int32),
     ]
 
 
@@ -186,6 +187,7 @@ class SlabArgs(Structure):
         ("v", Tensor3), ("lambda_v", Tensor3), ("k", Tensor3), ("q", Tensor3),
         ("a", c_void_p), ("p", c_void_p), ("lam0", c_void_p), ("eta0", c_void_p),
         ("dy", Tensor3), ("dy_var", Tensor3), ("out", c_void_p), ("chunks", c_int64), ("chunk_len", c_int64),
+        ("lambda_v_is_log_variance", c_int32), ("obs_var_min", c_float), ("obs_var_max", c_float),
     ]
 
 

@@ -60,6 +60,10 @@ struct alignas(64) AggParams {
     Tensor3 v, lv, k, q, dy, dyv;      // dy, dyv, q: adjoint only
     const float *a, *p, *lam0, *eta0;  // lam0/eta0: adjoint only (nullptr = unit prior)
     float *out;                        // [entries, M, S, 8]
+    // lv holds log-variances, as in FwdParams: every warp turns its channels of a tile into precisions, into kLam bytes behind
+    // the stages (one buffer: a warp is done with a tile before it meets the next)
+    int lv_log_sigma;
+    float obs_var_min, obs_var_max;
     ChunkCtl chunk;
     WaitCtl wait;
 };
@@ -74,9 +78,12 @@ struct AggSmem {
     static constexpr size_t kKq = ((sizeof(float) * (ADJ ? 2 : 1) * kAggTT * kSPad + 127) / 128) * 128;
     static constexpr size_t kIn = 2 * kTileI + (ADJ ? 2 * kTileO : 0) + kKq;
     static constexpr size_t kTotal = kBars + kAggStages * kIn;
+    static constexpr size_t kLam = sizeof(float) * kAggTT * kMC;
 };
 
-template <typename T, typename TO, int SPT, int LPC, int NW, bool ADJ, bool PRIOR>
+// LOGV (AggParams::lv_log_sigma) is a separate instantiation: a test in every step cost plain inference at B=1 L=1501
+// M=1536 float32 2 of its 64 us.
+template <typename T, typename TO, int SPT, int LPC, int NW, bool ADJ, bool PRIOR, bool LOGV>
 __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_constant__ AggParams prm) {
     using Sm = AggSmem<T, TO, SPT, LPC, NW, ADJ>;
     constexpr int TT = kAggTT, NS = kAggStages, MC = Sm::kMC, SPAD = Sm::kSPad, CLS = 32 / LPC;
@@ -105,6 +112,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
     if (prm.chunk.n > 1 && be % prm.chunk.n == (ADJ ? 0 : prm.chunk.n - 1)) return;
     const int NT = (L + TT - 1) / TT;
     const bool has_dyv = ADJ && prm.dyv.ptr != nullptr;
+    float *lam_tile = reinterpret_cast<float *>(smem + Sm::kTotal);  // [TT][MC], with LOGV
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
@@ -149,7 +157,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
         }
 
         auto step = [&](const T *vrow, const T *lrow, const TO *dyrow, const TO *dyvrow, const float *kqrow, int tt) {
-            const float2 lv = dup2(to_f32<T>(lrow[tt * MC])), vv = dup2(to_f32<T>(vrow[tt * MC]));
+            const float2 lv = dup2(LOGV ? lam_tile[tt * MC + cw] : to_f32<T>(lrow[tt * MC])), vv = dup2(to_f32<T>(vrow[tt * MC]));
             const float *row = kqrow + tt * NK * SPAD;
             float2 kk[HP], qq[HP];
             if constexpr (SPT == 4) {
@@ -206,6 +214,11 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
         for (int tile = 0; tile < NT; ++tile) {
             const int s = tile % NS, t0 = tile * TT;
             if (!mbar_wait(prm.wait, &full_in[s], (tile / NS) & 1, 31)) break;
+            if constexpr (LOGV) {
+                precisions_from_tile<T, TT, MC, CLS>(lstage(s) + warp * CLS, lam_tile + warp * CLS, prm.obs_var_min,
+                                                     prm.obs_var_max, lane);
+                __syncwarp();
+            }
             const T *vrow = vstage(s) + cw, *lrow = lstage(s) + cw;
             const TO *dyrow = dystage(s) + cw, *dyvrow = dyvstage(s) + cw;
             const float *kqrow = kqstage(s) + j * SPT;

@@ -688,6 +688,7 @@ int kla_b200_scan_fwd(const kla_b200_fwd_args *a, void *stream) {
     prm.y = t3(a->y); prm.yv = t3(a->y_var);
     prm.a = a->a; prm.p = a->p; prm.lam0 = a->lam0; prm.eta0 = a->eta0;
     prm.lam_fin = a->lam_fin; prm.eta_fin = a->eta_fin;
+    prm.sequence_state = prm.chunk.n > 1 && a->sequence_state != 0;
     prm.ckpt = static_cast<float2 *>(a->ckpt);
     prm.lv_log_sigma = a->lambda_v_is_log_variance != 0;
     prm.obs_var_min = a->obs_var_min; prm.obs_var_max = a->obs_var_max;
@@ -800,6 +801,8 @@ int kla_b200_slab_aggregate(const kla_b200_slab_args *a, void *stream) {
     prm.v = t3(a->v); prm.lv = t3(a->lambda_v); prm.k = t3(a->k); prm.q = t3(a->q);
     prm.dy = t3(a->dy); prm.dyv = t3(a->dy_var);
     prm.a = a->a; prm.p = a->p; prm.lam0 = a->lam0; prm.eta0 = a->eta0; prm.out = a->out;
+    prm.lv_log_sigma = a->lambda_v_is_log_variance != 0;
+    prm.obs_var_min = a->obs_var_min; prm.obs_var_max = a->obs_var_max;
     if ((rc = wait_ctl(&prm.wait))) return rc;
     prm.wait.skip_tile = -1;  // the hook is for the scan kernels
     return dispatch_slab(a->in_dtype, a->out_dtype, a->decode_from_prior != 0, lpc_for(a->S), prm, *a,

@@ -47,6 +47,7 @@ struct alignas(64) FwdParams {
     Tensor3 v, lv, k, q, y, yv;
     const float *a, *p, *lam0, *eta0;
     float *lam_fin, *eta_fin;
+    int sequence_state;  // lam_fin, eta_fin are per sequence, its last chunk's, instead of per chunk
     float2 *ckpt;  // [entries, NC, M, S] (P, mean) before every kCkptInterval-th step, or nullptr
     int vec_y, vec_yv, vec_raw;
     // lv holds the sensor projection's raw log-variance output instead of the precision:
@@ -395,9 +396,11 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI
                 const int s = i * LPC + j;
                 if (m < M && s < S) {
                     if (last_seg) {
+                        if (prm.sequence_state && be % prm.chunk.n != prm.chunk.n - 1) continue;
                         const float lam = 1.0f / pair_el(P[ci], i);
-                        prm.lam_fin[((long long)be * M + m) * S + s] = lam;
-                        prm.eta_fin[((long long)be * M + m) * S + s] = pair_el(mean[ci], i) * lam;
+                        const long long at = ((long long)(prm.sequence_state ? be / prm.chunk.n : be) * M + m) * S + s;
+                        prm.lam_fin[at] = lam;
+                        prm.eta_fin[at] = pair_el(mean[ci], i) * lam;
                     } else {
                         __stcg(hand + ((long long)be * M + m) * S + s, make_float2(pair_el(P[ci], i), pair_el(mean[ci], i)));
                     }

@@ -167,7 +167,7 @@ bool canonical(const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor 
 // ------------------------------------------------------------------------------------------------------ the scan
 
 // kla_b200_scan_fwd. segments: give the kernel working memory so that a forward without checkpoints can hand sequences
-// from CTA to CTA. chunks > 1: lam0, eta0 and the returned states are per chunk.
+// from CTA to CTA. chunks > 1: lam0 and eta0 are per chunk.
 std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> scan_fwd(
     const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const OptTensor &lam0,
     const OptTensor &eta0, bool prior, bool out_bf16, bool need_ckpt, bool segments, const SensorArg &sensors, const OptTensor &z,
@@ -177,7 +177,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> scan_fwd(
     const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2), E = B * chunks;
     const auto TO = out_type(out_bf16);
     Tensor y = fresh(v, {B, L, M}, TO), yv = fresh(v, {B, L, M}, TO);
-    Tensor lam = f32(v, {E, M, S}), eta = f32(v, {E, M, S});
+    Tensor lam = f32(v, {B, M, S}), eta = f32(v, {B, M, S});
     OptTensor ckpt, work;
     if (need_ckpt && L > 0) ckpt = fresh(v, {(int64_t)lib.ckpt_bytes(E, chunks > 1 ? chunk_len : L, M, S)}, at::kByte);
     else if (segments) work = fresh(v, {(int64_t)lib.segment_scratch_bytes(B, M, S)}, at::kByte);
@@ -194,7 +194,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> scan_fwd(
     if (skip) { f.z = t3(z); f.lambda_skip = fp(*skip); f.lambda_skip_len = (int32_t)skip->numel(); }
     if (gate) { f.gate = t3(*gate); f.gate_activation = gate_act; }
     f.y_raw = t3(y_raw); f.y_var_raw = t3(yv_raw);
-    if (chunks > 1) { f.chunks = chunks; f.chunk_len = chunk_len; }
+    if (chunks > 1) { f.chunks = chunks; f.chunk_len = chunk_len; f.sequence_state = 1; }
     check(lib.scan_fwd(&f, stream_of(v)));
     return {y, yv, lam, eta, ckpt};
 }
@@ -228,7 +228,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_
 // kla_b200_slab_aggregate -> [B*chunks, M, S, 8]; the adjoint aggregate when dy is given
 Tensor slab_aggregate(const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &a, const Tensor &p, const OptTensor &q,
                       const OptTensor &dy, const OptTensor &dyv, const OptTensor &lam0, const OptTensor &eta0, bool prior,
-                      int64_t chunks, int64_t chunk_len) {
+                      const SensorArg &sensors, int64_t chunks, int64_t chunk_len) {
     const c10::cuda::CUDAGuard guard(v.device());
     const int64_t B = v.size(0), L = v.size(1), M = v.size(2), S = k.size(2);
     Tensor out = f32(v, {B * chunks, M, S, 8});
@@ -239,6 +239,8 @@ Tensor slab_aggregate(const Tensor &v, const Tensor &lv, const Tensor &k, const 
     s.v = t3(v); s.lambda_v = t3(lv); s.k = t3(k); s.q = t3(q);
     s.a = fp(a); s.p = fp(p); s.lam0 = fp(lam0); s.eta0 = fp(eta0);
     s.dy = t3(dy); s.dy_var = t3(dyv); s.out = fp(out);
+    const Sensors sen(sensors);
+    s.lambda_v_is_log_variance = sen.on; s.obs_var_min = sen.vmin; s.obs_var_max = sen.vmax;
     if (chunks > 1) { s.chunks = chunks; s.chunk_len = chunk_len; }
     check(lib.slab_aggregate(&s, stream_of(v)));
     return out;
@@ -261,23 +263,23 @@ std::tuple<Tensor, Tensor> chunk_fold(const Tensor &agg, int64_t C, const OptTen
 // checkpoints and every chunk's start state (both for the backward).
 std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor, Tensor, Tensor> scan_fwd_chunked(
     const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const OptTensor &lam0,
-    const OptTensor &eta0, bool prior, bool out_bf16, bool need_ckpt, int64_t chunks, int64_t chunk_len) {
-    const Tensor agg = slab_aggregate(v, lv, k, a, p, {}, {}, {}, {}, {}, false, chunks, chunk_len);
+    const OptTensor &eta0, bool prior, bool out_bf16, bool need_ckpt, const SensorArg &sensors, const OptTensor &z,
+    const OptTensor &skip, const OptTensor &gate, int gate_act, const OptTensor &y_raw, const OptTensor &yv_raw, int64_t chunks,
+    int64_t chunk_len) {
+    const Tensor agg = slab_aggregate(v, lv, k, a, p, {}, {}, {}, {}, {}, false, sensors, chunks, chunk_len);
     auto [lam_in, eta_in] = chunk_fold(agg, chunks, lam0, eta0, {}, {}, false);
-    auto [y, yv, lam, eta, ckpt] = scan_fwd(v, lv, k, q, a, p, lam_in, eta_in, prior, out_bf16, need_ckpt, false, {}, {}, {}, {}, 0, {},
-                                            {}, chunks, chunk_len);
-    const int64_t B = v.size(0), M = v.size(2), S = k.size(2);
-    auto last = [&](const Tensor &t) { return t.view({B, chunks, M, S}).select(1, chunks - 1); };
-    return {y, yv, last(lam), last(eta), ckpt, lam_in, eta_in};
+    auto [y, yv, lam, eta, ckpt] = scan_fwd(v, lv, k, q, a, p, lam_in, eta_in, prior, out_bf16, need_ckpt, false, sensors, z, skip,
+                                            gate, gate_act, y_raw, yv_raw, chunks, chunk_len);
+    return {y, yv, lam, eta, ckpt, lam_in, eta_in};
 }
 
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_bwd_chunked(
     const Tensor &v, const Tensor &lv, const Tensor &k, const Tensor &q, const Tensor &a, const Tensor &p, const Tensor &lam_in,
     const Tensor &eta_in, const OptTensor &ckpt, const Tensor &dy, const OptTensor &dyv, const OptTensor &dlam_fin,
-    const OptTensor &deta_fin, bool prior, bool out_bf16, int64_t chunks, int64_t chunk_len) {
-    const Tensor agg = slab_aggregate(v, lv, k, a, p, q, dy, dyv, lam_in, eta_in, prior, chunks, chunk_len);
+    const OptTensor &deta_fin, bool prior, bool out_bf16, const SensorArg &sensors, int64_t chunks, int64_t chunk_len) {
+    const Tensor agg = slab_aggregate(v, lv, k, a, p, q, dy, dyv, lam_in, eta_in, prior, sensors, chunks, chunk_len);
     auto [dlam_seed, deta_seed] = chunk_fold(agg, chunks, dlam_fin, deta_fin, lam_in, eta_in, true);
-    auto r = scan_bwd(v, lv, k, q, a, p, lam_in, eta_in, ckpt, dy, dyv, dlam_seed, deta_seed, prior, out_bf16, {}, chunks, chunk_len);
+    auto r = scan_bwd(v, lv, k, q, a, p, lam_in, eta_in, ckpt, dy, dyv, dlam_seed, deta_seed, prior, out_bf16, sensors, chunks, chunk_len);
     const int64_t B = v.size(0), M = v.size(2), S = k.size(2);
     auto first = [&](const Tensor &t) { return t.view({B, chunks, M, S}).select(1, 0); };
     std::get<6>(r) = first(std::get<6>(r));

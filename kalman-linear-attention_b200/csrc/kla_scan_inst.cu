@@ -64,19 +64,20 @@ template <typename T, typename TO, int LPC, bool PRIOR>
 cudaError_t launch_agg(const AggParams &prm, bool adjoint, cudaStream_t st) {
     constexpr int MC = kNW * (32 / LPC);
     dim3 grid((unsigned)((prm.M + MC - 1) / MC), (unsigned)prm.B);
-    cudaError_t e;
+    auto go = [&](auto kern, size_t smem) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, (kNW + 1) * 32, smem, st>>>(prm);
+        return cudaGetLastError();
+    };
     if (adjoint) {
-        auto kern = kla_agg_kernel<T, TO, kSPT, LPC, kNW, true, PRIOR>;
-        constexpr size_t smem = AggSmem<T, TO, kSPT, LPC, kNW, true>::kTotal;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
-        kern<<<grid, (kNW + 1) * 32, smem, st>>>(prm);
-    } else {
-        auto kern = kla_agg_kernel<T, TO, kSPT, LPC, kNW, false, false>;
-        constexpr size_t smem = AggSmem<T, TO, kSPT, LPC, kNW, false>::kTotal;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
-        kern<<<grid, (kNW + 1) * 32, smem, st>>>(prm);
+        using Sm = AggSmem<T, TO, kSPT, LPC, kNW, true>;
+        return prm.lv_log_sigma ? go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, true, PRIOR, true>, Sm::kTotal + Sm::kLam)
+                                : go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, true, PRIOR, false>, Sm::kTotal);
     }
-    return cudaGetLastError();
+    using Sm = AggSmem<T, TO, kSPT, LPC, kNW, false>;
+    return prm.lv_log_sigma ? go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, false, false, true>, Sm::kTotal + Sm::kLam)
+                            : go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, false, false, false>, Sm::kTotal);
 }
 
 #define KLA_INST_AGG_ONE(T, TO, LPC)                                                       \

@@ -98,6 +98,14 @@ def _forward_segments(lib, dev: torch.device, B: int, L: int, M: int, S: int) ->
     return lib.kla_b200_plan_segments(B * ((M + per_cta - 1) // per_cta), L, 0, _SM_COUNT[idx], -1, None) > 1
 
 
+def _epilogue_args(epilogue, raw):
+    """z, lambda_skip, gate, its activation and the buffers of the scan's own outputs, as the host module takes them."""
+    epi = epilogue or {}
+    gate = epi.get("gate")
+    return (epi.get("z"), epi.get("lambda_skip"), gate,
+            0 if gate is None else _lib.ACT[epi.get("gate_activation", "silu")], *(raw or (None, None)))
+
+
 def _launch_fwd(v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype, need_ckpt: bool, sensors=None,
                 epilogue=None, raw=None):
     """Allocate outputs (and the checkpoint scratch when a backward will follow)
@@ -105,12 +113,18 @@ def _launch_fwd(v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype, nee
     # without checkpoints the kernel still hands long lists of sequences from CTA to CTA in segments, given a little
     # working memory
     segments = not need_ckpt and _forward_segments(_lib.load(), v.device, v.shape[0], v.shape[1], v.shape[2], k.shape[2])
-    epi = epilogue or {}
-    gate = epi.get("gate")
     return _lib.host().scan_fwd(
         v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype == torch.bfloat16, need_ckpt, segments, sensors,
-        epi.get("z"), epi.get("lambda_skip"), gate, 0 if gate is None else _lib.ACT[epi.get("gate_activation", "silu")],
-        *(raw or (None, None)), 1, 0)
+        *_epilogue_args(epilogue, raw), 1, 0)
+
+
+def _launch_fwd_chunked(v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype, need_ckpt: bool, chunks: int, sensors=None,
+                        epilogue=None, raw=None):
+    """:func:`_launch_fwd` with the chunks of every sequence running side by side from exact start states, which are
+    returned as well."""
+    return _lib.host().scan_fwd_chunked(
+        v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype == torch.bfloat16, need_ckpt, sensors,
+        *_epilogue_args(epilogue, raw), chunks, _chunk_len(v.shape[1], chunks))
 
 
 def _launch_bwd(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin,
@@ -124,7 +138,7 @@ def slab_aggregate(v, lambda_v, k, a, p, *, q=None, dy=None, dy_var=None, lam0=N
                    prior: bool = False) -> torch.Tensor:
     """Launch ``kla_b200_slab_aggregate``: one record per lane that describes how a whole time slab acts on
     the filter state (``dy`` None) or on the backward carry (``dy`` given). Returns [B, M, S, 8] float32."""
-    return _lib.host().slab_aggregate(v, lambda_v, k, a, p, q, dy, dy_var, lam0, eta0, prior, 1, 0)
+    return _lib.host().slab_aggregate(v, lambda_v, k, a, p, q, dy, dy_var, lam0, eta0, prior, None, 1, 0)
 
 
 # CTAs the backward kernel keeps resident on a B200: 148 SMs x 2
@@ -148,9 +162,11 @@ def _row_bytes(tensors) -> int:
     return n
 
 
-def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = None, tensors=(), training: bool = False) -> int:
+def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = None, tensors=(), training: bool = False,
+                     layer: bool = False) -> int:
     """Number of time chunks for the time-parallel scan. 1 = the plain lane-serial kernels. ``tensors``: the activations,
-    for the alignment of their rows; ``training``: a backward follows.
+    for the alignment of their rows; ``training``: a backward follows; ``layer``: the scan also forms the precisions or
+    applies the output path.
 
     The kernels put one CTA on every 32 / 16 / 8 ... channels (d_state 16 / 32 / 64 ...) of every batch element.
     When that grid leaves most of the GPU empty, the sequence is cut into C chunks that run as B*C batch entries;
@@ -183,6 +199,19 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
             row = _row_bytes(tensors)
             if row == 16 or not (training or (row < 4 and L >= 900)):
                 return 1
+        # With the layer's sensors and output path inside, both forms take longer, the uncut one in its slowest warps and
+        # the cut one in the pass over the log-variances: the lines lie further out. Forward / training step in us, uncut
+        # and cut, bfloat16: 48 CTAs (B=2 M=768) L=640 59 / 236 and 55 / 274, L=720 65 / 240 and 54 / 270, L=1000 87 / 307
+        # and 72 / 272; 64 CTAs (B=1 M=2048) L=900 80 / 286 and 78 / 284, L=1000 87 / 311 and 83 / 270, L=4096 335 / 1180
+        # and 237 / 750; 80 CTAs (B=1 M=2560) L=1000 87 / 319 and 93 / 302, L=1500 127 / 463 and 130 / 418, L=2048 171 / 616
+        # and 158 / 503; 98 CTAs (B=1 M=3136) L=2048 172 / 626 and 189 / 614, L=4096 340 / 1221 and 341 / 1101. Above 32
+        # states the forward with the output path holds an SM alone, and only a nearly empty GPU has room for chunks: 16
+        # CTAs (S=64 B=1 M=128) L=1000 137 / 466 and 89 / 266, 48 CTAs (B=2 M=192) 139 / 470 and 190 / 413, L=4096 540 / 1879
+        # and 650 / 1681, 72 CTAs (B=1 M=576) 542 / 1911 and 885 / 2201.
+        if layer and lpc >= 16 and (lpc > 16 or ctas > 16):
+            return 1
+        if layer and L < (1000 if training or 48 < ctas <= 75 else 700 if ctas <= 48 else 2048 if ctas <= 84 else 8000):
+            return 1
         # Whole rounds of the resident slots: enough chunks for one, more rounds while chunks are longer than about 256
         # steps, which evens out the last one. Measured on B200, forward / training step in us: B=1 L=1536 M=1536
         # (48 CTAs) 3 chunks 79 / 233, 4 91 / 287, 6 69 / 208, 8 73 / 227, 16 74 / 235, uncut 108 / 380; B=1 L=8192 M=2048
@@ -220,6 +249,22 @@ def _as_chunks(t: Optional[torch.Tensor], C: int) -> Optional[torch.Tensor]:
     return t.as_strided((B * C, L // C, X), (t.stride(1) * (L // C), t.stride(1), t.stride(2)), t.storage_offset())
 
 
+def _scan_backward(ctx, v, lambda_v, k, q, a, p, lam0, eta0, ckpt, chunk_state, dy, dy_var, dlam_fin, deta_fin):
+    """The scan's gradients, cut into chunks where its forward was (``chunk_state``: their start states)."""
+    if (dlam_fin is None) != (deta_fin is None):
+        zero = torch.zeros((v.shape[0], v.shape[2], k.shape[2]), device=v.device, dtype=torch.float32)
+        dlam_fin = zero if dlam_fin is None else dlam_fin
+        deta_fin = zero if deta_fin is None else deta_fin
+    if dlam_fin is not None:
+        dlam_fin, deta_fin = dlam_fin.float().contiguous(), deta_fin.float().contiguous()
+    if ctx.chunks > 1:
+        return _lib.host().scan_bwd_chunked(
+            v, lambda_v, k, q, a, p, *chunk_state, ckpt, dy, dy_var, dlam_fin, deta_fin, ctx.prior,
+            ctx.out_dtype == torch.bfloat16, ctx.sensors, ctx.chunks, _chunk_len(v.shape[1], ctx.chunks))
+    return _launch_bwd(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin, ctx.prior, ctx.out_dtype,
+                       ctx.sensors)
+
+
 class _KLAScanB200(torch.autograd.Function):
     """Forward and exact backward of the fused scan, both as single kernels.
 
@@ -232,13 +277,10 @@ class _KLAScanB200(torch.autograd.Function):
                 chunks: int = 1):
         need_grad = any(ctx.needs_input_grad[:8])
         ctx.set_materialize_grads(False)  # an output without a gradient costs nothing below
-        C = chunks if sensors is None else 1
-        ctx.chunks = C
-        if C > 1:
-            # time-parallel: the chunks of every sequence run side by side from exact start states
-            y, y_var, lam_fin, eta_fin, ckpt, lam_in, eta_in = _lib.host().scan_fwd_chunked(
-                v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype == torch.bfloat16, need_grad, C,
-                _chunk_len(v.shape[1], C))
+        ctx.chunks = chunks
+        if chunks > 1:
+            y, y_var, lam_fin, eta_fin, ckpt, lam_in, eta_in = _launch_fwd_chunked(
+                v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, need_grad, chunks, sensors)
             ctx.save_for_backward(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, lam_in, eta_in)
         else:
             y, y_var, lam_fin, eta_fin, ckpt = _launch_fwd(
@@ -254,7 +296,6 @@ class _KLAScanB200(torch.autograd.Function):
     def backward(ctx, dy, dy_var, dlam_fin, deta_fin):
         v, lambda_v, k, q, a, p, lam0, eta0, ckpt, *chunk_state = ctx.saved_tensors
         B, L, M = v.shape
-        S = k.shape[2]
         dev = v.device
         od = ctx.out_dtype
 
@@ -269,21 +310,8 @@ class _KLAScanB200(torch.autograd.Function):
         dy_var = grad_in(dy_var)
         if dy is None:
             dy = torch.zeros((B, L, M), device=dev, dtype=od)
-        if (dlam_fin is None) != (deta_fin is None):
-            z = torch.zeros((B, M, S), device=dev, dtype=torch.float32)
-            dlam_fin = z if dlam_fin is None else dlam_fin
-            deta_fin = z if deta_fin is None else deta_fin
-        if dlam_fin is not None:
-            dlam_fin = dlam_fin.float().contiguous()
-            deta_fin = deta_fin.float().contiguous()
-        C = ctx.chunks
-        if C > 1:
-            dv, dlv, dk, dq, da, dp, dlam0, deta0 = _lib.host().scan_bwd_chunked(
-                v, lambda_v, k, q, a, p, *chunk_state, ckpt, dy, dy_var, dlam_fin, deta_fin, ctx.prior,
-                od == torch.bfloat16, C, _chunk_len(L, C))
-        else:
-            dv, dlv, dk, dq, da, dp, dlam0, deta0 = _launch_bwd(
-                v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin, ctx.prior, od, ctx.sensors)
+        dv, dlv, dk, dq, da, dp, dlam0, deta0 = _scan_backward(
+            ctx, v, lambda_v, k, q, a, p, lam0, eta0, ckpt, chunk_state, dy, dy_var, dlam_fin, deta_fin)
         if k.dtype != torch.float32:
             dk, dq = dk.to(k.dtype), dq.to(k.dtype)
         has_state = lam0 is not None
@@ -297,7 +325,7 @@ class _KLAScanEpilogueB200(torch.autograd.Function):
     adjoint (one memory-bound kernel) and then the scan's backward kernel."""
 
     @staticmethod
-    def forward(ctx, v, lambda_v, k, q, a, p, lam0, eta0, z, gate, skip, prior, out_dtype, sensors, gate_act):
+    def forward(ctx, v, lambda_v, k, q, a, p, lam0, eta0, z, gate, skip, prior, out_dtype, sensors, gate_act, chunks: int = 1):
         ctx.set_materialize_grads(False)
         need_grad = any(ctx.needs_input_grad[:11])
         B, L, M = v.shape
@@ -311,9 +339,15 @@ class _KLAScanEpilogueB200(torch.autograd.Function):
         raw = None
         if need_grad and gate is not None:
             raw = (torch.empty((B, L, M), device=v.device, dtype=out_dtype), torch.empty((B, L, M), device=v.device, dtype=out_dtype))
-        y, y_var, lam_fin, eta_fin, ckpt = _launch_fwd(v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, need_grad,
-                                                       sensors, epi, raw)
-        ctx.save_for_backward(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, z, gate, skip_flat, *(raw or ()))
+        chunk_state = (None, None)
+        if chunks > 1:
+            y, y_var, lam_fin, eta_fin, ckpt, *chunk_state = _launch_fwd_chunked(
+                v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, need_grad, chunks, sensors, epi, raw)
+        else:
+            y, y_var, lam_fin, eta_fin, ckpt = _launch_fwd(v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, need_grad,
+                                                           sensors, epi, raw)
+        ctx.save_for_backward(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, z, gate, skip_flat, *chunk_state, *(raw or ()))
+        ctx.chunks = chunks
         ctx.prior, ctx.sensors, ctx.out_dtype, ctx.gate_act = prior, sensors, out_dtype, gate_act
         ctx.skip_shape, ctx.skip_dtype = (None, None) if skip is None else (skip.shape, skip.dtype)
         return y, y_var, lam_fin, eta_fin
@@ -321,9 +355,8 @@ class _KLAScanEpilogueB200(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, dout, dout_var, dlam_fin, deta_fin):
-        v, lambda_v, k, q, a, p, lam0, eta0, ckpt, z, gate, skip_flat, *raw = ctx.saved_tensors
+        v, lambda_v, k, q, a, p, lam0, eta0, ckpt, z, gate, skip_flat, lam_in, eta_in, *raw = ctx.saved_tensors
         B, L, M = v.shape
-        S = k.shape[2]
         dev, od = v.device, ctx.out_dtype
 
         def grad_in(g):
@@ -334,19 +367,13 @@ class _KLAScanEpilogueB200(torch.autograd.Function):
             dout = torch.zeros((B, L, M), device=dev, dtype=od)
         dy, dy_var, dz, dgate, dskip = _lib.host().epilogue_bwd(
             v, od == torch.bfloat16, dout, dout_var, *(raw or (None, None)), z, gate, skip_flat, _lib.ACT[ctx.gate_act])
-        if (dlam_fin is None) != (deta_fin is None):
-            zero = torch.zeros((B, M, S), device=dev, dtype=torch.float32)
-            dlam_fin = zero if dlam_fin is None else dlam_fin
-            deta_fin = zero if deta_fin is None else deta_fin
-        if dlam_fin is not None:
-            dlam_fin, deta_fin = dlam_fin.float().contiguous(), deta_fin.float().contiguous()
-        dv, dlv, dk, dq, da, dp, dlam0, deta0 = _launch_bwd(
-            v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin, ctx.prior, od, ctx.sensors)
+        dv, dlv, dk, dq, da, dp, dlam0, deta0 = _scan_backward(
+            ctx, v, lambda_v, k, q, a, p, lam0, eta0, ckpt, (lam_in, eta_in), dy, dy_var, dlam_fin, deta_fin)
         if k.dtype != torch.float32:
             dk, dq = dk.to(k.dtype), dq.to(k.dtype)
         has_state = lam0 is not None
         return (dv, dlv, dk, dq, da, dp, dlam0 if has_state else None, deta0 if has_state else None,
-                dz, dgate, None if dskip is None else dskip.reshape(ctx.skip_shape).to(ctx.skip_dtype), None, None, None, None)
+                dz, dgate, None if dskip is None else dskip.reshape(ctx.skip_shape).to(ctx.skip_dtype), None, None, None, None, None)
 
 
 def kla_scan_b200(
@@ -465,15 +492,21 @@ def kla_scan_b200(
         gate_act = epi.get("gate_activation", "silu")
         if gate_act not in ("silu", "gelu", "relu"):
             raise ValueError("gate_activation must be 'silu', 'gelu' or 'relu'")
-        if not _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip):
+        training = _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip)
+        chunks = _chunks_of(v, lambda_v, k, q, time_chunks, training, True)
+        if not training:
             if skip is not None:
                 epi["lambda_skip"] = skip.float().reshape(-1).contiguous()
-            y, y_var, lam_fin, eta_fin, _ = _launch_fwd(
-                v, lambda_v, k, q, a, p, lam0, eta0, bool(decode_from_prior), out_dtype, False, log_variance, epi)
+            if chunks > 1:
+                y, y_var, lam_fin, eta_fin, *_ = _launch_fwd_chunked(
+                    v, lambda_v, k, q, a, p, lam0, eta0, bool(decode_from_prior), out_dtype, False, chunks, log_variance, epi)
+            else:
+                y, y_var, lam_fin, eta_fin, _ = _launch_fwd(
+                    v, lambda_v, k, q, a, p, lam0, eta0, bool(decode_from_prior), out_dtype, False, log_variance, epi)
             return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)
         y, y_var, lam_fin, eta_fin = _KLAScanEpilogueB200.apply(
             v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip, bool(decode_from_prior),
-            out_dtype, log_variance, gate_act)
+            out_dtype, log_variance, gate_act, chunks)
         return y, y_var, _state_cls()(lam=lam_fin, eta=eta_fin)
     return _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, decode_from_prior, out_dtype, log_variance, time_chunks)
 
@@ -494,19 +527,26 @@ def _check_log_variance(log_variance):
     return float(log_variance[0]), None if log_variance[1] is None else float(log_variance[1])
 
 
+def _chunks_of(v, lambda_v, k, q, time_chunks, training: bool, layer: bool) -> int:
+    """Time chunks of a call with canonical arguments."""
+    B, L, M = v.shape
+    if L == 0:
+        return 1
+    chunks = pick_time_chunks(B, L, M, k.shape[2], time_chunks, (v, lambda_v), training, layer)
+    if chunks > 1 and time_chunks is not None and not all(_chunkable(t, B, L) for t in (v, lambda_v, k, q)):
+        return 1  # an explicit count is taken for sequences that lie back to back
+    return chunks
+
+
 def _run_scan(v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype, log_variance, time_chunks):
     """The scan of canonical arguments, without an epilogue."""
     log_variance = _check_log_variance(log_variance)
-    B, L, M = v.shape
     training = _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0)
-    chunks = pick_time_chunks(B, L, M, k.shape[2], time_chunks, (v, lambda_v), training) if L > 0 and log_variance is None else 1
-    if chunks > 1 and time_chunks is not None and not all(_chunkable(t, B, L) for t in (v, lambda_v, k, q)):
-        chunks = 1  # an explicit count is taken for sequences that lie back to back
+    chunks = _chunks_of(v, lambda_v, k, q, time_chunks, training, log_variance is not None)
     if not training:  # inference: no autograd node, no checkpoints
         if chunks > 1:
-            y, y_var, lam_fin, eta_fin, *_ = _lib.host().scan_fwd_chunked(
-                v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype == torch.bfloat16, False, chunks,
-                _chunk_len(L, chunks))
+            y, y_var, lam_fin, eta_fin, *_ = _launch_fwd_chunked(
+                v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype, False, chunks, log_variance)
         else:
             y, y_var, lam_fin, eta_fin, _ = _launch_fwd(
                 v, lambda_v, k, q, a, p, lam0, eta0, bool(prior), out_dtype, False, log_variance)

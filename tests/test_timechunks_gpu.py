@@ -110,3 +110,51 @@ def test_views_that_cannot_be_chunked_fall_back(kb):
         y4, _, _ = kb.kla_scan_b200(v, *rest, time_chunks=4)
         y1, _, _ = kb.kla_scan_b200(v.contiguous(), *rest, time_chunks=1)
     assert torch.equal(y4, y1)
+
+
+@pytest.mark.parametrize("B,L,M,S,dtype,chunks,layer", [
+    (2, 256, 40, 16, torch.float32, 4, "sensors"),
+    (2, 256, 40, 16, torch.float32, 4, "output"),
+    (2, 256, 40, 16, torch.bfloat16, 2, "both"),
+    (1, 1001, 41, 5, torch.bfloat16, None, "both"),   # a shorter last chunk, rows that TMA cannot read, dead states
+    (3, 1030, 33, 64, torch.float32, None, "both"),  # few channels per CTA
+])
+@pytest.mark.parametrize("grad", [False, True])
+def test_scans_with_the_layers_sensors_and_output_path_in_chunks(kb, B, L, M, S, dtype, chunks, layer, grad):
+    """log_variance and epilogue with the time axis cut, against the same call uncut. Both lie within 1 and 2 of
+    1e-6 + 1e-5 |ref| of the float64 oracle, so outputs and state agree to 3e-5 of their largest value (times a gate of at
+    most 4 here: 1.2e-4), the gradients' sums to 1e-4, and bfloat16 results to one rounding (2^-8) as well."""
+    F = torch.nn.functional
+    g = torch.Generator().manual_seed(L + M)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    act = lambda t: t.cuda().to(dtype).requires_grad_(grad)
+    f32 = lambda t: t.cuda().requires_grad_(grad)
+    ins = [act(rn(B, L, M)), act(rn(B, L, M) if layer != "output" else 1 / F.softplus(rn(B, L, M))),
+           act(F.normalize(rn(B, L, S), dim=-1)), act(F.normalize(rn(B, L, S), dim=-1)),
+           f32(torch.sigmoid(rn(M, S))), f32(F.softplus(rn(M, S)))]
+    init = kb.KLAState(f32(F.softplus(rn(B, M, S)) + 0.5), f32(rn(B, M, S)))
+    kw = dict(out_dtype=dtype, initial_state=init)
+    leaves = [*ins, *init]
+    if layer != "output":
+        kw["log_variance"] = (1e-3, 2.0)
+    if layer != "sensors":
+        epi = dict(z=act(rn(B, L, M)), lambda_skip=f32(rn(M)), gate=act(rn(B, L, M)), gate_activation="silu")
+        kw["epilogue"] = epi
+        leaves += [epi["z"], epi["lambda_skip"], epi["gate"]]
+    ups = [rn(B, L, M).cuda().to(dtype), rn(B, L, M).cuda().to(dtype), rn(B, M, S).cuda(), rn(B, M, S).cuda()]
+    assert chunks is not None or ops.pick_time_chunks(B, L, M, S, None, tuple(ins[:2]), grad, True) > 1
+
+    def run(c):
+        before = ops._lib.load().kla_b200_launch_count()
+        y, y_var, st = kb.kla_scan_b200(*ins, time_chunks=c, **kw)
+        assert ops._lib.load().kla_b200_launch_count() - before == (1 if c == 1 else 3)
+        assert st.lam.is_contiguous() and st.eta.is_contiguous()  # what an in-place step asks for
+        outs = [y, y_var, st.lam, st.eta]
+        return outs, torch.autograd.grad(outs, leaves, ups) if grad else []
+
+    (o1, g1), (oc, gc) = run(1), run(chunks)
+    for x, y in zip(oc, o1):
+        y = y.detach()
+        assert rel_err(x.float(), y.double().cpu().numpy()) < 1.2e-4 + (2.0 ** -8 if y.dtype == torch.bfloat16 else 0.0)
+    for x, y in zip(gc, g1):
+        assert rel_err(x.float(), y.double().cpu().numpy()) < (1e-2 if y.dtype == torch.bfloat16 else 1e-4)
