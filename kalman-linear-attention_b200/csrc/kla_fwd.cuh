@@ -516,41 +516,48 @@ __global__ void __launch_bounds__((NW + NH) * 32, LPC > 16 || NH == 6 ? 1 : !EPI
                     const T *zs = prm.z.ptr ? zstage(e) : nullptr, *gs = prm.gate.ptr ? gstage(e) : nullptr;
                     TO *yr = prm.y_raw.ptr ? static_cast<TO *>(prm.y_raw.ptr) + (long long)b * prm.y_raw.sb + (long long)(t_off + t0) * prm.y_raw.st : nullptr;
                     TO *yvr = prm.y_raw.ptr ? static_cast<TO *>(prm.yv_raw.ptr) + (long long)b * prm.yv_raw.sb + (long long)(t_off + t0) * prm.yv_raw.st : nullptr;
-                    output_pass<TO, LPC, MC, MCP, TT, kDrainers>(
-                        ystage(o), yb + (long long)t0 * prm.y.st, prm.y.st, prm.vec_y,
-                        yvb + (long long)t0 * prm.yv.st, prm.yv.st, prm.vec_yv, min(TT, L - t0), m_cta, M, dtid,
-                        // (y, y_var) of two neighbouring channels; z, gate and the raw outputs move as pairs (B=16 L=2048 M=1536
-                        // bfloat16 in training 822 -> 796 us)
-                        [&](float2 &y0, float2 &y1, int tt, int c, bool both) {
-                            if (yr != nullptr) {  // the scan's own outputs, for the epilogue's adjoint
-                                TO *pr = yr + (long long)tt * prm.y_raw.st + m_cta + c, *pvr = yvr + (long long)tt * prm.yv_raw.st + m_cta + c;
-                                if (both && prm.vec_raw) {
-                                    store_pair(pr, y0.x, y1.x);
-                                    store_pair(pvr, y0.y, y1.y);
-                                } else {
-                                    pr[0] = from_f32<TO>(y0.x);
-                                    pvr[0] = from_f32<TO>(y0.y);
-                                    if (both) {
-                                        pr[1] = from_f32<TO>(y1.x);
-                                        pvr[1] = from_f32<TO>(y1.y);
+                    // One pass per kind of gate, chosen once a tile: with the choice inside, around GELU's code, the bodies of a
+                    // thread's pairs could not overlap (bfloat16 with sensors: B=4 L=1500 M=1152 136 -> 122 us, as without a
+                    // gate; B=2 L=8192 M=2048 663 -> 631; the layer's training step at B=16 L=2048 M=1536 3313 -> 3262).
+                    auto pass = [&](auto act) {
+                        output_pass<TO, LPC, MC, MCP, TT, kDrainers>(
+                            ystage(o), yb + (long long)t0 * prm.y.st, prm.y.st, prm.vec_y,
+                            yvb + (long long)t0 * prm.yv.st, prm.yv.st, prm.vec_yv, min(TT, L - t0), m_cta, M, dtid,
+                            // (y, y_var) of two neighbouring channels; z, gate and the raw outputs move as pairs (B=16 L=2048 M=1536
+                            // bfloat16 in training 822 -> 796 us)
+                            [&](float2 &y0, float2 &y1, int tt, int c, bool both) {
+                                if (yr != nullptr) {  // the scan's own outputs, for the epilogue's adjoint
+                                    TO *pr = yr + (long long)tt * prm.y_raw.st + m_cta + c, *pvr = yvr + (long long)tt * prm.yv_raw.st + m_cta + c;
+                                    if (both && prm.vec_raw) {
+                                        store_pair(pr, y0.x, y1.x);
+                                        store_pair(pvr, y0.y, y1.y);
+                                    } else {
+                                        pr[0] = from_f32<TO>(y0.x);
+                                        pvr[0] = from_f32<TO>(y0.y);
+                                        if (both) {
+                                            pr[1] = from_f32<TO>(y1.x);
+                                            pvr[1] = from_f32<TO>(y1.y);
+                                        }
                                     }
                                 }
-                            }
-                            // a drainer thread meets the same pair of channels in every tile: its skip values are in registers
-                            if (zs != nullptr) {
-                                const float2 z = load_pair(zs + tt * MC + c);
-                                y0.x = fmaf(skip0, z.x, y0.x);
-                                y1.x = fmaf(skip1, z.y, y1.x);
-                            }
-                            if (gs != nullptr) {
-                                const float2 gp = load_pair(gs + tt * MC + c);
-                                const float g0 = activate_fast(gp.x, prm.gate_act), g1 = activate_fast(gp.y, prm.gate_act);
-                                y0.x *= g0;
-                                y0.y *= g0 * g0;
-                                y1.x *= g1;
-                                y1.y *= g1 * g1;
-                            }
-                        });
+                                // a drainer thread meets the same pair of channels in every tile: its skip values are in registers
+                                if (zs != nullptr) {
+                                    const float2 z = load_pair(zs + tt * MC + c);
+                                    y0.x = fmaf(skip0, z.x, y0.x);
+                                    y1.x = fmaf(skip1, z.y, y1.x);
+                                }
+                                if (gs != nullptr) {
+                                    const float2 gp = load_pair(gs + tt * MC + c);
+                                    const float g0 = act(gp.x), g1 = act(gp.y);
+                                    y0.x *= g0;
+                                    y0.y *= g0 * g0;
+                                    y1.x *= g1;
+                                    y1.y *= g1 * g1;
+                                }
+                            });
+                    };
+                    if (prm.gate_act == kActSilu) pass([](float x) { return activate_fast(x, kActSilu); });
+                    else pass([&](float x) { return activate_fast(x, prm.gate_act); });
                     __syncwarp();
                     if (hlane == 0) mbar_arrive(&epi_empty[e]);
                 } else {
