@@ -199,18 +199,19 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
             row = _row_bytes(tensors)
             if row == 16 or not (training or (row < 4 and L >= 900)):
                 return 1
-        # With the layer's sensors and output path inside, both forms take longer, the uncut one in its slowest warps and
-        # the cut one in the pass over the log-variances: the lines lie further out. Forward / training step in us, uncut
-        # and cut, bfloat16: 48 CTAs (B=2 M=768) L=640 59 / 236 and 55 / 274, L=720 65 / 240 and 54 / 270, L=1000 87 / 307
-        # and 72 / 272; 64 CTAs (B=1 M=2048) L=900 80 / 286 and 78 / 284, L=1000 87 / 311 and 83 / 270, L=4096 335 / 1180
-        # and 237 / 750; 80 CTAs (B=1 M=2560) L=1000 87 / 319 and 93 / 302, L=1500 127 / 463 and 130 / 418, L=2048 171 / 616
-        # and 158 / 503; 98 CTAs (B=1 M=3136) L=2048 172 / 626 and 189 / 614, L=4096 340 / 1221 and 341 / 1101. Above 32
+        # With the layer's sensors and output path inside, the call stands in a layer, whose host takes longer than a short
+        # scan: cutting adds launches and has to shorten what the GPU does beyond that. Whole prompts of one layer in us,
+        # uncut and cut, bfloat16: B=1 d_model=512 L=1000 162 and 170, L=1500 172 and 169, L=2048 215 and 169; training steps
+        # between the projections, B=1 M=1024 L=1000 727 and 770, L=2048 775 and 780, L=2400 875 and 765. By the GPU alone
+        # (forward / training step, bfloat16): 48 CTAs (B=2 M=768) L=1000 87 / 307 and 72 / 272; 64 CTAs (B=1 M=2048) L=1000
+        # 87 / 311 and 83 / 270, L=4096 335 / 1180 and 237 / 750; 80 CTAs (B=1 M=2560) L=1500 127 / 463 and 130 / 418, L=2048
+        # 171 / 616 and 158 / 503; 98 CTAs (B=1 M=3136) L=4096 340 / 1221 and 341 / 1101. Above 32
         # states the forward with the output path holds an SM alone, and only a nearly empty GPU has room for chunks: 16
         # CTAs (S=64 B=1 M=128) L=1000 137 / 466 and 89 / 266, 48 CTAs (B=2 M=192) 139 / 470 and 190 / 413, L=4096 540 / 1879
         # and 650 / 1681, 72 CTAs (B=1 M=576) 542 / 1911 and 885 / 2201.
         if layer and lpc >= 16 and (lpc > 16 or ctas > 16):
             return 1
-        if layer and L < (1000 if training or 48 < ctas <= 75 else 700 if ctas <= 48 else 2048 if ctas <= 84 else 8000):
+        if layer and L < (2400 if training else 1600 if ctas <= 75 else 2048 if ctas <= 84 else 8000):
             return 1
         # Whole rounds of the resident slots: enough chunks for one, more rounds while chunks are longer than about 256
         # steps, which evens out the last one. Measured on B200, forward / training step in us: B=1 L=1536 M=1536

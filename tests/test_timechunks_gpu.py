@@ -116,8 +116,8 @@ def test_views_that_cannot_be_chunked_fall_back(kb):
     (2, 256, 40, 16, torch.float32, 4, "sensors"),
     (2, 256, 40, 16, torch.float32, 4, "output"),
     (2, 256, 40, 16, torch.bfloat16, 2, "both"),
-    (1, 1001, 41, 5, torch.bfloat16, None, "both"),   # a shorter last chunk, rows that TMA cannot read, dead states
-    (3, 1030, 33, 64, torch.float32, None, "both"),  # few channels per CTA
+    (1, 2401, 41, 5, torch.bfloat16, None, "both"),   # a shorter last chunk, rows that TMA cannot read, dead states
+    (3, 2410, 33, 64, torch.float32, None, "both"),  # few channels per CTA
 ])
 @pytest.mark.parametrize("grad", [False, True])
 def test_scans_with_the_layers_sensors_and_output_path_in_chunks(kb, B, L, M, S, dtype, chunks, layer, grad):
