@@ -16,6 +16,7 @@ can; nothing falls back silently, and there is no CPU or Triton path.
 
 from __future__ import annotations
 
+import os
 import sys
 from typing import NamedTuple, Optional
 
@@ -98,14 +99,6 @@ def _forward_segments(lib, dev: torch.device, B: int, L: int, M: int, S: int) ->
     return lib.kla_b200_plan_segments(B * ((M + per_cta - 1) // per_cta), L, 0, _SM_COUNT[idx], -1, None) > 1
 
 
-def _epilogue_args(epilogue, raw):
-    """z, lambda_skip, gate, its activation and the buffers of the scan's own outputs, as the host module takes them."""
-    epi = epilogue or {}
-    gate = epi.get("gate")
-    return (epi.get("z"), epi.get("lambda_skip"), gate,
-            0 if gate is None else _lib.ACT[epi.get("gate_activation", "silu")], *(raw or (None, None)))
-
-
 def _launch_fwd(v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype, need_ckpt: bool, sensors=None,
                 epilogue=None, raw=None):
     """Allocate outputs (and the checkpoint scratch when a backward will follow)
@@ -113,18 +106,24 @@ def _launch_fwd(v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype, nee
     # without checkpoints the kernel still hands long lists of sequences from CTA to CTA in segments, given a little
     # working memory
     segments = not need_ckpt and _forward_segments(_lib.load(), v.device, v.shape[0], v.shape[1], v.shape[2], k.shape[2])
+    epi = epilogue or {}
+    gate = epi.get("gate")
     return _lib.host().scan_fwd(
         v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype == torch.bfloat16, need_ckpt, segments, sensors,
-        *_epilogue_args(epilogue, raw), 1, 0)
+        epi.get("z"), epi.get("lambda_skip"), gate, 0 if gate is None else _lib.ACT[epi.get("gate_activation", "silu")],
+        *(raw or (None, None)), 1, 0)
 
 
 def _launch_fwd_chunked(v, lambda_v, k, q, a, p, lam0, eta0, prior: bool, out_dtype, need_ckpt: bool, chunks: int, sensors=None,
                         epilogue=None, raw=None):
     """:func:`_launch_fwd` with the chunks of every sequence running side by side from exact start states, which are
     returned as well."""
+    epi = epilogue or {}
+    gate = epi.get("gate")
     return _lib.host().scan_fwd_chunked(
         v, lambda_v, k, q, a, p, lam0, eta0, prior, out_dtype == torch.bfloat16, need_ckpt, sensors,
-        *_epilogue_args(epilogue, raw), chunks, _chunk_len(v.shape[1], chunks))
+        epi.get("z"), epi.get("lambda_skip"), gate, 0 if gate is None else _lib.ACT[epi.get("gate_activation", "silu")],
+        *(raw or (None, None)), chunks, _chunk_len(v.shape[1], chunks))
 
 
 def _launch_bwd(v, lambda_v, k, q, a, p, lam0, eta0, ckpt, dy, dy_var, dlam_fin, deta_fin,
@@ -144,6 +143,7 @@ def slab_aggregate(v, lambda_v, k, a, p, *, q=None, dy=None, dy_var=None, lam0=N
 # CTAs the backward kernel keeps resident on a B200: 148 SMs x 2
 _RESIDENT_CTAS = 296
 _MIN_CHUNK_STEPS = 64
+_LAYER_CHUNKS_FROM = 1600  # steps from which scans with the layer's sensors or output path can be cut (pick_time_chunks)
 
 
 def _chunkable(t: Optional[torch.Tensor], B: int, L: int) -> bool:
@@ -173,9 +173,8 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
     building the chunks' start states costs about 0.7x of a forward + backward pass on top, so chunking is only
     chosen when the plain grid fills less than a third of the resident CTA slots; then up to 16 chunks. Chunks keep at least 64 steps and are equally long where the count divides L, else
     a multiple of 16 steps with a shorter last one (:func:`_chunk_len`). ``requested`` (or the environment variable
-    KLA_B200_TIME_CHUNKS) overrides the choice; it is lowered to the nearest usable divisor of L."""
-    import os
-
+    KLA_B200_TIME_CHUNKS, not looked at where an output path is applied to fewer than 1600 steps) overrides the choice; it is
+    lowered to the nearest usable divisor of L."""
     if requested is None and os.environ.get("KLA_B200_TIME_CHUNKS"):
         requested = int(os.environ["KLA_B200_TIME_CHUNKS"])
     lpc = 1
@@ -211,7 +210,7 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
         # and 650 / 1681, 72 CTAs (B=1 M=576) 542 / 1911 and 885 / 2201.
         if layer and lpc >= 16 and (lpc > 16 or ctas > 16):
             return 1
-        if layer and L < (2400 if training else 1600 if ctas <= 75 else 2048 if ctas <= 84 else 8000):
+        if layer and L < (2400 if training else _LAYER_CHUNKS_FROM if ctas <= 75 else 2048 if ctas <= 84 else 8000):
             return 1
         # Whole rounds of the resident slots: enough chunks for one, more rounds while chunks are longer than about 256
         # steps, which evens out the last one. Measured on B200, forward / training step in us: B=1 L=1536 M=1536
@@ -494,7 +493,8 @@ def kla_scan_b200(
         if gate_act not in ("silu", "gelu", "relu"):
             raise ValueError("gate_activation must be 'silu', 'gelu' or 'relu'")
         training = _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip)
-        chunks = _chunks_of(v, lambda_v, k, q, time_chunks, training, True)
+        # short prompts are bound by the host: not even the rule is asked for them (3 of 160 us)
+        chunks = 1 if L < _LAYER_CHUNKS_FROM and time_chunks is None else _chunks_of(v, lambda_v, k, q, time_chunks, training, True)
         if not training:
             if skip is not None:
                 epi["lambda_skip"] = skip.float().reshape(-1).contiguous()
