@@ -31,8 +31,12 @@
 //   true initial state, i.e. it runs after the forward fold. With a2 = a^2 and
 //   r - phi mean_t = g (r - phi a mean_{t-1}) the diagonal is one product,
 //   K00 = K11^2, and K01 = K11 R with R' = R + K11' (r - phi a mean): 19 pair
-//   operations a step instead of 25. (a2's floor of 1e-12, which binds where
-//   |a| < 1e-6, is left out of K00: 1e-12 of the carry at the most.)
+//   operations a step instead of 25.
+//
+// Both forms take a2 for a^2, which it is but for its floor of 1e-12, binding where |a| < 1e-6. A chain that the floor binds
+// forgets what came before within a few steps, 1e-6 a step at least, so the floor shows in the records of stretches of a few steps
+// and in the first terms of b0. Stretches of up to kAggFloorSteps steps are composed with it by kla_agg_short_kernel (forward),
+// and the adjoint walks that many steps of such a chain once more.
 //
 // Both walks keep -a, -a2 and -p as their constants and -Pp, -1/d as they go:
 // every product then has the sign the next sum needs, since a pair instruction
@@ -52,6 +56,7 @@ namespace kla {
 
 constexpr int kAggStages = 3;
 constexpr int kAggTT = 32;  // steps per tile
+constexpr int kAggFloorSteps = 8;  // after which 1e-6 a step leaves less than float32 holds
 
 struct alignas(64) AggParams {
     CUtensorMap tm_v, tm_lv, tm_dy, tm_dyv;  // rank-3 (M, L, B) maps with box (MC, kAggTT, 1); valid when use_tma
@@ -80,6 +85,72 @@ struct AggSmem {
     static constexpr size_t kTotal = kBars + kAggStages * kIn;
     static constexpr size_t kLam = sizeof(float) * kAggTT * kMC;
 };
+
+// The first steps of a stretch of L steps from t_off on, one chain, with the floor of a2: the adjoint's five sums, which with the
+// run from (0, 0) are also how the forward's posterior depends on P0 and m0 (K00 in place of A^2, K01 in place of A eta). Writes
+// the record of a stretch that these are all steps of, or adds to the adjoint's b0 what the form without the floor left out.
+template <typename T, typename TO, bool ADJ, bool PRIOR, bool LOGV>
+__device__ __forceinline__ void walk_with_floor(const AggParams &prm, int be, int b, int t_off, int L, int m, int s, float a) {
+    const long long ms = (long long)m * prm.S + s, at = (long long)be * prm.M * prm.S + ms;
+    const float a2 = fmaxf(a * a, kEps), p = fmaxf(prm.p[ms], kPMin);
+    float P = 0.0f, mean = 0.0f;
+    if (ADJ) {
+        P = prm.lam0 != nullptr ? 1.0f / fmaxf(prm.lam0[at], kLamMin) : 1.0f;
+        if (prm.lam0 != nullptr) mean = prm.eta0[at] * P;
+    }
+    float K00 = 1.0f, K01 = 0.0f, K11 = 1.0f, R = 0.0f, J = 0.0f, b0 = 0.0f, b1 = 0.0f, missed = 0.0f;
+    const int n = min(L, kAggFloorSteps);
+#pragma unroll 1
+    for (int tt = 0; tt < n; ++tt) {
+        auto load = [&](const Tensor3 &x, int column) { return (long long)b * x.sb + (long long)(t_off + tt) * x.st + column; };
+        float lv = to_f32<T>(static_cast<const T *>(prm.lv.ptr)[load(prm.lv, m)]);
+        if (LOGV) lv = precision_from_log_variance_fast(lv, prm.obs_var_min, prm.obs_var_max);
+        const float v = to_f32<T>(static_cast<const T *>(prm.v.ptr)[load(prm.v, m)]), k = to_f32<T>(static_cast<const T *>(prm.k.ptr)[load(prm.k, s)]);
+        const float phi = lv * k * k, r = v * (lv * k);
+        const float Pp = fmaf(a2, P, p), g = 1.0f / fmaf(phi, Pp, 1.0f), t = fmaf(-phi, a * mean, r);
+        J = fmaf(phi * a2, K00 * g, J);
+        K00 *= a2 * g * g;
+        K01 = fmaf(K00, t, K01 * (a * g));
+        K11 *= a * g;
+        P = Pp * g;
+        mean = g * fmaf(Pp, r, a * mean);
+        if constexpr (ADJ) {
+            const float q = to_f32<T>(static_cast<const T *>(prm.q.ptr)[load(prm.q, s)]);
+            float e0 = 0.0f, e1 = to_f32<TO>(static_cast<const TO *>(prm.dy.ptr)[load(prm.dy, m)]) * q;
+            if (prm.dyv.ptr != nullptr) e0 = to_f32<TO>(static_cast<const TO *>(prm.dyv.ptr)[load(prm.dyv, m)]) * q * q;
+            if (PRIOR) e1 *= a;
+            R = fmaf(K11, t, R);
+            b0 += K00 * (PRIOR ? a2 : 1.0f) * e0 + K01 * e1;
+            b1 = fmaf(K11, e1, b1);
+            missed += (K00 * (PRIOR ? a2 : 1.0f) - K11 * K11 * (PRIOR ? a * a : 1.0f)) * e0 + (K01 - K11 * R) * e1;
+        }
+    }
+    float4 *o = reinterpret_cast<float4 *>(prm.out + at * 8);
+    if constexpr (ADJ) {
+        if (L > n) {
+            prm.out[at * 8 + 3] += missed;
+            return;
+        }
+        o[0] = make_float4(K00, K01, K11, b0);
+        o[1] = make_float4(b1, P, mean, 0.0f);
+    } else {
+        const float sc = 1.0f / (1.0f + J);
+        o[0] = make_float4(sc, J * sc, P * sc, fmaf(P, J, K00) * sc);
+        o[1] = make_float4(mean * sc, fmaf(mean, J, K01) * sc, K11 * sc, 0.0f);
+    }
+}
+
+// Forward records of stretches of up to kAggFloorSteps steps, a thread per chain.
+template <typename T, bool LOGV>
+__global__ void __launch_bounds__(128) kla_agg_short_kernel(const __grid_constant__ AggParams prm) {
+    const long long lanes = (long long)prm.M * prm.S, gid = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (gid >= prm.B * lanes) return;
+    const int be = (int)(gid / lanes);
+    const long long ms = gid % lanes;
+    const ChunkSpan span = chunk_span(prm.chunk, be, prm.L);
+    if (prm.chunk.n > 1 && be % prm.chunk.n == prm.chunk.n - 1) return;  // as kla_agg_kernel
+    walk_with_floor<T, float, false, false, LOGV>(prm, be, span.b, span.t_off, span.L, (int)(ms / prm.S), (int)(ms % prm.S), prm.a[ms]);
+}
 
 // LOGV (AggParams::lv_log_sigma) is a separate instantiation: a test in every step cost plain inference at B=1 L=1501
 // M=1536 float32 2 of its 64 us.
@@ -251,6 +322,18 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
                     o[0] = make_float4(x[0] * x[0], x[0] * x[1], x[0], x[2]);
                     o[1] = make_float4(x[3], x[4], x[5], 0.0f);
                 }
+            }
+        }
+        // Chains that the floor of a2 binds. Here, from global memory, the walk costs the loop above no registers (inside it, or
+        // as a call, up to 32).
+        if constexpr (ADJ) {
+#pragma unroll 1
+            for (int i = 0; i < SPT; ++i) {
+                const int s = i * LPC + j;
+                if (m >= M || s >= S) break;
+                const long long ms = (long long)m * S + s;
+                const float a = prm.a[ms];
+                if (a * a < kEps) walk_with_floor<T, TO, ADJ, PRIOR, LOGV>(prm, be, b, t_off, L, m, s, a);
             }
         }
     } else {

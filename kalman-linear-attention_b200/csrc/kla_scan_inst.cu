@@ -75,6 +75,12 @@ cudaError_t launch_agg(const AggParams &prm, bool adjoint, cudaStream_t st) {
         return prm.lv_log_sigma ? go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, true, PRIOR, true>, Sm::kTotal + Sm::kLam)
                                 : go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, true, PRIOR, false>, Sm::kTotal);
     }
+    if ((prm.chunk.n > 1 ? prm.chunk.len : prm.L) <= kAggFloorSteps) {
+        const unsigned ctas = (unsigned)(((long long)prm.B * prm.M * prm.S + 127) / 128);
+        if (prm.lv_log_sigma) kla_agg_short_kernel<T, true><<<ctas, 128, 0, st>>>(prm);
+        else kla_agg_short_kernel<T, false><<<ctas, 128, 0, st>>>(prm);
+        return cudaGetLastError();
+    }
     using Sm = AggSmem<T, TO, kSPT, LPC, kNW, false>;
     return prm.lv_log_sigma ? go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, false, false, true>, Sm::kTotal + Sm::kLam)
                             : go(kla_agg_kernel<T, TO, kSPT, LPC, kNW, false, false, false>, Sm::kTotal);

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 import torch
 
+import slab_math
 from oracle import kla_oracle as O
 from test_scan_gpu import INPUTS, REDUCED_SLACK, _oracle, _seeded, ratio, rel_err
 
@@ -110,6 +111,51 @@ def test_views_that_cannot_be_chunked_fall_back(kb):
         y4, _, _ = kb.kla_scan_b200(v, *rest, time_chunks=4)
         y1, _, _ = kb.kla_scan_b200(v.contiguous(), *rest, time_chunks=1)
     assert torch.equal(y4, y1)
+
+
+@pytest.mark.parametrize("prior", [False, True])
+@pytest.mark.parametrize("L", [1, 2, 8, 9, 70])
+def test_aggregates_keep_the_floor_of_a_squared(kb, L, prior):
+    """|a| < 1e-6: a^2 is 1e-12 there, and that is all a chain without process noise keeps of what came before. Held to 1e-5 of the
+    float64 restatement's values, chain by chain (a few float32 operations, no cancellation but in b0's sum)."""
+    g = _seeded(2, L, 5, 12, seed=27)
+    g["a"].reshape(-1)[::2] = np.resize([0.0, 1e-9, -5e-7, 0.9999e-6], 30)
+    g["p"].reshape(-1)[::4] = 0.0
+    dev = {n: torch.tensor(g[n], dtype=torch.float32, device="cuda") for n in (*INPUTS, "dy", "dyvar", "lam0", "eta0")}
+    g = {n: t.double().cpu().numpy() for n, t in dev.items()}
+    v, lv, k, q, a, p = (dev[n] for n in INPUTS)
+    low = np.broadcast_to(np.abs(g["a"]) < 1e-6, (2, 5, 12))
+    fa = ops.slab_aggregate(v, lv, k, a, p).double().cpu().numpy()
+    ref = slab_math.forward_aggregate(*[g[n] for n in ("v", "lambda_v", "k", "a", "p")])
+
+    def apply(A, P0, m0):
+        x = A[..., 0] + A[..., 1] * P0
+        return (A[..., 2] + A[..., 3] * P0) / x, (A[..., 4] + A[..., 5] * P0 + A[..., 6] * m0) / x
+
+    for P0, m0 in ((1.0, 0.0), (1e3, -0.7)):
+        for got, want in zip(apply(fa, P0, m0), apply(ref, P0, m0)):
+            assert np.all(np.abs(got - want)[low] <= 1e-5 * np.abs(want)[low] + 1e-30)
+    aa = ops.slab_aggregate(v, lv, k, a, p, q=q, dy=dev["dy"], dy_var=dev["dyvar"], lam0=dev["lam0"], eta0=dev["eta0"], prior=prior)
+    aa = aa.double().cpu().numpy()
+    ref = slab_math.adjoint_aggregate(*[g[n] for n in INPUTS], g["dy"], g["dyvar"], g["lam0"], g["eta0"], prior)
+    for i in (0, 2, 3, 4, 5, 6):  # (K01 is a difference of two numbers; its share is in b0)
+        scale = np.abs(ref[..., i]) if i != 3 else np.abs(ref[..., 3]) + np.abs(ref[..., 0]) + 1e-14
+        assert np.all(np.abs(aa[..., i] - ref[..., i])[low] <= 2e-5 * scale[low] + 1e-37), i
+
+
+def test_gradients_through_the_floor_of_a_squared_cross_a_cut(kb):
+    """a = 0, and only the steps behind the cut are read: what the steps in front of it get comes through the floor alone. The uncut
+    kernels form it without cancellation: equal to 1e-5. The oracle, in information form, takes it as the difference of two numbers
+    of order one: 2.2e-16 of them is 2.2e-4 of 1e-12, so 1e-3."""
+    g = _seeded(2, 128, 16, 16, seed=28)
+    g["a"][:] = 0.0
+    g["dy"][:, :64] = g["dyvar"][:, :64] = 0.0
+    _, b = _oracle(g)
+    cut, uncut = (_run(kb, g, c)[3] for c in (2, 1))
+    for i, want in ((1, b.dlambda_v), (2, b.dk)):
+        got, plain, want = cut[i].double().cpu().numpy()[:, 63], uncut[i].double().cpu().numpy()[:, 63], want[:, 63]
+        assert 0 < np.abs(want).max() < 1e-9
+        assert np.linalg.norm(got - plain) <= 1e-5 * np.linalg.norm(plain) and np.linalg.norm(got - want) <= 1e-3 * np.linalg.norm(want)
 
 
 @pytest.mark.parametrize("B,L,M,S,dtype,chunks,layer", [
