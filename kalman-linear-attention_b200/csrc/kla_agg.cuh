@@ -325,7 +325,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) kla_agg_kernel(const __grid_con
             }
         }
         // Chains that the floor of a2 binds. Here, from global memory, the walk costs the loop above no registers (inside it, or
-        // as a call, up to 32); reading a again to find them cost 1.6 of the 197 us of a training step at B=2 L=1024 M=1024.
+        // as a call, up to 32), and where there are none, nothing: 33.7 us at B=2 L=1024 M=1024 float32 in 4 chunks, 34.0 without.
         if constexpr (ADJ) {
             unsigned floored = 0;
 #pragma unroll
