@@ -222,14 +222,16 @@ class _TokenGraph:
         return logits
 
     def reset(self):
-        """The prior state, ordered behind whatever used the buffers last. They are memory of the stream that captured the
-        step: another stream that uses them says so to the allocator."""
+        """The prior state, ordered behind whatever used the buffers last. They are memory of the stream whose call made the
+        step, the kernel's working memory of the side stream that captured it: a stream that uses them says so to the allocator."""
         stream = torch.cuda.current_stream(self.token.device)
         if self.done is not None:
             stream.wait_event(self.done)
         if stream != self.stream:
-            for t in (self.token, *self.work, *(t for layer in self.state for t in layer if t is not None)):
+            for t in (self.token, *(t for layer in self.state for t in layer if t is not None)):
                 t.record_stream(stream)
+        for t in self.work:  # of the stream it was captured on
+            t.record_stream(stream)
         for conv, lam, eta in self.state:
             if conv is not None:
                 conv.zero_()

@@ -181,3 +181,27 @@ def test_a_wait_for_words_that_never_come_runs_out_and_is_reported():
     finally:
         L.kla_b200_test_hooks(0, -1)
     assert torch.equal(dec._step_blocks(x, dec.init_state(2, "cuda", torch.bfloat16)), want) and lib.device_status() == 0
+
+
+def test_a_captured_tokens_working_memory_is_kept_until_its_replays_are_done():
+    """It was allocated on the side stream of the capture and is used on the caller's: a graph that is dropped with its replays
+    still to run must not give it to what that side stream allocates next (streams come from a pool of 32)."""
+    decode = import_module("kalman-linear-attention_b200.decode")
+    dec = stack(64, 128, 16, 2, 176, {}, False)
+    graph = decode._TokenGraph(dec, 2, torch.device("cuda", torch.cuda.current_device()), torch.bfloat16, True)
+    (work,) = graph.work
+    at, size = work.data_ptr(), work.numel()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # 0.1 s
+    graph.reset()
+    graph.graph.replay()
+    graph.release()
+    still = graph.done
+    del graph, work
+    taken = []
+    for _ in range(40):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            taken += [torch.empty(size, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    assert not still.query()  # the replay has it all to do
+    assert all(not t.data_ptr() <= at < t.data_ptr() + size for t in taken)
+    torch.cuda.synchronize()
