@@ -438,16 +438,36 @@ bool few_rows(const Tensor &x, const Tensor &w, const OptTensor &bias, const Opt
 //    89 M  32 rows 1024 x 2720 9.0 / 8.2                   101 M  32 rows 4096 x 768 16.3 / 15.9
 //   144 M  17 rows 4128 x 2048 7.6 / 6.4                   134 M  32 rows 4096 x 1024 12.5 / 9.9
 bool kernel_pays(int64_t rows, int64_t N, int64_t K) { return rows <= 16 || rows * N * K <= 80'000'000; }
-// Rows up to which a token is one kernel. Blocks of a model, in a graph, us, one kernel / separate ones: 12 layers d_model 768
-// 8 rows 270 / 328, 1 row 248 / 264, d_model 128 8 rows 199 / 211, d_model 1024 4 rows 314 / 354; 4 layers d_model 2048 8 rows
-// 244 / 256. (Two groups of eight rows, as the kernel was tried: 12 layers d_model 768 16 rows 377 / 371.)
+// Rows up to which a token can be one kernel. (Two groups of eight rows, as the kernel was tried: 12 layers d_model 768 16 rows
+// 377 us against 371 of the separate kernels.)
 constexpr int64_t kTokenRows = KLA_B200_TOKEN_MAX_ROWS;
+// Whether that is the faster way for a block, issued from a graph: time of the separate kernels over that of the one, M = 2 d_model,
+// swiglu of 8/3 d_model (without an MLP), W from HBM; d_model 128 to 4096, 8 to 128 states, 1, 2, 4, 6 and 8 rows.
+// * The filter's units (32 / lanes channels of a row) are dealt one to a warp, and a second round of them costs more from state to
+//   state. One round: 1.05 to 1.25 from two rows on, at all sizes; two rounds or more: 16 states 1.02 to 1.23 (0.98 to 1.25), 32 states
+//   1.00 to 1.06 up to d_model 1536, 1.00 at 2048 and 8 rows (0.95), 64 states 0.93 to 1.06, 128 states 0.85 to 1.08.
+// * One row: up to d_model 384 1.06 to 1.15; beyond, with 32768 states a row or fewer, 1.02 to 1.14 up to d_model 768, 0.98 at 1024
+//   (1.07), with more 0.90 to 1.01; d_model 1280 and 1536 0.95 and 1.01 with any; from 2048 on 1.06.
+// * Wide projections are slow as kernels of their own: d_model 2560 with its MLP and 3072 1.05 to 1.40 up to 4 M states in all, 0.95
+//   to 1.06 with more. Past 6144 channels x leaves W two stages of the ring: d_model 4096 0.81 to 1.00.
+// What the rule takes gains 0.97 to 1.40 with an MLP; without one the same but for three points of few and full CTAs of filter units (32
+// states d_model 384 and 640 2 rows, 64 states 384 1 row: 0.87 to 0.94).
+bool token_pays(int64_t rows, int64_t M, int64_t S, int64_t widest, int64_t sms) {
+    if (M > 6144) return false;
+    if (widest >= 12288) return rows * M * S <= 4'000'000;
+    if (rows == 1 && M > 768 && (M <= 2048 ? M * S > 32768 : M < 4096)) return false;
+    int64_t lanes = 1;
+    while (4 * lanes < S) lanes *= 2;
+    const int64_t channels = 32 / lanes, units = rows * ((M + channels - 1) / channels);
+    return units <= 16 * sms || (S <= 32 && rows * M * S <= 800'000);
+}
 // A lone layer's token is one kernel only where it is issued call by call, four launches costing the host 21 us whatever the
 // sizes, and where the kernel takes less than that. us, one kernel / separate ones, eager: 8 rows d_model 256 14.4 / 20.6, 768
 // 17.9 / 20.2, 1024 18.7 / 20.7, 2048 40.8 / 39.6; with 32 states 768 21.0 / 21.9, 1024 22.6 / 20.7. Captured, where the kernel's
 // working memory is cleared with every replay, the separate ones win: 8 rows d_model 256 16.4 / 14.3, 1024 20.5 / 19.8.
+bool few_weights(int64_t d, int64_t M, int64_t S) { return 3 * M * d + 2 * M * (M + S) <= 16'000'000; }
 bool lone_token_pays(int64_t B, int64_t d, int64_t M, int64_t S) {
-    return 3 * M * d + 2 * M * (M + S) <= 16'000'000 && B * M * S <= 400'000 &&
+    return few_weights(d, M, S) && B * M * S <= 400'000 &&
            c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
 }
 // Who runs a projection that few_rows() takes: whoever is faster, or what the caller says.
@@ -751,7 +771,7 @@ bool token_rows(const Tensor &x, int64_t most) {
            !wants_grad({&x}) && sm100(x.device());
 }
 
-// One token through all blocks of a model, or None where a block or the rows are not ones kla_b200_token takes. blocks: per
+// One token through all blocks of a model, or None where a block or the rows are not ones kla_b200_token takes or is the faster way for. blocks: per
 // block (weights, config, conv window, lam, eta, a_bar, p_bar, skip, conv weights, conv bias, w_value, w_var, norm weight) and,
 // with a swiglu MLP behind the mixer, (norm weight, w12, bias, w3, bias).
 using BlockArgs = std::tuple<py::dict, py::dict, OptTensor, Tensor, Tensor, Tensor, Tensor, OptTensor, OptTensor, OptTensor, int64_t, int64_t, Tensor>;
@@ -760,9 +780,15 @@ py::object model_token(const Tensor &x, const std::vector<BlockArgs> &blocks, co
     if (!token_rows(x, kTokenRows) || blocks.empty() || (!mlps.empty() && mlps.size() != blocks.size())) return py::none();
     const c10::cuda::CUDAGuard guard(x.device());
     std::vector<kla_b200_token_layer> layers(blocks.size());
+    const int64_t rows = x.size(0), d = x.size(1), sms = at::cuda::getDeviceProperties(x.device().index())->multiProcessorCount;
+    // Issued call by call, a block's separate kernels cost the host 30 us, which is more than they take up to the sizes of a lone
+    // layer's rule.
+    const bool replayed = works || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
     for (size_t i = 0; i < blocks.size(); ++i) {
         const auto &[w, cfg, conv_state, lam, eta, a_bar, p_bar, skip, conv_w, conv_b, w_value, w_var, norm_w] = blocks[i];
         if (!token_layer(x, LayerArgs{w, cfg, conv_state, lam, eta, a_bar, p_bar, skip, conv_w, conv_b, w_value, w_var}, norm_w, layers[i])) return py::none();
+        const int64_t M = layers[i].M, S = layers[i].S, hidden_out = mlps.empty() || std::get<1>(mlps[i]).dim() != 2 ? 0 : std::get<1>(mlps[i]).size(0);
+        if ((replayed || !few_weights(d, M, S)) && !token_pays(rows, M, S, std::max((layers[i].gated ? 2 : 1) * M, hidden_out), sms)) return py::none();
         if (mlps.empty()) continue;
         const auto &[mlp_norm, w12, b12, w3, b3] = mlps[i];
         const int64_t hidden = w12.dim() == 2 ? w12.size(0) / 2 : 0;
@@ -953,6 +979,7 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("step", &step);
     m.def("layer_step", &layer_step);
     m.def("model_token", &model_token);
+    m.def("token_pays", &token_pays);
     m.def("add_norm", &add_norm);
     m.def("swiglu", &swiglu);
     m.def("argmax", &argmax);

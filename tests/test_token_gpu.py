@@ -127,6 +127,25 @@ def test_a_lone_layers_token_is_that_of_the_separate_kernels(B, d, M, S, cfg, n)
         assert torch.equal(out[0] if cfg.get("return_variance") else out, wants[i])
 
 
+@pytest.mark.parametrize("B,d,M,S,hidden,one", [(1, 64, 768, 64, 176, True), (1, 64, 776, 64, 176, False), (2, 64, 776, 64, 176, True),
+                                                (8, 64, 592, 64, 0, True), (8, 64, 600, 64, 0, False), (8, 64, 600, 32, 0, True)])
+def test_a_captured_token_is_one_kernel_where_that_is_faster(B, d, M, S, hidden, one):
+    """Both sides of the rule's lines on 148 SMs (2368 units of 32 lanes): one launch or the separate kernels, the same bits. Call by
+    call the host is slower than either, and a token is one kernel."""
+    assert torch.cuda.get_device_properties(0).multi_processor_count == 148
+    dec = stack(d, M, S, 1, hidden, {}, False)
+    x = torch.randn(B, d, device="cuda").bfloat16()
+    a, b = (dec.init_state(B, "cuda", torch.bfloat16) for _ in range(2))
+    want, n = launches(lambda: dec._step_blocks(x, b))
+    assert n == 1
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got, n = launches(lambda: dec._step_blocks(x, a))
+    assert (n == 1) == one
+    graph.replay()
+    assert torch.equal(got, want) and same(flat(a), flat(b))
+
+
 def test_tokens_on_streams_and_in_graphs_do_not_meet():
     """Eager tokens of one decoder on several streams and threads, and a captured one replayed meanwhile."""
     dec = stack(256, 512, 16, 2, 688, {}, False)
