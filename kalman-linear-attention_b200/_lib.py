@@ -56,6 +56,7 @@ class Tensor3(Structure):
 
 ACT = {"silu": 0, "gelu": 1, "relu": 2, None: 3}
 MAX_CONV_TAPS = 8
+TOKEN_MAX_ROWS = 8
 
 
 class ConvStepArgs(Structure):

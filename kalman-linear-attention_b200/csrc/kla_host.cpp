@@ -961,6 +961,14 @@ py::bytes stamp(const std::vector<OptTensor> &ts) {
     return py::bytes(reinterpret_cast<const char *>(v.data()), v.size() * sizeof(int64_t));
 }
 
+// Whether the GPU is past a recorded event; while another thread captures a graph as well, which a plain query would end.
+bool event_done(uintptr_t event) {
+    const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    if (cudaEventQuery(reinterpret_cast<cudaEvent_t>(event)) != cudaErrorNotReady) return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_kla_host, m) {
@@ -980,6 +988,7 @@ PYBIND11_MODULE(_kla_host, m) {
     m.def("layer_step", &layer_step);
     m.def("model_token", &model_token);
     m.def("token_pays", &token_pays);
+    m.def("event_done", &event_done);
     m.def("add_norm", &add_norm);
     m.def("swiglu", &swiglu);
     m.def("argmax", &argmax);

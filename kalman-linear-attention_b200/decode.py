@@ -191,11 +191,41 @@ class LayerDecoder:
         return out
 
 
+_under_way: dict = {}  # by device: [stream, model, event behind it or None] of models' calls not known to have ended
+_under_way_lock = threading.Lock()
+
+
+@contextlib.contextmanager
+def _announced(model, device):
+    """Whether a ``generate`` or ``prefill`` of ``model`` has the GPU to itself, as far as models' calls go: none of another model on
+    another stream is still being issued or run. (Those of one model share its kept step and follow one another.) Others see this
+    call until the GPU is done with it."""
+    if torch.cuda.is_current_stream_capturing():
+        yield True
+        return
+    mine = [torch.cuda.current_stream(device), id(model), None]
+    with _under_way_lock:
+        calls = _under_way.setdefault(mine[0].device_index, [])
+        calls[:] = [c for c in calls if c[2] is None or not _lib.host().event_done(c[2].cuda_event)]
+        alone = all(c[0] == mine[0] or c[1] == mine[1] for c in calls)
+        calls.append(mine)
+    try:
+        yield alone
+        event = torch.cuda.Event()
+        event.record(mine[0])
+        mine[2] = event
+    except BaseException:
+        with _under_way_lock:
+            calls[:] = [c for c in calls if c is not mine]
+        raise
+
+
 class _TokenGraph:
     """The decode step of a :class:`ModelDecoder` captured once: state, token and logits buffers and the graph that
     advances them by one token."""
 
-    def __init__(self, dec: "ModelDecoder", batch: int, device, dtype, greedy: bool):
+    def __init__(self, dec: "ModelDecoder", batch: int, device, dtype, greedy: bool, whole: bool = True):
+        self.whole = whole
         self.state = dec.init_state(batch, device, dtype)
         self.token = torch.zeros(batch, device=device, dtype=torch.long)
         self.work = []  # of the kernel that a whole token is, made by its first run here; replays follow one another
@@ -216,7 +246,7 @@ class _TokenGraph:
         torch.cuda.current_stream(device).wait_stream(side)
 
     def _token(self, dec, greedy):
-        logits = dec._token_logits(self.token, self.state, self.work)
+        logits = dec._token_logits(self.token, self.state, self.work, self.whole)
         if greedy:
             _lib.host().argmax(logits, self.token)
         return logits
@@ -270,12 +300,20 @@ class ModelDecoder:
     A block is ``x += mixer(norm(x))`` then ``x += mlp(norm(x))`` (sequence_model.py:47-98). For one token of up to eight
     sequences in bfloat16 all blocks are one kernel (``kla_b200_token``), for up to 16 a block is six: the projections with norm,
     convolution step, gate and residual sum folded in, and the filter step. For up to 32 sequences large projections are library GEMMs. For a prompt the projections are library GEMMs and what stands between them one kernel each.
+    That one kernel holds every SM: the tokens of two streams follow one another where separate kernels overlap, and a token waits for
+    all that another stream has running. 256 tokens of 12 blocks of d_model 768, 8 rows each, ms, one kernel / separate ones: one
+    ``generate`` 82 / 97, two models at once 174 / 112, four 394 / 157, one beside prompts on another stream 475 / 201. A ``generate``
+    that finds another model's ``generate`` or ``prefill`` under way on another stream of its device therefore takes the separate
+    kernels, with the same results. ``whole_gpu``, set on a decoder, says which: False where other work of the program shares the GPU, True for
+    the one kernel at any time.
     One decoded token is a fixed sequence of launches over state that is updated in place, so ``generate`` captures it in
     a CUDA graph, which it keeps for calls with the same batch, types and weights, and replays it: a token then costs no
     host work but one replay, where the reference's loop issues several hundred small launches per token from Python.
 
     Built from plain tensors (``SequenceModel.state_dict()``) and plain config dicts; ``from_model`` reads them
     off a reference model. The reference package is not needed at run time."""
+
+    whole_gpu = None  # or True, False
 
     def __init__(self, weights: dict, layer_configs, model_config: dict):
         missing = [k for k in MODEL_KEYS if k not in model_config]
@@ -291,7 +329,7 @@ class ModelDecoder:
             pre = f"blocks.{i}.mixer."
             lw = {k[len(pre):]: v for k, v in weights.items() if k.startswith(pre)}
             self.layers.append(LayerDecoder(lw, layer_configs[i]))
-        self._slot = _GraphSlot()
+        self._slot, self._shared_slot = _GraphSlot(), _GraphSlot()
 
     @classmethod
     def from_model(cls, model) -> "ModelDecoder":
@@ -308,7 +346,7 @@ class ModelDecoder:
         out.__dict__.update(self.__dict__)
         out.w = {k: v.to(device) for k, v in self.w.items()}
         out.layers = [layer.to(device) for layer in self.layers]
-        out._slot = _GraphSlot()
+        out._slot, out._shared_slot = _GraphSlot(), _GraphSlot()
         return out
 
     def init_state(self, batch: int, device, dtype=torch.float32):
@@ -336,13 +374,14 @@ class ModelDecoder:
         cap = self.cfg["logit_softcap"]
         return logits if cap is None else cap * torch.tanh(logits / cap)
 
-    def _step_blocks(self, x, state, work=None):
-        """One token through the blocks: of up to eight sequences in bfloat16 all of them as one kernel (``work``: a list of
-        its working memory where the caller keeps it); otherwise norm, mixer and residual sum of a block are the layer's step with
-        the norm folded into its first projection and the sum into its last, and the MLP likewise."""
+    def _step_blocks(self, x, state, work=None, whole=True):
+        """One token through the blocks: of up to eight sequences in bfloat16 all of them as one kernel, at sizes where that pays
+        (``work``: a list of its working memory where the caller keeps it; ``whole``: it may take the whole GPU); otherwise norm, mixer
+        and residual sum of a block are the layer's step with the norm folded into its first projection and the sum into its last, and
+        the MLP likewise."""
         _require_cuda(x)
         host, w, eps, mlp = _lib.host(), self.w, self.cfg["norm_eps"], self.cfg["mlp"]
-        if mlp in ("swiglu", "none") and x.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
+        if whole and mlp in ("swiglu", "none") and x.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
             blocks = [(m.w, m.cfg, *st, m.a_bar, m.p_bar, m.skip, m.conv_w, getattr(m, "conv_b", None), m.w_value, m.w_var,
                        w[f"blocks.{i}.mixer_norm.weight"]) for i, (m, st) in enumerate(zip(self.layers, state))]
             mlps = [] if mlp == "none" else [
@@ -381,17 +420,19 @@ class ModelDecoder:
     def prefill(self, input_ids: torch.Tensor, state=None):
         """A prompt: ``input_ids`` [B, L] -> (logits [B, L, vocab], state ready for ``step``)."""
         x = F.embedding(input_ids, self.w["embedding.weight"])
+        _require_cuda(x)
         if state is None:
             state = self.init_state(x.shape[0], x.device, x.dtype)
-        return self._head(*self._prompt_blocks(x, state)), state
+        with _announced(self, x.device):
+            return self._head(*self._prompt_blocks(x, state)), state
 
     @torch.no_grad()
     def step(self, token: torch.Tensor, state):
         """One token per sequence: ``token`` [B] -> logits [B, vocab]; ``state`` is updated in place."""
-        return self._token_logits(token, state)
+        return self._token_logits(token, state, whole=self.whole_gpu is not False)
 
-    def _token_logits(self, token, state, work=None):
-        x = self._step_blocks(F.embedding(token, self.w["embedding.weight"]), state, work)
+    def _token_logits(self, token, state, work=None, whole=True):
+        x = self._step_blocks(F.embedding(token, self.w["embedding.weight"]), state, work, whole)
         return self._cap(_lib.host().project(x, self.w["lm_head.weight"], None, self.w["norm_f.weight"], self.cfg["norm_eps"], None))
 
     @torch.no_grad()
@@ -402,9 +443,14 @@ class ModelDecoder:
         one CUDA graph replay; sampling happens between replays, on the device."""
         x = F.embedding(input_ids, self.w["embedding.weight"])
         _require_cuda(x)
+        with _announced(self, x.device) as alone:
+            return self._generate(input_ids, x, max_new_tokens, temperature, top_k, use_graph, alone if self.whole_gpu is None else self.whole_gpu)
+
+    def _generate(self, input_ids, x, max_new_tokens, temperature, top_k, use_graph, whole):
         B, P = input_ids.shape
         greedy = temperature <= 0
-        graph_ctx = self._token_graph(B, x.device, x.dtype, greedy) if use_graph and max_new_tokens > 1 else contextlib.nullcontext()
+        whole = whole or x.dtype != torch.bfloat16 or B > _lib.TOKEN_MAX_ROWS  # (tokens that are separate kernels anyway)
+        graph_ctx = self._token_graph(B, x.device, x.dtype, greedy, whole) if use_graph and max_new_tokens > 1 else contextlib.nullcontext()
         with graph_ctx as graph:
             state = graph.reset() if graph is not None else self.init_state(B, x.device, x.dtype)
             # the head sees the last position: the prompt's other logits are not needed
@@ -418,7 +464,7 @@ class ModelDecoder:
             tok_buf = token[:, 0].clone() if graph is None else graph.token.copy_(token[:, 0])
             for i in range(P + 1, P + max_new_tokens):
                 if graph is None:
-                    tok_buf.copy_(self._sample(self.step(tok_buf, state), temperature, top_k)[:, 0])
+                    tok_buf.copy_(self._sample(self._token_logits(tok_buf, state, whole=whole), temperature, top_k)[:, 0])
                 else:
                     graph.graph.replay()
                     if not greedy:
@@ -427,15 +473,16 @@ class ModelDecoder:
         return out
 
     @contextlib.contextmanager
-    def _token_graph(self, batch: int, device, dtype, greedy: bool):
-        """The captured decode step for this batch: the kept one when it fits and is free, else a new one."""
+    def _token_graph(self, batch: int, device, dtype, greedy: bool, whole: bool = True):
+        """The captured decode step for this batch: the kept one when it fits and is free, else a new one. Steps that may take
+        the whole GPU and others are kept apart."""
         own = [t for name, t in self.w.items() if ".mixer." not in name]
         layers = [t for layer in self.layers
                   for t in (*layer.w.values(), layer.a_bar, layer.p_bar, layer.skip, layer.conv_w, getattr(layer, "conv_b", None))]
         key = (batch, device, dtype, greedy, torch.is_autocast_enabled("cuda"), torch.get_autocast_dtype("cuda"),
                torch.is_inference_mode_enabled(), _lib.host().stamp(own + layers), dict(self.cfg),
                [(dict(layer.cfg), layer.w_value, layer.w_var) for layer in self.layers])
-        slot = self._slot
+        slot = self._slot if whole else self._shared_slot
         kept = slot.lock.acquire(blocking=False)
         try:
             if kept and slot.key == key:
@@ -444,7 +491,7 @@ class ModelDecoder:
                 if kept and slot.graph is not None:
                     slot.graph.done.synchronize()  # its buffers go back to the allocator: nothing may still read them
                     slot.key = slot.graph = None
-                graph = _TokenGraph(self, batch, device, dtype, greedy)
+                graph = _TokenGraph(self, batch, device, dtype, greedy, whole)
                 if kept:
                     slot.key, slot.graph = key, graph
             try:

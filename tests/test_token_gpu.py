@@ -224,3 +224,40 @@ def test_a_captured_tokens_working_memory_is_kept_until_its_replays_are_done():
     assert not still.query()  # the replay has it all to do
     assert all(not t.data_ptr() <= at < t.data_ptr() + size for t in taken)
     torch.cuda.synchronize()
+
+
+def test_a_generate_beside_another_stream_leaves_it_room():
+    """Another model's call on another stream that the GPU is not done with: separate kernels, the same tokens. Not for calls on the
+    same stream or of the same model, nor once the other is done or has failed."""
+    a, b = (stack(64, 128, 16, 2, 176, {}, False, seed=s) for s in (0, 1))
+    ids = torch.arange(12, device="cuda").view(2, 6)
+    want = [m.generate(ids, 24) for m in (a, b)]
+    own = b._slot.graph
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for busy in (lambda: a.generate(ids, 24), lambda: a.prefill(ids)):
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200_000_000)  # 0.1 s
+            other = busy()
+            assert torch.equal(b.generate(ids, 24), want[1]) and b._shared_slot.graph is None  # behind it on its stream
+            torch.cuda._sleep(200_000_000)
+            other = busy()
+        assert torch.equal(a.generate(ids, 24), want[0]) and a._shared_slot.graph is None  # they share a's kept step
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200_000_000)
+            other = busy()
+        got = b.generate(ids, 24)
+        assert b._shared_slot.graph is not None and not b._shared_slot.graph.whole
+        torch.cuda.synchronize()
+        assert torch.equal(got, want[1]) and (isinstance(other, tuple) or torch.equal(other, want[0]))
+        b._shared_slot.key = b._shared_slot.graph = None
+    with torch.cuda.stream(side), pytest.raises(RuntimeError):
+        a.generate(ids, 4, temperature=1.0, top_k=1000)  # of 64
+    assert torch.equal(b.generate(ids, 24), want[1]) and b._shared_slot.graph is None
+    assert b._slot.graph is own
+    for whole in (True, False):
+        c = stack(64, 128, 16, 2, 176, {}, False)
+        c.whole_gpu = whole
+        assert torch.equal(c.generate(ids, 24), want[0]) and torch.equal(c.generate(ids, 24, use_graph=False), want[0])
+        assert (c._slot.graph is not None) == whole and (c._shared_slot.graph is None) == whole
+        assert launches(lambda: c.step(ids[:, 0], c.init_state(2, "cuda", torch.bfloat16)))[1] < 4 or not whole
