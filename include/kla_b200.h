@@ -237,11 +237,13 @@ int kla_b200_slab_aggregate(const kla_b200_slab_args *args, void *stream);
  * y + lambda_skip * z, then the gate on y and its square on y_var). One
  * memory-bound pass: from the gradients of the gated outputs it forms the
  * gradients kla_b200_scan_bwd takes as dy, dy_var, plus dz, dgate and
- * dlambda_skip (accumulated with atomic adds after the library zeroes it).
+ * dlambda_skip (accumulated with atomic adds after the library zeroes it; one
+ * value for everything in double precision, given work to do it in).
  * z/dz and lambda_skip, or gate/dgate, are NULL when that half of the path is
  * absent. Activation tensors (z, gate, dz, dgate) are in_dtype, the others
  * out_dtype, as in the forward.
  */
+#define KLA_B200_SKIP_SUM_BYTES 16
 typedef struct kla_b200_epilogue_bwd_args {
     int64_t B, L, M;
     int32_t in_dtype, out_dtype;
@@ -254,6 +256,8 @@ typedef struct kla_b200_epilogue_bwd_args {
     kla_b200_tensor3 dy, dy_var;    /* out [B, L, M], out_dtype */
     kla_b200_tensor3 dz, dgate;     /* out [B, L, M], in_dtype */
     float *dlambda_skip;            /* out [lambda_skip_len] float32 */
+    void *work;                     /* KLA_B200_SKIP_SUM_BYTES, 8-byte aligned, for lambda_skip_len 1: its gradient is then
+                                     * added up in double. NULL: in float32, in the order the CTAs end */
 } kla_b200_epilogue_bwd_args;
 
 int kla_b200_epilogue_bwd(const kla_b200_epilogue_bwd_args *args, void *stream);

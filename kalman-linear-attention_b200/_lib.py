@@ -161,6 +161,7 @@ class EpilogueBwdArgs(Structure):
         ("dout", Tensor3), ("dout_var", Tensor3), ("y_raw", Tensor3), ("y_var_raw", Tensor3),
         ("z", Tensor3), ("gate", Tensor3), ("lambda_skip", c_void_p),
         ("dy", Tensor3), ("dy_var", Tensor3), ("dz", Tensor3), ("dgate", Tensor3), ("dlambda_skip", c_void_p),
+        ("work", c_void_p),
     ]
 
 

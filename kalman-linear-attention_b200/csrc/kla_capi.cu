@@ -821,9 +821,12 @@ int kla_b200_epilogue_bwd(const kla_b200_epilogue_bwd_args *a, void *stream) {
     const size_t esz = a->in_dtype == KLA_B200_F32 ? 4 : 2, osz = a->out_dtype == KLA_B200_F32 ? 4 : 2;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e;
-    if (has_skip && (e = cudaMemsetAsync(a->dlambda_skip, 0, sizeof(float) * (size_t)a->lambda_skip_len, st)) != cudaSuccess)
+    const bool empty = a->B == 0 || a->L == 0 || a->M == 0, wide_sum = a->lambda_skip_len == 1 && a->work != nullptr && !empty;
+    if (wide_sum && !aligned(a->work, 8)) return KLA_B200_EALIGN;
+    if (has_skip && (e = wide_sum ? cudaMemsetAsync(a->work, 0, sizeof(SkipSum), st)
+                                  : cudaMemsetAsync(a->dlambda_skip, 0, sizeof(float) * (size_t)a->lambda_skip_len, st)) != cudaSuccess)
         return cuda_fail(e);
-    if (a->B == 0 || a->L == 0 || a->M == 0) return KLA_B200_OK;
+    if (empty) return KLA_B200_OK;
     int rc;
     if ((rc = check_t3(a->dout, osz, true)) || (rc = check_t3(a->dout_var, osz, false)) || (rc = check_t3(a->dy, osz, true)) ||
         (rc = check_t3(a->dy_var, osz, true)))
@@ -838,6 +841,8 @@ int kla_b200_epilogue_bwd(const kla_b200_epilogue_bwd_args *a, void *stream) {
     prm.B = (int)a->B; prm.L = (int)a->L; prm.M = (int)a->M;
     prm.dout = t3(a->dout); prm.dout_var = t3(a->dout_var); prm.y_raw = t3(a->y_raw); prm.yv_raw = t3(a->y_var_raw);
     if (has_skip) { prm.z = t3(a->z); prm.dz = t3(a->dz); prm.skip = a->lambda_skip; prm.skip_len = a->lambda_skip_len; prm.dskip = a->dlambda_skip; }
+    static_assert(sizeof(SkipSum) == KLA_B200_SKIP_SUM_BYTES, "as the header says");
+    prm.sum = wide_sum ? static_cast<SkipSum *>(a->work) : nullptr;
     if (has_gate) { prm.gate = t3(a->gate); prm.dgate = t3(a->dgate); prm.gate_act = a->gate_activation; }
     prm.dy = t3(a->dy); prm.dy_var = t3(a->dy_var);
     // four channels per thread when every tensor can be read and written as 4-element vectors, eight when they are all

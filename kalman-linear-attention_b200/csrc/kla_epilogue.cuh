@@ -13,7 +13,10 @@
 // y and y_var are the scan's outputs before the path was applied; the forward stores them for this purpose.
 // Memory-bound: 6 tensors in, 4 out, one element of each per (b, t, m). A thread owns one channel and walks
 // kEpiRows time steps, so consecutive lanes touch consecutive addresses and the skip gradient needs one atomic
-// add per thread.
+// add per thread, or for a scalar skip one per CTA: that sum runs over all of [B, L, M] and can be a small difference of large shares
+// (B=16 L=2048 M=1536: 5e7 terms; added up in float32 in the order of the CTAs, its last 1e-3 to 1e-2 were another number each
+// time), so the CTAs' shares are added in double, and the last CTA rounds (192.1 -> 194.6 us there, the wait for its own share
+// before a CTA counts itself done).
 #pragma once
 
 #include "kla_common.cuh"
@@ -21,6 +24,11 @@
 namespace kla {
 
 constexpr int kEpiRows = 32, kEpiFewRows = 4;  // the latter where 32 would leave SMs without work
+
+struct SkipSum {
+    double sum;
+    unsigned done, pad;  // CTAs
+};
 
 struct EpilogueBwdParams {
     int B, L, M;
@@ -32,6 +40,7 @@ struct EpilogueBwdParams {
     Tensor3 dy, dy_var;       // TO, out
     Tensor3 dz, dgate;        // T, out (nullptr when the operand is absent)
     float *dskip;             // [skip_len], accumulated
+    SkipSum *sum;             // a scalar skip's sum, zeroed, or nullptr: accumulated in dskip
 };
 
 // The gate activation and its derivative from one exponential (or error function) and one reciprocal: taken separately
@@ -179,13 +188,27 @@ __global__ void __launch_bounds__(128) kla_epilogue_bwd_kernel(const EpilogueBwd
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) atomicAdd(prm.dskip + m + e, dskip[e]);
             }
-        } else {  // scalar skip: one sum over everything; add the warp's share with one atomic
-            float s = 0.0f;
+        } else {  // scalar skip: one sum over everything
+            double s = 0.0;
 #pragma unroll
             for (int e = 0; e < VEC; ++e) s += dskip[e];
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-            if ((threadIdx.x & 31) == 0) atomicAdd(prm.dskip, s);
+            __shared__ double share[4];
+            if ((threadIdx.x & 31) == 0) share[threadIdx.x / 32] = s;
+            __syncthreads();
+            if (threadIdx.x != 0) return;
+            s = (share[0] + share[1]) + (share[2] + share[3]);
+            if (prm.sum == nullptr) {
+                atomicAdd(prm.dskip, (float)s);
+                return;
+            }
+            atomicAdd(&prm.sum->sum, s);
+            __threadfence();
+            if (atomicAdd(&prm.sum->done, 1u) == gridDim.x * gridDim.y * gridDim.z - 1) {
+                __threadfence();
+                *prm.dskip = (float)atomicAdd(&prm.sum->sum, 0.0);
+            }
         }
     }
 }

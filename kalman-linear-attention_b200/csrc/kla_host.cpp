@@ -296,10 +296,11 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> epilogue_bwd(const T
     const int64_t B = v.size(0), L = v.size(1), M = v.size(2);
     const auto TO = out_type(out_bf16);
     Tensor dy = fresh(v, {B, L, M}, TO), dyv = fresh(v, {B, L, M}, TO);
-    OptTensor dz, dgate, dskip;
+    OptTensor dz, dgate, dskip, work;
     if (z) dz = fresh(v, {B, L, M});
     if (gate) dgate = fresh(v, {B, L, M});
     if (skip) dskip = at::empty_like(*skip);
+    if (skip && skip->numel() == 1) work = fresh(v, {KLA_B200_SKIP_SUM_BYTES}, at::kByte);
     kla_b200_epilogue_bwd_args e{};
     e.B = B; e.L = L; e.M = M;
     e.in_dtype = dt(v.scalar_type()); e.out_dtype = dt(TO);
@@ -308,6 +309,7 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> epilogue_bwd(const T
     e.dout = t3(dout); e.dout_var = t3(dout_var); e.y_raw = t3(y_raw); e.y_var_raw = t3(yv_raw);
     e.z = t3(z); e.gate = t3(gate); e.lambda_skip = fp(skip);
     e.dy = t3(dy); e.dy_var = t3(dyv); e.dz = t3(dz); e.dgate = t3(dgate); e.dlambda_skip = fp(dskip);
+    e.work = work ? work->data_ptr() : nullptr;
     check(lib.epilogue_bwd(&e, stream_of(v)));
     return {dy, dyv, dz, dgate, dskip};
 }

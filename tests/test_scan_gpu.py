@@ -638,3 +638,35 @@ def test_training_epilogue_keeps_raw_outputs_at_any_width(M, dtype):
     s = F.silu(gf)
     want, = torch.autograd.grad([(y0.float() + skip * z.float()) * s, yv0.float() * s * s], [gf], [dy.float(), dyv.float()])
     assert (got.float() - want).norm() <= (4 * 2 ** -8 if dtype == torch.bfloat16 else 1e-5) * want.norm()
+
+
+@pytest.mark.parametrize("B,L,M,dtype,gated", [
+    (2, 1, 1, torch.float32, True), (2, 37, 129, torch.float32, False),  # one channel per thread; a few CTAs
+    (2, 700, 516, torch.float32, True), (4, 2048, 768, torch.bfloat16, True),  # four, eight; few rows and many per CTA
+])
+def test_a_scalar_skips_gradient_is_summed_in_double(B, L, M, dtype, gated):
+    """Half the batch with the other half's gradients negated: the sum is 0, and what each CTA adds has its exact opposite. Up to n
+    CTAs' shares in double are off by n 2^-53 of the terms' sum at the most; in float32, in the order of the CTAs, by 1e-9 of it.
+    With the halves alike it is float64's sum to the rounding of 32 float32 terms per thread (32 2^-24)."""
+    import torch.nn.functional as F
+
+    import kla_b200
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    both = lambda t: torch.cat((t, t)).to(dtype)
+    b, S = B // 2, 16
+    v, z, gate, dy = (both(rn(b, L, M)) for _ in range(4))
+    lv = F.softplus(v.float()).reciprocal().to(dtype)
+    k, q = (both(F.normalize(rn(b, L, S), dim=-1)) for _ in range(2))
+    a, p, skip = torch.sigmoid(rn(M, S)), F.softplus(rn(M, S)), torch.tensor(-0.7, device="cuda", requires_grad=True)
+    epi = dict(z=z, lambda_skip=skip, **(dict(gate=gate, gate_activation="silu") if gated else {}))
+    terms = (dy.double() * z.double() * (F.silu(gate.double()) if gated else 1.0)).flatten()
+    for sign in (1.0, -1.0):
+        dout = torch.cat((dy[:b], sign * dy[b:]))
+        y, _, _ = kla_b200.kla_scan_b200(v, lv, k, q, a, p, out_dtype=dtype, epilogue=epi)
+        got = torch.autograd.grad([y], [skip], [dout])[0].double().item()
+        if sign > 0:
+            assert abs(got - terms.sum().item()) <= (32 * 2 ** -24 + 4e-6) * terms.abs().sum().item()  # (the fast sigmoid: 4e-6)
+        else:
+            assert abs(got) <= 2 ** -40 * terms.abs().sum().item()
