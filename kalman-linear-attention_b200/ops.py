@@ -173,8 +173,7 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
     building the chunks' start states costs about 0.7x of a forward + backward pass on top, so chunking is only
     chosen when the plain grid fills less than a third of the resident CTA slots; then up to 16 chunks. Chunks keep at least 64 steps and are equally long where the count divides L, else
     a multiple of 16 steps with a shorter last one (:func:`_chunk_len`). ``requested`` (or the environment variable
-    KLA_B200_TIME_CHUNKS, not looked at where an output path is applied to fewer than 1600 steps) overrides the choice; it is
-    lowered to the nearest usable divisor of L."""
+    KLA_B200_TIME_CHUNKS) overrides the choice; it is lowered to the nearest usable divisor of L."""
     if requested is None and os.environ.get("KLA_B200_TIME_CHUNKS"):
         requested = int(os.environ["KLA_B200_TIME_CHUNKS"])
     lpc = 1
@@ -199,7 +198,8 @@ def pick_time_chunks(B: int, L: int, M: int, S: int, requested: Optional[int] = 
             if row == 16 or not (training or (row < 4 and L >= 900)):
                 return 1
         # With the layer's sensors and output path inside, the call stands in a layer, whose host takes longer than a short
-        # scan: cutting adds launches and has to shorten what the GPU does beyond that. Whole prompts of one layer in us,
+        # scan: cutting adds launches and has to shorten what the GPU does beyond that. (The lines are those of calls issued one
+        # by one; a captured call, which the GPU's times below would cut from 1000 steps on, is not told apart.) Whole prompts of one layer in us,
         # uncut and cut, bfloat16: B=1 d_model=512 L=1000 162 and 170, L=1500 172 and 169, L=2048 215 and 169; training steps
         # between the projections, B=1 M=1024 L=1000 727 and 770, L=2048 775 and 780, L=2400 875 and 765. By the GPU alone
         # (forward / training step, bfloat16): 48 CTAs (B=2 M=768) L=1000 87 / 307 and 72 / 272; 64 CTAs (B=1 M=2048) L=1000
@@ -493,8 +493,9 @@ def kla_scan_b200(
         if gate_act not in ("silu", "gelu", "relu"):
             raise ValueError("gate_activation must be 'silu', 'gelu' or 'relu'")
         training = _wants_grad(v, lambda_v, k, q, a, p, lam0, eta0, epi.get("z"), epi.get("gate"), skip)
-        # short prompts are bound by the host: not even the rule is asked for them (3 of 160 us)
-        chunks = 1 if L < _LAYER_CHUNKS_FROM and time_chunks is None else _chunks_of(v, lambda_v, k, q, time_chunks, training, True)
+        # short prompts are bound by the host: not even the rule is asked for them (3 of 160 us), unless a count is given
+        ask = L >= _LAYER_CHUNKS_FROM or time_chunks is not None or os.environ.get("KLA_B200_TIME_CHUNKS")
+        chunks = _chunks_of(v, lambda_v, k, q, time_chunks, training, True) if ask else 1
         if not training:
             if skip is not None:
                 epi["lambda_skip"] = skip.float().reshape(-1).contiguous()

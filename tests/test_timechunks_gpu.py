@@ -204,3 +204,21 @@ def test_scans_with_the_layers_sensors_and_output_path_in_chunks(kb, B, L, M, S,
         assert rel_err(x.float(), y.double().cpu().numpy()) < 1.2e-4 + (2.0 ** -8 if y.dtype == torch.bfloat16 else 0.0)
     for x, y in zip(gc, g1):
         assert rel_err(x.float(), y.double().cpu().numpy()) < (1e-2 if y.dtype == torch.bfloat16 else 1e-4)
+
+
+@pytest.mark.parametrize("layer", [False, True])
+def test_the_environment_variable_holds_at_any_length(kb, monkeypatch, layer):
+    g = _seeded(2, 256, 16, 16, seed=25, state=False)
+    ins = [torch.tensor(g[n], dtype=torch.float32, device="cuda") for n in INPUTS]
+    kw = dict(epilogue=dict(z=ins[0], lambda_skip=ins[4][:, 0].contiguous())) if layer else {}
+
+    def run():
+        before = ops._lib.load().kla_b200_launch_count()
+        y = kb.kla_scan_b200(*ins, **kw)[0]
+        return y, ops._lib.load().kla_b200_launch_count() - before
+
+    y1, n1 = run()
+    monkeypatch.setenv("KLA_B200_TIME_CHUNKS", "4")
+    y4, n4 = run()
+    assert (n1, n4) == (1, 3)
+    torch.testing.assert_close(y4, y1, rtol=2e-5, atol=2e-6)
