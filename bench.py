@@ -457,7 +457,7 @@ def run_b200(args):
                          "unit": "GB/s", "frac": ach_bwd / peak, "traffic": NCU_TRAFFIC["kla_bwd_kernel"] * B / 8 if "kla_bwd_kernel" in NCU_TRAFFIC else None,
                          "peak_source": peak_src, "algorithmic_bytes": bwd_bytes, "ms": bwd_ms,
                          "nominal_peak_gbs": 8000.0, "frac_of_nominal": ach_bwd / 8000.0,
-                         "note": "not HBM-bound at d_state=16: 43.5 warp-instructions per 32 lane-steps against 24.8 KB per "
+                         "note": "not HBM-bound at d_state=16: 43.1 warp-instructions per 32 lane-steps against 24.8 KB per "
                                  "token; bound by the FP32 pipe's register reads (ncu: issue slots 56 % busy, FP32 pipe 58 %; the "
                                  "256 sequences run as 16 segments each, handed from CTA to CTA)"},
             "roofline_fwd": {"bound": "hbm", "kernel": "kla_fwd_kernel", "achieved": ach_fwd, "peak": peak,

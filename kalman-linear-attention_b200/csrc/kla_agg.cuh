@@ -46,8 +46,9 @@
 // states of one channel as pairs (paired fp32 instructions), and one loader warp
 // that brings tiles of TT steps in: v, lambda_v (and dy, dy_var) as TMA tiles
 // signalled on mbarriers, k (and q) regrouped by owning lane. Nothing is written but the final record.
-// Measured on B200, B=2 L=1024 M=1024 S=16 in 16 chunks, float32, against the form with matrices: forward 29.7 -> 27.3 us,
-// adjoint 39.8 -> 34.3; bound by the FP32 pipe (17.7 of the 27.3 us) and by the start of CTAs of two tiles each.
+// Measured on B200, B=2 L=1024 M=1024 S=16 in 4 chunks, float32, against the form with matrices: forward 29.7 -> 26.7 us,
+// adjoint 39.8 -> 33.7; 192 CTAs of eight tiles: bound by the FP32 pipe of the 44 SMs that hold two (17.7 of the forward's time)
+// and by the latency of the first and last tile. In 8 chunks of 512 steps (L=4096, 448 CTAs) 94 and 119 us.
 #pragma once
 
 #include "kla_common.cuh"

@@ -49,14 +49,14 @@
 // on; the state its walk starts from needs no hand-over, the replay group computes it from the checkpoints.
 //
 // Measured on B200 at T=4096, M=1024, S=16, float32, against the kernel with one channel per thread and scalar
-// arithmetic: B=8 1.42 -> 1.13 ms, B=4 0.88 -> 0.69 ms, B=16 2.59 -> 2.13 ms; 43.5 instead of 66 warp instructions per 32
+// arithmetic: B=8 1.42 -> 1.14 ms, B=4 0.88 -> 0.69 ms, B=16 2.59 -> 2.13 ms; 43.1 instead of 66 warp instructions per 32
 // lane-steps. What bounds it is the FP32 pipe's register reads: 29 pair operations per two chains and step in the
 // reverse walk and 8 in the replay, 12 and 2 of them three-operand FMAs at 3.75 cycles (kla_common.cuh), add up to about
-// 235 of the 291 cycles a scheduler spends on a warp's step. Not limits: shared memory (the trajectory through tensor
+// 230 of the 289 cycles a scheduler spends on a warp's step. Not limits: shared memory (the trajectory through tensor
 // memory, a third less shared-memory traffic, takes the same 1.17 ms), the helpers (1.12 ms without their sums), the
 // replay (1.08 ms without its arithmetic). Scalar FMAs in place of the pair FMAs: 1.25 ms. Fetching a step's inputs
 // before the previous step's arithmetic and unrolling the whole tile gave 1.20 -> 1.17 ms; shares of dk, dq summed as halves
-// and doubled once per CTA 1.144 -> 1.132.
+// and doubled once per CTA 1.148 -> 1.141.
 #pragma once
 
 #include <type_traits>

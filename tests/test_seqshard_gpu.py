@@ -55,8 +55,8 @@ def test_slabs_equal_one_shot_scan(mods, cuts, prior):
 
 
 def test_eight_long_slabs_against_oracle(mods):
-    """B=1, M=32, S=16, T=32768 in 8 slabs of 4096 steps: each slab's aggregate is a product of 4096 step maps in
-    float32, rescaled every other step. Forward state, y and all gradients against the float64 oracle."""
+    """B=1, M=32, S=16, T=32768 in 8 slabs of 4096 steps: each slab's aggregate is the map of 4096 steps in
+    float32. Forward state, y and all gradients against the float64 oracle."""
     _check_slabs(mods, 1, 32768, 32, 16, tuple(range(0, 32768 + 1, 4096)), False, seed=33, long=True)
 
 

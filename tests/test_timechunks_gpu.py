@@ -76,7 +76,7 @@ def test_time_chunks_agree_with_the_plain_kernels_bf16_and_no_state(kb):
 
 
 def test_long_sequence_in_chunks_against_oracle(kb):
-    """B=1, T=32768 in 8 chunks of 4096: the aggregates are products of 4096 step maps, rescaled as they go.
+    """B=1, T=32768 in 8 chunks of 4096: the aggregates are maps of 4096 steps each.
     State, y and all gradients against the float64 oracle."""
     g = _seeded(1, 32768, 32, 16, seed=23)
     f, b = _oracle(g)
