@@ -806,13 +806,14 @@ py::object model_token(const Tensor &x, const std::vector<BlockArgs> &blocks, co
 }
 
 // One token of a layer (LayerDecoder.step), with the block's norm before it and its residual sum after it when norm_w is given
-// (ModelDecoder): three projections, the convolution's step and the fused filter step. conv_state
+// (ModelDecoder): three projections, the convolution's step and the fused filter step, or one kernel where that pays and may take
+// the whole GPU. conv_state
 // (absent without a convolution), lam and eta are updated in place. Returns the layer's output and the gated variance, which
 // a config that returns variances projects as well.
 std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, const Tensor &x, const OptTensor &conv_state,
                                       const Tensor &lam, const Tensor &eta, const Tensor &a_bar, const Tensor &p_bar,
                                       const OptTensor &skip, const OptTensor &conv_w, const OptTensor &conv_b, int64_t w_value,
-                                      int64_t w_var, const OptTensor &norm_w, double norm_eps) {
+                                      int64_t w_var, const OptTensor &norm_w, double norm_eps, bool whole) {
     const c10::cuda::CUDAGuard guard(x.device());
     const Weights w{w_};
     auto get = [&cfg](const char *name) {
@@ -842,7 +843,7 @@ std::tuple<Tensor, Tensor> layer_step(const py::dict &w_, const py::dict &cfg, c
     const bool in_model = norm_w.has_value();  // other kernels of the token, or the embedding's, are in front
     require(in_w.dim() == 2 && in_w.size(0) == (gated ? 2 * M : M), "in_proj must have one output per channel, two with a gate");
     require(sensor_w.dim() == 2 && sensor_w.size(0) == w_value + w_var + 2 * S, "sensor_proj must have one output per sensor signal");
-    if (!in_model && token_rows(x, kTokenRows) && lone_token_pays(B, x.size(1), M, S)) {
+    if (whole && !in_model && token_rows(x, kTokenRows) && lone_token_pays(B, x.size(1), M, S)) {
         std::vector<kla_b200_token_layer> one(1);
         if (token_layer(x, LayerArgs{w_, cfg, conv_state, lam, eta, a_bar, p_bar, skip, conv_w, conv_b, w_value, w_var}, {}, one[0])) {
             const Tensor yv = fresh(x, {B, M});

@@ -59,6 +59,11 @@ def _require_cuda(x: torch.Tensor) -> None:
 
 
 class LayerDecoder:
+    # False where other work of the program shares the GPU: a small layer's token, which as one kernel holds every SM and waits for
+    # all that another stream has running, then always takes the separate kernels. 8 rows of d_model 1024 call by call, us a token,
+    # one kernel / separate: alone 18.5 / 21.9, beside prompts on another stream 55 / 23, beside training 107 / 23.
+    whole_gpu = None  # as ModelDecoder.whole_gpu; None is True here
+
     def __init__(self, weights: dict, config: dict):
         missing = [k for k in CONFIG_KEYS if k not in config]
         if missing:
@@ -177,7 +182,7 @@ class LayerDecoder:
         conv_state, lam, eta = state
         return _lib.host().layer_step(self.w, self.cfg, x, conv_state, lam, eta, self.a_bar, self.p_bar, self.skip,
                                       self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var, norm_weight,
-                                      norm_eps)[0]
+                                      norm_eps, False)[0]
 
     def step(self, x: torch.Tensor, state):
         """One token. ``x``: [B, d_model]; ``state``: the tuple of ``init_state``, updated in place.
@@ -185,7 +190,8 @@ class LayerDecoder:
         _require_cuda(x)
         conv_state, lam, eta = state
         out, y_var = _lib.host().layer_step(self.w, self.cfg, x, conv_state, lam, eta, self.a_bar, self.p_bar, self.skip,
-                                            self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var, None, 0.0)
+                                            self.conv_w, getattr(self, "conv_b", None), self.w_value, self.w_var, None, 0.0,
+                                            self.whole_gpu is not False)
         if self.cfg["return_variance"]:
             return out, F.linear(y_var, self.w["out_proj.weight"].pow(2))
         return out

@@ -260,4 +260,7 @@ def test_a_generate_beside_another_stream_leaves_it_room():
         c.whole_gpu = whole
         assert torch.equal(c.generate(ids, 24), want[0]) and torch.equal(c.generate(ids, 24, use_graph=False), want[0])
         assert (c._slot.graph is not None) == whole and (c._shared_slot.graph is None) == whole
-        assert launches(lambda: c.step(ids[:, 0], c.init_state(2, "cuda", torch.bfloat16)))[1] < 4 or not whole
+        assert (launches(lambda: c.step(ids[:, 0], c.init_state(2, "cuda", torch.bfloat16)))[1] < 4) == whole
+        layer, x = c.layers[0], torch.randn(2, 64, device="cuda").bfloat16()
+        layer.whole_gpu = whole
+        assert launches(lambda: layer.step(x, layer.init_state(2, "cuda", torch.bfloat16)))[1] == (1 if whole else 4)
